@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "self.cuh"
+#include "smooth.cuh"
 #include "bem3_internal.h"
 
 // ------------------------------------------------------------------------------------------
@@ -152,21 +153,26 @@ struct RegWarp {
 #define REGP_SMEM_BYTES (sizeof(RegWarp) * 8 * REGP_PAIRS + sizeof(AccP) * 256 * REGP_PAIRS)
 
 // One warp's unit of regular periodic work: the pairs first, first + 1, ... (REGP_PAIRS of them,
-// those < np) of the chunk that starts at pair p0 of the domain.  Lane l takes the points l, l + 32,
+// those < np) of the chunk that starts at pair p0 of the domain, or of the list of pairs of that
+// chunk (list != nullptr, np entries).  Lane l takes the points l, l + 32,
 // ... of the pairs' concatenated point lists.  sw: the warp's REGP_PAIRS pair slots; sacc: the
 // block's per-thread accumulators (shared memory).
 __device__ __forceinline__ void reg_periodic_unit(const AssembleArgs& A, const QPLattice& L, long long p0, long long np,
-                                                  long long first, double3* Fp, unsigned* gh_list, unsigned* gh_count,
-                                                  unsigned gh_cap, int* status, RegWarp* sw, AccP (*sacc)[256], int lane)
+                                                  long long first, const unsigned* list, double3* Fp, unsigned* gh_list,
+                                                  unsigned* gh_count, unsigned gh_cap, int* status, RegWarp* sw,
+                                                  AccP (*sacc)[256], int lane)
 {
   int npts[REGP_PAIRS];
+  long long pidx[REGP_PAIRS];  // pair within the chunk
   PairIdx q[REGP_PAIRS];
   __syncwarp();  // a warp that runs several units reuses its slots: the last unit's reads are done
 #pragma unroll
   for (int j = 0; j < REGP_PAIRS; j++) {
     npts[j] = 0;
+    pidx[j] = first + j;
     if (first + j >= np) continue;
-    q[j] = pair_of(p0 + first + j, A.ne);
+    if (list) pidx[j] = list[first + j];
+    q[j] = pair_of(p0 + pidx[j], A.ne);
     const int at = abs(A.sid[q[j].t]);
     const int tnn = (int)A.geo[(size_t)at * GEO_STRIDE + GEO_NN];
     if ((q[j].tn == 3 && tnn == 3) || q[j].s == q[j].t) continue;
@@ -181,11 +187,15 @@ __device__ __forceinline__ void reg_periodic_unit(const AssembleArgs& A, const Q
     accp_zero(sacc[j][threadIdx.x]);
   }
   __syncwarp();
-  const int ntot = npts[0] + (REGP_PAIRS > 1 ? npts[1] : 0);
+  // a list's order varies from run to run: each of its pairs starts at lane 0, whatever its neighbour,
+  // so that its sums are the same
+  const int off1 = list ? (npts[0] + 31) & ~31 : npts[0];
+  const int ntot = off1 + npts[1];
   int err = 0, nterms = 0;
   for (int k = lane; k < ntot; k += 32) {
-    const int j = (k < npts[0]) ? 0 : 1;
-    const int kk = j ? k - npts[0] : k;
+    const int j = (k < off1) ? 0 : 1;
+    const int kk = j ? k - off1 : k;
+    if (kk >= npts[j]) continue;
     const RegWarp& W = sw[j];
     double z, e, wt;
     rule_point(W.es.nn, 12, c_xl, c_wl, kk, z, e, wt);
@@ -233,7 +243,7 @@ __device__ __forceinline__ void reg_periodic_unit(const AssembleArgs& A, const Q
       fs = 0.0625 * EL_SQ3 * EL_I_SPSQ3;
     }
     const double dFz = acc[17] * fs, dFe = acc[18] * fs;
-    const long long pi = first + j;
+    const long long pi = j ? pidx[REGP_PAIRS - 1] : pidx[0];
     if (needs_gh(dFz, dFe)) {
       if (lane == 0) {
         unsigned slot = atomicAdd(gh_count, 1u);
@@ -260,20 +270,23 @@ __device__ __forceinline__ void reg_periodic_unit(const AssembleArgs& A, const Q
   }
 }
 
-// Regular periodic pairs of one chunk: one warp per REGP_PAIRS consecutive pairs.
+// Regular periodic pairs of one chunk summed point by point: one warp per REGP_PAIRS pairs, striding
+// over all pairs of the chunk, or (plan on) over the list of pairs that the tabulated kernel left.
 __global__ void __launch_bounds__(256, REGP_MIN_BLOCKS) k_reg_periodic(AssembleArgs A, const __grid_constant__ QPLattice L,
-                                                                       long long p0, long long np, double3* Fp,
-                                                                       unsigned* gh_list, unsigned* gh_count,
+                                                                       const SmoothPlan* plan, const unsigned* list,
+                                                                       const unsigned* nlist, long long p0, long long np,
+                                                                       double3* Fp, unsigned* gh_list, unsigned* gh_count,
                                                                        unsigned gh_cap, int* status)
 {
   extern __shared__ __align__(16) unsigned char regp_smem[];  // REGP_SMEM_BYTES
   RegWarp(*sw)[REGP_PAIRS] = reinterpret_cast<RegWarp(*)[REGP_PAIRS]>(regp_smem);
   AccP(*sacc)[256] = reinterpret_cast<AccP(*)[256]>(regp_smem + sizeof(RegWarp) * 8 * REGP_PAIRS);
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const long long first = w * REGP_PAIRS;  // pair index within the chunk
-  if (first >= np) return;  // uniform across the warp
-  reg_periodic_unit(A, L, p0, np, first, Fp, gh_list, gh_count, gh_cap, status, sw[wib], sacc, lane);
+  const bool on = plan && plan->on;
+  if (on) np = *nlist;
+  const long long stride = (long long)gridDim.x * (blockDim.x >> 5) * REGP_PAIRS;
+  for (long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * REGP_PAIRS; first < np; first += stride)
+    reg_periodic_unit(A, L, p0, np, first, on ? list : nullptr, Fp, gh_list, gh_count, gh_cap, status, sw[wib], sacc, lane);
 }
 
 // Near-singular periodic pair w of the chunk starting at pair p0, 64x64 rule, by the whole CTA
@@ -488,12 +501,16 @@ __device__ __forceinline__ void self_periodic_row(const AssembleArgs& A, const Q
   store_pair(A, row, t, CC, dCz, dCe, Fself, row, -1);
 }
 
-__global__ void __launch_bounds__(SELF_THREADS, 2) k_self_periodic(AssembleArgs A, const __grid_constant__ QPLattice L, double3* Fself, int* status)
+__global__ void __launch_bounds__(SELF_THREADS, 2) k_self_periodic(AssembleArgs A, const __grid_constant__ QPLattice L,
+                                                                   const SmoothPlan* plan, double3* Fself, int* status)
 {
+  if (plan && plan->on) return;
   __shared__ double red[SELF_THREADS / 32][24];
   __shared__ int serr[SELF_THREADS / 32];
   self_periodic_row(A, L, blockIdx.x, Fself, status, red, serr);
 }
+
+#include "assemble_smooth.cuh"
 
 // ==========================================================================================
 // Host side
@@ -542,7 +559,12 @@ static int ensure_tables(void)
   if (cudaFuncSetAttribute(k_reg_periodic, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
       cudaFuncSetAttribute(k_reg_periodic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGP_SMEM_BYTES) !=
-          cudaSuccess)
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_reg_smooth, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+      cudaFuncSetAttribute(k_reg_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(SMT_WARPS * sizeof(SmoothWarp))) != cudaSuccess ||
+      cudaFuncSetAttribute(k_smooth_spectral, cudaFuncAttributeMaxDynamicSharedMemorySize, SMT_SPEC_SMEM) != cudaSuccess)
     return -1;
   if (dev < 64) g_tables_ready[dev] = 1;
   return 0;
@@ -552,13 +574,15 @@ extern "C" void bem3_gauss_legendre(int n, double* x, double* w) { gauleg_host(n
 
 // Scratch layout of bem3_assemble_run for a chunk of `rows` rows, each part starting on a 256-byte
 // boundary: self-pair F sums (4 ne double3), the work-list counters (256 B), the chunk's per-pair F
-// terms (rows * ne double3), the near-singular work list (rows * ne / 8 + 4096 u32).
+// terms (rows * ne double3), the near-singular work list (rows * ne / 8 + 4096 u32), and for a table of
+// `cap` coefficients (periodic domains; 0: none) the plan, the list of in-plane pairs (rows * ne u32),
+// the coefficients and the samples.
 static inline size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 struct ScratchLayout {
-  size_t fself, counters, fp, gh_list, end;
+  size_t fself, counters, fp, gh_list, plan, ip_list, tab, smp, end;
   unsigned gh_cap;
 };
-static ScratchLayout scratch_layout(int ne, int rows)
+static ScratchLayout scratch_layout(int ne, int rows, long long cap)
 {
   ScratchLayout l;
   const size_t np = (size_t)rows * ne;
@@ -567,10 +591,18 @@ static ScratchLayout scratch_layout(int ne, int rows)
   l.counters = round256((size_t)4 * ne * sizeof(double3));
   l.fp = l.counters + 256;
   l.gh_list = l.fp + round256(np * sizeof(double3));
-  l.end = l.gh_list + round256((size_t)l.gh_cap * sizeof(unsigned));
+  l.plan = l.gh_list + round256((size_t)l.gh_cap * sizeof(unsigned));
+  l.ip_list = l.plan + (cap ? round256(sizeof(SmoothPlan)) : 0);
+  l.tab = l.ip_list + (cap ? round256(np * sizeof(unsigned)) : 0);
+  l.smp = l.tab + round256((size_t)cap * sizeof(cplx));
+  l.end = l.smp + round256((size_t)cap * 2 * sizeof(cplx));
   return l;
 }
-size_t bem3_scratch_bytes(int ne, int rows) { return scratch_layout(ne, rows).end; }
+size_t bem3_scratch_bytes(int ne, int rows, long long cap) { return scratch_layout(ne, rows, cap).end; }
+
+// Coefficients a domain's table may hold: enough for the cheapest plans of the configurations (0.1 M
+// for 96 elements, 0.9 M for 1536), more where more pairs pay for it.
+long long bem3_smooth_cap(int ne) { return ne < 256 ? 1LL << 19 : ne < 1024 ? 1LL << 20 : 1LL << 21; }
 
 // Runs the whole domain on `stream` using caller-provided scratch (see bem3_scratch_bytes).
 // Returns 0, or a negative code (see bem3_qd2_b200.h).
@@ -581,13 +613,17 @@ __global__ void k_acc_count(const unsigned* __restrict__ cnt, unsigned long long
 }
 
 int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, size_t scratch_bytes, int rows_per_chunk,
-                      int* d_status, cudaStream_t st, AssembleStats* stats, const ChunkHook* hook)
+                      long long cap, int* d_status, cudaStream_t st, AssembleStats* stats, const ChunkHook* hook)
 {
   if (ensure_tables() != 0) return BEM3_ERR_CUDA;
   const int ne = A.ne;
   const int nrows = 4 * ne;
   if (rows_per_chunk <= 0 || rows_per_chunk > nrows) rows_per_chunk = nrows;
-  const ScratchLayout lay = scratch_layout(ne, rows_per_chunk);
+  SmoothArgs M;
+  memset(&M, 0, sizeof M);
+  if (A.periodic && cap > 0) smooth_lattice(*L, M.S);
+  if (!M.S.ok) cap = 0;
+  const ScratchLayout lay = scratch_layout(ne, rows_per_chunk, cap);
   if (lay.end > scratch_bytes) return BEM3_ERR_SCRATCH;  // every part below ends inside the scratch
   char* base = (char*)scratch;
   double3* Fself = (double3*)(base + lay.fself);
@@ -596,6 +632,17 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, 
   double3* Fp = (double3*)(base + lay.fp);
   unsigned* gh_list = (unsigned*)(base + lay.gh_list);
   const unsigned gh_cap = lay.gh_cap;
+  // tabulated pairs: their near-singular list fills gh_list, the in-plane pairs' (ip_list) the same
+  // way after them; both lists' counters
+  unsigned* smt_count = (unsigned*)(base + lay.counters + 16);
+  unsigned* ip_count = (unsigned*)(base + lay.counters + 20);
+  unsigned* ip_list = (unsigned*)(base + lay.ip_list);
+  if (cap) {
+    M.plan = (SmoothPlan*)(base + lay.plan);
+    M.tab = (cplx*)(base + lay.tab);
+    M.smp = (cplx*)(base + lay.smp);
+    M.cap = cap;
+  }
 
   const size_t N = (size_t)nrows;
   if (cudaMemsetAsync(A.G, 0, N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
@@ -622,10 +669,23 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, 
     }
     return ms;
   };
+  // the table of the smooth remainder
+  if (M.plan) {
+    tic();
+    k_smooth_plan<<<1, SMT_PLAN_THREADS, 0, st>>>(A, *L, M);
+    k_smooth_spectral<<<148 * 4, SMT_SPEC_THREADS, smooth_spec_smem(M.S), st>>>(*L, M);
+    k_smooth_project<<<148 * 8, SMT_PROJ_THREADS, 0, st>>>(*L, M);
+    toc(1);
+    launches += 3;
+  }
   // self pairs
   tic();
-  if (A.periodic) k_self_periodic<<<nrows, SELF_THREADS, 0, st>>>(A, *L, Fself, d_status);
-  else bem3_launch_self_interior(A, Fself, d_status, st);
+  if (A.periodic) {
+    if (M.plan) { k_self_smooth<<<nrows, SELF_THREADS, 0, st>>>(A, *L, M, Fself); launches++; }
+    k_self_periodic<<<nrows, SELF_THREADS, 0, st>>>(A, *L, M.plan, Fself, d_status);
+  } else {
+    bem3_launch_self_interior(A, Fself, d_status, st);
+  }
   toc(0);
   launches++;
 
@@ -634,11 +694,30 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, 
     long long p0 = (long long)r0 * ne, np = (long long)nr * ne;
     cudaMemsetAsync(gh_count, 0, sizeof(unsigned), st);
     if (A.periodic) {
-      long long threads = (np + REGP_PAIRS - 1) / REGP_PAIRS * 32;
-      unsigned blocks = (unsigned)((threads + 255) / 256);
+      const long long units = (np + REGP_PAIRS - 1) / REGP_PAIRS;
+      // without a table every pair has its warp; with one, a resident grid strides over what it left
+      const long long want = (units * 32 + 255) / 256;
+      const unsigned blocks = (unsigned)((M.plan && want > 148 * REGP_MIN_BLOCKS) ? 148 * REGP_MIN_BLOCKS : want);
       tic();
-      k_reg_periodic<<<blocks, 256, REGP_SMEM_BYTES, st>>>(A, *L, p0, np, Fp, gh_list, gh_count, gh_cap, d_status);
-      const float ms = toc(1);
+      if (M.plan) {
+        cudaMemsetAsync(smt_count, 0, 2 * sizeof(unsigned), st);
+        const long long su = (long long)((ne + SMT_PAIRS - 1) / SMT_PAIRS) * nr;
+        k_reg_smooth<<<(unsigned)((su + SMT_WARPS - 1) / SMT_WARPS), SMT_WARPS * 32, SMT_WARPS * sizeof(SmoothWarp), st>>>(
+            A, *L, M, r0, nr, Fp, gh_list, smt_count, gh_cap, ip_list, ip_count, d_status);
+        launches++;
+      }
+      float ms = toc(1);
+      tic();
+      if (M.plan) {
+        k_gh_smooth<<<148 * 4, 256, 0, st>>>(A, *L, M, p0, Fp, gh_list, smt_count, gh_cap);
+        k_acc_count<<<1, 1, 0, st>>>(smt_count, gh_total);
+        launches += 2;
+      }
+      toc(2);
+      tic();
+      k_reg_periodic<<<blocks, 256, REGP_SMEM_BYTES, st>>>(A, *L, M.plan, ip_list, ip_count, p0, np, Fp, gh_list, gh_count,
+                                                           gh_cap, d_status);
+      ms += toc(1);
       if (timing) {
         stats->reg_periodic_ms += ms;
         stats->reg_periodic_launches++;

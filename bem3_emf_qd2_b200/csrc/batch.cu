@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256, REGP_MIN_BLOCKS) k_batch_reg_periodic(con
       const int i = seg_find(S, u);
       const BatchDomain& d = D[S.dom[i]];
       const long long np = 4LL * d.A.ne * d.A.ne;
-      reg_periodic_unit(d.A, d.L, 0, np, (u - S.base[i]) * REGP_PAIRS, d.Fp, d.gh_list, d.gh_count, d.gh_cap, d.status,
+      reg_periodic_unit(d.A, d.L, 0, np, (u - S.base[i]) * REGP_PAIRS, nullptr, d.Fp, d.gh_list, d.gh_count, d.gh_cap, d.status,
                         sw[wib], sacc, lane);
     }
   }

@@ -40,7 +40,9 @@ struct ChunkHook {
   void* user;
 };
 
-size_t bem3_scratch_bytes(int ne, int rows);
+// cap: coefficients of the periodic domain's table of the smooth remainder (0: none)
+long long bem3_smooth_cap(int ne);
+size_t bem3_scratch_bytes(int ne, int rows, long long cap);
 int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, size_t scratch_bytes, int rows_per_chunk,
-                      int* d_status, cudaStream_t st, AssembleStats* stats, const ChunkHook* hook = nullptr);
+                      long long cap, int* d_status, cudaStream_t st, AssembleStats* stats, const ChunkHook* hook = nullptr);
 void bem3_launch_self_interior(const AssembleArgs& A, double3* Fself, int* d_status, cudaStream_t st);

@@ -192,7 +192,8 @@ static int enqueue_domain(const double* geo_dev, int Ne, const int* sid_dev, int
     int e = lattice_from(qd, &L);
     if (e) return e;
   }
-  size_t need = bem3_scratch_bytes(Ne_d, rows);
+  const long long cap = periodic ? bem3_smooth_cap(Ne_d) : 0;
+  size_t need = bem3_scratch_bytes(Ne_d, rows, cap);
   DevRes* R = nullptr;
   int e = ensure_scratch(need, &R);
   if (e) return e;
@@ -215,7 +216,7 @@ static int enqueue_domain(const double* geo_dev, int Ne, const int* sid_dev, int
   memset(&run.S, 0, sizeof run.S);
   run.S.time_kernels = t_profiling;
   run.R = R;
-  return bem3_assemble_run(A, &L, R->scratch, R->scratch_bytes, rows, R->status, st, &run.S, hook);
+  return bem3_assemble_run(A, &L, R->scratch, R->scratch_bytes, rows, cap, R->status, st, &run.S, hook);
 }
 
 // Waits for `st` and returns the kernels' status; fills this thread's counters.
@@ -373,7 +374,7 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
     r = r < 64 ? 64 : r;
     r = r > default_rows_per_chunk(Ne_d[d]) ? default_rows_per_chunk(Ne_d[d]) : r;
     rows[d] = r;
-    const size_t b = bem3_scratch_bytes(Ne_d[d], r);
+    const size_t b = bem3_scratch_bytes(Ne_d[d], r, (periodic && d == 0) ? bem3_smooth_cap(Ne_d[d]) : 0);
     need = b > need ? b : need;
   }
   double* dgeo = nullptr;
@@ -553,8 +554,15 @@ extern "C" int bem3_assemble_domain_dev_noalloc(const double* geo_dev, int Ne, c
   void* scratch = (char*)base + head;
   const size_t avail = BEM3_NOALLOC_SCRATCH_BYTES - head;
   int rows = default_rows_per_chunk(Ne_d);
-  while (rows > 4 && bem3_scratch_bytes(Ne_d, rows) > avail) rows = rows / 2 > 4 ? rows / 2 : 4;
-  if (bem3_scratch_bytes(Ne_d, rows) > avail) return BEM3_ERR_SCRATCH;  // domain too large for the array
+  while (rows > 4 && bem3_scratch_bytes(Ne_d, rows, 0) > avail) rows = rows / 2 > 4 ? rows / 2 : 4;
+  if (bem3_scratch_bytes(Ne_d, rows, 0) > avail) return BEM3_ERR_SCRATCH;  // domain too large for the array
+  // a table of up to 0.25 M coefficients where at least 64 rows still fit beside it
+  long long cap = 0;
+  if (periodic) {
+    int rc = default_rows_per_chunk(Ne_d);
+    while (rc > 64 && bem3_scratch_bytes(Ne_d, rc, 1LL << 18) > avail) rc = rc / 2 > 64 ? rc / 2 : 64;
+    if (bem3_scratch_bytes(Ne_d, rc, 1LL << 18) <= avail) { cap = 1LL << 18; rows = rc; }
+  }
   cudaStream_t st = (cudaStream_t)stream;
   AssembleArgs A;
   A.geo = geo_dev; A.sid = sid_dev; A.ne = Ne_d; A.did = did; A.periodic = periodic ? 1 : 0;
@@ -570,7 +578,7 @@ extern "C" int bem3_assemble_domain_dev_noalloc(const double* geo_dev, int Ne, c
   if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return BEM3_ERR_CUDA;
   AssembleStats S;
   memset(&S, 0, sizeof S);
-  int e = bem3_assemble_run(A, &L, scratch, avail, rows, status, st, &S);
+  int e = bem3_assemble_run(A, &L, scratch, avail, rows, cap, status, st, &S);
   if (e) return e;
   int hs = 0;
   unsigned long long gh = 0;

@@ -1,0 +1,156 @@
+// Host build of the tabulated smooth remainder of the quasi-periodic Green's function (csrc/smooth.cuh):
+// a domain's plan and table on the CPU, and one pair by it and by the plain lattice sums.
+#include <string.h>
+
+#include <vector>
+
+#include "smooth.cuh"
+
+namespace {
+struct Domain {
+  QPLattice L;
+  std::vector<QPProp> prop;
+  SmoothPlan P;
+  std::vector<cplx> tab;
+  std::vector<char> have;
+  SmoothLat S;
+};
+Domain D;
+
+void centre_coefs(int slot)
+{
+  SmoothPlan& P = D.P;
+  if (D.have[slot]) return;
+  D.have[slot] = 1;
+  SmoothCell c;
+  smooth_centre(D.L, P, slot % P.N1 - P.I, slot / P.N1 % P.N2 - P.J, slot / P.N1 / P.N2, c);
+  std::vector<cplx> smp(P.nth * P.nph), a(P.nth), b(P.nth);
+  std::vector<double> pts(3 * P.nth * P.nph);
+  for (int p = 0; p < P.nth * P.nph; p++) {
+    smooth_sample_point(P, c, p, &pts[3 * p]);
+    smp[p] = smooth_real(D.L, D.S, c, &pts[3 * p]);
+  }
+  for (int t = 0; t < P.nth; t++)  // a theta's samples share their height
+    for (int a = 0; a < D.S.no1; a++)
+      for (int b = 0; b < D.S.no2; b++) {
+        double ax, ay;
+        const cplx f = smooth_order(D.L, D.S, D.S.o1 + a, D.S.o2 + b, fabs(pts[3 * t * P.nph + 2]), &ax, &ay);
+        if (f.re == 0.0 && f.im == 0.0) continue;
+        for (int q = t * P.nph; q < (t + 1) * P.nph; q++) smp[q] += f * expi(ax * pts[3 * q] + ay * pts[3 * q + 1]);
+      }
+  cplx* al = D.tab.data() + (size_t)slot * smt_ncoef(P.L);
+  for (int m = 0; m <= P.L; m++) {
+    for (int t = 0; t < P.nth; t++) smooth_azimuth(P, smp.data(), t, m, a[t], b[t]);
+    for (int l = m; l <= P.L; l++) {
+      cplx A = mk(0, 0), B = mk(0, 0);
+      for (int t = 0; t < P.nth; t++) {
+        A += a[t] * P.proj[(size_t)smt_lm(P.L, m, l) * P.nth + t];
+        B += b[t] * P.proj[(size_t)smt_lm(P.L, m, l) * P.nth + t];
+      }
+      *al++ = A;
+      if (m) *al++ = B;
+    }
+  }
+}
+}  // namespace
+
+extern "C" {
+
+// Plan of the elements 1..ne of geo; lat = k, vkx, vky, d1, d2; degree 0: the cheapest.  info: on, L,
+// centres, points of the quad and triangle rules.  Returns 1 when a plan exists.
+int sh_plan(const double* lat, const double* geo, int ne, double npairs, int degree, int* info)
+{
+  memset((void*)&D.L, 0, sizeof D.L);
+  if (qp_lattice_init(D.L, lat[0], lat[1], lat[2], lat[3], lat[4], lat[5], lat[6]) != 0) return 0;
+  D.prop.resize(QP_PROP_CAP);
+  D.L.nprop = qp_prop_list(D.L, D.prop.data(), QP_PROP_CAP);
+  D.L.prop = D.prop.data();
+  SmoothLat& S = D.S;
+  smooth_lattice(D.L, S);
+  double he = 0, ra = 0, be = 0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+  int tri = 0;
+  for (int i = 1; i <= ne; i++) {
+    Elem e;
+    load_elem(geo, i, e);
+    smooth_extent(D.L, e, &he, &ra, &be, lo, hi);
+    tri |= (e.nn == 3);
+  }
+  const SmoothExt X = {he, hi[2] - lo[2], hi[0] - lo[0], hi[1] - lo[1], ra, be};
+  double best = 1e300;
+  SmoothGrid g;
+  for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
+    double c;
+    if (degree && d != degree) continue;
+    smooth_choose(D.L, S, X, npairs, tri, 1LL << 40, d, g, c);
+    if (c < best) { best = c; *static_cast<SmoothGrid*>(&D.P) = g; }
+  }
+  info[0] = best < 1e300 ? D.P.on : 0;
+  if (best >= 1e300) return 0;
+  info[1] = D.P.L; info[2] = D.P.ncent; info[3] = D.P.nq4; info[4] = D.P.nq3;
+  smooth_tables_a(D.P, 0, 1);
+  smooth_tables_b(D.P, 0, 1);
+  smooth_tables_c(D.P, D.L.k, 0, 1);
+  D.tab.assign((size_t)D.P.ncent * smt_ncoef(D.P.L), mk(0, 0));
+  D.have.assign(D.P.ncent, 0);
+  return 1;
+}
+
+// Sums G[4], H[4], F, dF0, dF1 (19 doubles, scaled as the matrices hold them) of the pair (node tn of
+// element t, element s) by the n x n rule: by the plan (plain 0) or the lattice sums (plain 1).
+// Returns the lowest status; in_plane: whether the plan leaves the pair to the lattice sums.
+int sh_pair(const double* geo, int t, int tn, int s, int plain, int n, const double* x, const double* w, double* out,
+            int* in_plane)
+{
+  Elem es, et;
+  load_elem(geo, s, es);
+  load_elem(geo, t, et);
+  double v0[3], v1[3];
+  node_tangents(et, tn, v0, v1);
+  const double* rt = geo + (size_t)t * GEO_STRIDE + GEO_REN + 3 * tn;
+  *in_plane = smooth_in_plane(D.L, es, rt[2]);
+  const int npts = (es.nn == 4) ? n * n : 3 * n * n;
+  AccP a;
+  accp_zero(a);
+  int err = 0;
+  cplx ph = mk(1.0, 0.0);
+  if (plain) {
+    for (int q = 0; q < npts; q++) {
+      double z, e, wt;
+      rule_point(es.nn, n, x, w, q, z, e, wt);
+      const int st = accp_point(es, D.L, rt, v0, v1, z, e, wt, a);
+      if (st < 0) err = st;
+    }
+  } else {
+    const double v[3] = {es.cr[0][0] - rt[0], es.cr[1][0] - rt[1], es.cr[2][0] - rt[2]};
+    double sx, sy;
+    const int sh = smooth_shift(D.L, v, &sx, &sy);
+    for (int q = 0; q < npts; q++) {
+      double z, e, wt;
+      rule_point(es.nn, n, x, w, q, z, e, wt);
+      smooth_near(es, D.L.k, rt, v0, v1, sx, sy, sh, z, e, wt, a);
+    }
+    for (int i = 0; i < 4; i++) { a.G[i] = a.G[i] * EL_I_FP; a.H[i] = a.H[i] * EL_I_FP; }
+    const int nq = es.nn == 4 ? D.P.nq4 : D.P.nq3;
+    const double* tq = es.nn == 4 ? D.P.q4 : D.P.q3;
+    for (int q = 0; q < nq; q++) {
+      double r[3], W[3], rad[SMT_LMAX + 2], N[4], z, e;
+      point_geom(es, tq[3 * q], tq[3 * q + 1], rt, r, W);
+      SmoothCell c;
+      smooth_cell(D.L, D.P, r[0] + sx, r[1] + sy, fabs(r[2]), c);
+      centre_coefs(c.slot);
+      cplx gw, hw;
+      smooth_point(es, D.L, D.P, D.tab.data(), rt, sx, sy, q, rad, 1, gw, hw, z, e);
+      if (es.nn == 4) bil_N4(z, e, N);
+      else { lit_N3(z, e, N); N[3] = 0.0; }
+      for (int i = 0; i < 4; i++) { a.G[i] += gw * N[i]; a.H[i] += hw * N[i]; }
+    }
+    if (sh) ph = expi(D.L.vkx * sx + D.L.vky * sy);
+  }
+  cplx CC[9], dCz[9], dCe[9];
+  accp_finish(es, a, CC, dCz, dCe);
+  for (int i = 0; i < 8; i++) { CC[i] = CC[i] * ph; out[2 * i] = CC[i].re; out[2 * i + 1] = CC[i].im; }
+  out[16] = CC[8].re; out[17] = dCz[8].re; out[18] = dCe[8].re;
+  return err;
+}
+
+}
