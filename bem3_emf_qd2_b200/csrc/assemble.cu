@@ -600,9 +600,9 @@ static ScratchLayout scratch_layout(int ne, int rows, long long cap)
 }
 size_t bem3_scratch_bytes(int ne, int rows, long long cap) { return scratch_layout(ne, rows, cap).end; }
 
-// Coefficients a domain's table may hold: enough for the cheapest plans of the configurations (0.1 M
-// for 96 elements, 0.9 M for 1536), more where more pairs pay for it.
-long long bem3_smooth_cap(int ne) { return ne < 256 ? 1LL << 19 : ne < 1024 ? 1LL << 20 : 1LL << 21; }
+// Coefficients a domain's table may hold (48 bytes of scratch each, with the samples): enough for the
+// cheapest plans of the configurations (0.4 M for 96 elements, 1.1 M for 384, 2.1 M for 864).
+long long bem3_smooth_cap(int ne) { return ne < 256 ? 1LL << 19 : ne < 640 ? 1LL << 21 : 1LL << 22; }
 
 // Runs the whole domain on `stream` using caller-provided scratch (see bem3_scratch_bytes).
 // Returns 0, or a negative code (see bem3_qd2_b200.h).

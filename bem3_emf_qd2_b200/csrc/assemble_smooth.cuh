@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(SMT_SPEC_THREADS) k_smooth_spectral(const __gr
             q += im;
             if (q >= P.n1) q -= P.n1;
           }
-          const double u = (double)(ii - P.I) / P.n1, v = (double)(j0 + jj - P.J) / P.n2;
+          const double u = (ii - P.I) * P.rn1, v = (j0 + jj - P.J) * P.rn2;
           const cplx ph = expi(-(L.vkx * (u * L.d1x + v * L.d2x) + L.vky * (u * L.d1y + v * L.d2y)));
           const long long slot = ((long long)m * P.N2 + j0 + jj) * P.N1 + ii;
           M.smp[slot * ns + t * P.nph + f] = s * ph;
@@ -250,6 +250,9 @@ __global__ void __launch_bounds__(SMT_PROJ_THREADS) k_smooth_project(const __gri
 // them up: no reduction over lanes.
 #define SMT_PAIRS 4
 #define SMT_WARPS 4
+#ifndef SMT_BLOCKS
+#define SMT_BLOCKS 4
+#endif
 #define SMT_BUF 160  // smooth points of a pass over the list
 struct SmoothWarp {
   Elem es[SMT_PAIRS];
@@ -258,14 +261,16 @@ struct SmoothWarp {
   double rt[3], v0[3], v1[3];
   double sx[SMT_PAIRS], sy[SMT_PAIRS];
   int sh[SMT_PAIRS];
-  double rad[(SMT_LMAX + 2) * 32];
   union {
-    double slot[32 * 19];      // the lanes' nearest-image sums
-    cplx buf[SMT_BUF][2];      // smooth points: g w |W|, h w
+    double slot[32 * 19];              // the lanes' nearest-image sums
+    struct {
+      cplx buf[SMT_BUF][2];            // smooth points: g w |W|, h w
+      double rad[(SMT_LMAX + 2) * 32]; // f_l of the lanes' points
+    };
   };
 };
 
-__global__ void __launch_bounds__(SMT_WARPS * 32, 4)
+__global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS)
     k_reg_smooth(AssembleArgs A, const __grid_constant__ QPLattice L, SmoothArgs M, int r0, int nr, double3* Fp,
                  unsigned* gh_list, unsigned* gh_count, unsigned gh_cap, unsigned* ip_list, unsigned* ip_count, int* status)
 {

@@ -12,10 +12,9 @@
 // few Gauss points that a smooth integrand of that size needs (smooth_nq), and S is not summed at
 // all: it solves Helmholtz's equation, so on a ball around a centre c of a grid over the cell it is
 //
-//   S(c + d) = sum_{l <= L} jh_l(k |d|) sum_m [A_lm Re + B_lm Im] R_lm(d)
+//   S(c + d) = sum_{l <= L} f_l(|d|) sum_m [A_lm Re + B_lm Im] R_lm(d)
 //
-// with (L + 1)^2 complex coefficients per centre (jh_l(x) = (2l+1)!! j_l(x) / x^l, R_lm the solid
-// harmonics), where polynomials of the same degree would need (L+1)(L+2)(L+3)/6.  The coefficients
+// with (L + 1)^2 complex coefficients per centre (f_l(r) = j_l(k r) / r^l, R_lm the solid harmonics), where polynomials of the same degree would need (L+1)(L+2)(L+3)/6.  The coefficients
 // come from 2 (L + 1)^2 values of S on a sphere around c (Gauss-Legendre in cos(theta), equal steps
 // in phi).  Those values are Ewald sums with ONE split parameter and fixed sets of terms for the whole
 // table: the spheres of a layer of centres share their heights, so an order's height function is
@@ -39,7 +38,8 @@
 #define SMT_NQMAX 12
 #define SMT_ZPLANE 1e-11
 #define SMT_PMAX (SMT_NQMAX * (SMT_NQMAX + 1))
-#define SMT_TOL 1e-16
+#define SMT_TOL 1e-16   // truncation of the expansions
+#define SMT_QTOL 5e-16  // worst-direction error of the smooth rules
 #define SMT_EXPM 1.0     // bound of (k veps)^2 of the table's Ewald sums
 #define SMT_CUT 38.5     // their terms below e^-38.5 = 2e-17 are left out
 #define SMT_ORDERS 5000  // most spectral orders (of the rectangle that holds them) of a table: shared memory
@@ -48,13 +48,13 @@
 // R_l^m = z R_{l-1}^m - c_lm r^2 R_{l-2}^m, R_m^m = (x + iy)^m, R_{m-1}^m = 0.
 struct SmtRec {
   double c[SMT_LMAX + 2][SMT_LMAX + 2];  // [m][l]
-  double g[SMT_LMAX + 2];                // 1 / (2l + 3)
-  constexpr SmtRec() : c{}, g{}
+  double inv[2 * SMT_LMAX + 32];         // 1 / i
+  constexpr SmtRec() : c{}, inv{}
   {
     for (int m = 0; m < SMT_LMAX + 2; m++)
       for (int l = 0; l < SMT_LMAX + 2; l++)
         c[m][l] = (l >= m + 2) ? ((l - 1.0) * (l - 1.0) - 1.0 * m * m) / ((2.0 * l - 1.0) * (2.0 * l - 3.0)) : 0.0;
-    for (int l = 0; l < SMT_LMAX + 2; l++) g[l] = 1.0 / (2.0 * l + 3.0);
+    for (int i = 1; i < 2 * SMT_LMAX + 32; i++) inv[i] = 1.0 / i;
   }
 };
 #if defined(__CUDACC__)
@@ -66,6 +66,7 @@ static const SmtRec smt_rec = SmtRec();
 // What the plan needs from the lattice alone (host): distances, and the table's Ewald split.
 struct SmoothLat {
   int ok;
+  cplx e1, e2;   // Bloch phases e^{i k||.d1}, e^{i k||.d2}
   double dimg;   // distance from the cell to the nearest image other than the origin
   double dblk;   // ... to the nearest image outside a point's 2 x 2 block
   double terms;  // lattice terms of one full evaluation (estimate)
@@ -84,6 +85,9 @@ struct SmoothGrid {
   int ncent;
   int nq4, nq3;           // points of the smooth rules (quads, triangles)
   double hz, rs;          // vertical spacing; sphere radius
+  double rn1, rn2, rhz;   // 1 / n1, 1 / n2, 1 / hz
+  double top;             // k^{L+1} / (2L+3)!!
+  cplx e1, e2;            // the lattice's Bloch phases
 };
 struct SmoothPlan : SmoothGrid {
   double cth[SMT_LMAX + 1], sth[SMT_LMAX + 1], wth[SMT_LMAX + 1];
@@ -128,6 +132,8 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S)
           if (!(inu && inv)) db = fmin(db, d);
         }
     }
+  S.e1 = expi(L.vkx * L.d1x + L.vky * L.d1y);
+  S.e2 = expi(L.vkx * L.d2x + L.vky * L.d2y);
   S.dimg = sqrt(d0);
   S.dblk = sqrt(db);
   // Ewald terms of a per-point sum, at the split parameter the clamp gives near the origin
@@ -153,28 +159,30 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S)
   S.ok = 1;
 }
 
-// Gauss points per direction for a smooth integrand on an edge of half length h: a wave of number k
-// and images at distance d, times the (linear) shape functions.  The error term of the n-point rule,
-// 2^{2n+1} (n!)^4 / ((2n+1) ((2n)!)^3) f^{(2n)} h^{2n+1}, and the ellipse of analyticity through an
-// image on the edge's line; and the area factor |W|, whose branch points lie 1 / bend half edges away.
-// 0 when SMT_NQMAX points do not reach 2e-16.
+// Gauss points per direction for a smooth integrand on an edge of half length h: a wave of number k and
+// images at distance d, times the (linear) shape functions, and the area factor |W| of an element whose
+// normal turns by `bend`.  The error of the n-point rule is K_n f^{(2n)} h^{2n} / (2n)!, K_n = 2^{2n}
+// (n!)^4 / ((2n+1) ((2n)!)^2) (mean over the edge); for the images it is the ellipse of analyticity
+// through one on the edge's line; |W| = |W0| sqrt(1 + bend^2 x^2) has the Taylor coefficient
+// binom(1/2, n) bend^{2n} ~ bend^{2n} / (2 sqrt(pi) n^{3/2}).  The smallest n whose errors, for the worst
+// direction, stay below SMT_QTOL; 0 when SMT_NQMAX points do not reach it.
 BEM_HD int smooth_nq(double k, double h, double d, double bend)
 {
   const double x = k * h, q = d / h;
   if (!(q > 1.5)) return 0;
   const double rho = q + sqrt(q * q - 1.0);
-  const double rhw = (1.0 + sqrt(1.0 + bend * bend)) / (bend > 1e-9 ? bend : 1e-9);
+  const double lb = log(bend > 1e-9 ? bend : 1e-9), lx = log(x), lr = log(rho);
   double lf = 0.0;   // ln n!
   double lf2 = 0.0;  // ln (2n)!
   for (int n = 1; n <= SMT_NQMAX; n++) {
     lf += log((double)n);
     lf2 += log((double)(2 * n - 1)) + log((double)(2 * n));
     if (n < 4) continue;
-    const double c = (2 * n) * 0.6931471805599453 + 4.0 * lf - log(2.0 * n + 1.0) - 3.0 * lf2;
-    const double e1 = exp(c + (2 * n - 1) * log(x)) * (x + 2 * n);
-    const double e2 = 4.0 * exp(-(2 * n - 1) * log(rho));
-    const double e3 = 4.0 * exp(-2 * n * log(rhw));
-    if (e1 <= 2e-16 && e2 <= 2e-16 && e3 <= 2e-16) return n;
+    const double K = (2 * n) * 0.6931471805599453 + 4.0 * lf - log(2.0 * n + 1.0) - 2.0 * lf2;
+    const double e1 = exp(K - lf2 + (2 * n - 1) * lx) * (x + 2 * n);
+    const double e2 = 4.0 * exp(-(2 * n - 1) * lr);
+    const double e3 = exp(K + 2 * n * lb) * 0.29 / (n * sqrt((double)n));
+    if (e1 <= SMT_QTOL && e2 <= SMT_QTOL && e3 <= SMT_QTOL) return n;
   }
   return 0;
 }
@@ -234,79 +242,106 @@ BEM_HD double smooth_cost(const SmoothLat& S, double det, double pts, double nce
   return pts * (14.0 * nc + 400.0) + ncent * 2.0 * nc * (8.0 * (S.no1 + S.no2) + real);
 }
 
-// jh_l(x) for l = 0 .. L + 1 into out[l * st], x2 = x^2 (x <= 2.5): the top two from the series, the
-// rest by the downward recurrence.
-BEM_HD void smooth_radial(double x2, int L, double* out, int st)
+// f_l(r) = j_l(k r) / r^l for l = 0 .. L + 1 into out[l * st], r2 = r^2 (k r <= 2.5): the top two from
+// the series j_l(x) = x^l / (2l+1)!! (1 - x^2 / (2 (2l+3)) + ...), the rest by f_{l-1} = ((2l+1) f_l -
+// k r^2 f_{l+1}) / k.  top = k^{L+1} / (2L+3)!!.
+BEM_HD void smooth_radial(double k, double r2, int L, double top, double* out, int st)
 {
-  const double t = -0.5 * x2;
-  double top[2];
+  const double t = -0.5 * k * k * r2, ik = 1.0 / k;
+  double f[2];
   for (int q = 0; q < 2; q++) {
     const int l = L + 1 - q;
     double s = 1.0, term = 1.0;
     for (int i = 1; i <= 12; i++) {
-      term *= t / ((double)i * (2.0 * l + 2.0 * i + 1.0));
+      term *= t * smt_rec.inv[i] * smt_rec.inv[2 * l + 2 * i + 1];
       s += term;
       if (fabs(term) < 1e-18) break;
     }
-    top[q] = s;
+    f[q] = s * top;
+    top *= (2.0 * L + 3.0) * ik;
   }
-  double hi = top[0], lo = top[1];
+  double hi = f[0], lo = f[1];
   out[(L + 1) * st] = hi;
   out[L * st] = lo;
+  const double kr2 = k * r2;
   for (int l = L; l >= 1; l--) {
-    const double n = lo - x2 * (smt_rec.g[l - 1] * smt_rec.g[l]) * hi;  // 1 / ((2l + 1)(2l + 3))
+    const double n = ((2.0 * l + 1.0) * lo - kr2 * hi) * ik;
     hi = lo;
     lo = n;
     out[(l - 1) * st] = n;
   }
 }
 
+// Coefficient i of a centre (16-byte load; the table is 256-byte aligned).
+BEM_HD cplx smt_ld(const cplx* __restrict__ al, int i)
+{
+#if defined(__CUDA_ARCH__)
+  const double2 v = __ldg(reinterpret_cast<const double2*>(al) + i);
+  return mk(v.x, v.y);
+#else
+  return al[i];
+#endif
+}
+
 // S and W . grad S at the offset (x, y, z) from a centre, from its coefficients al; rad as
-// smooth_radial fills it for (k r)^2.
+// smooth_radial fills it.  The coefficients are one stream; the next pair of it is loaded a
+// step ahead (up to 2 past the centre's: the table has SMT_PAD more).
+#define SMT_PAD 4
 BEM_HD void smooth_eval(const cplx* __restrict__ al, int L, double k, double x, double y, double z, double Wx, double Wy,
                         double Wz, const double* rad, int st, cplx& S, cplx& D)
 {
   const double r2 = x * x + y * y + z * z;
   const double wd = Wx * x + Wy * y + Wz * z;
-  const double wd2 = 2.0 * wd, kw = -k * k * wd;
+  const double wd2 = 2.0 * wd, kw = -k * wd;  // d f_l / dr = -k r f_{l+1}
   double Sr = 0.0, Si = 0.0, Dr = 0.0, Di = 0.0;
-  {  // m = 0
+  cplx A = smt_ld(al, 0);
+  {  // m = 0: R_l^0, its derivative along W; v, u: value and derivative times f_l
     double a = 1.0, d = 0.0, b = 0.0, e = 0.0;
     double j = rad[0];
     for (int l = 0; l <= L; l++) {
+      const cplx An = smt_ld(al, l + 1);
       const double jn = rad[(l + 1) * st];
-      const double v = j * a, u = j * d + (kw * smt_rec.g[l] * jn) * a;
-      const cplx A = al[l];
+      const double v = j * a, u = j * d + (kw * jn) * a;
       Sr += A.re * v; Si += A.im * v; Dr += A.re * u; Di += A.im * u;
       const double c = smt_rec.c[0][l + 1], t1 = c * r2, t2 = c * wd2;
       const double na = z * a - t1 * b, nd = z * d + Wz * a - t2 * b - t1 * e;
       b = a; e = d; a = na; d = nd;
       j = jn;
+      A = An;
     }
   }
   al += L + 1;
+  cplx B = smt_ld(al, 1);
   double pr = x, pi = y, qr = Wx, qi = Wy;  // R_m^m and its derivative along W
   for (int m = 1; m <= L; m++) {
     double ar = pr, ai = pi, dr = qr, di = qi, br = 0.0, bi = 0.0, er = 0.0, ei = 0.0;
-    double j = rad[m * st];
-#if defined(__CUDA_ARCH__)
-#pragma unroll 2
-#endif
-    for (int l = m; l <= L; l++) {
-      const double jn = rad[(l + 1) * st];
-      const double g = kw * smt_rec.g[l] * jn;
-      const double vr = j * ar, vi = j * ai, ur = j * dr + g * ar, ui = j * di + g * ai;
-      const cplx A = al[0], B = al[1];
+    const double* rl = rad + m * st;
+    const double* rc = &smt_rec.c[m][m + 1];
+    double j = rl[0];
+    // one degree: adds the terms of R_l^m = (ar, ai), then (br, bi) becomes R_{l+1}^m
+    auto step = [&](double& ar, double& ai, double& dr, double& di, double& br, double& bi, double& er, double& ei) {
       al += 2;
+      const cplx An = smt_ld(al, 0), Bn = smt_ld(al, 1);
+      rl += st;
+      const double jn = *rl;
+      const double g = kw * jn;
+      const double vr = j * ar, vi = j * ai, ur = j * dr + g * ar, ui = j * di + g * ai;
       Sr += A.re * vr; Si += A.im * vr; Dr += A.re * ur; Di += A.im * ur;
       Sr += B.re * vi; Si += B.im * vi; Dr += B.re * ui; Di += B.im * ui;
-      const double c = smt_rec.c[m][l + 1], t1 = c * r2, t2 = c * wd2;
-      const double nr = z * ar - t1 * br, ni = z * ai - t1 * bi;
-      const double ndr = z * dr + Wz * ar - t2 * br - t1 * er, ndi = z * di + Wz * ai - t2 * bi - t1 * ei;
-      br = ar; bi = ai; er = dr; ei = di;
-      ar = nr; ai = ni; dr = ndr; di = ndi;
+      const double c = *rc++, t1 = c * r2, t2 = c * wd2;
+      er = z * dr + Wz * ar - t2 * br - t1 * er;
+      ei = z * di + Wz * ai - t2 * bi - t1 * ei;
+      br = z * ar - t1 * br;
+      bi = z * ai - t1 * bi;
       j = jn;
+      A = An; B = Bn;
+    };
+    int l = m;
+    for (; l < L; l += 2) {
+      step(ar, ai, dr, di, br, bi, er, ei);
+      step(br, bi, er, ei, ar, ai, dr, di);
     }
+    if (l == L) step(ar, ai, dr, di, br, bi, er, ei);
     const double nr = pr * x - pi * y, ni = pr * y + pi * x;
     const double mr = qr * x - qi * y + pr * Wx - pi * Wy, mi = qr * y + qi * x + pr * Wy + pi * Wx;
     pr = nr; pi = ni; qr = mr; qi = mi;
@@ -334,7 +369,7 @@ struct SmoothCell {
 BEM_HD void smooth_centre(const QPLattice& L, const SmoothPlan& P, int i, int j, int m, SmoothCell& c)
 {
   c.slot = (m * P.N2 + (j + P.J)) * P.N1 + (i + P.I);
-  const double u = (double)i / P.n1, v = (double)j / P.n2;
+  const double u = i * P.rn1, v = j * P.rn2;
   c.cx = u * L.d1x + v * L.d2x;
   c.cy = u * L.d1y + v * L.d2y;
   c.cz = m * P.hz;
@@ -345,7 +380,7 @@ BEM_HD void smooth_centre(const QPLattice& L, const SmoothPlan& P, int i, int j,
 BEM_HD void smooth_cell(const QPLattice& L, const SmoothPlan& P, double x, double y, double z, SmoothCell& c)
 {
   const double u = (x * L.d2y - y * L.d2x) * L.idd, v = (y * L.d1x - x * L.d1y) * L.idd;
-  int i = (int)rint(u * P.n1), j = (int)rint(v * P.n2), m = (int)rint(z / P.hz);
+  int i = (int)rint(u * P.n1), j = (int)rint(v * P.n2), m = (int)rint(z * P.rhz);
   i = i < -P.I ? -P.I : (i > P.I ? P.I : i);
   j = j < -P.J ? -P.J : (j > P.J ? P.J : j);
   m = m < 0 ? 0 : (m >= P.N3 ? P.N3 - 1 : m);
@@ -363,8 +398,9 @@ BEM_HD void smooth_rest(const QPLattice& L, const SmoothPlan& P, const cplx* __r
   SmoothCell c;
   smooth_cell(L, P, r[0], r[1], z, c);
   const double x = r[0] - c.cx, y = r[1] - c.cy, zz = z - c.cz;
-  smooth_radial(L.k * L.k * (x * x + y * y + zz * zz), P.L, rad, st);
+  smooth_radial(L.k, x * x + y * y + zz * zz, P.L, P.top, rad, st);
   smooth_eval(tab + (size_t)c.slot * smt_ncoef(P.L), P.L, L.k, x, y, zz, W[0], W[1], Wz, rad, st, g, h);
+  const cplx p1 = c.su > 0.0 ? P.e1 : conj(P.e1), p2 = c.sv > 0.0 ? P.e2 : conj(P.e2);
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
@@ -373,7 +409,7 @@ BEM_HD void smooth_rest(const QPLattice& L, const SmoothPlan& P, const cplx* __r
     const double X = a * L.d1x + b * L.d2x, Y = a * L.d1y + b * L.d2y;
     cplx gi, hi;
     smooth_image(L.k, r[0] + X, r[1] + Y, z, W[0], W[1], Wz, gi, hi);
-    const cplx ph = expi(L.vkx * X + L.vky * Y);
+    const cplx ph = q == 1 ? p1 : q == 2 ? p2 : p1 * p2;
     g += ph * gi;
     h += ph * hi;
   }
@@ -501,7 +537,7 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   if (n4 == 0) return;
   const double a = smooth_radius(degree, L.k, S.dblk);
   const double nc = smooth_grid(L, X, a, P);
-  if (!(nc > 0.0) || nc * smt_ncoef(degree) > (double)cap) return;
+  if (!(nc > 0.0) || nc * smt_ncoef(degree) + SMT_PAD > (double)cap) return;
   P.L = degree;
   P.nth = degree + 1;
   P.nph = 2 * degree + 2;
@@ -512,6 +548,10 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   cost = smooth_cost(S, fabs(L.detd), npairs * nq, nc, degree);
   const double plain = npairs * (tri ? 432.0 : 144.0) * S.terms * 200.0;
   if (cost < 0.8 * plain) P.on = 1;
+  P.rn1 = 1.0 / P.n1; P.rn2 = 1.0 / P.n2; P.rhz = 1.0 / P.hz;
+  P.e1 = S.e1; P.e2 = S.e2;
+  P.top = L.k / 3.0;
+  for (int l = 1; l <= degree; l++) P.top *= L.k / (2.0 * l + 3.0);
   // the sphere: the ball of the grid cell's half diagonal, off the origin's image by 5 % of it
   const double ax = L.d1x / P.n1, ay = L.d1y / P.n1, bx = L.d2x / P.n2, by = L.d2y / P.n2;
   const double dp = (ax + bx) * (ax + bx) + (ay + by) * (ay + by), dm = (ax - bx) * (ax - bx) + (ay - by) * (ay - by);
@@ -562,7 +602,7 @@ BEM_HD void smooth_tables_a(SmoothPlan& P, int part, int nparts)
     P.q3[3 * q + 2] = 6.0 * wa * wb * u;
   }
 }
-// projection weights: w_t p_lm(theta_t) / (norm rs^l jh_l(k rs)) x (1 or 2) / nph.  Stage b fills
+// projection weights: w_t p_lm(theta_t) / (norm rs^l f_l(rs)) x (1 or 2) / nph.  Stage b fills
 // p_lm(theta_t), stage c scales each (m, l).
 BEM_HD void smooth_tables_b(SmoothPlan& P, int part, int nparts)
 {
@@ -581,7 +621,7 @@ BEM_HD void smooth_tables_b(SmoothPlan& P, int part, int nparts)
 BEM_HD void smooth_tables_c(SmoothPlan& P, double k, int part, int nparts)
 {
   double rad[SMT_LMAX + 2];
-  smooth_radial(k * k * P.rs * P.rs, P.L, rad, 1);
+  smooth_radial(k, P.rs * P.rs, P.L, P.top, rad, 1);
   for (int i = part; i < (P.L + 1) * (P.L + 1); i += nparts) {
     const int m = i / (P.L + 1), l = i - m * (P.L + 1);
     if (l < m) continue;

@@ -90,7 +90,7 @@ int sh_plan(const double* lat, const double* geo, int ne, double npairs, int deg
   smooth_tables_a(D.P, 0, 1);
   smooth_tables_b(D.P, 0, 1);
   smooth_tables_c(D.P, D.L.k, 0, 1);
-  D.tab.assign((size_t)D.P.ncent * smt_ncoef(D.P.L), mk(0, 0));
+  D.tab.assign((size_t)D.P.ncent * smt_ncoef(D.P.L) + SMT_PAD, mk(0, 0));
   D.have.assign(D.P.ncent, 0);
   return 1;
 }

@@ -2,7 +2,7 @@
 the host build, against an Ewald sum with a small split parameter (numpy, scipy's w and erfcx) and
 against the plain lattice sums of the same build.
 
-Tolerance: the expansions and the smooth rules are truncated below 2e-16 (SMT_TOL, smooth_nq), rounding
+Tolerance: the expansions and the smooth rules are truncated below 5e-16 (SMT_TOL, SMT_QTOL), rounding
 adds a few 1e-15 of the parts' size, so G and H of a pair must agree with the reference to 1e-13 of its
 largest entry of each kind plus 1e-14 of the size the cancelling parts have (the pair's near and smooth
 parts, at most a few times the largest G times 1 / distance).  The plain sums' own error grows with the
