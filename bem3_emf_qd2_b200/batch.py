@@ -42,14 +42,23 @@ def domain_output_bytes(ne: int) -> int:
 
 
 # scratch the batch allocates for a domain (bem3_batch_scratch_bytes, per domain): per-pair F
-# terms (24 B per pair), self-pair terms, the near-singular list, the propagating-order list
+# terms (24 B per pair), self-pair terms, the near-singular list; for periodic domains the
+# propagating-order list and the table of the smooth remainder with its plan and lists
 PROP_LIST_BYTES = 32 * 2048
+PLAN_BYTES = 48 << 10
+
+
+def table_coefficients(ne: int) -> int:
+    """Coefficients a periodic domain's table may hold (48 bytes each with its samples)."""
+    return 1 << 19 if ne < 256 else (1 << 21 if ne < 640 else 1 << 22)
 
 
 def domain_scratch_bytes(ne: int, periodic: bool) -> int:
     np_ = 4 * ne * ne
     b = 24 * np_ + 96 * ne + 4 * (np_ // 8 + 4096) + 4 * 256
-    return b + (PROP_LIST_BYTES if periodic else 0)
+    if periodic:
+        b += PROP_LIST_BYTES + PLAN_BYTES + 48 * table_coefficients(ne) + 4 * np_ + 4 * (np_ // 8 + 4096)
+    return b
 
 
 def instance_domains(p) -> List[Tuple[int, int, bool]]:

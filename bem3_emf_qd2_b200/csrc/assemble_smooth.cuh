@@ -128,11 +128,11 @@ static inline size_t smooth_spec_smem(const SmoothLat& S)
 {
   return sizeof(cplx) * ((size_t)2 * S.no1 * S.no2 + (size_t)S.no1 * SMT_JT);
 }
-__global__ void __launch_bounds__(SMT_SPEC_THREADS) k_smooth_spectral(const __grid_constant__ QPLattice L, SmoothArgs M)
+__device__ __forceinline__ void smooth_spectral_block(const QPLattice& L, const SmoothArgs& M, int first, int stride,
+                                                      unsigned char* spec_smem)
 {
   const SmoothPlan& P = *M.plan;
   if (!P.on) return;
-  extern __shared__ __align__(16) unsigned char spec_smem[];
   const SmoothLat& S = M.S;
   const int no = S.no1 * S.no2, ns = P.nth * P.nph;
   cplx* F = (cplx*)spec_smem;  // height functions of this block's height
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(SMT_SPEC_THREADS) k_smooth_spectral(const __gr
   for (int i = threadIdx.x; i < P.n1; i += blockDim.x) tw1[i] = expi(2.0 * QP_PI * i / P.n1);
   for (int i = threadIdx.x; i < P.n2; i += blockDim.x) tw2[i] = expi(2.0 * QP_PI * i / P.n2);
   const int items = P.N3 * P.nth * SMT_FG;
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+  for (int it = first; it < items; it += stride) {
     const int g = it % SMT_FG, t = it / SMT_FG % P.nth, m = it / (SMT_FG * P.nth);
     const double z = fabs(m * P.hz + P.rs * P.cth[t]);
     __syncthreads();
@@ -199,15 +199,21 @@ __global__ void __launch_bounds__(SMT_SPEC_THREADS) k_smooth_spectral(const __gr
   }
 }
 
+__global__ void __launch_bounds__(SMT_SPEC_THREADS) k_smooth_spectral(const __grid_constant__ QPLattice L, SmoothArgs M)
+{
+  extern __shared__ __align__(16) unsigned char spec_smem[];
+  smooth_spectral_block(L, M, blockIdx.x, gridDim.x, spec_smem);
+}
+
 #define SMT_PROJ_THREADS 128
-__global__ void __launch_bounds__(SMT_PROJ_THREADS) k_smooth_project(const __grid_constant__ QPLattice L, SmoothArgs M)
+__device__ __forceinline__ void smooth_project_block(const QPLattice& L, const SmoothArgs& M, int first, int stride)
 {
   const SmoothPlan& P = *M.plan;
   if (!P.on) return;
   __shared__ cplx smp[2 * (SMT_LMAX + 1) * (SMT_LMAX + 1)];
   __shared__ cplx ca[(SMT_LMAX + 1) * (SMT_LMAX + 1)], cb[(SMT_LMAX + 1) * (SMT_LMAX + 1)];
   const int ns = P.nth * P.nph, L1 = P.L + 1, nc = smt_ncoef(P.L);
-  for (int slot = blockIdx.x; slot < P.ncent; slot += gridDim.x) {
+  for (int slot = first; slot < P.ncent; slot += stride) {
     const cplx* in = M.smp + (size_t)slot * ns;
     SmoothCell c;
     smooth_slot(L, P, slot, c);
@@ -242,6 +248,11 @@ __global__ void __launch_bounds__(SMT_PROJ_THREADS) k_smooth_project(const __gri
   }
 }
 
+__global__ void __launch_bounds__(SMT_PROJ_THREADS) k_smooth_project(const __grid_constant__ QPLattice L, SmoothArgs M)
+{
+  smooth_project_block(L, M, blockIdx.x, gridDim.x);
+}
+
 // ------------------------------------------------------------------------------------------
 // Regular pairs.  A warp takes SMT_PAIRS consecutive sources of one row: their rule points for the
 // nearest image and the solid angle (32 points of one pair at a time, sums in registers), then their
@@ -270,21 +281,15 @@ struct SmoothWarp {
   };
 };
 
-__global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS)
-    k_reg_smooth(AssembleArgs A, const __grid_constant__ QPLattice L, SmoothArgs M, int r0, int nr, double3* Fp,
-                 unsigned* gh_list, unsigned* gh_count, unsigned gh_cap, unsigned* ip_list, unsigned* ip_count, int* status)
+// Unit `unit` of the rows r0, r0 + 1, ...: sources 4 (unit mod upr) .. + 3 of row r0 + unit / upr, by one
+// warp.  xl, wl: the 12-point Gauss rule in shared memory.
+__device__ __forceinline__ void reg_smooth_unit(const AssembleArgs& A, const QPLattice& L, const SmoothArgs& M, int r0,
+                                                long long unit, double3* Fp, unsigned* gh_list, unsigned* gh_count,
+                                                unsigned gh_cap, unsigned* ip_list, unsigned* ip_count, int* status,
+                                                SmoothWarp& w, const double* xl, const double* wl, int lane)
 {
   const SmoothPlan& P = *M.plan;
-  if (!P.on) return;
-  extern __shared__ __align__(16) unsigned char smt_smem[];
-  __shared__ double xl[12], wl[12];
-  if (threadIdx.x < 12) { xl[threadIdx.x] = c_xl[threadIdx.x]; wl[threadIdx.x] = c_wl[threadIdx.x]; }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  SmoothWarp& w = reinterpret_cast<SmoothWarp*>(smt_smem)[threadIdx.x >> 5];
   const int upr = (A.ne + SMT_PAIRS - 1) / SMT_PAIRS;
-  const long long unit = (long long)blockIdx.x * SMT_WARPS + (threadIdx.x >> 5);
-  if (unit >= (long long)upr * nr) return;  // uniform across the warp; no block barrier below
   const int rr = (int)(unit / upr), s0 = (int)(unit - (long long)rr * upr) * SMT_PAIRS;
   const int row = r0 + rr, t = row >> 2, tn = row & 3;
   double rt[3], v0[3], v1[3];
@@ -421,6 +426,22 @@ __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS)
       if (it == 0) Fp[pair] = make_double3(tot[16] * fs, dFz, dFe);
     }
   }
+}
+
+__global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS)
+    k_reg_smooth(AssembleArgs A, const __grid_constant__ QPLattice L, SmoothArgs M, int r0, int nr, double3* Fp,
+                 unsigned* gh_list, unsigned* gh_count, unsigned gh_cap, unsigned* ip_list, unsigned* ip_count, int* status)
+{
+  if (!M.plan->on) return;
+  extern __shared__ __align__(16) unsigned char smt_smem[];
+  __shared__ double xl[12], wl[12];
+  if (threadIdx.x < 12) { xl[threadIdx.x] = c_xl[threadIdx.x]; wl[threadIdx.x] = c_wl[threadIdx.x]; }
+  __syncthreads();
+  const int wib = threadIdx.x >> 5;
+  const long long unit = (long long)blockIdx.x * SMT_WARPS + wib;
+  if (unit >= (long long)((A.ne + SMT_PAIRS - 1) / SMT_PAIRS) * nr) return;  // uniform across the warp
+  reg_smooth_unit(A, L, M, r0, unit, Fp, gh_list, gh_count, gh_cap, ip_list, ip_count, status,
+                  reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xl, wl, threadIdx.x & 31);
 }
 
 // Near-singular pair w of the chunk starting at pair p0, by the whole CTA: the 64 x 64 rule for the

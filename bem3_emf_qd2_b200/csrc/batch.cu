@@ -9,20 +9,24 @@
 //
 //   descriptor table  BatchDomain[nd] in device memory: the domain's AssembleArgs, its own
 //                     QPLattice (Bloch wave vector, Ewald split parameter veps0, propagating
-//                     orders) and its scratch (per-pair F terms, near-singular work list,
-//                     status word);
+//                     orders), its scratch (per-pair F terms, near-singular work list,
+//                     status word) and, for periodic domains, the plan and table of the smooth
+//                     remainder (assemble_smooth.cuh), which every run makes anew;
 //   work segments     per pair class, the cumulative work of the domains of that class
 //                     (rows, pairs or pair units); a launch maps its global work index to
 //                     (domain, local index) by binary search over them;
-//   persistent kernel k_batch_reg_periodic, the dominant class: every warp takes `grab` units of
-//                     REGP_PAIRS pairs at a time from one device counter until the batch's
-//                     regular periodic pairs are exhausted, whatever domain they belong to;
-//   graph             reset, zero, then two branches -- periodic (self, regular, near-singular)
-//                     and interior (self, regular, near-singular) -- joined before the row sums.
+//   persistent kernel k_batch_reg_periodic, the pairs summed point by point (domains without a
+//                     table, and the pairs in one plane that a table leaves): every warp takes
+//                     `grab` units of REGP_PAIRS pairs at a time from one device counter until they
+//                     are exhausted, whatever domain they belong to;
+//   graph             reset, zero, then two branches -- periodic (tables, self, regular,
+//                     near-singular) and interior (self, regular, near-singular) -- joined before the
+//                     row sums.
 //
 // Every pair is computed by the same device functions, in the same order of operations, as in
 // the one-domain kernels (assemble.cu), so a domain's matrices do not depend on what else is in
-// the batch.
+// the batch.  Measured on a B200, four two-layer problems of 192 quads with creation and wait: 218 ms
+// with point-by-point periodic sums, 25.5 ms with the tables.
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -40,6 +44,10 @@ struct BatchDomain {
   unsigned* gh_count;  // entries appended (may exceed gh_cap: then status -900)
   unsigned gh_cap;
   int* status;         // the domain's status word (first error code)
+  SmoothArgs M;        // periodic domains: plan and table (plan == nullptr: none)
+  unsigned* ip_list;   // [4 ne * ne] pairs in one plane, left to the point-by-point sums
+  unsigned* smt_list;  // [gh_cap] near-singular pairs of the tabulated ones
+  unsigned* smt_count; // entries of smt_list, then of ip_list
 };
 
 // Cumulative work of the domains of one class: base[0] = 0, base[n] = total, domain dom[i]
@@ -69,6 +77,7 @@ __global__ void k_batch_reset(BatchDomain* D, int nd, unsigned long long* next)
   if (i == 0) next[0] = 0ull;
   if (i < nd) {
     *D[i].gh_count = 0u;
+    if (D[i].smt_count) D[i].smt_count[0] = D[i].smt_count[1] = 0u;
     *D[i].status = 0;
   }
 }
@@ -94,6 +103,29 @@ __global__ void k_batch_zero(const BatchDomain* __restrict__ D)
   for (size_t i = i0; i < N; i += stride) d.Fself[i] = make_double3(0.0, 0.0, 0.0);
 }
 
+// Tables of the periodic domains dom[blockIdx.y].
+__global__ void __launch_bounds__(SMT_PLAN_THREADS) k_batch_smooth_plan(const BatchDomain* __restrict__ D,
+                                                                        const int* __restrict__ dom)
+{
+  const BatchDomain& d = D[dom[blockIdx.x]];
+  if (d.M.plan) smooth_plan_block(d.A, d.L, d.M);
+}
+__global__ void __launch_bounds__(SMT_SPEC_THREADS) k_batch_smooth_spectral(const BatchDomain* __restrict__ D,
+                                                                            const int* __restrict__ dom)
+{
+  extern __shared__ __align__(16) unsigned char spec_smem[];
+  const BatchDomain& d = D[dom[blockIdx.y]];
+  if (d.M.plan) smooth_spectral_block(d.L, d.M, blockIdx.x, gridDim.x, spec_smem);
+}
+__global__ void __launch_bounds__(SMT_PROJ_THREADS) k_batch_smooth_project(const BatchDomain* __restrict__ D,
+                                                                           const int* __restrict__ dom)
+{
+  const BatchDomain& d = D[dom[blockIdx.y]];
+  if (d.M.plan) smooth_project_block(d.L, d.M, blockIdx.x, gridDim.x);
+}
+
+__device__ __forceinline__ bool batch_smooth(const BatchDomain& d) { return d.M.plan && d.M.plan->on; }
+
 __global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_periodic(const BatchDomain* __restrict__ D, BatchSeg S)
 {
   __shared__ double red[SELF_THREADS / 32][24];
@@ -101,7 +133,39 @@ __global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_periodic(const B
   const long long g = blockIdx.x;
   const int i = seg_find(S, g);
   const BatchDomain& d = D[S.dom[i]];
+  if (batch_smooth(d)) return;
   self_periodic_row(d.A, d.L, (int)(g - S.base[i]), d.Fself, d.status, red, serr);
+}
+
+__global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_smooth(const BatchDomain* __restrict__ D, BatchSeg S)
+{
+  __shared__ double red[SELF_THREADS / 32][24];
+  __shared__ double xl[12], wl[12], xh[64], wh[64];
+  const long long g = blockIdx.x;
+  const int i = seg_find(S, g);
+  const BatchDomain& d = D[S.dom[i]];
+  if (!batch_smooth(d)) return;
+  if (threadIdx.x < 12) { xl[threadIdx.x] = c_xl[threadIdx.x]; wl[threadIdx.x] = c_wl[threadIdx.x]; }
+  if (threadIdx.x < 64) { xh[threadIdx.x] = c_xh[threadIdx.x]; wh[threadIdx.x] = c_wh[threadIdx.x]; }
+  __syncthreads();
+  self_smooth_row(d.A, d.L, *d.M.plan, d.M.tab, (int)(g - S.base[i]), d.Fself, red, xl, wl, xh, wh);
+}
+
+// Tabulated regular pairs: S counts units of SMT_PAIRS sources (reg_smooth_unit), one warp each.
+__global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth(const BatchDomain* __restrict__ D, BatchSeg S)
+{
+  extern __shared__ __align__(16) unsigned char smt_smem[];
+  __shared__ double xl[12], wl[12];
+  if (threadIdx.x < 12) { xl[threadIdx.x] = c_xl[threadIdx.x]; wl[threadIdx.x] = c_wl[threadIdx.x]; }
+  __syncthreads();
+  const int wib = threadIdx.x >> 5;
+  const long long u = (long long)blockIdx.x * SMT_WARPS + wib;
+  if (u >= S.base[S.n]) return;  // uniform across the warp
+  const int i = seg_find(S, u);
+  const BatchDomain& d = D[S.dom[i]];
+  if (!batch_smooth(d)) return;
+  reg_smooth_unit(d.A, d.L, d.M, 0, u - S.base[i], d.Fp, d.smt_list, d.smt_count, d.gh_cap, d.ip_list, d.smt_count + 1,
+                  d.status, reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xl, wl, threadIdx.x & 31);
 }
 
 __global__ void __launch_bounds__(SI_THREADS) k_batch_self_interior(const BatchDomain* __restrict__ D, BatchSeg S)
@@ -133,8 +197,11 @@ __global__ void __launch_bounds__(256, REGP_MIN_BLOCKS) k_batch_reg_periodic(con
     for (long long u = (long long)u0; u < uend; u++) {
       const int i = seg_find(S, u);
       const BatchDomain& d = D[S.dom[i]];
-      const long long np = 4LL * d.A.ne * d.A.ne;
-      reg_periodic_unit(d.A, d.L, 0, np, (u - S.base[i]) * REGP_PAIRS, nullptr, d.Fp, d.gh_list, d.gh_count, d.gh_cap, d.status,
+      const bool on = batch_smooth(d);  // then only the pairs in one plane are left
+      const long long np = on ? (long long)d.smt_count[1] : 4LL * d.A.ne * d.A.ne;
+      const long long first = (u - S.base[i]) * REGP_PAIRS;
+      if (first >= np) continue;
+      reg_periodic_unit(d.A, d.L, 0, np, first, on ? d.ip_list : nullptr, d.Fp, d.gh_list, d.gh_count, d.gh_cap, d.status,
                         sw[wib], sacc, lane);
     }
   }
@@ -159,6 +226,21 @@ __global__ void __launch_bounds__(256, 2) k_batch_gh_periodic(const BatchDomain*
     const BatchDomain& d = D[dom[i]];
     const unsigned cnt = min(*d.gh_count, d.gh_cap);
     for (unsigned it = blockIdx.x; it < cnt; it += gridDim.x) gh_periodic_pair(d.A, d.L, 0, d.gh_list[it], d.Fp, d.status, red, serr);
+  }
+}
+
+__global__ void __launch_bounds__(256, 2) k_batch_gh_smooth(const BatchDomain* __restrict__ D, const int* __restrict__ dom, int n)
+{
+  __shared__ double red[8][19];
+  __shared__ double xh[64], wh[64];
+  if (threadIdx.x < 64) { xh[threadIdx.x] = c_xh[threadIdx.x]; wh[threadIdx.x] = c_wh[threadIdx.x]; }
+  __syncthreads();
+  for (int i = 0; i < n; i++) {
+    const BatchDomain& d = D[dom[i]];
+    if (!batch_smooth(d)) continue;
+    const unsigned cnt = min(d.smt_count[0], d.gh_cap);
+    for (unsigned it = blockIdx.x; it < cnt; it += gridDim.x)
+      gh_smooth_pair(d.A, d.L, *d.M.plan, d.M.tab, 0, d.smt_list[it], d.Fp, red, xh, wh);
   }
 }
 
@@ -245,7 +327,12 @@ extern "C" size_t bem3_batch_scratch_bytes(const bem3_batch_domain* doms, int n)
     const size_t np = 4 * ne * ne;
     total += ((np * sizeof(double3) + 255) & ~(size_t)255) + ((4 * ne * sizeof(double3) + 255) & ~(size_t)255) +
              (((np / 8 + 4096) * sizeof(unsigned) + 255) & ~(size_t)255) + 256;
-    if (doms[i].periodic) total += (sizeof(QPProp) * QP_PROP_CAP + 255) & ~(size_t)255;
+    if (doms[i].periodic) {
+      total += (sizeof(QPProp) * QP_PROP_CAP + 255) & ~(size_t)255;
+      // the table (48 bytes a coefficient with its samples), its plan and lists
+      total += (size_t)bem3_smooth_cap((int)ne) * 48 + ((sizeof(SmoothPlan) + 255) & ~(size_t)255) + np * sizeof(unsigned) +
+               (np / 8 + 4096) * sizeof(unsigned) + 1024;
+    }
   }
   // table, status words and segments
   total += (((sizeof(BatchDomain) + 2 * sizeof(long long) + 5 * sizeof(int)) * (size_t)n + 8 * sizeof(long long)) * 5 +
@@ -273,6 +360,12 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
   if (cudaFuncSetAttribute(k_batch_reg_periodic, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
       cudaFuncSetAttribute(k_batch_reg_periodic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGP_SMEM_BYTES) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_batch_reg_smooth, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+      cudaFuncSetAttribute(k_batch_reg_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(SMT_WARPS * sizeof(SmoothWarp))) != cudaSuccess ||
+      cudaFuncSetAttribute(k_batch_smooth_spectral, cudaFuncAttributeMaxDynamicSharedMemorySize, SMT_SPEC_SMEM) !=
           cudaSuccess)
     return BEM3_ERR_CUDA;
 
@@ -283,7 +376,8 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
   // host descriptors, lattices and propagating orders
   std::vector<BatchDomain> hD((size_t)n);
   std::vector<std::vector<QPProp>> props((size_t)n);
-  SegHost selfP, selfI, regP, regI, rows;
+  SegHost selfP, selfI, regP, regI, rows, smtP;
+  size_t spec_smem = 0;
   std::vector<int> pdom, idom;
   for (int i = 0; i < n; i++) {
     const bem3_batch_domain& d = doms[i];
@@ -305,6 +399,12 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
       B.L.nprop = np;
       selfP.add(i, 4 * ne);
       regP.add(i, (4 * ne * ne + REGP_PAIRS - 1) / REGP_PAIRS);
+      smtP.add(i, 4 * ne * ((ne + SMT_PAIRS - 1) / SMT_PAIRS));
+      smooth_lattice(B.L, B.M.S);
+      if (B.M.S.ok) {
+        B.M.cap = bem3_smooth_cap((int)ne);
+        spec_smem = std::max(spec_smem, smooth_spec_smem(B.M.S));
+      }
       pdom.push_back(i);
     } else {
       selfI.add(i, 4 * ne);
@@ -319,15 +419,17 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
   const size_t oD = Lay.take(sizeof(BatchDomain) * (size_t)n);
   const size_t oStatus = Lay.take(sizeof(int) * (size_t)n);
   const size_t oNext = Lay.take(sizeof(unsigned long long) * 4);
-  SegHost* segs[5] = {&selfP, &selfI, &regP, &regI, &rows};
-  size_t oBase[5], oDom[5];
-  for (int k = 0; k < 5; k++) {
+  constexpr int NSEG = 6;
+  SegHost* segs[NSEG] = {&selfP, &selfI, &regP, &regI, &rows, &smtP};
+  size_t oBase[NSEG], oDom[NSEG];
+  for (int k = 0; k < NSEG; k++) {
     oBase[k] = Lay.take(sizeof(long long) * segs[k]->base.size());
     oDom[k] = Lay.take(sizeof(int) * (segs[k]->dom.size() + 1));
   }
   const size_t oPdom = Lay.take(sizeof(int) * (pdom.size() + 1));
   const size_t oIdom = Lay.take(sizeof(int) * (idom.size() + 1));
   std::vector<size_t> oFp((size_t)n), oFself((size_t)n), oList((size_t)n), oCount((size_t)n), oProp((size_t)n, 0);
+  std::vector<size_t> oPlan((size_t)n), oTab((size_t)n), oSmp((size_t)n), oIp((size_t)n), oSl((size_t)n), oSc((size_t)n);
   for (int i = 0; i < n; i++) {
     const size_t ne = (size_t)doms[i].Ne_d, np = 4 * ne * ne;
     oFp[(size_t)i] = Lay.take(np * sizeof(double3));
@@ -336,6 +438,14 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     oList[(size_t)i] = Lay.take((size_t)hD[(size_t)i].gh_cap * sizeof(unsigned));
     oCount[(size_t)i] = Lay.take(sizeof(unsigned));
     if (doms[i].periodic && !props[(size_t)i].empty()) oProp[(size_t)i] = Lay.take(sizeof(QPProp) * props[(size_t)i].size());
+    if (hD[(size_t)i].M.cap) {
+      oPlan[(size_t)i] = Lay.take(sizeof(SmoothPlan));
+      oTab[(size_t)i] = Lay.take(sizeof(cplx) * (size_t)hD[(size_t)i].M.cap);
+      oSmp[(size_t)i] = Lay.take(sizeof(cplx) * 2 * (size_t)hD[(size_t)i].M.cap);
+      oIp[(size_t)i] = Lay.take(np * sizeof(unsigned));
+      oSl[(size_t)i] = Lay.take((size_t)hD[(size_t)i].gh_cap * sizeof(unsigned));
+      oSc[(size_t)i] = Lay.take(2 * sizeof(unsigned));
+    }
   }
   b->bytes = Lay.off;
   if (cudaMalloc(&b->mem, b->bytes) != cudaSuccess) { b->mem = nullptr; batch_free(b); return BEM3_ERR_CUDA; }
@@ -350,12 +460,20 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     B.gh_list = (unsigned*)(m + oList[(size_t)i]);
     B.gh_count = (unsigned*)(m + oCount[(size_t)i]);
     B.status = b->dstatus + i;
+    if (B.M.cap) {
+      B.M.plan = (SmoothPlan*)(m + oPlan[(size_t)i]);
+      B.M.tab = (cplx*)(m + oTab[(size_t)i]);
+      B.M.smp = (cplx*)(m + oSmp[(size_t)i]);
+      B.ip_list = (unsigned*)(m + oIp[(size_t)i]);
+      B.smt_list = (unsigned*)(m + oSl[(size_t)i]);
+      B.smt_count = (unsigned*)(m + oSc[(size_t)i]);
+    }
     if (doms[i].periodic) B.L.prop = props[(size_t)i].empty() ? nullptr : (QPProp*)(m + oProp[(size_t)i]);
   }
   // uploads (synchronous: creation is outside the timed path)
   bool ok = cudaMemcpy(b->dD, hD.data(), sizeof(BatchDomain) * (size_t)n, cudaMemcpyHostToDevice) == cudaSuccess;
-  BatchSeg S[5];
-  for (int k = 0; k < 5 && ok; k++) {
+  BatchSeg S[NSEG];
+  for (int k = 0; k < NSEG && ok; k++) {
     ok = cudaMemcpy(m + oBase[k], segs[k]->base.data(), sizeof(long long) * segs[k]->base.size(), cudaMemcpyHostToDevice) ==
          cudaSuccess;
     if (ok && !segs[k]->dom.empty())
@@ -395,6 +513,18 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     cudaEventRecord(fork, s0);
     cudaStreamWaitEvent(s1, fork, 0);
     // periodic branch
+    if (spec_smem > 0) {
+      const unsigned npd = (unsigned)pdom.size();
+      const int* dp = (const int*)(m + oPdom);
+      k_batch_smooth_plan<<<npd, SMT_PLAN_THREADS, 0, s0>>>(b->dD, dp);
+      k_batch_smooth_spectral<<<dim3((unsigned)(4 * sms), npd), SMT_SPEC_THREADS, spec_smem, s0>>>(b->dD, dp);
+      k_batch_smooth_project<<<dim3((unsigned)(8 * sms), npd), SMT_PROJ_THREADS, 0, s0>>>(b->dD, dp);
+      k_batch_self_smooth<<<(unsigned)selfP.total(), SELF_THREADS, 0, s0>>>(b->dD, S[0]);
+      k_batch_reg_smooth<<<(unsigned)((smtP.total() + SMT_WARPS - 1) / SMT_WARPS), SMT_WARPS * 32,
+                           SMT_WARPS * sizeof(SmoothWarp), s0>>>(b->dD, S[5]);
+      k_batch_gh_smooth<<<(unsigned)(sms * T.gh_blocks_per_sm), 256, 0, s0>>>(b->dD, dp, (int)npd);
+      launches += 6;
+    }
     if (selfP.total() > 0) { k_batch_self_periodic<<<(unsigned)selfP.total(), SELF_THREADS, 0, s0>>>(b->dD, S[0]); launches++; }
     if (regP.total() > 0) {
       const long long want = (regP.total() * 32 + 255) / 256;  // CTAs that would give every warp one unit
