@@ -12,7 +12,8 @@
 //   k_self_periodic / k_self_interior : one CTA per self pair (t == s), polar rule;
 //   k_reg_periodic : one warp per regular pair, lanes over the 144 (quad) / 432 (triangle)
 //                    Gauss points, one quasi-periodic Green's function per point;
-//   k_reg_interior : one thread per regular pair (free-space kernel, uniform cost);
+//   k_reg_interior : one thread per regular pair (free-space kernel, uniform cost), a warp per 32
+//                    sources of a row;
 //   k_gh_*         : pairs whose GL dF/dv exceeds CBD_SDF, recomputed with the 64x64 rule from a
 //                    compacted device work list (no host round trip);
 //   k_rowsum       : deterministic per-row sums of F, dF/dt over s, H diagonal += (1+)F.
@@ -93,29 +94,6 @@ __device__ __forceinline__ void accp_unpack(const double* v, AccP& a)
   for (int i = 0; i < 4; i++) { a.G[i] = mk(v[2 * i], v[2 * i + 1]); a.H[i] = mk(v[8 + 2 * i], v[9 + 2 * i]); }
   a.F = v[16]; a.dF0 = v[17]; a.dF1 = v[18];
 }
-// AccI <-> flat array (51 doubles)
-__device__ __forceinline__ void acci_pack(const AccI& a, double* v)
-{
-  for (int i = 0; i < 4; i++) {
-    v[2 * i] = a.G[i].re; v[2 * i + 1] = a.G[i].im;
-    v[8 + 2 * i] = a.H[i].re; v[9 + 2 * i] = a.H[i].im;
-    v[16 + 2 * i] = a.dG0[i].re; v[17 + 2 * i] = a.dG0[i].im;
-    v[24 + 2 * i] = a.dH0[i].re; v[25 + 2 * i] = a.dH0[i].im;
-    v[32 + 2 * i] = a.dG1[i].re; v[33 + 2 * i] = a.dG1[i].im;
-    v[40 + 2 * i] = a.dH1[i].re; v[41 + 2 * i] = a.dH1[i].im;
-  }
-  v[48] = a.F; v[49] = a.dF0; v[50] = a.dF1;
-}
-__device__ __forceinline__ void acci_unpack(const double* v, AccI& a)
-{
-  for (int i = 0; i < 4; i++) {
-    a.G[i] = mk(v[2 * i], v[2 * i + 1]); a.H[i] = mk(v[8 + 2 * i], v[9 + 2 * i]);
-    a.dG0[i] = mk(v[16 + 2 * i], v[17 + 2 * i]); a.dH0[i] = mk(v[24 + 2 * i], v[25 + 2 * i]);
-    a.dG1[i] = mk(v[32 + 2 * i], v[33 + 2 * i]); a.dH1[i] = mk(v[40 + 2 * i], v[41 + 2 * i]);
-  }
-  a.F = v[48]; a.dF0 = v[49]; a.dF1 = v[50];
-}
-
 // Store one pair's coefficients in the reference layout.  Done by lanes of a warp (lane l
 // stores item l) or by a single thread (lane = -1 stores all).
 __device__ __forceinline__ void store_pair(const AssembleArgs& A, int row, int s, const cplx* CC, const cplx* dCz,
@@ -345,87 +323,391 @@ __global__ void __launch_bounds__(256, 2) k_gh_periodic(AssembleArgs A, const __
 }
 
 // ==========================================================================================
-// Regular interior pair w of the chunk starting at pair p0, by one thread.
-__device__ __forceinline__ void reg_interior_pair(const AssembleArgs& A, long long p0, long long w, double3* Fp,
-                                                  unsigned* gh_list, unsigned* gh_count, unsigned gh_cap, int* status)
+// Regular interior pairs: one thread per pair, a warp's 32 pairs being consecutive sources of one row.
+//
+// The 12 x 12 rule (three of them on triangles) is walked by rows of the first coordinate a.  Along a
+// row the position, the normal, their products with the node's tangents and the shape functions are
+// linear in the second coordinate b:
+//   r - rt = P + Q b,  W = C + D b,  N_i = al_i + be_i b,
+// so a point adds a few scalars to moments sum f b^m instead of evaluating six integrands and four
+// shape functions each; the moments become shape-function sums once per row, kept in shared memory
+// (48 doubles a thread: in registers they would leave room for 8 warps an SM).  With q = (ikR - 1) e^{ikR}
+// / R^3 and e5 = ((kR)^2 + 3 (ikR - 1)) e^{ikR} (R.W) / R^5 the integrands are
+//   G = e |W| / R,  H = q (R.W),  dG_v = q |W| (R.v),  dH_v = e5 (R.v) - q (W.v).
+// e^{ikR} along a row is e^{ikR0} (its middle) times a Taylor sum in k (R - R0), without reductions and
+// branches, where every element of the warp is smaller than the sums' range.  At the end the warp writes
+// its row segments of each matrix from shared memory, 512 contiguous bytes an instruction.
+#define REGI_WARPS 4
+#define REGI_LD 33  // leading dimension of the sums (pad: the transposed read of the stores)
+#define REGI_SMEM_BYTES (sizeof(double) * 48 * REGI_LD * REGI_WARPS)
+// Ranges of the Taylor sums: cos and sin to x^18 and x^17 (next terms below 1e-17 for |x| <= 0.9), e^-y
+// to y^10 (below 1e-17 for |y| <= 0.12).
+#define REGI_XMAX 0.9
+#define REGI_YMAX 0.12
+
+__device__ __forceinline__ cplx taylor_cis(double x)
 {
-  long long p = p0 + w;
-  PairIdx q = pair_of(p, A.ne);
-  int tnn;
-  double rt[3], vtz[3], vte[3];
-  target_info(A.geo, A.sid, q.t, q.tn, rt, vtz, vte, tnn);
-  if ((q.tn == 3 && tnn == 3) || q.s == q.t) return;
-  int sd = A.sid[q.s];
-  Elem es;
-  load_elem(A.geo, abs(sd), es);
-  const int npts = (es.nn == 4) ? 144 : 432;
-  const cplx k = mk(A.kre, A.kim);
-  AccI a;
-  acci_zero(a);
-  for (int kq = 0; kq < npts; kq++) {
-    double z, e, wt;
-    rule_point(es.nn, 12, c_xl, c_wl, kq, z, e, wt);
-    acci_point(es, k, rt, vtz, vte, z, e, wt, a);
-  }
-  cplx CC[9], dCz[9], dCe[9];
-  acci_finish(es, a, sd < 0, CC, dCz, dCe);
-  if (needs_gh(dCz[8].re, dCe[8].re)) {
-    unsigned slot = atomicAdd(gh_count, 1u);
-    if (slot < gh_cap) gh_list[slot] = (unsigned)w;
-    else record_status(status, -900);
+  const double t = x * x;
+  double c = -1.0 / 6402373705728000.0, s = 1.0 / 355687428096000.0;
+  c = fma(c, t, 1.0 / 20922789888000.0);
+  s = fma(s, t, -1.0 / 1307674368000.0);
+  c = fma(c, t, -1.0 / 87178291200.0);
+  s = fma(s, t, 1.0 / 6227020800.0);
+  c = fma(c, t, 1.0 / 479001600.0);
+  s = fma(s, t, -1.0 / 39916800.0);
+  c = fma(c, t, -1.0 / 3628800.0);
+  s = fma(s, t, 1.0 / 362880.0);
+  c = fma(c, t, 1.0 / 40320.0);
+  s = fma(s, t, -1.0 / 5040.0);
+  c = fma(c, t, -1.0 / 720.0);
+  s = fma(s, t, 1.0 / 120.0);
+  c = fma(c, t, 1.0 / 24.0);
+  s = fma(s, t, -1.0 / 6.0);
+  c = fma(c, t, -0.5);
+  return mk(fma(c, t, 1.0), fma(s, t * x, x));
+}
+__device__ __forceinline__ double taylor_expm(double y)  // e^{-y}
+{
+  double s = 1.0 / 3628800.0;
+  s = fma(s, y, -1.0 / 362880.0);
+  s = fma(s, y, 1.0 / 40320.0);
+  s = fma(s, y, -1.0 / 5040.0);
+  s = fma(s, y, 1.0 / 720.0);
+  s = fma(s, y, -1.0 / 120.0);
+  s = fma(s, y, 1.0 / 24.0);
+  s = fma(s, y, -1.0 / 6.0);
+  s = fma(s, y, 0.5);
+  s = fma(s, y, -1.0);
+  return fma(s, y, 1.0);
+}
+
+// Moments of one row: with b the second coordinate and w its weight
+struct RegiRow {
+  cplx g0, g1;          // G:        sum g, g b
+  cplx h0, h1;          // H
+  cplx a0, a1, a2;      // q |W|:    sum, b, b^2
+  cplx e0, e1, e2;      // e5
+  cplx q0, q1, q2;      // q
+  double F, s0, s1, t0, t1;  // (R.W) / R^3; 3 (R.W) / R^5 and 1 / R^3: sum, b
+};
+
+// Row a (coordinate a of part `part` of a triangle's rule) of element e seen from rt: the linear forms,
+// the weight factor and the shape functions N_i = al[i] + be[i] b.
+struct RegiLine {
+  double P[3], Q[3], C[3], D[3], wf0, wf1, al[4], be[4];
+};
+__device__ __forceinline__ void regi_line(const Elem& e, const double* rt, int part, double a, RegiLine& y)
+{
+  if (e.nn == 4) {
+    y.wf0 = 1.0;
+    y.wf1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      y.P[i] = e.cr[i][0] + e.cr[i][1] * a - rt[i];
+      y.Q[i] = e.cr[i][2] + e.cr[i][3] * a;
+      y.C[i] = e.cw[i][0] + e.cw[i][1] * a;
+      y.D[i] = e.cw[i][2];
+    }
+    const double i_a = 1.0 / EL_P44_N;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      y.al[i] = (i == 0 || i == 3) ? 0.25 * (1.0 - a * i_a) : 0.25 * (1.0 + a * i_a);
+      y.be[i] = (i < 2) ? -y.al[i] * i_a : y.al[i] * i_a;
+    }
     return;
   }
-  store_pair(A, q.row, q.s, CC, dCz, dCe, Fp, w, -1);
+  double z0, z1, n0, n1;  // lit_part_point: zeta = z0 + z1 b, eta = n0 + n1 b
+  if (part == 0) {
+    z0 = 0.125 * (3.0 + 2.0 * a); z1 = 0.125 * (2.0 + a);
+    n0 = -0.125 * EL_SQ3 * a; n1 = 0.125 * EL_SQ3;
+  } else if (part == 1) {
+    z0 = 0.0625 * (-3.0 + a); z1 = 0.0625 * (-5.0 - a);
+    n0 = 0.0625 * EL_SQ3 * (3.0 + 3.0 * a); n1 = 0.0625 * EL_SQ3 * (1.0 + a);
+  } else {
+    z0 = 0.0625 * (-3.0 - 5.0 * a); z1 = 0.0625 * (1.0 - a);
+    n0 = 0.0625 * EL_SQ3 * (-3.0 - a); n1 = 0.0625 * EL_SQ3 * (-3.0 - a);
+  }
+  y.wf0 = 1.0 + 0.25 * a;
+  y.wf1 = 0.25;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    y.P[i] = e.cr[i][0] + e.cr[i][1] * z0 + e.cr[i][2] * n0 - rt[i];
+    y.Q[i] = e.cr[i][1] * z1 + e.cr[i][2] * n1;
+    y.C[i] = e.cw[i][0];
+    y.D[i] = 0.0;
+  }
+  const double h = 0.5 / EL_P34_N0 / 3.0;
+  y.al[0] = 1.0 / 3.0 - h * (z0 + EL_SQ3 * n0); y.be[0] = -h * (z1 + EL_SQ3 * n1);
+  y.al[1] = 1.0 / 3.0 + 2.0 * h * z0;           y.be[1] = 2.0 * h * z1;
+  y.al[2] = 1.0 / 3.0 - h * (z0 - EL_SQ3 * n0); y.be[2] = -h * (z1 - EL_SQ3 * n1);
+  y.al[3] = y.be[3] = 0.0;
 }
 
-// Regular interior pairs of one chunk: one thread per pair.
-__global__ void __launch_bounds__(128) k_reg_interior(AssembleArgs A, long long p0, long long np, double3* Fp,
-                                                      unsigned* gh_list, unsigned* gh_count, unsigned gh_cap, int* status)
+// Points j0 .. j1 - 1 of a row (nodes xs, weights ws).  SHORT: the Taylor sums' range holds.
+template <bool SHORT>
+__device__ __forceinline__ void regi_row(const RegiLine& line, const double* xs, const double* ws, int j0, int j1, bool tri,
+                                         double kre, double kim, RegiRow& m)
 {
-  long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= np) return;
-  reg_interior_pair(A, p0, w, Fp, gh_list, gh_count, gh_cap, status);
-}
-
-// Near-singular interior pair w of the chunk starting at pair p0, 64x64 rule, by one warp.
-__device__ __forceinline__ void gh_interior_pair(const AssembleArgs& A, long long p0, long long w, double3* Fp, int lane)
-{
-  const cplx k = mk(A.kre, A.kim);
-  {
-    PairIdx q = pair_of(p0 + w, A.ne);
-    int tnn;
-    double rt[3], vtz[3], vte[3];
-    target_info(A.geo, A.sid, q.t, q.tn, rt, vtz, vte, tnn);
-    int sd = A.sid[q.s];
-    Elem es;
-    load_elem(A.geo, abs(sd), es);
-    const int npts = (es.nn == 4) ? 4096 : 3 * 4096;
-    AccI a;
-    acci_zero(a);
-    for (int kq = lane; kq < npts; kq += 32) {
-      double z, e, wt;
-      rule_point(es.nn, 64, c_xh, c_wh, kq, z, e, wt);
-      acci_point(es, k, rt, vtz, vte, z, e, wt, a);
+  const double *P = line.P, *Q = line.Q, *C = line.C, *D = line.D;
+  cplx e0 = mk(1.0, 0.0);
+  double R0 = 0.0;
+  if (SHORT) {
+    R0 = vnorm3(P);
+    e0 = expi(kre * R0) * exp(-kim * R0);
+  }
+  const bool damped = kim != 0.0;
+#pragma unroll 1
+  for (int j = j0; j < j1; j++) {
+    const double b = xs[j], w = ws[j] * fma(line.wf1, b, line.wf0);
+    const double x = fma(Q[0], b, P[0]), y = fma(Q[1], b, P[1]), z = fma(Q[2], b, P[2]);
+    const double Wx = fma(D[0], b, C[0]), Wy = fma(D[1], b, C[1]), Wz = fma(D[2], b, C[2]);
+    const double R2 = x * x + y * y + z * z;
+    const double iR = rsqrt_(R2), R = R2 * iR, i2 = iR * iR;
+    const double RW = x * Wx + y * Wy + z * Wz;
+    double wG = w;
+    if (!tri) {
+      const double W2 = Wx * Wx + Wy * Wy + Wz * Wz;
+      wG = w * (W2 * rsqrt_(W2));
     }
-    double v[51];
-    acci_pack(a, v);
-    warp_sum_arr<51>(v);
-    acci_unpack(v, a);
-    cplx CC[9], dCz[9], dCe[9];
-    acci_finish(es, a, sd < 0, CC, dCz, dCe);
-    store_pair(A, q.row, q.s, CC, dCz, dCe, Fp, w, lane);
+    const cplx kR = mk(kre * R, kim * R);
+    cplx u;
+    if (SHORT) {
+      const double d = R - R0;
+      u = e0 * taylor_cis(kre * d);
+      if (damped) u = u * taylor_expm(kim * d);
+    } else {
+      u = expi(kR.re);
+      if (damped) u = u * exp(-kR.im);
+    }
+    const double w3 = i2 * iR;
+    const cplx g = u * (wG * iR);
+    const cplx cb = mk(-kR.im - 1.0, kR.re);
+    const cplx q = (cb * u) * w3;
+    const cplx qa = q * wG, qw = q * w;
+    const cplx h = qw * RW;
+    const cplx k3 = mk(kR.re * kR.re - kR.im * kR.im + 3.0 * cb.re, 2.0 * kR.re * kR.im + 3.0 * cb.im);
+    const double t5 = w3 * w, s5 = t5 * i2 * RW;
+    const cplx e5 = (k3 * u) * s5;
+    const double b2 = b * b;
+    m.g0 += g; m.g1.re = fma(g.re, b, m.g1.re); m.g1.im = fma(g.im, b, m.g1.im);
+    m.h0 += h; m.h1.re = fma(h.re, b, m.h1.re); m.h1.im = fma(h.im, b, m.h1.im);
+    m.a0 += qa; m.a1.re = fma(qa.re, b, m.a1.re); m.a1.im = fma(qa.im, b, m.a1.im);
+    m.a2.re = fma(qa.re, b2, m.a2.re); m.a2.im = fma(qa.im, b2, m.a2.im);
+    m.e0 += e5; m.e1.re = fma(e5.re, b, m.e1.re); m.e1.im = fma(e5.im, b, m.e1.im);
+    m.e2.re = fma(e5.re, b2, m.e2.re); m.e2.im = fma(e5.im, b2, m.e2.im);
+    m.q0 += qw; m.q1.re = fma(qw.re, b, m.q1.re); m.q1.im = fma(qw.im, b, m.q1.im);
+    m.q2.re = fma(qw.re, b2, m.q2.re); m.q2.im = fma(qw.im, b2, m.q2.im);
+    m.F = fma(t5, RW, m.F);
+    const double s3 = 3.0 * s5;
+    m.s0 += s3; m.s1 = fma(s3, b, m.s1);
+    m.t0 += t5; m.t1 = fma(t5, b, m.t1);
   }
 }
 
-// Near-singular interior pairs of one chunk: one warp per listed pair (at most gh_cap of them).
-__global__ void __launch_bounds__(256) k_gh_interior(AssembleArgs A, long long p0, double3* Fp, const unsigned* gh_list,
-                                                     const unsigned* gh_count, unsigned gh_cap)
+// |r - r(b = 0)| <= regi_reach along every row: the Taylor sums' range
+__device__ __forceinline__ bool regi_brief(const Elem& e, double kre, double kim)
 {
+  double reach = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double d = (e.nn == 3) ? 0.4 * fabs(e.cr[i][1]) + 0.4 * fabs(e.cr[i][2]) : fabs(e.cr[i][2]) + fabs(e.cr[i][3]);
+    reach += d * d;
+  }
+  reach = sqrt(reach);
+  return fabs(kre) * reach <= REGI_XMAX && fabs(kim) * reach <= REGI_YMAX;
+}
+
+// Adds a row's moments, times its weight wr, to the 48 shape-function sums v[(8 q + 2 i + part) ld] of the
+// quantities q = G, H, dG0, dG1, dH0, dH1, and to F, dF0, dF1.
+__device__ __forceinline__ void regi_add(const RegiLine& y, const RegiRow& m, const double* v0, const double* v1, double wr,
+                                         double* v, int ld, double& F, double& dF0, double& dF1)
+{
+  const double C0 = dot3(y.C, v0), D0 = dot3(y.D, v0), C1 = dot3(y.C, v1), D1 = dot3(y.D, v1);
+  const double P0 = dot3(y.P, v0), Q0 = dot3(y.Q, v0), P1 = dot3(y.P, v1), Q1 = dot3(y.Q, v1);
+  // sums of f and f b of the integrands
+  const cplx f0[6] = {m.g0, m.h0, m.a0 * P0 + m.a1 * Q0, m.a0 * P1 + m.a1 * Q1,
+                      m.e0 * P0 + m.e1 * Q0 - (m.q0 * C0 + m.q1 * D0), m.e0 * P1 + m.e1 * Q1 - (m.q0 * C1 + m.q1 * D1)};
+  const cplx f1[6] = {m.g1, m.h1, m.a1 * P0 + m.a2 * Q0, m.a1 * P1 + m.a2 * Q1,
+                      m.e1 * P0 + m.e2 * Q0 - (m.q1 * C0 + m.q2 * D0), m.e1 * P1 + m.e2 * Q1 - (m.q1 * C1 + m.q2 * D1)};
+  F += wr * m.F;
+  dF0 += wr * (P0 * m.s0 + Q0 * m.s1 - (C0 * m.t0 + D0 * m.t1));
+  dF1 += wr * (P1 * m.s0 + Q1 * m.s1 - (C1 * m.t0 + D1 * m.t1));
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const double al = wr * y.al[i], be = wr * y.be[i];
+#pragma unroll
+    for (int c = 0; c < 6; c++) {
+      double* p = v + (c * 8 + 2 * i) * ld;
+      p[0] += al * f0[c].re + be * f1[c].re;
+      p[ld] += al * f0[c].im + be * f1[c].im;
+    }
+  }
+}
+
+__device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row, int s, int lane, double3* Fp,
+                                                  long long fidx, unsigned* gh_list, unsigned* gh_count, unsigned gh_cap,
+                                                  int* status, double* acc)
+{
+  const int t = row >> 2, tn = row & 3;
+  const bool in = s < A.ne;
+  int tnn;
+  double rt[3], v0[3], v1[3];
+  target_info(A.geo, A.sid, t, tn, rt, v0, v1, tnn);
+  const bool blank = (tn == 3 && tnn == 3);  // a triangle's fourth row stays zero
+  const int sd = A.sid[in ? s : 0];
+  Elem e;
+  load_elem(A.geo, abs(sd), e);
+  const bool tri = e.nn == 3;
+  double* my = acc + lane;
+#pragma unroll
+  for (int i = 0; i < 48; i++) my[i * REGI_LD] = 0.0;
+  double F = 0.0, dF0 = 0.0, dF1 = 0.0;
+  const int nrow = (blank || !in || s == t) ? 0 : (tri ? 36 : 12);
+  const bool brief = __all_sync(0xffffffffu, nrow == 0 || regi_brief(e, A.kre, A.kim));
+#pragma unroll 1
+  for (int ar = 0; ar < nrow; ar++) {
+    const int part = ar / 12, ia = ar - 12 * part;
+    RegiLine y;
+    regi_line(e, rt, part, c_xl[ia], y);
+    RegiRow m;
+    memset(&m, 0, sizeof m);
+    if (brief) regi_row<true>(y, c_xl, c_wl, 0, 12, tri, A.kre, A.kim, m);
+    else regi_row<false>(y, c_xl, c_wl, 0, 12, tri, A.kre, A.kim, m);
+    regi_add(y, m, v0, v1, c_wl[ia], my, REGI_LD, F, dF0, dF1);
+  }
+  // scalings of acci_finish; an element seen from its other side flips H and F
+  double cg = EL_I_FP, ch = EL_I_FP, cf = EL_I_FP;
+  if (tri) {
+    const double V[3] = {e.cw[0][0], e.cw[1][0], e.cw[2][0]}, c = 0.0625 * EL_SQ3 * EL_I_SPSQ3;
+    cg = c * vnorm3(V);
+    ch = cf = c;
+  }
+  if (sd < 0) { ch = -ch; cf = -cf; }
+#pragma unroll
+  for (int i = 0; i < 48; i++) {
+    const int q = i >> 3;  // G, H, dG0, dG1, dH0, dH1
+    my[i * REGI_LD] *= q == 0 ? cg : (q == 2 || q == 3) ? -cg : ch;
+  }
+  const double dFz = dF0 * cf, dFe = dF1 * cf;
+  if (in && s != t && !blank) {
+    if (needs_gh(dFz, dFe)) {  // its entries and F are written again from the list
+      const unsigned slot = atomicAdd(gh_count, 1u);
+      if (slot < gh_cap) gh_list[slot] = (unsigned)fidx;
+      else record_status(status, -900);
+    } else {
+      Fp[fidx] = make_double3(F * cf, dFz, dFe);
+    }
+  }
+  __syncwarp();
+  const size_t N = (size_t)4 * A.ne;
+  const int s0 = s - lane;
+  double* const mat[6] = {A.G, A.H, A.dG, A.dG, A.dH, A.dH};
+#pragma unroll 1
+  for (int q = 0; q < 6; q++) {
+    if (!mat[q]) continue;
+    const size_t r = (q < 2) ? (size_t)row : (size_t)2 * row + (q & 1);
+    cplx* out = (cplx*)mat[q] + r * N + (size_t)4 * s0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int k = c * 32 + lane, sl = k >> 2, i = k & 3;
+      if (s0 + sl >= A.ne || (s0 + sl == t && !blank)) continue;
+      const double* v = acc + (q * 8 + 2 * i) * REGI_LD + sl;
+      *reinterpret_cast<double2*>(out + k) = make_double2(v[0], v[REGI_LD]);
+    }
+  }
+  __syncwarp();
+}
+
+// Regular interior pairs of one chunk (rows r0 .. r0 + nr - 1).  One B200, the shell of 1,728 quads
+// (11.9 M pairs, complex wave number): REGI_MS.
+#ifndef REGI_BLOCKS
+#define REGI_BLOCKS 4
+#endif
+__global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_reg_interior(AssembleArgs A, int r0, int nr, double3* Fp,
+                                                                     unsigned* gh_list, unsigned* gh_count, unsigned gh_cap,
+                                                                     int* status)
+{
+  extern __shared__ __align__(16) double regi_smem[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpr = (A.ne + 31) >> 5;
+  const long long w = (long long)blockIdx.x * REGI_WARPS + wib;
+  if (w >= (long long)wpr * nr) return;  // uniform across the warp
+  const int rr = (int)(w / wpr), s = (int)(w - (long long)rr * wpr) * 32 + lane;
+  reg_interior_warp(A, r0 + rr, s, lane, Fp, (long long)rr * A.ne + s, gh_list, gh_count, gh_cap, status,
+                    regi_smem + wib * 48 * REGI_LD);
+}
+
+// Near-singular interior pair w of the chunk starting at pair p0, 64 x 64 rule, by the whole CTA
+// (GHI_THREADS threads): a thread takes half a row of 64 points at a time, by the regular rule's moments.
+#define GHI_THREADS 128
+__device__ __forceinline__ void gh_interior_pair(const AssembleArgs& A, long long p0, long long w, double3* Fp,
+                                                 const double* xh, const double* wh, double (*red)[51])
+{
+  const PairIdx q = pair_of(p0 + w, A.ne);
+  int tnn;
+  double rt[3], v0[3], v1[3];
+  target_info(A.geo, A.sid, q.t, q.tn, rt, v0, v1, tnn);
+  const int sd = A.sid[q.s];
+  Elem e;
+  load_elem(A.geo, abs(sd), e);
+  const bool tri = e.nn == 3;
+  const bool brief = regi_brief(e, A.kre, A.kim);
+  double v[51];
+#pragma unroll
+  for (int i = 0; i < 51; i++) v[i] = 0.0;
+  const int items = tri ? 3 * 64 * 2 : 64 * 2;
+#pragma unroll 1
+  for (int it = threadIdx.x; it < items; it += GHI_THREADS) {
+    const int half = it & 1, ar = it >> 1, part = ar >> 6, ia = ar & 63;
+    RegiLine y;
+    regi_line(e, rt, part, xh[ia], y);
+    RegiRow m;
+    memset(&m, 0, sizeof m);
+    if (brief) regi_row<true>(y, xh, wh, 32 * half, 32 * half + 32, tri, A.kre, A.kim, m);
+    else regi_row<false>(y, xh, wh, 32 * half, 32 * half + 32, tri, A.kre, A.kim, m);
+    regi_add(y, m, v0, v1, wh[ia], v, 1, v[48], v[49], v[50]);
+  }
+  warp_sum_arr<51>(v);
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0)
+    for (int i = 0; i < 51; i++) red[wid][i] = v[i];
+  __syncthreads();
+  if (threadIdx.x < 51) {
+    double t = 0.0;
+    for (int i = 0; i < GHI_THREADS / 32; i++) t += red[i][threadIdx.x];
+    red[0][threadIdx.x] = t;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    AccI a;
+    const double* r = red[0];
+    for (int i = 0; i < 4; i++) {
+      a.G[i] = mk(r[2 * i], r[2 * i + 1]);
+      a.H[i] = mk(r[8 + 2 * i], r[9 + 2 * i]);
+      a.dG0[i] = mk(r[16 + 2 * i], r[17 + 2 * i]);
+      a.dG1[i] = mk(r[24 + 2 * i], r[25 + 2 * i]);
+      a.dH0[i] = mk(r[32 + 2 * i], r[33 + 2 * i]);
+      a.dH1[i] = mk(r[40 + 2 * i], r[41 + 2 * i]);
+    }
+    a.F = r[48]; a.dF0 = r[49]; a.dF1 = r[50];
+    cplx CC[9], dCz[9], dCe[9];
+    acci_finish(e, a, sd < 0, CC, dCz, dCe);
+    store_pair(A, q.row, q.s, CC, dCz, dCe, Fp, w, lane);
+  }
+  __syncthreads();
+}
+
+// Near-singular interior pairs of one chunk: one CTA per listed pair (at most gh_cap of them).
+__global__ void __launch_bounds__(GHI_THREADS, 4) k_gh_interior(AssembleArgs A, long long p0, double3* Fp,
+                                                                const unsigned* gh_list, const unsigned* gh_count,
+                                                                unsigned gh_cap)
+{
+  __shared__ double red[GHI_THREADS / 32][51];
+  __shared__ double xh[64], wh[64];
   const unsigned n = min(*gh_count, gh_cap);
-  const int lane = threadIdx.x & 31;
-  const unsigned wglob = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const unsigned nw = (gridDim.x * blockDim.x) >> 5;
-  for (unsigned it = wglob; it < n; it += nw) gh_interior_pair(A, p0, gh_list[it], Fp, lane);
+  if (blockIdx.x >= n) return;
+  if (threadIdx.x < 64) { xh[threadIdx.x] = c_xh[threadIdx.x]; wh[threadIdx.x] = c_wh[threadIdx.x]; }
+  __syncthreads();
+  for (unsigned it = blockIdx.x; it < n; it += gridDim.x) gh_interior_pair(A, p0, gh_list[it], Fp, xh, wh, red);
 }
 
 // ==========================================================================================
@@ -566,6 +848,11 @@ static int ensure_tables(void)
                            (int)(SMT_WARPS * sizeof(SmoothWarp))) != cudaSuccess ||
       cudaFuncSetAttribute(k_smooth_spectral, cudaFuncAttributeMaxDynamicSharedMemorySize, SMT_SPEC_SMEM) != cudaSuccess)
     return -1;
+  if (cudaFuncSetAttribute(k_reg_interior, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+      cudaFuncSetAttribute(k_reg_interior, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGI_SMEM_BYTES) !=
+          cudaSuccess)
+    return -1;
   if (dev < 64) g_tables_ready[dev] = 1;
   return 0;
 }
@@ -645,10 +932,12 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, 
   }
 
   const size_t N = (size_t)nrows;
-  if (cudaMemsetAsync(A.G, 0, N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
-  if (cudaMemsetAsync(A.H, 0, N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
-  if (A.dG && cudaMemsetAsync(A.dG, 0, 2 * N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
-  if (A.dH && cudaMemsetAsync(A.dH, 0, 2 * N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
+  if (A.periodic) {  // its kernels skip the triangles' fourth rows and the derivatives (all zero)
+    if (cudaMemsetAsync(A.G, 0, N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
+    if (cudaMemsetAsync(A.H, 0, N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
+    if (A.dG && cudaMemsetAsync(A.dG, 0, 2 * N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
+    if (A.dH && cudaMemsetAsync(A.dH, 0, 2 * N * N * 16, st) != cudaSuccess) return BEM3_ERR_CUDA;
+  }
   if (A.dF && cudaMemsetAsync(A.dF, 0, N * 3 * sizeof(double), st) != cudaSuccess) return BEM3_ERR_CUDA;
   cudaMemsetAsync(Fself, 0, N * sizeof(double3), st);
   cudaMemsetAsync(gh_total, 0, sizeof(unsigned long long), st);
@@ -726,12 +1015,13 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, 
       k_gh_periodic<<<148 * 4, 256, 0, st>>>(A, *L, p0, Fp, gh_list, gh_count, gh_cap, d_status);
       toc(2);
     } else {
-      unsigned blocks = (unsigned)((np + 127) / 128);
+      const long long warps = (long long)((ne + 31) / 32) * nr;
       tic();
-      k_reg_interior<<<blocks, 128, 0, st>>>(A, p0, np, Fp, gh_list, gh_count, gh_cap, d_status);
+      k_reg_interior<<<(unsigned)((warps + REGI_WARPS - 1) / REGI_WARPS), REGI_WARPS * 32, REGI_SMEM_BYTES, st>>>(
+          A, r0, nr, Fp, gh_list, gh_count, gh_cap, d_status);
       toc(1);
       tic();
-      k_gh_interior<<<148 * 4, 256, 0, st>>>(A, p0, Fp, gh_list, gh_count, gh_cap);
+      k_gh_interior<<<148 * 8, GHI_THREADS, 0, st>>>(A, p0, Fp, gh_list, gh_count, gh_cap);
       toc(2);
     }
     tic();

@@ -96,9 +96,11 @@ __global__ void k_batch_zero(const BatchDomain* __restrict__ D)
   double2* H = (double2*)d.A.H;
   double2* dG = (double2*)d.A.dG;
   double2* dH = (double2*)d.A.dH;
-  for (size_t i = i0; i < nn; i += stride) { G[i] = z; H[i] = z; }
-  if (dG) for (size_t i = i0; i < 2 * nn; i += stride) dG[i] = z;
-  if (dH) for (size_t i = i0; i < 2 * nn; i += stride) dH[i] = z;
+  if (d.A.periodic) {  // the interior kernels write every entry
+    for (size_t i = i0; i < nn; i += stride) { G[i] = z; H[i] = z; }
+    if (dG) for (size_t i = i0; i < 2 * nn; i += stride) dG[i] = z;
+    if (dH) for (size_t i = i0; i < 2 * nn; i += stride) dH[i] = z;
+  }
   if (d.A.dF) for (size_t i = i0; i < 3 * N; i += stride) d.A.dF[i] = 0.0;
   for (size_t i = i0; i < N; i += stride) d.Fself[i] = make_double3(0.0, 0.0, 0.0);
 }
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth
                   d.status, reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xl, wl, threadIdx.x & 31);
 }
 
-__global__ void __launch_bounds__(SI_THREADS) k_batch_self_interior(const BatchDomain* __restrict__ D, BatchSeg S)
+__global__ void __launch_bounds__(SI_THREADS, 2) k_batch_self_interior(const BatchDomain* __restrict__ D, BatchSeg S)
 {
   __shared__ double red[SI_NW * SELF_NV];
   __shared__ double res[4][SELF_NV];
@@ -207,17 +209,23 @@ __global__ void __launch_bounds__(256, REGP_MIN_BLOCKS) k_batch_reg_periodic(con
   }
 }
 
-__global__ void __launch_bounds__(128) k_batch_reg_interior(const BatchDomain* __restrict__ D, BatchSeg S)
+// Regular interior pairs: S counts warps, each 32 sources of a row (reg_interior_warp).
+__global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_batch_reg_interior(const BatchDomain* __restrict__ D, BatchSeg S)
 {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= S.base[S.n]) return;
-  const int i = seg_find(S, g);
+  extern __shared__ __align__(16) double regi_smem[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const long long w = (long long)blockIdx.x * REGI_WARPS + wib;
+  if (w >= S.base[S.n]) return;  // uniform across the warp
+  const int i = seg_find(S, w);
   const BatchDomain& d = D[S.dom[i]];
-  reg_interior_pair(d.A, 0, g - S.base[i], d.Fp, d.gh_list, d.gh_count, d.gh_cap, d.status);
+  const int wpr = (d.A.ne + 31) >> 5;
+  const long long u = w - S.base[i];
+  const int row = (int)(u / wpr), s = (int)(u - (long long)row * wpr) * 32 + lane;
+  reg_interior_warp(d.A, row, s, lane, d.Fp, (long long)row * d.A.ne + s, d.gh_list, d.gh_count, d.gh_cap, d.status,
+                    regi_smem + wib * 48 * REGI_LD);
 }
 
-// Near-singular pairs: the domains' lists in turn, CTAs (periodic) or warps (interior) striding
-// over each.
+// Near-singular pairs: the domains' lists in turn, CTAs striding over each.
 __global__ void __launch_bounds__(256, 2) k_batch_gh_periodic(const BatchDomain* __restrict__ D, const int* __restrict__ dom, int n)
 {
   __shared__ double red[8][19];
@@ -244,15 +252,17 @@ __global__ void __launch_bounds__(256, 2) k_batch_gh_smooth(const BatchDomain* _
   }
 }
 
-__global__ void __launch_bounds__(256) k_batch_gh_interior(const BatchDomain* __restrict__ D, const int* __restrict__ dom, int n)
+__global__ void __launch_bounds__(GHI_THREADS, 4) k_batch_gh_interior(const BatchDomain* __restrict__ D,
+                                                                      const int* __restrict__ dom, int n)
 {
-  const int lane = threadIdx.x & 31;
-  const unsigned wglob = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const unsigned nw = (gridDim.x * blockDim.x) >> 5;
+  __shared__ double red[GHI_THREADS / 32][51];
+  __shared__ double xh[64], wh[64];
+  if (threadIdx.x < 64) { xh[threadIdx.x] = c_xh[threadIdx.x]; wh[threadIdx.x] = c_wh[threadIdx.x]; }
+  __syncthreads();
   for (int i = 0; i < n; i++) {
     const BatchDomain& d = D[dom[i]];
     const unsigned cnt = min(*d.gh_count, d.gh_cap);
-    for (unsigned it = wglob; it < cnt; it += nw) gh_interior_pair(d.A, 0, d.gh_list[it], d.Fp, lane);
+    for (unsigned it = blockIdx.x; it < cnt; it += gridDim.x) gh_interior_pair(d.A, 0, d.gh_list[it], d.Fp, xh, wh, red);
   }
 }
 
@@ -366,6 +376,10 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
       cudaFuncSetAttribute(k_batch_reg_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)(SMT_WARPS * sizeof(SmoothWarp))) != cudaSuccess ||
       cudaFuncSetAttribute(k_batch_smooth_spectral, cudaFuncAttributeMaxDynamicSharedMemorySize, SMT_SPEC_SMEM) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_batch_reg_interior, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+      cudaFuncSetAttribute(k_batch_reg_interior, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGI_SMEM_BYTES) !=
           cudaSuccess)
     return BEM3_ERR_CUDA;
 
@@ -408,7 +422,7 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
       pdom.push_back(i);
     } else {
       selfI.add(i, 4 * ne);
-      regI.add(i, 4 * ne * ne);
+      regI.add(i, 4 * ne * ((ne + 31) / 32));
       idom.push_back(i);
     }
     rows.add(i, 4 * ne);
@@ -537,8 +551,9 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     // interior branch
     if (selfI.total() > 0) { k_batch_self_interior<<<(unsigned)selfI.total(), SI_THREADS, 0, s1>>>(b->dD, S[1]); launches++; }
     if (regI.total() > 0) {
-      k_batch_reg_interior<<<(unsigned)((regI.total() + 127) / 128), 128, 0, s1>>>(b->dD, S[3]);
-      k_batch_gh_interior<<<(unsigned)(sms * T.gh_blocks_per_sm), 256, 0, s1>>>(b->dD, (const int*)(m + oIdom),
+      k_batch_reg_interior<<<(unsigned)((regI.total() + REGI_WARPS - 1) / REGI_WARPS), REGI_WARPS * 32, REGI_SMEM_BYTES, s1>>>(
+          b->dD, S[3]);
+      k_batch_gh_interior<<<(unsigned)(2 * sms * T.gh_blocks_per_sm), GHI_THREADS, 0, s1>>>(b->dD, (const int*)(m + oIdom),
                                                                              (int)idom.size());
       launches += 2;
     }

@@ -61,6 +61,13 @@ BEM_HD double rsqrt_(double x) {  // 1/sqrt(x)
   return 1.0 / sqrt(x);
 #endif
 }
+BEM_HD double recip_(double x) {  // 1/x
+#if defined(__CUDA_ARCH__)
+  return __drcp_rn(x);
+#else
+  return 1.0 / x;
+#endif
+}
 BEM_HD cplx cexp_(cplx z) {  // e^{z}
   double e = exp(z.re);
   cplx p = expi(z.im);

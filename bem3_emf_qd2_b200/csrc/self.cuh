@@ -20,8 +20,6 @@
 
 #include "elem.cuh"
 
-BEM_HD cplx ccos_(cplx z) { return mk(cos(z.re) * cosh(z.im), -sin(z.re) * sinh(z.im)); }
-BEM_HD cplx csin_(cplx z) { return mk(sin(z.re) * cosh(z.im), cos(z.re) * sinh(z.im)); }
 BEM_HD void acc_put(double* v, int i, cplx z) { v[2 * i] += z.re; v[2 * i + 1] += z.im; }
 BEM_HD cplx acc_get(const double* v, int i) { return mk(v[2 * i], v[2 * i + 1]); }
 
@@ -96,119 +94,254 @@ BEM_HD double lit_dN(int n, double cth, double sth)
 #define SELF_NV 40  // accumulator length of every piece
 
 // ---- interior pieces -------------------------------------------------------------------------
+// Along a ray (fixed theta) the map's K, the normal W, the products K.T with the tangents and the shape
+// functions are polynomials in r (degrees 1, 1, 1, 2):
+//   K = K0 + K1 r,  W = W0 + W1 r,  K.Tz = z0 + z1 r,  K.Te = e0 + e1 r,  N_i = a_i + b_i r + c_i r^2.
+// Each piece's points therefore add a few scalars to moments sum f r^m, without shape functions, and the
+// moments become the shape functions' sums once per ray.  The trigonometry of theta (its sine and
+// cosine, three more sines for the edge distance) is also done once per ray, not at each of its points.
+struct SelfRay {
+  double cth, sth, K0[3], K1[3], W0[3], W1[3], z0, z1, e0, e1;
+};
+BEM_HD void self_ray(const SelfInfo& S, double theta, SelfRay& Y)
+{
+#if defined(__CUDA_ARCH__)
+  sincos(theta, &Y.sth, &Y.cth);
+#else
+  Y.sth = sin(theta);
+  Y.cth = cos(theta);
+#endif
+  const Elem& e = S.e;
+  for (int i = 0; i < 3; i++) {
+    Y.K0[i] = e.cr[i][1] * Y.cth + e.cr[i][2] * Y.sth + e.cr[i][3] * (S.zt * Y.sth + S.et * Y.cth);
+    Y.K1[i] = e.cr[i][3] * (Y.cth * Y.sth);
+    Y.W0[i] = e.cw[i][0] + e.cw[i][1] * S.zt + e.cw[i][2] * S.et;
+    Y.W1[i] = e.cw[i][1] * Y.cth + e.cw[i][2] * Y.sth;
+  }
+  Y.z0 = dot3(Y.K0, S.Tz); Y.z1 = dot3(Y.K1, S.Tz);
+  Y.e0 = dot3(Y.K0, S.Te); Y.e1 = dot3(Y.K1, S.Te);
+}
+BEM_HD double ray_K2(const SelfRay& Y, double r)  // |K|^2
+{
+  const double x = Y.K0[0] + Y.K1[0] * r, y = Y.K0[1] + Y.K1[1] * r, z = Y.K0[2] + Y.K1[2] * r;
+  return x * x + y * y + z * z;
+}
+BEM_HD double ray_aW(const SelfInfo& S, const SelfRay& Y, double r)  // |W| (1 on triangles)
+{
+  if (!S.bil) return 1.0;
+  const double x = Y.W0[0] + Y.W1[0] * r, y = Y.W0[1] + Y.W1[1] * r, z = Y.W0[2] + Y.W1[2] * r;
+  const double w2 = x * x + y * y + z * z;
+  return w2 * rsqrt_(w2);
+}
+// N_i = n[0] + n[1] r + n[2] r^2 along the ray
+BEM_HD void ray_N(const SelfInfo& S, const SelfRay& Y, int i, double* n)
+{
+  if (S.bil) {
+    const double i_a = 1.0 / EL_P44_N;
+    const double u = (i == 0 || i == 3) ? -i_a : i_a, v = (i < 2) ? -i_a : i_a;
+    const double a = 1.0 + u * S.zt, b = 1.0 + v * S.et;
+    n[0] = 0.25 * a * b;
+    n[1] = 0.25 * (a * v * Y.sth + b * u * Y.cth);
+    n[2] = 0.25 * u * v * Y.cth * Y.sth;
+    return;
+  }
+  n[2] = 0.0;
+  if (i == 3) { n[0] = n[1] = 0.0; return; }
+  const double h = 0.5 / EL_P34_N0 / 3.0;
+  const double u = (i == 1) ? 2.0 * h : -h, v = (i == 1) ? 0.0 : (i == 0 ? -h * EL_SQ3 : h * EL_SQ3);
+  n[0] = 1.0 / 3.0 + u * S.zt + v * S.et;
+  n[1] = u * Y.cth + v * Y.sth;
+}
+// e^{i z} of a complex z
+BEM_HD cplx self_cis(cplx z)
+{
+  cplx u = expi(z.re);
+  if (z.im != 0.0) u = u * exp(-z.im);
+  return u;
+}
+BEM_HD void csincos_(cplx z, cplx& s, cplx& c)
+{
+  const cplx u = expi(z.re);
+  double ch = 1.0, sh = 0.0;
+  if (z.im != 0.0) { ch = cosh(z.im); sh = sinh(z.im); }
+  s = mk(u.im * ch, u.re * sh);
+  c = mk(u.re * ch, -u.im * sh);
+}
+// Moments of a ray: g (times K.T) and p (times K.T, of the curved part), q: sums f r^m
+struct SelfMom {
+  cplx g[4], p[4], q[3];
+  double f0, f1, f2;  // w / (r |K|^5): 1, r; w / (r |K|^3)
+};
+BEM_HD void mom_zero(SelfMom& m)
+{
+  for (int i = 0; i < 4; i++) { m.g[i] = mk(0, 0); m.p[i] = mk(0, 0); }
+  for (int i = 0; i < 3; i++) m.q[i] = mk(0, 0);
+  m.f0 = m.f1 = m.f2 = 0.0;
+}
+template <int N>
+BEM_HD void mom_add(cplx* m, cplx f, double r)
+{
+  m[0] += f;
+  double t = r;
+  for (int i = 1; i < N; i++) {
+    m[i].re += f.re * t;
+    m[i].im += f.im * t;
+    t *= r;
+  }
+}
+// Adds a ray's moments to the sums of the pieces 2-4 (layout below): dG from g, dH and dF from p, q, f.
+BEM_HD void ray_add(const SelfInfo& S, const SelfRay& Y, const SelfMom& m, double* v)
+{
+  cplx gz[3], ge[3], hz[3], he[3];
+  const double cs = Y.cth * Y.sth;
+  for (int k = 0; k < 3; k++) {
+    gz[k] = m.g[k] * Y.z0 + m.g[k + 1] * Y.z1;
+    ge[k] = m.g[k] * Y.e0 + m.g[k + 1] * Y.e1;
+    if (S.curved) {
+      hz[k] = (m.p[k] * Y.z0 + m.p[k + 1] * Y.z1) * cs - m.q[k] * Y.sth;
+      he[k] = (m.p[k] * Y.e0 + m.p[k + 1] * Y.e1) * cs - m.q[k] * Y.cth;
+    }
+  }
+  for (int i = 0; i < 4; i++) {
+    double n[3];
+    ray_N(S, Y, i, n);
+    acc_put(v, i, gz[0] * n[0] + gz[1] * n[1] + gz[2] * n[2]);
+    acc_put(v, 4 + i, ge[0] * n[0] + ge[1] * n[1] + ge[2] * n[2]);
+    if (S.curved) {
+      acc_put(v, 8 + i, hz[0] * n[0] + hz[1] * n[1] + hz[2] * n[2]);
+      acc_put(v, 12 + i, he[0] * n[0] + he[1] * n[1] + he[2] * n[2]);
+    }
+  }
+  if (S.curved) {
+    v[32] += Y.sth * (3.0 * Y.cth * (Y.z0 * m.f0 + Y.z1 * m.f1) - m.f2);
+    v[33] += Y.cth * (3.0 * Y.sth * (Y.e0 * m.f0 + Y.e1 * m.f1) - m.f2);
+  }
+}
+
 // piece 1 layout: G[4] 0..7, H[4] 8..15, F 16
 BEM_HD void self_int_piece1(const SelfInfo& S, const double* xl, const double* wl, const double* xh, const double* wh,
                             int lane, int nlanes, double* v)
 {
-  const int n = S.P.nsub * 128 * 12;
-  for (int q = lane; q < n; q += nlanes) {
-    int ir = q % 12, tq = q / 12, j = tq >> 7, m2 = tq & 127;
+  const int n = S.P.nsub * 128;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+  for (int tq = lane; tq < n; tq += nlanes) {
+    const int j = tq >> 7, m2 = tq & 127;
     double theta, wt;
     polar_theta(S.P, j, m2, xh, wh, theta, wt);
-    double rm = polar_rm(S.P, j, theta);
-    double cth = cos(theta), sth = sin(theta);
-    double r = 0.5 * rm * (xl[ir] + 1.0);
-    double w = wt * 0.5 * rm * wl[ir];
-    double zeta = r * cth + S.zt, eta = r * sth + S.et;
-    double K[3], N[4];
-    self_K(S, r, cth, sth, K);
-    self_N(S, zeta, eta, N);
-    double aK = vnorm3(K);
-    cplx kR = S.k * (aK * r);
-    cplx ce = cexp_(mul_i(kR));
-    cplx g = ce * (w / aK * self_aW(S, zeta, eta));
-    for (int i = 0; i < 4; i++) acc_put(v, i, g * N[i]);
-    if (S.curved) {
-      double i3 = 1.0 / (aK * aK * aK);
-      cplx h = mk(-kR.im - 1.0, kR.re) * ce * (w * i3 * cth * sth);  // (i kR - 1) e^{ikR} cs/|K|^3
-      for (int i = 0; i < 4; i++) acc_put(v, 4 + i, h * N[i]);
-      v[16] += w * i3 * cth * sth;
+    const double rm = polar_rm(S.P, j, theta);
+    SelfRay Y;
+    self_ray(S, theta, Y);
+    cplx g[3] = {mk(0, 0), mk(0, 0), mk(0, 0)}, h[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
+    double f = 0.0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int ir = 0; ir < 12; ir++) {
+      const double r = 0.5 * rm * (xl[ir] + 1.0), w = wt * 0.5 * rm * wl[ir];
+      const double K2 = ray_K2(Y, r), iK = rsqrt_(K2);
+      const cplx kR = S.k * (K2 * iK * r);
+      const cplx ce = self_cis(kR);
+      mom_add<3>(g, ce * (w * iK * ray_aW(S, Y, r)), r);
+      if (S.curved) {
+        const double i3 = iK * iK * iK * w;
+        mom_add<3>(h, (mk(-kR.im - 1.0, kR.re) * ce) * i3, r);  // (i kR - 1) e^{ikR} / |K|^3
+        f += i3;
+      }
     }
+    const double cs = Y.cth * Y.sth;
+    for (int i = 0; i < 4; i++) {
+      double N[3];
+      ray_N(S, Y, i, N);
+      acc_put(v, i, g[0] * N[0] + g[1] * N[1] + g[2] * N[2]);
+      if (S.curved) acc_put(v, 4 + i, (h[0] * N[0] + h[1] * N[1] + h[2] * N[2]) * cs);
+    }
+    if (S.curved) v[16] += f * cs;
   }
 }
 
-// piece 2 (D̄ε) layout: dGz[4] 0..7, dGe[4] 8..15, dHz[4] 16..23, dHe[4] 24..31, dFz 32, dFe 33
+// piece 2 (D̄ε) layout: dGz[4] 0..7, dGe[4] 8..15, dHz[4] 16..23, dHe[4] 24..31, dFz 32, dFe 33.
+// Items: a ray and one half of its 64 points.
 BEM_HD void self_int_piece2(const SelfInfo& S, const double* xh, const double* wh, int lane, int nlanes, double* v)
 {
-  const int n = S.P.nsub * 128 * 64;
+  const int n = S.P.nsub * 128 * 2;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
   for (int q = lane; q < n; q += nlanes) {
-    int ir = q & 63, tq = q >> 6, j = tq >> 7, m2 = tq & 127;
+    const int half = q & 1, tq = q >> 1, j = tq >> 7, m2 = tq & 127;
     double theta, wt;
     polar_theta(S.P, j, m2, xh, wh, theta, wt);
-    double rm = polar_rm(S.P, j, theta);
-    double cth = cos(theta), sth = sin(theta);
-    double r = 0.5 * (rm - EL_DEPS) * xh[ir] + 0.5 * (rm + EL_DEPS);
-    double w = wt * 0.5 * (rm - EL_DEPS) * wh[ir];
-    double zeta = r * cth + S.zt, eta = r * sth + S.et;
-    double K[3], N[4];
-    self_K(S, r, cth, sth, K);
-    self_N(S, zeta, eta, N);
-    double aK = vnorm3(K), i_aK = 1.0 / aK;
-    cplx kR = S.k * (aK * r);
-    cplx ca = mul_i(kR);
-    cplx cb = mk(ca.re - 1.0, ca.im);
-    cplx ce = cexp_(ca);
-    double KTz = dot3(K, S.Tz), KTe = dot3(K, S.Te);
-    cplx gb = cb * ce * (w * i_aK * i_aK / r * self_aW(S, zeta, eta));
-    for (int i = 0; i < 4; i++) {
-      acc_put(v, i, gb * (KTz * i_aK * N[i]));
-      acc_put(v, 4 + i, gb * (KTe * i_aK * N[i]));
+    const double rm = polar_rm(S.P, j, theta);
+    SelfRay Y;
+    self_ray(S, theta, Y);
+    SelfMom m;
+    mom_zero(m);
+    const double hr = 0.5 * (rm - EL_DEPS), cr = 0.5 * (rm + EL_DEPS);
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int ir = 32 * half; ir < 32 * half + 32; ir++) {
+      const double r = hr * xh[ir] + cr, w = wt * hr * wh[ir];
+      const double K2 = ray_K2(Y, r), iK = rsqrt_(K2), i2 = iK * iK;
+      const cplx kR = S.k * (K2 * iK * r);
+      const cplx cb = mk(-kR.im - 1.0, kR.re);
+      const cplx ce = self_cis(kR);
+      const double w3 = w * i2 * iK * recip_(r);
+      const cplx qm = (cb * ce) * w3;  // (ikR - 1) e^{ikR} w / (r |K|^3)
+      mom_add<4>(m.g, qm * ray_aW(S, Y, r), r);
+      if (S.curved) {
+        const double w5 = w3 * i2;
+        mom_add<4>(m.p, ((kR * kR + 3.0 * cb) * ce) * w5, r);
+        mom_add<3>(m.q, qm, r);
+        m.f0 += w5;
+        m.f1 += w5 * r;
+        m.f2 += w3;
+      }
     }
-    if (S.curved) {
-      double aK2 = aK * aK, i5r = 1.0 / (r * aK2 * aK2 * aK);
-      cplx kR2p3 = kR * kR + 3.0 * cb;
-      cplx hz = ce * (kR2p3 * (KTz * cth) - cb * aK2) * (w * sth * i5r);
-      cplx he = ce * (kR2p3 * (KTe * sth) - cb * aK2) * (w * cth * i5r);
-      for (int i = 0; i < 4; i++) { acc_put(v, 8 + i, hz * N[i]); acc_put(v, 12 + i, he * N[i]); }
-      v[32] += w * sth * i5r * (3.0 * KTz * cth - aK2);
-      v[33] += w * cth * i5r * (3.0 * KTe * sth - aK2);
-    }
+    ray_add(S, Y, m, v);
   }
 }
 
-// piece 3 (Dε) layout: dGz[4] 0..7, dGe[4] 8..15, dHz[4] 16..23, dHe[4] 24..31
+// piece 3 (Dε) layout: dGz[4] 0..7, dGe[4] 8..15, dHz[4] 16..23, dHe[4] 24..31 (32, 33 are not used)
 BEM_HD void self_int_piece3(const SelfInfo& S, const double* xl, const double* wl, const double* xh, const double* wh,
                             int lane, int nlanes, double* v)
 {
   const cplx k = S.k;
   if (S.bil) {
     // theta in 4 quarter pieces of [-pi, pi] (64 nodes each), r in [0, DEPS] (12 nodes)
-    for (int q = lane; q < 4 * 64 * 12; q += nlanes) {
-      int ir = q % 12, tq = q / 12, piece = tq >> 6, m = tq & 63;
-      double theta = 0.25 * QP_PI * xh[m] + (-0.75 + 0.5 * piece) * QP_PI;
-      double w = 0.25 * QP_PI * wh[m] * 0.5 * EL_DEPS * wl[ir];
-      double r = 0.5 * EL_DEPS * (xl[ir] + 1.0);
-      double cth = cos(theta), sth = sin(theta);
-      double zeta = r * cth + S.zt, eta = r * sth + S.et;
-      double K[3], N[4];
-      self_K(S, r, cth, sth, K);
-      self_N(S, zeta, eta, N);
-      double aW = self_aW(S, zeta, eta);
-      double aK = vnorm3(K), i_aK = 1.0 / aK;
-      cplx kR = k * (aK * r);
-      cplx ca = mul_i(kR);
-      cplx cb = mk(ca.re - 1.0, ca.im);
-      cplx cc = ccos_(kR), cs = csin_(kR);
-      double KTz = dot3(K, S.Tz), KTe = dot3(K, S.Te);
-      cplx gd = (cb * cs + kR * cc) * (w * i_aK * i_aK / r * aW);
-      for (int i = 0; i < 4; i++) {
-        acc_put(v, i, gd * (KTz * i_aK * N[i]));
-        acc_put(v, 4 + i, gd * (KTe * i_aK * N[i]));
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int tq = lane; tq < 4 * 64; tq += nlanes) {
+      const int piece = tq >> 6, mm = tq & 63;
+      const double theta = 0.25 * QP_PI * xh[mm] + (-0.75 + 0.5 * piece) * QP_PI;
+      SelfRay Y;
+      self_ray(S, theta, Y);
+      SelfMom m;
+      mom_zero(m);
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+      for (int ir = 0; ir < 12; ir++) {
+        const double w = 0.25 * QP_PI * wh[mm] * 0.5 * EL_DEPS * wl[ir], r = 0.5 * EL_DEPS * (xl[ir] + 1.0);
+        const double K2 = ray_K2(Y, r), iK = rsqrt_(K2), i2 = iK * iK;
+        const cplx kR = k * (K2 * iK * r);
+        const cplx cb = mk(-kR.im - 1.0, kR.re);
+        cplx cs, cc;
+        csincos_(kR, cs, cc);
+        const double w3 = w * i2 * iK * recip_(r);
+        mom_add<4>(m.g, (cb * cs + kR * cc) * (w3 * ray_aW(S, Y, r)), r);
+        if (S.curved) {
+          // e^{ikR} (k kR + 3ik) / |K|^4 - i 3 sin(kR) / (r |K|^5), and e^{ikR} ik / |K|^2 - i sin(kR) / (r |K|^3)
+          const cplx ce = cc + mul_i(cs), ik = mul_i(k);
+          const double w5 = w3 * i2;
+          mom_add<4>(m.p, (ce * (k * kR + 3.0 * ik)) * (w * i2 * i2) - mul_i(cs) * (3.0 * w5), r);
+          mom_add<3>(m.q, (ce * ik) * (w * i2) - mul_i(cs) * w3, r);
+        }
       }
-      if (S.curved) {
-        double aK2 = aK * aK;
-        cplx ce = cexp_(ca);
-        cplx cbk = mul_i(k);                 // i k
-        cplx kkR3 = k * kR + 3.0 * cbk;      // k kR + 3 i k
-        double i4 = 1.0 / (aK2 * aK2), i5r = 1.0 / (aK2 * aK2 * aK * r);
-        cplx h0z = ce * (kkR3 * (KTz * cth) - cbk * aK2) * i4;
-        cplx h1z = cs * ((3.0 * KTz * cth - aK2) * i5r);
-        cplx h0e = ce * (kkR3 * (KTe * sth) - cbk * aK2) * i4;
-        cplx h1e = cs * ((3.0 * KTe * sth - aK2) * i5r);
-        cplx hz = (h0z - mul_i(h1z)) * (w * sth);
-        cplx he = (h0e - mul_i(h1e)) * (w * cth);
-        for (int i = 0; i < 4; i++) { acc_put(v, 8 + i, hz * N[i]); acc_put(v, 12 + i, he * N[i]); }
-      }
+      ray_add(S, Y, m, v);  // f0 .. f2 are zero: no solid-angle part here
     }
   } else {
     // triangle: closed form in r; theta in 4 quarter pieces (64 nodes each)
@@ -221,7 +354,8 @@ BEM_HD void self_int_piece3(const SelfInfo& S, const double* xl, const double* w
       self_K(S, 0.0, cth, sth, K);
       double aK = vnorm3(K), i_aK = 1.0 / aK;
       cplx keK = k * (EL_DEPS * aK);
-      cplx cc = ccos_(keK), cs = csin_(keK);
+      cplx cc, cs;
+      csincos_(keK, cs, cc);
       // (keK + i) sin + (2 - i keK) cos - 2
       cplx f = mk(keK.re, keK.im + 1.0) * cs + mk(2.0 + keK.im, -keK.re) * cc - mk(2.0, 0.0);
       double i3 = i_aK * i_aK * i_aK;
@@ -234,46 +368,46 @@ BEM_HD void self_int_piece3(const SelfInfo& S, const double* xl, const double* w
   }
 }
 
-// piece 4 (principal-value correction) layout as piece 2
+// piece 4 (principal-value correction) layout as piece 2.  Items: a line through the node (the rays
+// theta and theta + pi) and one half of its 12 distances.  The line at -r is the same polynomial in -r.
 BEM_HD void self_int_piece4(const SelfInfo& S, const double* xl, const double* wl, const double* xh, const double* wh,
                             int lane, int nlanes, double* v)
 {
   const cplx k = S.k;
   if (S.bil) {
-    for (int q = lane; q < 2 * 64 * 12; q += nlanes) {
-      int ir = q % 12, tq = q / 12, piece = tq >> 6, m = tq & 63;
-      double theta = 0.25 * QP_PI * xh[m] + (0.25 + 0.5 * piece) * QP_PI;
-      double w = 0.25 * QP_PI * wh[m] * 0.5 * EL_DEPS * wl[ir];
-      double r = 0.5 * EL_DEPS * (xl[ir] + 1.0);
-      double cth = cos(theta), sth = sin(theta);
-      double zp = r * cth + S.zt, ep = r * sth + S.et, zm = -r * cth + S.zt, em = -r * sth + S.et;
-      double Kp[3], Km[3], Np[4], Nm[4];
-      bil_K(S.e, S.zt, S.et, r, cth, sth, Kp);
-      bil_K(S.e, S.zt, S.et, -r, cth, sth, Km);
-      bil_N4(zp, ep, Np);
-      bil_N4(zm, em, Nm);
-      double aKp = vnorm3(Kp), aKm = vnorm3(Km), aWp = self_aW(S, zp, ep), aWm = self_aW(S, zm, em);
-      cplx ccp = ccos_(k * (aKp * r)), ccm = ccos_(k * (aKm * r));
-      double KpTz = dot3(Kp, S.Tz), KmTz = dot3(Km, S.Tz), KpTe = dot3(Kp, S.Te), KmTe = dot3(Km, S.Te);
-      double ip2 = 1.0 / (aKp * aKp), im2 = 1.0 / (aKm * aKm);
-      for (int i = 0; i < 4; i++) {
-        cplx gz = ccp * (ip2 * KpTz / aKp * Np[i] * aWp) - ccm * (im2 * KmTz / aKm * Nm[i] * aWm);
-        cplx ge = ccp * (ip2 * KpTe / aKp * Np[i] * aWp) - ccm * (im2 * KmTe / aKm * Nm[i] * aWm);
-        acc_put(v, i, gz * (w / r));
-        acc_put(v, 4 + i, ge * (w / r));
-      }
-      if (S.curved) {
-        double p2 = aKp * aKp, m2 = aKm * aKm;
-        double i5p = 1.0 / (p2 * p2 * aKp), i5m = 1.0 / (m2 * m2 * aKm);
-        double az_p = (3.0 * KpTz * cth - p2) * i5p, az_m = (3.0 * KmTz * cth - m2) * i5m;
-        double ae_p = (3.0 * KpTe * sth - p2) * i5p, ae_m = (3.0 * KmTe * sth - m2) * i5m;
-        for (int i = 0; i < 4; i++) {
-          acc_put(v, 8 + i, (ccp * (az_p * Np[i]) - ccm * (az_m * Nm[i])) * (w * sth / r));
-          acc_put(v, 12 + i, (ccp * (ae_p * Np[i]) - ccm * (ae_m * Nm[i])) * (w * cth / r));
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int q = lane; q < 2 * 64 * 2; q += nlanes) {
+      const int half = q & 1, tq = q >> 1, piece = tq >> 6, mm = tq & 63;
+      const double theta = 0.25 * QP_PI * xh[mm] + (0.25 + 0.5 * piece) * QP_PI;
+      SelfRay Y;
+      self_ray(S, theta, Y);
+      SelfMom m;
+      mom_zero(m);
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+      for (int ir = 12 * half; ir < 12 * half + 12; ir++) {
+        // ir = 2 n (+ r_n) and 2 n + 1 (- r_n), n of the half
+        const int n = ir >> 1;
+        const double r0 = 0.5 * EL_DEPS * (xl[n] + 1.0), r = (ir & 1) ? -r0 : r0;
+        const double w = 0.25 * QP_PI * wh[mm] * 0.5 * EL_DEPS * wl[n];
+        const double K2 = ray_K2(Y, r), iK = rsqrt_(K2), i2 = iK * iK;
+        cplx cs, cc;
+        csincos_(k * (K2 * iK * r0), cs, cc);
+        const double w3 = w * i2 * iK * recip_(r);  // the point at -r enters with the opposite sign
+        mom_add<4>(m.g, cc * (w3 * ray_aW(S, Y, r)), r);
+        if (S.curved) {
+          const double w5 = w3 * i2;
+          mom_add<4>(m.p, cc * (3.0 * w5), r);
+          mom_add<3>(m.q, cc * w3, r);
+          m.f0 += w5;
+          m.f1 += w5 * r;
+          m.f2 += w3;
         }
-        v[32] += w * sth / r * (az_p - az_m);
-        v[33] += w * cth / r * (ae_p - ae_m);
       }
+      ray_add(S, Y, m, v);
     }
   } else {
     for (int q = lane; q < 2 * 64; q += nlanes) {
@@ -284,7 +418,8 @@ BEM_HD void self_int_piece4(const SelfInfo& S, const double* xl, const double* w
       double K[3];
       self_K(S, 0.0, cth, sth, K);
       double aK = vnorm3(K), i_aK = 1.0 / aK;
-      cplx cs = csin_(k * (aK * EL_DEPS));
+      cplx cc, cs;
+      csincos_(k * (aK * EL_DEPS), cs, cc);
       double i3 = i_aK * i_aK * i_aK;
       for (int i = 0; i < 3; i++) {
         double dn = lit_dN(i, cth, sth);

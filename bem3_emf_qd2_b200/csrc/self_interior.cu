@@ -88,7 +88,7 @@ __device__ __forceinline__ void self_interior_row(const AssembleArgs& A, int row
   Fself[row] = make_double3(CC[8].re, dCz[8].re, dCe[8].re);
 }
 
-__global__ void __launch_bounds__(SI_THREADS) k_self_interior(AssembleArgs A, double3* Fself)
+__global__ void __launch_bounds__(SI_THREADS, 2) k_self_interior(AssembleArgs A, double3* Fself)
 {
   __shared__ double red[SI_NW * SELF_NV];
   __shared__ double res[4][SELF_NV];
