@@ -45,7 +45,16 @@ __device__ __forceinline__ double block_reduce(double v, double* red, bool mx)
   return r;
 }
 
-__device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const QPLattice& L, const SmoothArgs& M)
+// What the table is for: the pairs of a domain, or (points) evaluations at points of heights zlo .. zhi
+// against every element, `evals` of them (near = 0: each a single point; else elements with a rule of
+// `near` points per quad).
+struct SmoothUse {
+  int points;
+  double zlo, zhi, evals, near;
+};
+
+__device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const QPLattice& L, const SmoothArgs& M,
+                                                  const SmoothUse U = SmoothUse{0, 0.0, 0.0, 0.0, 0.0})
 {
   __shared__ double red[SMT_PLAN_THREADS];
   __shared__ SmoothGrid best;
@@ -65,14 +74,17 @@ __device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const Q
   for (int i = 0; i < 3; i++) {
     const double a = block_reduce(lo[i], red, false), b = block_reduce(hi[i], red, true);
     (i == 0 ? X.ulen : i == 1 ? X.vlen : X.zlen) = b - a;
+    if (i == 2 && U.points) X.zlen = fmax(fmax(U.zhi - a, b - U.zlo), 0.0);
   }
-  const double np = 4.0 * (double)A.ne * A.ne;
+  if (U.points) X.ulen = X.vlen = 1.0;  // points anywhere in the cell
+  const double np = U.points ? U.evals : 4.0 * (double)A.ne * A.ne;
+  const double near = U.points ? U.near : 144.0;
   const int d = SMT_LMIN + (int)threadIdx.x;
   SmoothGrid g;
   g.on = 0;
   double c = 1e300;
   if (d <= SMT_LMAX) {
-    smooth_choose(L, M.S, X, np, tri > 0.0, M.cap, d, g, c);
+    smooth_choose(L, M.S, X, np, near, tri > 0.0, M.cap, d, g, c);
     if (!g.on) c = 1e300;
     costs[d] = c;
   }
@@ -108,6 +120,13 @@ __global__ void __launch_bounds__(SMT_PLAN_THREADS) k_smooth_plan(AssembleArgs A
                                                                   SmoothArgs M)
 {
   smooth_plan_block(A, L, M);
+}
+
+// A table for evaluations at field points.
+__global__ void __launch_bounds__(SMT_PLAN_THREADS) k_field_plan(AssembleArgs A, const __grid_constant__ QPLattice L,
+                                                                 SmoothArgs M, double zlo, double zhi, double evals, double near)
+{
+  smooth_plan_block(A, L, M, SmoothUse{1, zlo, zhi, evals, near});
 }
 
 __device__ __forceinline__ void smooth_slot(const QPLattice& L, const SmoothPlan& P, int slot, SmoothCell& c)

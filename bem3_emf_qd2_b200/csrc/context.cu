@@ -771,8 +771,7 @@ int run_domain_id(bem3_ctx c, const FieldArgs& A, int n, const double* r, DevBuf
   int rc;
   if ((rc = upload(dr, r, (size_t)3 * n))) return rc;
   if (ddid.alloc(sizeof(int) * (size_t)n) || dcell.alloc(sizeof(int2) * (size_t)n)) return BEM3_ERR_CUDA;
-  k_domain_id<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256>>>(A, n, dr.as<double>(), ddid.as<int>(),
-                                                                  dcell.as<int2>());
+  k_domain_id<<<(unsigned)n, DOMID_THREADS>>>(A, n, dr.as<double>(), ddid.as<int>(), dcell.as<int2>());
   return cudaGetLastError() == cudaSuccess ? 0 : BEM3_ERR_CUDA;
 }
 
@@ -790,6 +789,70 @@ extern "C" int bem3_ctx_domain_id(bem3_ctx c, int n, const double* r, int* did)
   return cudaMemcpy(did, ddid.p, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost) == cudaSuccess ? 0 : BEM3_ERR_CUDA;
 }
 
+namespace {
+
+// How the open region's Green's function is evaluated at n field points (rule `type`): by warps where
+// the rule's points are few (FIELD_WARP_MAX evaluations: 17 ns each against ~1.3 ms for a table and its
+// plan), else from a table of the smooth remainder made for the points' heights.
+#define FIELD_WARP_MAX 60000
+struct FieldPlanHost {
+  FieldGreen g;
+  bool warp = false;
+};
+
+int field_plan(bem3_ctx c, const FieldArgs& A, int n, const double* r, int type, bool grad, FieldPlanHost& P)
+{
+  memset(&P.g, 0, sizeof P.g);
+  P.warp = false;
+  if (c->ps != 1) return 0;
+  const int ne = (int)c->sid[0].size();
+  if (type <= 1) {
+    smooth_lattice(c->L, P.g.W, EWW_EXPM);
+    if (P.g.W.ok && (grad || (double)n * ne * (type == 0 ? 4 : 9) <= FIELD_WARP_MAX)) {
+      P.warp = true;
+      return 0;
+    }
+  }
+  if (grad) return 0;
+  SmoothArgs& M = P.g.M;
+  smooth_lattice(c->L, M.S);
+  if (!M.S.ok) return 0;
+  M.cap = 1LL << 21;
+  const size_t plan = round256(sizeof(SmoothPlan));
+  DevRes* R = nullptr;
+  int rc = ensure_scratch(plan + (size_t)M.cap * 48, &R);
+  if (rc) return rc;
+  M.plan = (SmoothPlan*)R->scratch;
+  M.tab = (cplx*)((char*)R->scratch + plan);
+  M.smp = M.tab + M.cap;
+  double zlo = r[2], zhi = r[2];
+  for (int i = 1; i < n; i++) { zlo = fmin(zlo, r[3 * i + 2]); zhi = fmax(zhi, r[3 * i + 2]); }
+  AssembleArgs B;
+  memset(&B, 0, sizeof B);
+  B.geo = A.geo; B.sid = A.sid[0]; B.ne = ne;
+  const double evals = (double)n * ne * (type == 0 ? 4 : type == 1 ? 9 : 1);
+  k_field_plan<<<1, SMT_PLAN_THREADS>>>(B, c->L, M, zlo, zhi, evals, type >= 2 ? (type == 2 ? 144.0 : 4096.0) : 0.0);
+  k_smooth_spectral<<<148 * 4, SMT_SPEC_THREADS, smooth_spec_smem(M.S)>>>(c->L, M);
+  k_smooth_project<<<148 * 8, SMT_PROJ_THREADS>>>(c->L, M);
+  return cudaGetLastError() == cudaSuccess ? 0 : BEM3_ERR_CUDA;
+}
+
+// Points a launch takes so that its partial sums (`bytes` a point) stay within 256 MB.
+int field_chunk(int n, size_t bytes)
+{
+  const size_t m = (256u << 20) / bytes;
+  return (size_t)n <= m ? n : (m > 0 ? (int)m : 1);
+}
+
+int max_elements(bem3_ctx c)
+{
+  size_t m = 0;
+  for (const auto& s : c->sid) m = s.size() > m ? s.size() : m;
+  return (int)m;
+}
+
+}  // namespace
+
 // E, H (pot false) or U (pot true) at n points; mode 0 scattered / interior, 1 total, 2 incident.
 static int ctx_field_run(bem3_ctx c, int n, const double* r, int type, int mode, bool pot, double* E, double* H,
                          int* did)
@@ -798,23 +861,56 @@ static int ctx_field_run(bem3_ctx c, int n, const double* r, int type, int mode,
     return BEM3_ERR_ARG;
   if (n == 0) return 0;
   DeviceGuard g(c->dev);
-  if (type >= 2 && ensure_tables() != 0) return BEM3_ERR_CUDA;  // Gauss-Legendre tables
+  if (ensure_tables() != 0) return BEM3_ERR_CUDA;  // Gauss-Legendre tables, kernel attributes
   FieldArgs A = field_view(c);
-  DevBuf dr, ddid, dcell, dE, dH;
+  DevBuf dr, ddid, dcell, dE, dH, dpart;
   int rc = run_domain_id(c, A, n, r, dr, ddid, dcell);
   if (rc) return rc;
   const size_t eo = (size_t)n * (pot ? 8 : 6) * sizeof(double);
   if (dE.alloc(eo) || (!pot && dH.alloc((size_t)n * 6 * sizeof(double)))) return BEM3_ERR_CUDA;
-  cudaMemset(c->status.p, 0, sizeof(int));
-  if (pot)
-    k_field_t<true><<<(unsigned)n, FIELD_THREADS>>>(A, c->L, n, dr.as<double>(), ddid.as<int>(), dcell.as<int2>(), type,
-                                                    mode, dE.as<double>(), nullptr, c->status.as<int>());
-  else
-    k_field_t<false><<<(unsigned)n, FIELD_THREADS>>>(A, c->L, n, dr.as<double>(), ddid.as<int>(), dcell.as<int2>(), type,
-                                                     mode, dE.as<double>(), dH.as<double>(), c->status.as<int>());
+  int nb = 1, epb = 1, chunk = n;
+  int* status = c->status.as<int>();
+  if (cudaMemsetAsync(status, 0, sizeof(int), cudaStreamPerThread) != cudaSuccess) return BEM3_ERR_CUDA;
+  auto sum = [&](int p0, int m) {
+    const double* pr = dr.as<double>() + 3 * (size_t)p0;
+    const int* pd = ddid.as<int>() + p0;
+    const int2* pc = dcell.as<int2>() + p0;
+    if (pot)
+      k_field_sum<true><<<(unsigned)m, FIELD_THREADS>>>(A, pr, pd, pc, mode, dpart.as<double>(), nb, epb,
+                                                        dE.as<double>() + 8 * (size_t)p0, nullptr);
+    else
+      k_field_sum<false><<<(unsigned)m, FIELD_THREADS>>>(A, pr, pd, pc, mode, dpart.as<double>(), nb, epb,
+                                                         dE.as<double>() + 6 * (size_t)p0, dH.as<double>() + 6 * (size_t)p0);
+  };
+  if (mode != 2) {
+    FieldPlanHost P;
+    if ((rc = field_plan(c, A, n, r, type, false, P))) return rc;
+    const int ne = max_elements(c);
+    epb = !P.warp ? FIELD_THREADS : ((long long)n * ne <= 4096 ? 1 : FIELD_EPB);
+    nb = (ne + epb - 1) / epb;
+    chunk = field_chunk(n, (size_t)nb * (pot ? 9 : 13) * sizeof(double));
+    if (dpart.alloc((size_t)chunk * nb * (pot ? 9 : 13) * sizeof(double))) return BEM3_ERR_CUDA;
+    for (int p0 = 0; p0 < n; p0 += chunk) {
+      const dim3 grid((unsigned)(chunk < n - p0 ? chunk : n - p0), (unsigned)nb);
+      const double* pr = dr.as<double>() + 3 * (size_t)p0;
+      const int* pd = ddid.as<int>() + p0;
+      const int2* pc = dcell.as<int2>() + p0;
+      double* pp = dpart.as<double>();
+      if (P.warp) {
+        if (pot) k_field_warp<true><<<grid, FIELD_THREADS>>>(A, c->L, P.g, epb, pr, pd, pc, type, pp, status);
+        else k_field_warp<false><<<grid, FIELD_THREADS>>>(A, c->L, P.g, epb, pr, pd, pc, type, pp, status);
+      } else {
+        if (pot) k_field_part<true><<<grid, FIELD_THREADS>>>(A, c->L, P.g, pr, pd, pc, type, pp, status);
+        else k_field_part<false><<<grid, FIELD_THREADS>>>(A, c->L, P.g, pr, pd, pc, type, pp, status);
+      }
+      sum(p0, (int)grid.x);
+    }
+  } else {
+    sum(0, n);
+  }
   if (cudaGetLastError() != cudaSuccess) return BEM3_ERR_CUDA;
   int hs = 0;
-  if (cudaMemcpy(&hs, c->status.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+  if (cudaMemcpy(&hs, status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
       cudaMemcpy(E, dE.p, eo, cudaMemcpyDeviceToHost) != cudaSuccess ||
       (!pot && cudaMemcpy(H, dH.p, (size_t)n * 6 * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) ||
       (did && cudaMemcpy(did, ddid.p, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost) != cudaSuccess))
@@ -838,15 +934,40 @@ extern "C" int bem3_ctx_field_memp(bem3_ctx c, int n, const double* r, int type,
   if (!c || n < 0 || (n > 0 && (!r || !E || !H)) || type < 0 || type > 3 || total < 0 || total > 2) return BEM3_ERR_ARG;
   if (n == 0) return 0;
   DeviceGuard g(c->dev);
-  if (type >= 2 && ensure_tables() != 0) return BEM3_ERR_CUDA;
+  if (ensure_tables() != 0) return BEM3_ERR_CUDA;
   FieldArgs A = field_view(c);
-  DevBuf dr, ddid, dcell, dE, dH;
+  DevBuf dr, ddid, dcell, dE, dH, dpart;
   int rc = run_domain_id(c, A, n, r, dr, ddid, dcell);
   if (rc) return rc;
   if (dE.alloc((size_t)n * 6 * sizeof(double)) || dH.alloc((size_t)n * 6 * sizeof(double))) return BEM3_ERR_CUDA;
-  cudaMemset(c->status.p, 0, sizeof(int));
-  k_eh_memp<<<(unsigned)n, FIELD_THREADS>>>(A, c->L, n, dr.as<double>(), ddid.as<int>(), dcell.as<int2>(), type, total,
-                                            c->lambda0, dE.as<double>(), dH.as<double>(), c->status.as<int>());
+  int* status = c->status.as<int>();
+  if (cudaMemsetAsync(status, 0, sizeof(int), cudaStreamPerThread) != cudaSuccess) return BEM3_ERR_CUDA;
+  int nb = 1, epb = 1, chunk = n;
+  auto sum = [&](int p0, int m) {
+    k_memp_sum<<<(unsigned)m, FIELD_THREADS>>>(A, dr.as<double>() + 3 * (size_t)p0, ddid.as<int>() + p0, dcell.as<int2>() + p0,
+                                               total, c->lambda0, dpart.as<double>(), nb, epb,
+                                               dE.as<double>() + 6 * (size_t)p0, dH.as<double>() + 6 * (size_t)p0);
+  };
+  if (total != 2) {
+    FieldPlanHost P;
+    if ((rc = field_plan(c, A, n, r, type, true, P))) return rc;
+    const int ne = max_elements(c);
+    epb = !P.warp ? FIELD_THREADS : ((long long)n * ne <= 4096 ? 1 : FIELD_EPB);
+    nb = (ne + epb - 1) / epb;
+    chunk = field_chunk(n, (size_t)nb * MEMP_NV * sizeof(double));
+    if (dpart.alloc((size_t)chunk * nb * MEMP_NV * sizeof(double))) return BEM3_ERR_CUDA;
+    for (int p0 = 0; p0 < n; p0 += chunk) {
+      const dim3 grid((unsigned)(chunk < n - p0 ? chunk : n - p0), (unsigned)nb);
+      const double* pr = dr.as<double>() + 3 * (size_t)p0;
+      const int* pd = ddid.as<int>() + p0;
+      const int2* pc = dcell.as<int2>() + p0;
+      if (P.warp) k_memp_warp<<<grid, FIELD_THREADS>>>(A, c->L, P.g, epb, pr, pd, pc, type, dpart.as<double>(), status);
+      else k_memp_part<<<grid, FIELD_THREADS>>>(A, c->L, pr, pd, pc, type, dpart.as<double>(), status);
+      sum(p0, (int)grid.x);
+    }
+  } else {
+    sum(0, n);
+  }
   if (cudaGetLastError() != cudaSuccess) return BEM3_ERR_CUDA;
   int hs = 0;
   if (cudaMemcpy(&hs, c->status.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||

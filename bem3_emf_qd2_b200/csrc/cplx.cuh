@@ -10,9 +10,11 @@
 #if defined(__CUDACC__)
 #define BEM_HD __host__ __device__ __forceinline__
 #define BEM_HD_NOINLINE __host__ __device__ __noinline__
+#define BEM_HD_MEMBER __host__ __device__ __forceinline__
 #else
 #define BEM_HD static inline
 #define BEM_HD_NOINLINE static
+#define BEM_HD_MEMBER inline
 #endif
 
 struct cplx {

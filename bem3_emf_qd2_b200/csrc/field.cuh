@@ -17,6 +17,7 @@
 #pragma once
 
 #include "elem.cuh"
+#include "ewald_warp.cuh"
 
 // quadrature tables (init_elem_const, d3qd2_setup.c:1194-1217): the standard 3x3 Gauss-Legendre
 // product rule, and the 4- and 7-point triangle rules on the reference triangle with vertices
@@ -73,27 +74,97 @@ struct FieldKer {
   double tD, aW;
 };
 
-template <bool PER>
-BEM_HD int field_kernel(const QPLattice& L, cplx k, const double* vR, const double* vW, FieldKer& o)
+// The parts that do not depend on the Green's function.
+BEM_HD void field_kernel_geom(const double* vR, const double* vW, FieldKer& o)
 {
   const double aR = vnorm3(vR);
   const double i_aR = 1.0 / aR;
   o.aW = vnorm3(vW);
   o.tD = dot3(vR, vW) * i_aR * i_aR * i_aR;
-  if (PER) {
-    QPVal v;
-    int err = qpgf_eval<QP_V1>(L, vR, v);
-    o.g = v.G;
-    o.hn = v.dG[0] * vW[0] + v.dG[1] * vW[1] + v.dG[2] * vW[2];
-    return err;
-  }
-  // free space: e^{ikR}/R and its normal derivative, without the 1/(4 pi) applied later
-  cplx ca = mul_i(k) * aR;
-  cplx ce = (k.im == 0.0) ? expi(k.re * aR) : cexp_(ca);
-  o.g = ce * i_aR;
-  o.hn = (ca - mk(1.0, 0.0)) * ce * o.tD;
-  return 0;
 }
+
+// Evaluators of a rule's points: point i of the rule at vR with normal vW.
+// The lattice sums with the reference's rules (PER), or free space.
+template <bool PER>
+struct FieldPlain {
+  const QPLattice& L;
+  cplx k;
+  BEM_HD_MEMBER int operator()(int i, const double* vR, const double* vW, FieldKer& o) const
+  {
+    (void)i;
+    field_kernel_geom(vR, vW, o);
+    if (PER) {
+      QPVal v;
+      int err = qpgf_eval<QP_V1>(L, vR, v);
+      o.g = v.G;
+      o.hn = v.dG[0] * vW[0] + v.dG[1] * vW[1] + v.dG[2] * vW[2];
+      return err;
+    }
+    // free space: e^{ikR}/R and its normal derivative, without the 1/(4 pi) applied later
+    const double aR = vnorm3(vR), i_aR = 1.0 / aR;
+    cplx ca = mul_i(k) * aR;
+    cplx ce = (k.im == 0.0) ? expi(k.re * aR) : cexp_(ca);
+    o.g = ce * i_aR;
+    o.hn = (ca - mk(1.0, 0.0)) * ce * o.tD;
+    return 0;
+  }
+};
+
+// One copy of the lattice sums for the rare points that need them.
+BEM_HD_NOINLINE int field_plain_v1(const QPLattice& L, const double* r, QPVal& v) { return qpgf_eval<QP_V1>(L, r, v); }
+BEM_HD_NOINLINE int field_plain_opt(const QPLattice& L, const double* r, QPVal& v) { return qpgf_eval<QP_V1, true>(L, r, v); }
+
+// A point in the plane of the field point (within SMT_ZPLANE periods): only the reference's sums and stop
+// rules give the reference's value there (smooth.cuh).
+BEM_HD int field_in_plane(const QPLattice& L, double z) { return z * z < SMT_ZPLANE * SMT_ZPLANE * fabs(L.detd); }
+
+// The tabulated remainder (smooth.cuh): the nearest image and the smooth part at the point reduced to the
+// cell.  Where the plan is off: the lattice sums in the assembly's form.
+struct FieldTable {
+  const QPLattice& L;
+  const SmoothPlan& P;
+  const cplx* tab;
+  double* rad;  // scratch, stride st
+  int st;
+  BEM_HD_MEMBER int operator()(int i, const double* vR, const double* vW, FieldKer& o) const
+  {
+    (void)i;
+    field_kernel_geom(vR, vW, o);
+    const int plane = field_in_plane(L, vR[2]);
+    if (plane || !P.on) {
+      QPVal v;
+      const int err = plane ? field_plain_v1(L, vR, v) : field_plain_opt(L, vR, v);
+      o.g = v.G;
+      o.hn = v.dG[0] * vW[0] + v.dG[1] * vW[1] + v.dG[2] * vW[2];
+      return err;
+    }
+    double sx, sy;
+    const int sh = smooth_shift(L, vR, &sx, &sy);
+    const double r[3] = {vR[0] + sx, vR[1] + sy, vR[2]};
+    cplx g, h, gi, hi;
+    smooth_rest(L, P, tab, r, vW, rad, st, g, h);
+    smooth_image(L.k, r[0], r[1], r[2], vW[0], vW[1], vW[2], gi, hi);
+    o.g = g + gi;
+    o.hn = h + hi;
+    if (sh) {
+      const cplx ph = expi(L.vkx * sx + L.vky * sy);
+      o.g = o.g * ph;
+      o.hn = o.hn * ph;
+    }
+    return 0;
+  }
+};
+
+// Values already computed, point by point of the rule.
+struct FieldStored {
+  const FieldKer* v;
+  BEM_HD_MEMBER int operator()(int i, const double* vR, const double* vW, FieldKer& o) const
+  {
+    (void)vR; (void)vW;
+    o = v[i];
+    return 0;
+  }
+};
 
 // Coefficients of source element `sd` (signed id) at point rt: CC[0..3] (Green's function times
 // shape functions), CC[4..7] (normal derivative), F.  Triangles leave CC[3], CC[7] zero.
@@ -147,17 +218,42 @@ BEM_HD int field_coef_gl(const double* geo, int sd, const double* rt, cplx k, in
   return err;
 }
 
-template <bool PER>
-BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int type, const QPLattice& L, cplx* CC,
-                      double& F, const FieldGL* gl = nullptr)
+// Points of the rules of types 0 and 1 on an element of nn vertices.
+BEM_HD int field_rule_points(int nn, int type) { return type == 0 ? 4 : (nn == 4 ? 9 : 7); }
+// Point i of them seen from rt, and the normal there (quads: Jacobian normal; triangles: one for all).
+BEM_HD void field_rule_point(const double* geo, int s, int type, int i, const double* rt, double* vR, double* vW)
+{
+  const double* g = geo + (size_t)s * GEO_STRIDE;
+  const int nn = (int)g[GEO_NN];
+  if (nn == 3)
+    for (int l = 0; l < 3; l++) vW[l] = (type == 0) ? g[GEO_WEN + l] : g[GEO_CW + 3 * l];
+  if (type == 0) {
+    for (int l = 0; l < 3; l++) {
+      vR[l] = g[GEO_REN + 3 * i + l] - rt[l];
+      if (nn == 4) vW[l] = g[GEO_WEN + 3 * i + l];
+    }
+    return;
+  }
+  Elem el;
+  load_elem(geo, s, el);
+  double z, e, w;
+  if (nn == 4) {
+    fq_gauss9(i, z, e, w);
+    bil_rw(el, z, e, vR, vW);
+  } else {
+    fq_tri7(i, z, e, w);
+    lit_r(el, z, e, vR);
+  }
+  for (int l = 0; l < 3; l++) vR[l] -= rt[l];
+}
+
+// Types 0 and 1 with the Green's function from `ev`.
+template <bool PER, class EVAL>
+BEM_HD int field_coef_by(const double* geo, int sd, const double* rt, int type, const EVAL& ev, cplx* CC, double& F)
 {
   for (int i = 0; i < 8; i++) CC[i] = mk(0.0, 0.0);
   F = 0.0;
   if (PER && sd < 0) return -1;
-  if (type == 2 || type == 3) {
-    if (!gl) return -1;
-    return field_coef_gl<PER>(geo, sd, rt, k, type, *gl, L, CC, F);
-  }
   if (type != 0 && type != 1) return -1;
   const int s = sd < 0 ? -sd : sd;
   const double* g = geo + (size_t)s * GEO_STRIDE;
@@ -169,7 +265,7 @@ BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int t
     if (type == 0) {
       for (int i = 0; i < 4; i++) {
         for (int l = 0; l < 3; l++) { vR[l] = g[GEO_REN + 3 * i + l] - rt[l]; vW[l] = g[GEO_WEN + 3 * i + l]; }
-        int e = field_kernel<PER>(L, k, vR, vW, q);
+        int e = ev(i, vR, vW, q);
         if (e < 0) err = e;
         CC[i] = q.g * q.aW;
         CC[i + 4] = q.hn;
@@ -183,7 +279,7 @@ BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int t
         fq_gauss9(i, z, e, w);
         bil_rw(el, z, e, vR, vW);
         for (int l = 0; l < 3; l++) vR[l] -= rt[l];
-        int st = field_kernel<PER>(L, k, vR, vW, q);
+        int st = ev(i, vR, vW, q);
         if (st < 0) err = st;
         bil_N4(z, e, N);
         cplx gw = q.g * (w * q.aW), hw = q.hn * w;
@@ -201,7 +297,7 @@ BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int t
     if (type == 0) {
       for (int i = 0; i < 4; i++) {
         for (int l = 0; l < 3; l++) vR[l] = g[GEO_REN + 3 * i + l] - rt[l];
-        int e = field_kernel<PER>(L, k, vR, vW, q);
+        int e = ev(i, vR, vW, q);
         if (e < 0) err = e;
         const double w = (i < 3) ? FQ_T4W0 : -FQ_T4W1;
         if (i < 3) {
@@ -222,7 +318,7 @@ BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int t
         fq_tri7(i, z, e, w);
         lit_r(el, z, e, vR);
         for (int l = 0; l < 3; l++) vR[l] -= rt[l];
-        int st = field_kernel<PER>(L, k, vR, vW, q);
+        int st = ev(i, vR, vW, q);
         if (st < 0) err = st;
         lit_N3(z, e, N);
         for (int ep = 0; ep < 3; ep++) { CC[ep] += q.g * (w * N[ep]); CC[ep + 4] += q.hn * (w * N[ep]); }
@@ -241,6 +337,62 @@ BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int t
   return err;
 }
 
+template <bool PER>
+BEM_HD int field_coef(const double* geo, int sd, const double* rt, cplx k, int type, const QPLattice& L, cplx* CC,
+                      double& F, const FieldGL* gl = nullptr)
+{
+  if ((type == 2 || type == 3) && !(PER && sd < 0)) {
+    for (int i = 0; i < 8; i++) CC[i] = mk(0.0, 0.0);
+    F = 0.0;
+    if (!gl) return -1;
+    return field_coef_gl<PER>(geo, sd, rt, k, type, *gl, L, CC, F);
+  }
+  return field_coef_by<PER>(geo, sd, rt, type, FieldPlain<PER>{L, k}, CC, F);
+}
+
+// Types 2 and 3 of a periodic element by the table: the rule's points for the nearest image, the smooth
+// points for the rest.
+BEM_HD int field_coef_gl_table(const double* geo, int sd, const double* rt, int type, const FieldGL& gl, const QPLattice& L,
+                               const SmoothPlan& P, const cplx* tab, double* rad, int st, cplx* CC, double& F)
+{
+  for (int i = 0; i < 8; i++) CC[i] = mk(0.0, 0.0);
+  F = 0.0;
+  if (sd < 0) return -1;
+  Elem el;
+  load_elem(geo, sd, el);
+  if (!P.on || smooth_in_plane(L, el, rt[2])) return field_coef_gl<true>(geo, sd, rt, mk(0.0, 0.0), type, gl, L, CC, F);
+  const int n = (type == 2) ? 12 : 64;
+  const double* x = (type == 2) ? gl.x12 : gl.x64;
+  const double* w = (type == 2) ? gl.w12 : gl.w64;
+  const int npts = (el.nn == 4) ? n * n : 3 * n * n, nq = (el.nn == 4) ? P.nq4 : P.nq3;
+  const double v0[3] = {0.0, 0.0, 0.0};
+  const double v[3] = {el.cr[0][0] - rt[0], el.cr[1][0] - rt[1], el.cr[2][0] - rt[2]};
+  double sx, sy;
+  const int sh = smooth_shift(L, v, &sx, &sy);
+  AccP a;
+  accp_zero(a);
+  for (int q = 0; q < npts; q++) {
+    double z, e, wt;
+    rule_point(el.nn, n, x, w, q, z, e, wt);
+    smooth_near(el, L.k, rt, v0, v0, sx, sy, sh, z, e, wt, a);
+  }
+  for (int i = 0; i < 4; i++) { a.G[i] = a.G[i] * EL_I_FP; a.H[i] = a.H[i] * EL_I_FP; }
+  for (int q = 0; q < nq; q++) {
+    cplx gw, hw;
+    double z, e, N[4];
+    smooth_point(el, L, P, tab, rt, sx, sy, q, rad, st, gw, hw, z, e);
+    if (el.nn == 4) bil_N4(z, e, N);
+    else { lit_N3(z, e, N); N[3] = 0.0; }
+    for (int i = 0; i < 4; i++) { a.G[i] += gw * N[i]; a.H[i] += hw * N[i]; }
+  }
+  cplx C9[9], dCz[9], dCe[9];
+  accp_finish(el, a, C9, dCz, dCe);
+  const cplx ph = sh ? expi(L.vkx * sx + L.vky * sy) : mk(1.0, 0.0);
+  for (int i = 0; i < 8; i++) CC[i] = C9[i] * ph;
+  F = C9[8].re;
+  return 0;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Coefficients and their gradients with respect to the point, for the fields computed from the
 // derivatives of the potentials (q0_dcoef_rt_grad d3qd2_elem.c:650-682 and dcoef_rt_grad
@@ -255,42 +407,66 @@ struct GradKer {
 // Kernel values at one quadrature point, R = r(point) - rt, W the normal used by the rule:
 // g, h = G and grad G . W; dg, dh their derivatives with respect to R (the rules apply the sign
 // of d/d rt); tD = (R . W) / |R|^3 and its derivative dF.  Free space without the 1/(4 pi).
-template <bool PER>
-BEM_HD int grad_kernel(const QPLattice& L, cplx k, const double* vR, const double* vW, GradKer& o)
+BEM_HD void grad_kernel_geom(const double* vR, const double* vW, GradKer& o, double& aR, double& rdW)
 {
-  const double aR = vnorm3(vR);
+  aR = vnorm3(vR);
   const double i_aR = 1.0 / aR, i3 = i_aR * i_aR * i_aR;
-  const double rdW = dot3(vR, vW) * i_aR;
+  rdW = dot3(vR, vW) * i_aR;
   o.tD = rdW * i_aR * i_aR;
   for (int p = 0; p < 3; p++) o.dF[p] = i3 * (3.0 * vR[p] * i_aR * rdW - vW[p]);
-  if (PER) {
-    QPVal2 v;
-    const int err = qpgf_eval2(L, vR, v);
-    o.g = v.G;
-    o.h = v.dG[0] * vW[0] + v.dG[1] * vW[1] + v.dG[2] * vW[2];
-    const cplx* d2 = v.d2G;  // xx, yy, zz, xy, yz, zx
-    o.dh[0] = d2[0] * vW[0] + d2[3] * vW[1] + d2[5] * vW[2];
-    o.dh[1] = d2[3] * vW[0] + d2[1] * vW[1] + d2[4] * vW[2];
-    o.dh[2] = d2[5] * vW[0] + d2[4] * vW[1] + d2[2] * vW[2];
-    for (int p = 0; p < 3; p++) o.dg[p] = v.dG[p];
-    return err;
-  }
-  const cplx kR = k * aR;
-  const cplx ca = mul_i(kR), cb = ca - mk(1.0, 0.0);
-  const cplx ce = (k.im == 0.0) ? expi(kR.re) : cexp_(ca);
-  o.g = ce * i_aR;
-  o.h = cb * ce * o.tD;
-  const cplx a3 = kR * kR + 3.0 * cb;
-  for (int p = 0; p < 3; p++) {
-    o.dg[p] = cb * ce * (i_aR * i_aR * vR[p] * i_aR);
-    o.dh[p] = ce * i3 * (a3 * (vR[p] * i_aR * rdW) - cb * vW[p]);
-  }
-  return 0;
 }
-
+// from the values G, dG, d2G (xx, yy, zz, xy, yz, zx)
+BEM_HD void grad_kernel_from(cplx G, const cplx* dG, const cplx* d2, const double* vW, GradKer& o)
+{
+  o.g = G;
+  o.h = dG[0] * vW[0] + dG[1] * vW[1] + dG[2] * vW[2];
+  o.dh[0] = d2[0] * vW[0] + d2[3] * vW[1] + d2[5] * vW[2];
+  o.dh[1] = d2[3] * vW[0] + d2[1] * vW[1] + d2[4] * vW[2];
+  o.dh[2] = d2[5] * vW[0] + d2[4] * vW[1] + d2[2] * vW[2];
+  for (int p = 0; p < 3; p++) o.dg[p] = dG[p];
+}
 template <bool PER>
-BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, int type, const QPLattice& L,
-                           const FieldGL* gl, cplx* CC, cplx (*dC)[8], double& F, double* dF)
+struct GradPlain {
+  const QPLattice& L;
+  cplx k;
+  BEM_HD_MEMBER int operator()(int i, const double* vR, const double* vW, GradKer& o) const
+  {
+    (void)i;
+    double aR, rdW;
+    grad_kernel_geom(vR, vW, o, aR, rdW);
+    if (PER) {
+      QPVal2 v;
+      const int err = qpgf_eval2(L, vR, v);
+      grad_kernel_from(v.G, v.dG, v.d2G, vW, o);
+      return err;
+    }
+    const double i_aR = 1.0 / aR, i3 = i_aR * i_aR * i_aR;
+    const cplx kR = k * aR;
+    const cplx ca = mul_i(kR), cb = ca - mk(1.0, 0.0);
+    const cplx ce = (k.im == 0.0) ? expi(kR.re) : cexp_(ca);
+    o.g = ce * i_aR;
+    o.h = cb * ce * o.tD;
+    const cplx a3 = kR * kR + 3.0 * cb;
+    for (int p = 0; p < 3; p++) {
+      o.dg[p] = cb * ce * (i_aR * i_aR * vR[p] * i_aR);
+      o.dh[p] = ce * i3 * (a3 * (vR[p] * i_aR * rdW) - cb * vW[p]);
+    }
+    return 0;
+  }
+};
+struct GradStored {
+  const GradKer* v;
+  BEM_HD_MEMBER int operator()(int i, const double* vR, const double* vW, GradKer& o) const
+  {
+    (void)vR; (void)vW;
+    o = v[i];
+    return 0;
+  }
+};
+
+template <bool PER, class EVAL>
+BEM_HD int field_grad_coef_by(const double* geo, int sd, const double* rt, int type, const EVAL& ev, const FieldGL* gl,
+                              cplx* CC, cplx (*dC)[8], double& F, double* dF)
 {
   for (int i = 0; i < 8; i++) {
     CC[i] = mk(0.0, 0.0);
@@ -330,7 +506,7 @@ BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, 
     if (type == 0) {  // the element's nodes, node weights 1 (q0_bil_dcoef_grad_4p, bil_dcoef_grad_4p)
       for (int i = 0; i < 4; i++) {
         for (int l = 0; l < 3; l++) { vR[l] = g[GEO_REN + 3 * i + l] - rt[l]; vW[l] = g[GEO_WEN + 3 * i + l]; }
-        const int st = grad_kernel<PER>(L, k, vR, vW, q);
+        const int st = ev(i, vR, vW, q);
         if (st < 0) err = st;
         double N[4] = {0.0, 0.0, 0.0, 0.0};
         N[i] = 1.0;
@@ -344,7 +520,7 @@ BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, 
         else rule_point(4, n, x, wq, i, z, e, w);
         bil_rw(el, z, e, vR, vW);
         for (int l = 0; l < 3; l++) vR[l] -= rt[l];
-        const int st = grad_kernel<PER>(L, k, vR, vW, q);
+        const int st = ev(i, vR, vW, q);
         if (st < 0) err = st;
         bil_N4(z, e, N);
         add(w, N, vnorm3(vW));
@@ -364,7 +540,7 @@ BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, 
     if (type == 0) {  // nodes 0-2 (weight 25/48) and the centroid (weight -27/48, shape functions 1/3)
       for (int i = 0; i < 4; i++) {
         for (int l = 0; l < 3; l++) vR[l] = g[GEO_REN + 3 * i + l] - rt[l];
-        const int st = grad_kernel<PER>(L, k, vR, vW, q);
+        const int st = ev(i, vR, vW, q);
         if (st < 0) err = st;
         double N[3] = {0.0, 0.0, 0.0};
         if (i < 3) N[i] = 1.0;
@@ -379,7 +555,7 @@ BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, 
         else rule_point(3, n, x, wq, i, z, e, w);
         lit_r(el, z, e, vR);
         for (int l = 0; l < 3; l++) vR[l] -= rt[l];
-        const int st = grad_kernel<PER>(L, k, vR, vW, q);
+        const int st = ev(i, vR, vW, q);
         if (st < 0) err = st;
         lit_N3(z, e, N);
         add(w, N, 1.0);
@@ -412,6 +588,23 @@ BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, 
     for (int p = 0; p < 3; p++) dF[p] = -dF[p];
   }
   return err;
+}
+
+// Point i of the periodic rules of types 0 and 1: as field_rule_point, but triangles use the node-0
+// normal in both.
+BEM_HD void field_grad_rule_point(const double* geo, int s, int type, int i, const double* rt, double* vR, double* vW)
+{
+  field_rule_point(geo, s, type, i, rt, vR, vW);
+  const double* g = geo + (size_t)s * GEO_STRIDE;
+  if (g[GEO_NN] == 3.0)
+    for (int l = 0; l < 3; l++) vW[l] = g[GEO_WEN + l];
+}
+
+template <bool PER>
+BEM_HD int field_grad_coef(const double* geo, int sd, const double* rt, cplx k, int type, const QPLattice& L,
+                           const FieldGL* gl, cplx* CC, cplx (*dC)[8], double& F, double* dF)
+{
+  return field_grad_coef_by<PER>(geo, sd, rt, type, GradPlain<PER>{L, k}, gl, CC, dC, F, dF);
 }
 
 // Solid angle of a flat triangle (or of a quad split into two triangles along 0-2) seen from the

@@ -108,7 +108,8 @@ BEM_HD int smt_ncoef(int L) { return (L + 1) * (L + 1); }
 // position of (m, l) in the coefficient order: m = 0: l = 0..L; then m = 1: l = 1..L; ...
 BEM_HD int smt_lm(int L, int m, int l) { return m * (L + 1) - m * (m - 1) / 2 + (l - m); }
 
-inline void smooth_lattice(const QPLattice& L, SmoothLat& S)
+// expm: bound of (k veps)^2 of the sums.
+inline void smooth_lattice(const QPLattice& L, SmoothLat& S, double expm = SMT_EXPM)
 {
   S.ok = 0;
   S.dimg = S.dblk = S.terms = S.ve = S.rmax = 0.0;
@@ -142,7 +143,7 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S)
   const double am2 = 37.0 / (ve * ve) + L.k * L.k, R = 2.0 * ve * 6.1, det = fabs(L.detd);
   S.terms = det / (4.0 * QP_PI) * am2 + QP_PI * R * R / det + 30.0;
   // the table's sums
-  S.ve = sqrt(SMT_EXPM) / L.k;
+  S.ve = sqrt(expm) / L.k;
   if (S.ve > L.veps0) S.ve = L.veps0;
   S.rmax = 2.0 * S.ve * sqrt(SMT_CUT + L.k * L.k * S.ve * S.ve);
   const double l1 = sqrt(L.d1x * L.d1x + L.d1y * L.d1y), l2 = sqrt(L.ad22);
@@ -156,6 +157,13 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S)
   S.o1 = (int)ceil(c1 - w1); S.o2 = (int)ceil(c2 - w2);
   S.no1 = (int)floor(c1 + w1) - S.o1 + 1; S.no2 = (int)floor(c2 + w2) - S.o2 + 1;
   if (S.no1 < 1 || S.no2 < 1 || S.no1 > 128 || S.no2 > 128 || S.no1 * S.no2 > SMT_ORDERS) return;
+  // a grazing order (beta_n = 0): the lattice sums report it
+  for (int a = 0; a < S.no1; a++)
+    for (int b = 0; b < S.no2; b++) {
+      const double ax = -L.vkx + (S.o1 + a) * L.g1x + (S.o2 + b) * L.g2x;
+      const double ay = -L.vky + (S.o1 + a) * L.g1y + (S.o2 + b) * L.g2y;
+      if (fabs(L.k * L.k - ax * ax - ay * ay) < 1e-13 * L.k * L.k) return;
+    }
   S.ok = 1;
 }
 
@@ -526,10 +534,11 @@ BEM_HD void smooth_gauss(int n, int i, double& x, double& w)
 
 // The plan's choice of degree and grid, then its tables; the tables are filled by part = 0, 1, ... of
 // nparts (threads), with a barrier between the two stages (smooth_tables_a, _b).
-BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothExt& X, double npairs, int tri, long long cap,
-                          int degree, SmoothGrid& P, double& cost)
+BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothExt& X, double npairs, double near, int tri,
+                          long long cap, int degree, SmoothGrid& P, double& cost)
 {
-  // degree L alone (the caller takes the cheapest)
+  // degree L alone (the caller takes the cheapest).  near: points of a quad's rule, three times that on a
+  // triangle; 0 where each "pair" is one point
   cost = 1e300;
   P.on = 0;
   if (!S.ok) return;
@@ -544,9 +553,9 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.ncent = (int)nc;
   P.nq4 = n4 * n4;
   P.nq3 = n4 * (n4 + 1);
-  const double nq = tri ? P.nq3 : P.nq4;
+  const double nq = near > 0.0 ? (tri ? P.nq3 : P.nq4) : 1.0;
   cost = smooth_cost(S, fabs(L.detd), npairs * nq, nc, degree);
-  const double plain = npairs * (tri ? 432.0 : 144.0) * S.terms * 200.0;
+  const double plain = npairs * (near > 0.0 ? (tri ? 3.0 * near : near) : 1.0) * S.terms * 200.0;
   if (cost < 0.8 * plain) P.on = 1;
   P.rn1 = 1.0 / P.n1; P.rn2 = 1.0 / P.n2; P.rhz = 1.0 / P.hz;
   P.e1 = S.e1; P.e2 = S.e2;

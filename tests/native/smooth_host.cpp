@@ -4,6 +4,7 @@
 
 #include <vector>
 
+#include "ewald_warp.cuh"
 #include "smooth.cuh"
 
 namespace {
@@ -81,7 +82,7 @@ int sh_plan(const double* lat, const double* geo, int ne, double npairs, int deg
   for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
     double c;
     if (degree && d != degree) continue;
-    smooth_choose(D.L, S, X, npairs, tri, 1LL << 40, d, g, c);
+    smooth_choose(D.L, S, X, npairs, 144.0, tri, 1LL << 40, d, g, c);
     if (c < best) { best = c; *static_cast<SmoothGrid*>(&D.P) = g; }
   }
   info[0] = best < 1e300 ? D.P.on : 0;
@@ -151,6 +152,37 @@ int sh_pair(const double* geo, int t, int tn, int s, int plain, int n, const dou
   for (int i = 0; i < 8; i++) { CC[i] = CC[i] * ph; out[2 * i] = CC[i].re; out[2 * i + 1] = CC[i].im; }
   out[16] = CC[8].re; out[17] = dCz[8].re; out[18] = dCe[8].re;
   return err;
+}
+
+// G, grad G, second derivatives (20 doubles a point) by the warps' sums (lanes lanes, added up) and by the
+// plain sums; returns 0 when the lattice has no such sums.
+int sh_ewald(const double* lat, const double* r, int n, int lanes, double* out, double* plain)
+{
+  QPLattice L;
+  memset((void*)&L, 0, sizeof L);
+  if (qp_lattice_init(L, lat[0], lat[1], lat[2], lat[3], lat[4], lat[5], lat[6]) != 0) return 0;
+  std::vector<QPProp> prop(QP_PROP_CAP);
+  L.nprop = qp_prop_list(L, prop.data(), QP_PROP_CAP);
+  L.prop = prop.data();
+  SmoothLat S;
+  smooth_lattice(L, S, EWW_EXPM);
+  if (!S.ok) return 0;
+  for (int i = 0; i < n; i++) {
+    double sum[20] = {0.0}, px = 0.0, py = 0.0;
+    EwaldVal o;
+    for (int l = 0; l < lanes; l++) {
+      ewald_terms<true>(L, S, r + 3 * i, l, lanes, o, &px, &py);
+      const double* t = reinterpret_cast<const double*>(&o);
+      for (int c = 0; c < 20; c++) sum[c] += t[c];
+    }
+    memcpy((void*)&o, sum, sizeof o);
+    ewald_phase<true>(L, px, py, o);
+    memcpy(out + 20 * i, (const void*)&o, sizeof o);
+    QPVal2 v;
+    if (qpgf_eval2(L, r + 3 * i, v) < 0) return 0;
+    memcpy(plain + 20 * i, (const void*)&v, sizeof v);
+  }
+  return 1;
 }
 
 }

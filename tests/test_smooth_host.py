@@ -33,6 +33,7 @@ def sh():
     vp, i, d = C.c_void_p, C.c_int, C.c_double
     lib.sh_plan.argtypes = [vp, vp, i, d, i, vp]
     lib.sh_pair.argtypes = [vp, i, i, i, i, i, vp, vp, vp, vp]
+    lib.sh_ewald.argtypes = [vp, vp, i, i, vp, vp]
     return lib
 
 
@@ -91,8 +92,11 @@ def _green(lat, r):
             cb = np.exp(1j * (kx * (a * d1[0] + b * d2[0]) + ky * (a * d1[1] + b * d2[1]))) / (4 * math.pi)
             cf = -cb * ef * (w.real / D - k * w.imag + 1 / (ve * math.sqrt(math.pi))) / (D * D)
             out += np.stack([cb * ef * w.real / D, cf * px, cf * py, cf * z], -1)
-    g1 = 2 * math.pi / det * np.array([d2[1], -d2[0]])
-    g2 = 2 * math.pi / det * np.array([-d1[1], d1[0]])
+    # the reciprocal vectors as the library rounds them: near a grazing order (k = |a|) the sum depends on
+    # their last bits
+    idd = 1.0 / det
+    g1 = np.array([2 * math.pi * idd * d2[1], -2 * math.pi * idd * d2[0]])
+    g2 = np.array([-2 * math.pi * idd * d1[1], 2 * math.pi * idd * d1[0]])
     amax = math.sqrt(42 / ve ** 2 + k * k) + math.hypot(kx, ky)
     az, sz, q = np.abs(z), np.where(z < 0, -1.0, 1.0), np.abs(z) / (2 * ve)
     for a in range(-int(amax * n1 / 6.28) - 2, int(amax * n1 / 6.28) + 3):
@@ -213,3 +217,24 @@ def test_in_plane_pairs_are_left_to_the_lattice_sums(sh):
         out, x = np.zeros(19), np.zeros(1)
         sh.sh_pair(g.ctypes.data, 1, 0, 2, 0, 0, x.ctypes.data, x.ctypes.data, out.ctypes.data, C.byref(ip))
         assert ip.value == want, dz
+
+
+@pytest.mark.parametrize("lattice", sorted(LATTICES))
+@pytest.mark.parametrize("lam", [0.4, 0.8, 2.5])
+def test_warp_sums_equal_the_reference_and_the_plain_second_derivatives(sh, lattice, lam):
+    """ewald_warp.cuh: G and grad G against the numpy sums, the second derivatives against qpgf_eval2, at
+    points of every height (0 and far among them) and in other cells.  Rounding: terms up to e^2 (the
+    plain sums e^3) times the sum, ~400 of them: 1e-13 and, for the plain sums at large wave numbers, 1e-11
+    of the largest value."""
+    rng = np.random.default_rng(int(lam * 100))
+    k = 2 * math.pi * 1.33 / lam
+    lat = np.array([k, 0.3 * k, -0.2 * k, *LATTICES[lattice]])
+    n = 12
+    r = np.concatenate([rng.uniform(-1.6, 1.6, (n, 2)), rng.uniform(-0.9, 0.9, (n, 1))], 1)
+    r[:4, 2] = [0.0, 1e-9, -2.5, 1.3]
+    r = np.ascontiguousarray(r)
+    out, plain = np.zeros((n, 20)), np.zeros((n, 20))
+    assert sh.sh_ewald(lat.ctypes.data, r.ctypes.data, n, 32, out.ctypes.data, plain.ctypes.data) == 1
+    out, plain, ref = out.view(complex), plain.view(complex), _green(lat, r)
+    assert np.max(np.abs(out[:, :4] - ref) / np.abs(ref).max(1, keepdims=True)) <= 1e-13
+    assert np.max(np.abs(out - plain) / np.abs(plain).max(1, keepdims=True)) <= 1e-11
