@@ -231,7 +231,7 @@ __device__ __forceinline__ void smooth_project_block(const QPLattice& L, const S
   if (!P.on) return;
   __shared__ cplx smp[2 * (SMT_LMAX + 1) * (SMT_LMAX + 1)];
   __shared__ cplx ca[(SMT_LMAX + 1) * (SMT_LMAX + 1)], cb[(SMT_LMAX + 1) * (SMT_LMAX + 1)];
-  const int ns = P.nth * P.nph, L1 = P.L + 1, nc = smt_ncoef(P.L);
+  const int ns = P.nth * P.nph, L1 = P.L + 1;
   for (int slot = first; slot < P.ncent; slot += stride) {
     const cplx* in = M.smp + (size_t)slot * ns;
     SmoothCell c;
@@ -244,7 +244,7 @@ __device__ __forceinline__ void smooth_project_block(const QPLattice& L, const S
     __syncthreads();
     for (int i = threadIdx.x; i < P.nth * L1; i += blockDim.x) smooth_azimuth(P, smp, i / L1, i % L1, ca[i], cb[i]);
     __syncthreads();
-    cplx* al = M.tab + (size_t)slot * nc;
+    cplx* al = smt_at(M.tab, P.L, slot);
     for (int i = threadIdx.x; i < L1 * L1; i += blockDim.x) {
       const int m = i / L1, l = i % L1;
       if (l < m) continue;

@@ -104,7 +104,17 @@ struct SmoothExt {
   double bend;  // largest variation of the normal over an element, |W(+-1)  - W(0)| / |W(0)| (quads)
 };
 
-BEM_HD int smt_ncoef(int L) { return (L + 1) * (L + 1); }
+// Coefficients of a centre, (L + 1)^2, and one more for even L: with the device table's first at an odd
+// place then (smt_at), every pair A, B of m >= 1 is one aligned 32-byte load.
+BEM_HD int smt_ncoef(int L) { return (L + 1) * (L + 1) + !(L & 1); }
+template <class T>
+BEM_HD T* smt_at(T* tab, int L, int slot)
+{
+#if defined(__CUDA_ARCH__)
+  tab += !(L & 1);
+#endif
+  return tab + (size_t)slot * smt_ncoef(L);
+}
 // position of (m, l) in the coefficient order: m = 0: l = 0..L; then m = 1: l = 1..L; ...
 BEM_HD int smt_lm(int L, int m, int l) { return m * (L + 1) - m * (m - 1) / 2 + (l - m); }
 
@@ -291,6 +301,16 @@ BEM_HD cplx smt_ld(const cplx* __restrict__ al, int i)
 #endif
 }
 
+// Coefficients i, i + 1 by one 32-byte load.
+BEM_HD void smt_ld2(const cplx* __restrict__ al, int i, cplx& A, cplx& B)
+{
+#if defined(__CUDA_ARCH__)
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(A.re), "=d"(A.im), "=d"(B.re), "=d"(B.im) : "l"(al + i));
+#else
+  A = al[i]; B = al[i + 1];
+#endif
+}
+
 // S and W . grad S at the offset (x, y, z) from a centre, from its coefficients al; rad as
 // smooth_radial fills it.  The coefficients are one stream; the next pair of it is loaded a
 // step ahead (up to 2 past the centre's: the table has SMT_PAD more).
@@ -312,44 +332,50 @@ BEM_HD void smooth_eval(const cplx* __restrict__ al, int L, double k, double x, 
       const double v = j * a, u = j * d + (kw * jn) * a;
       Sr += A.re * v; Si += A.im * v; Dr += A.re * u; Di += A.im * u;
       const double c = smt_rec.c[0][l + 1], t1 = c * r2, t2 = c * wd2;
-      const double na = z * a - t1 * b, nd = z * d + Wz * a - t2 * b - t1 * e;
+      const double na = fma(z, a, -(t1 * b)), nd = fma(z, d, fma(Wz, a, -fma(t2, b, t1 * e)));
       b = a; e = d; a = na; d = nd;
       j = jn;
       A = An;
     }
   }
   al += L + 1;
-  cplx B = smt_ld(al, 1);
-  double pr = x, pi = y, qr = Wx, qi = Wy;  // R_m^m and its derivative along W
+  cplx B;
+  smt_ld2(al, 0, A, B);
+  // m >= 1: R_l^m = q_l (x + i y)^m with q_l real.  Per m the sums over l of f_l q_l and of its derivative
+  // along W, times A and times B; the power of x + i y and its derivative come in once per m.
+  double pr = x, pi = y, qr = Wx, qi = Wy;  // (x + i y)^m and its derivative along W
   for (int m = 1; m <= L; m++) {
-    double ar = pr, ai = pi, dr = qr, di = qi, br = 0.0, bi = 0.0, er = 0.0, ei = 0.0;
+    double a = 1.0, d = 0.0, b = 0.0, e = 0.0;
+    double VAr = 0.0, VAi = 0.0, VBr = 0.0, VBi = 0.0, UAr = 0.0, UAi = 0.0, UBr = 0.0, UBi = 0.0;
     const double* rl = rad + m * st;
     const double* rc = &smt_rec.c[m][m + 1];
     double j = rl[0];
-    // one degree: adds the terms of R_l^m = (ar, ai), then (br, bi) becomes R_{l+1}^m
-    auto step = [&](double& ar, double& ai, double& dr, double& di, double& br, double& bi, double& er, double& ei) {
+    // one degree: adds the terms of q_l = a, then b becomes q_{l+1}
+    auto step = [&](double& a, double& d, double& b, double& e) {
       al += 2;
-      const cplx An = smt_ld(al, 0), Bn = smt_ld(al, 1);
+      cplx An, Bn;
+      smt_ld2(al, 0, An, Bn);
       rl += st;
       const double jn = *rl;
-      const double g = kw * jn;
-      const double vr = j * ar, vi = j * ai, ur = j * dr + g * ar, ui = j * di + g * ai;
-      Sr += A.re * vr; Si += A.im * vr; Dr += A.re * ur; Di += A.im * ur;
-      Sr += B.re * vi; Si += B.im * vi; Dr += B.re * ui; Di += B.im * ui;
+      const double v = j * a, u = j * d + (kw * jn) * a;
+      VAr += A.re * v; VAi += A.im * v; VBr += B.re * v; VBi += B.im * v;
+      UAr += A.re * u; UAi += A.im * u; UBr += B.re * u; UBi += B.im * u;
       const double c = *rc++, t1 = c * r2, t2 = c * wd2;
-      er = z * dr + Wz * ar - t2 * br - t1 * er;
-      ei = z * di + Wz * ai - t2 * bi - t1 * ei;
-      br = z * ar - t1 * br;
-      bi = z * ai - t1 * bi;
+      // the newest values (d, a) come in last: a step's dependent chain is two operations
+      e = fma(z, d, fma(Wz, a, -fma(t2, b, t1 * e)));
+      b = fma(z, a, -(t1 * b));
       j = jn;
       A = An; B = Bn;
     };
     int l = m;
     for (; l < L; l += 2) {
-      step(ar, ai, dr, di, br, bi, er, ei);
-      step(br, bi, er, ei, ar, ai, dr, di);
+      step(a, d, b, e);
+      step(b, e, a, d);
     }
-    if (l == L) step(ar, ai, dr, di, br, bi, er, ei);
+    if (l == L) step(a, d, b, e);
+    Sr += VAr * pr + VBr * pi; Si += VAi * pr + VBi * pi;
+    Dr += UAr * pr + UBr * pi + VAr * qr + VBr * qi;
+    Di += UAi * pr + UBi * pi + VAi * qr + VBi * qi;
     const double nr = pr * x - pi * y, ni = pr * y + pi * x;
     const double mr = qr * x - qi * y + pr * Wx - pi * Wy, mi = qr * y + qi * x + pr * Wy + pi * Wx;
     pr = nr; pi = ni; qr = mr; qi = mi;
@@ -407,7 +433,7 @@ BEM_HD void smooth_rest(const QPLattice& L, const SmoothPlan& P, const cplx* __r
   smooth_cell(L, P, r[0], r[1], z, c);
   const double x = r[0] - c.cx, y = r[1] - c.cy, zz = z - c.cz;
   smooth_radial(L.k, x * x + y * y + zz * zz, P.L, P.top, rad, st);
-  smooth_eval(tab + (size_t)c.slot * smt_ncoef(P.L), P.L, L.k, x, y, zz, W[0], W[1], Wz, rad, st, g, h);
+  smooth_eval(smt_at(tab, P.L, c.slot), P.L, L.k, x, y, zz, W[0], W[1], Wz, rad, st, g, h);
   const cplx p1 = c.su > 0.0 ? P.e1 : conj(P.e1), p2 = c.sv > 0.0 ? P.e2 : conj(P.e2);
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
