@@ -12,8 +12,7 @@
 //   k_self_periodic / k_self_interior : one CTA per self pair (t == s), polar rule;
 //   k_reg_periodic : one warp per regular pair, lanes over the 144 (quad) / 432 (triangle)
 //                    Gauss points, one quasi-periodic Green's function per point;
-//   k_reg_interior : one thread per regular pair (free-space kernel, uniform cost), a warp per 32
-//                    sources of a row;
+//   k_reg_interior : one thread per regular pair (free-space kernel), a warp per 32 sources of a row;
 //   k_gh_*         : pairs whose GL dF/dv exceeds CBD_SDF, recomputed with the 64x64 rule from a
 //                    compacted device work list (no host round trip);
 //   k_rowsum       : deterministic per-row sums of F, dF/dt over s, H diagonal += (1+)F.
@@ -32,6 +31,7 @@
 // ------------------------------------------------------------------------------------------
 // Constant tables: Gauss-Legendre nodes (12, 64) and the open-domain lattice.
 __constant__ double c_xl[12], c_wl[12], c_xh[64], c_wh[64];
+__constant__ double c_xr[RULE_TAB], c_wr[RULE_TAB];  // the rules of 6 to 12 points
 
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v)
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(256, 2) k_gh_periodic(AssembleArgs A, const __
 // ==========================================================================================
 // Regular interior pairs: one thread per pair, a warp's 32 pairs being consecutive sources of one row.
 //
-// The 12 x 12 rule (three of them on triangles) is walked by rows of the first coordinate a.  Along a
+// The n x n rule (three of them on triangles; n = 6 to 12, rule_order) is walked by rows of the first coordinate a.  Along a
 // row the position, the normal, their products with the node's tangents and the shape functions are
 // linear in the second coordinate b:
 //   r - rt = P + Q b,  W = C + D b,  N_i = al_i + be_i b,
@@ -562,18 +562,24 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
 #pragma unroll
   for (int i = 0; i < 48; i++) my[i * REGI_LD] = 0.0;
   double F = 0.0, dF0 = 0.0, dF1 = 0.0;
-  const int nrow = (blank || !in || s == t) ? 0 : (tri ? 36 : 12);
-  const bool brief = __all_sync(0xffffffffu, nrow == 0 || regi_brief(e, A.kre, A.kim));
+  const bool none = blank || !in || s == t;
+  const bool brief = __all_sync(0xffffffffu, none || regi_brief(e, A.kre, A.kim));
+  // the warp's pairs take the largest of their rules: one loop count, and nodes from constant memory
+  const double dx = e.cr[0][0] - rt[0], dy = e.cr[1][0] - rt[1], dz = e.cr[2][0] - rt[2];
+  const int n = __reduce_max_sync(
+      0xffffffffu, none ? RULE_NMIN : rule_order(e, dx * dx + dy * dy + dz * dz, fabs(A.kre) + 2.5 * fabs(A.kim)));
+  const double *xn = c_xr + RULE_OFF(n), *wn = c_wr + RULE_OFF(n);
+  const int nrow = none ? 0 : (tri ? 3 * n : n);
 #pragma unroll 1
   for (int ar = 0; ar < nrow; ar++) {
-    const int part = ar / 12, ia = ar - 12 * part;
+    const int part = (ar >= n) + (ar >= 2 * n), ia = ar - n * part;
     RegiLine y;
-    regi_line(e, rt, part, c_xl[ia], y);
+    regi_line(e, rt, part, xn[ia], y);
     RegiRow m;
     memset(&m, 0, sizeof m);
-    if (brief) regi_row<true>(y, c_xl, c_wl, 0, 12, tri, A.kre, A.kim, m);
-    else regi_row<false>(y, c_xl, c_wl, 0, 12, tri, A.kre, A.kim, m);
-    regi_add(y, m, v0, v1, c_wl[ia], my, REGI_LD, F, dF0, dF1);
+    if (brief) regi_row<true>(y, xn, wn, 0, n, tri, A.kre, A.kim, m);
+    else regi_row<false>(y, xn, wn, 0, n, tri, A.kre, A.kim, m);
+    regi_add(y, m, v0, v1, wn[ia], my, REGI_LD, F, dF0, dF1);
   }
   // scalings of acci_finish; an element seen from its other side flips H and F
   double cg = EL_I_FP, ch = EL_I_FP, cf = EL_I_FP;
@@ -619,7 +625,8 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
 }
 
 // Regular interior pairs of one chunk (rows r0 .. r0 + nr - 1).  One B200, the shell of 1,728 quads
-// (11.9 M pairs, complex wave number): 38.5 -> 25.2 ms.
+// (11.9 M pairs, complex wave number): 38.5 -> 25.2 ms by the moments, -> 18.7 ms by fewer points for
+// distant pairs (rule_order; 7 to 9 per direction for most).
 #ifndef REGI_BLOCKS
 #define REGI_BLOCKS 4
 #endif
@@ -836,6 +843,10 @@ static int ensure_tables(void)
   if (cudaMemcpyToSymbol(c_wl, wl, sizeof wl) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_xh, xh, sizeof xh) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_wh, wh, sizeof wh) != cudaSuccess) return -1;
+  double xr[RULE_TAB], wr[RULE_TAB];
+  for (int n = RULE_NMIN; n <= RULE_NMAX; n++) gauleg_host(n, xr + RULE_OFF(n), wr + RULE_OFF(n));
+  if (cudaMemcpyToSymbol(c_xr, xr, sizeof xr) != cudaSuccess) return -1;
+  if (cudaMemcpyToSymbol(c_wr, wr, sizeof wr) != cudaSuccess) return -1;
   // k_reg_periodic keeps ~80 KB of shared memory per block (dynamic, above the 48 KB static
   // limit): allow it, and ask for the largest carve-out so the L1 split does not cut occupancy
   if (cudaFuncSetAttribute(k_reg_periodic, cudaFuncAttributePreferredSharedMemoryCarveout,

@@ -12,6 +12,8 @@
 // Measured on a B200 against one lattice sum per point (k_reg_periodic, k_gh_periodic and
 // k_self_periodic, ~200 terms a point): the open region of 96 quads 41.4 -> 2.26 ms, of 864 quads
 // 1,767 -> 59.6 ms, of 352 triangles 437 -> 54 ms (33 ms of it the in-plane pairs, which stay there).
+// With k_reg_smooth's evaluation tuned since, 864 quads take 39.0 ms, and with eight lanes a pair and
+// fewer points for distant pairs in its nearest image (rule_order) 35.4 ms.
 //
 // Every kernel returns at once when the plan is off (SmoothPlan::on == 0); the point-by-point kernels
 // then do the domain.  Nothing is kept between calls: plan and table are made again by each assembly.
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(SMT_PROJ_THREADS) k_smooth_project(const __gri
 
 // ------------------------------------------------------------------------------------------
 // Regular pairs.  A warp takes SMT_PAIRS consecutive sources of one row: their rule points for the
-// nearest image and the solid angle (32 points of one pair at a time, sums in registers), then their
+// nearest image and the solid angle (eight lanes a pair, sums in registers), then their
 // smooth points, all four pairs' in one list so that few lanes idle (4 x 36 points: 4.5 of 5 passes).
 // The smooth points' values go to shared memory, from where two lanes per (pair, shape function) add
 // them up: no reduction over lanes.
@@ -290,7 +292,7 @@ struct SmoothWarp {
   cplx sm[SMT_PAIRS][4][2];    // smooth part: G, H per shape function
   double rt[3], v0[3], v1[3];
   double sx[SMT_PAIRS], sy[SMT_PAIRS];
-  int sh[SMT_PAIRS];
+  int sh[SMT_PAIRS], n[SMT_PAIRS];  // shifted or not; the nearest image's points per direction
   union {
     double slot[32 * 19];              // the lanes' nearest-image sums
     struct {
@@ -301,11 +303,11 @@ struct SmoothWarp {
 };
 
 // Unit `unit` of the rows r0, r0 + 1, ...: sources 4 (unit mod upr) .. + 3 of row r0 + unit / upr, by one
-// warp.  xl, wl: the 12-point Gauss rule in shared memory.
+// warp.  xr, wr: the Gauss rules of 6 to 12 points in shared memory.
 __device__ __forceinline__ void reg_smooth_unit(const AssembleArgs& A, const QPLattice& L, const SmoothArgs& M, int r0,
                                                 long long unit, double3* Fp, unsigned* gh_list, unsigned* gh_count,
                                                 unsigned gh_cap, unsigned* ip_list, unsigned* ip_count, int* status,
-                                                SmoothWarp& w, const double* xl, const double* wl, int lane)
+                                                SmoothWarp& w, const double* xr, const double* wr, int lane)
 {
   const SmoothPlan& P = *M.plan;
   const int upr = (A.ne + SMT_PAIRS - 1) / SMT_PAIRS;
@@ -332,37 +334,52 @@ __device__ __forceinline__ void reg_smooth_unit(const AssembleArgs& A, const QPL
     const double v[3] = {e.cr[0][0] - rt[0], e.cr[1][0] - rt[1], e.cr[2][0] - rt[2]};
     w.sh[lane] = smooth_shift(L, v, &w.sx[lane], &w.sy[lane]);
     ok = !smooth_in_plane(L, e, rt[2]);
+    // both the nearest image and (solid angle) the element itself are at least this far
+    const double x = v[0] + w.sx[lane], y = v[1] + w.sy[lane], h2 = v[0] * v[0] + v[1] * v[1];
+    w.n[lane] = rule_order(e, fmin(h2, x * x + y * y) + v[2] * v[2], L.k);
     if (!ok) ip_list[atomicAdd(ip_count, 1u)] = (unsigned)((long long)rr * A.ne + s0 + lane);
   }
   const unsigned valid = __ballot_sync(0xffffffffu, ok);
   if (valid == 0) return;
   __syncwarp();
-  // nearest image
-#pragma unroll 1
-  for (int j = 0; j < np; j++) {
-    if (!(valid >> j & 1)) continue;
-    const Elem& e = w.es[j];
-    const int npts = (e.nn == 4) ? 144 : 432;
-    const double sx = w.sx[j], sy = w.sy[j];
-    const int sh = w.sh[j];
+  // nearest image: eight lanes a pair, over its 36 to 144 points (three times that on triangles)
+  {
+    const int j = lane >> 3;
     AccP a;
     accp_zero(a);
+    if (valid >> j & 1) {
+      const Elem& e = w.es[j];
+      const int n = w.n[j], sh = w.sh[j];
+      const double sx = w.sx[j], sy = w.sy[j];
+      const double *xn = xr + RULE_OFF(n), *wn = wr + RULE_OFF(n);
+      int left = (e.nn == 4) ? n : 3 * n, part = 0, i = 0, c = lane & 7;  // rows left, part, row, column
+      if (c >= n) { c -= n; i++; left--; }
 #pragma unroll 1
-    for (int q = lane; q < npts; q += 32) {
-      double z, n, wt;
-      rule_point(e.nn, 12, xl, wl, q, z, n, wt);
-      smooth_near(e, L.k, w.rt, w.v0, w.v1, sx, sy, sh, z, n, wt, a);
+      while (left > 0) {
+        double zeta = xn[i], eta = xn[c], wt = wn[i] * wn[c];
+        if (e.nn != 4) {
+          wt *= 1.0 + 0.25 * zeta + 0.25 * eta;
+          lit_part_point(part, zeta, eta, zeta, eta);
+        }
+        smooth_near(e, L.k, w.rt, w.v0, w.v1, sx, sy, sh, zeta, eta, wt, a);
+        c += 8;
+        while (c >= n) { c -= n; i++; left--; }
+        if (i >= n) { i -= n; part++; }
+      }
     }
     accp_pack(a, &w.slot[lane * 19]);
-    __syncwarp();
-    if (lane < 19) {
-      double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int i = 0; i < 32; i++) s[i & 3] += w.slot[i * 19 + lane];
-      w.tot[j][lane] = (s[0] + s[1]) + (s[2] + s[3]);
-    }
-    __syncwarp();
   }
+  __syncwarp();
+#pragma unroll 1
+  for (int i = lane; i < SMT_PAIRS * 19; i += 32) {
+    const int j = i / 19, c = i - 19 * j;
+    const double* v = &w.slot[8 * j * 19 + c];
+    double s[2] = {0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 8; q++) s[q & 1] += v[q * 19];
+    w.tot[j][c] = s[0] + s[1];
+  }
+  __syncwarp();
   // smooth part
   int off[SMT_PAIRS + 1];
   off[0] = 0;
@@ -453,14 +470,14 @@ __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS)
 {
   if (!M.plan->on) return;
   extern __shared__ __align__(16) unsigned char smt_smem[];
-  __shared__ double xl[12], wl[12];
-  if (threadIdx.x < 12) { xl[threadIdx.x] = c_xl[threadIdx.x]; wl[threadIdx.x] = c_wl[threadIdx.x]; }
+  __shared__ double xr[RULE_TAB], wr[RULE_TAB];
+  if (threadIdx.x < RULE_TAB) { xr[threadIdx.x] = c_xr[threadIdx.x]; wr[threadIdx.x] = c_wr[threadIdx.x]; }
   __syncthreads();
   const int wib = threadIdx.x >> 5;
   const long long unit = (long long)blockIdx.x * SMT_WARPS + wib;
   if (unit >= (long long)((A.ne + SMT_PAIRS - 1) / SMT_PAIRS) * nr) return;  // uniform across the warp
   reg_smooth_unit(A, L, M, r0, unit, Fp, gh_list, gh_count, gh_cap, ip_list, ip_count, status,
-                  reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xl, wl, threadIdx.x & 31);
+                  reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xr, wr, threadIdx.x & 31);
 }
 
 // Near-singular pair w of the chunk starting at pair p0, by the whole CTA: the 64 x 64 rule for the

@@ -157,8 +157,8 @@ __global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_smooth(const Bat
 __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth(const BatchDomain* __restrict__ D, BatchSeg S)
 {
   extern __shared__ __align__(16) unsigned char smt_smem[];
-  __shared__ double xl[12], wl[12];
-  if (threadIdx.x < 12) { xl[threadIdx.x] = c_xl[threadIdx.x]; wl[threadIdx.x] = c_wl[threadIdx.x]; }
+  __shared__ double xr[RULE_TAB], wr[RULE_TAB];
+  if (threadIdx.x < RULE_TAB) { xr[threadIdx.x] = c_xr[threadIdx.x]; wr[threadIdx.x] = c_wr[threadIdx.x]; }
   __syncthreads();
   const int wib = threadIdx.x >> 5;
   const long long u = (long long)blockIdx.x * SMT_WARPS + wib;
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth
   const BatchDomain& d = D[S.dom[i]];
   if (!batch_smooth(d)) return;
   reg_smooth_unit(d.A, d.L, d.M, 0, u - S.base[i], d.Fp, d.smt_list, d.smt_count, d.gh_cap, d.ip_list, d.smt_count + 1,
-                  d.status, reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xl, wl, threadIdx.x & 31);
+                  d.status, reinterpret_cast<SmoothWarp*>(smt_smem)[wib], xr, wr, threadIdx.x & 31);
 }
 
 __global__ void __launch_bounds__(SI_THREADS, 2) k_batch_self_interior(const BatchDomain* __restrict__ D, BatchSeg S)

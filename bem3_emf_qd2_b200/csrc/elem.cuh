@@ -159,6 +159,61 @@ BEM_HD void rule_point(int nn, int n, const double* x, const double* wgt, int q,
   }
 }
 
+// Points per direction of a regular pair's rule: 12, or fewer where the element is far away.  The
+// integrands along a row are e^{ikR} / R times 1, 1/R, 1/R^2 and products of the position with vectors,
+// times polynomials up to degree 2 (shape functions, a triangle part's area factor) and, on quads, |W|.
+// For an edge of half length h whose nearest singularity is q h from its middle, the n-point rule's
+// error stays below 2e-16 of the integrand's size, which is below the rounding of the 12 x 12 sum, for
+//   q >= Q_n and (|Re k| + 2.5 |Im k|) h <= K_n
+// (largest error over the integrands, the singularity's direction and the phase of k, in extended
+// precision; Q_12 would be 4, so nearer pairs keep 12), and for |W| = |W0 + x W1|, |W1| <= b (|W0| - |W1|),
+// by its Taylor coefficients, b <= 0.132, 0.198, 0.267, 0.337, 0.406, 0.473.  The middles of the rows lie
+// within h of the element's middle, those of a triangle's three parts within 2 h.
+// d2: squared distance of the node from the element's middle; k: |Re k| + 2.5 |Im k|.
+#define RULE_NMIN 6
+#define RULE_NMAX 12
+#define RULE_OFF(n) ((n) * ((n) - 1) / 2 - 15)  // place of the n-point rule in the tables of 6 to 12 points
+#define RULE_TAB 63
+BEM_HD int rule_order(const Elem& e, double d2, double k)
+{
+  double h2, wb = 0.0, w0 = 1.0, off;
+  double s11 = 0.0, s22 = 0.0, s33 = 0.0, s13 = 0.0, s23 = 0.0, s12 = 0.0;
+  for (int i = 0; i < 3; i++) {
+    s11 += e.cr[i][1] * e.cr[i][1];
+    s22 += e.cr[i][2] * e.cr[i][2];
+    s12 += e.cr[i][1] * e.cr[i][2];
+  }
+  if (e.nn == 4) {
+    double w1 = 0.0, w2 = 0.0;
+    w0 = 0.0;
+    for (int i = 0; i < 3; i++) {
+      s33 += e.cr[i][3] * e.cr[i][3];
+      s13 += e.cr[i][1] * e.cr[i][3];
+      s23 += e.cr[i][2] * e.cr[i][3];
+      w0 += e.cw[i][0] * e.cw[i][0];
+      w1 += e.cw[i][1] * e.cw[i][1];
+      w2 += e.cw[i][2] * e.cw[i][2];
+    }
+    h2 = s33 + fmax(s11 + 2.0 * fabs(s13), s22 + 2.0 * fabs(s23));
+    wb = fmax(w1, w2);
+    off = 1.0;
+  } else {  // the parts' edges: 0.375 cr1 +- 0.2165 cr2, 0.433 cr2
+    h2 = fmax(0.140625 * s11 + 0.046875 * s22 + 0.16238 * fabs(s12), 0.1875 * s22);
+    off = 2.0;
+  }
+  const double k2 = k * k * h2;
+  auto fits = [&](double q, double kh, double b) {  // b: the bound above over 1 + itself
+    return d2 >= (q + off) * (q + off) * h2 && k2 <= kh * kh && wb <= b * b * w0;
+  };
+  if (fits(33.0, 0.25, 0.116)) return 6;
+  if (fits(17.0, 0.55, 0.165)) return 7;
+  if (fits(10.5, 0.95, 0.210)) return 8;
+  if (fits(7.4, 1.45, 0.252)) return 9;
+  if (fits(5.6, 2.0, 0.288)) return 10;
+  if (fits(4.6, 2.7, 0.320)) return 11;
+  return RULE_NMAX;
+}
+
 // =============================================================================================
 // Periodic (open-domain) pair, "cc" variant: CC[0..8], dC0[8], dC1[8]
 // (q0_bil_dcoef_v2_cc_GL/GH q0_bil_dcoef_v2_cc.c:129-281; q0_lit_dcoef_v2_cc_GL

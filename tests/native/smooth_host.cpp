@@ -1,7 +1,9 @@
 // Host build of the tabulated smooth remainder of the quasi-periodic Green's function (csrc/smooth.cuh):
 // a domain's plan and table on the CPU, and one pair by it and by the plain lattice sums.
+#include <math.h>
 #include <string.h>
 
+#include <complex>
 #include <vector>
 
 #include "ewald_warp.cuh"
@@ -51,6 +53,21 @@ void centre_coefs(int slot)
       *al++ = A;
       if (m) *al++ = B;
     }
+  }
+}
+typedef long double X;
+void gauss(int n, X* x, X* w)
+{
+  for (int i = 0; i < n; i++) {
+    X z = cosl(3.14159265358979323846L * (i + 0.75L) / (n + 0.5L)), d = 1;
+    for (int it = 0; it < 12; it++) {
+      X p = 1, q = 0;
+      for (int j = 1; j <= n; j++) { const X o = q; q = p; p = ((2 * j - 1) * z * q - (j - 1) * o) / j; }
+      d = n * (z * p - q) / (z * z - 1);
+      z -= p / d;
+    }
+    x[i] = z;
+    w[i] = 2 / ((1 - z * z) * d * d);
   }
 }
 }  // namespace
@@ -183,6 +200,66 @@ int sh_ewald(const double* lat, const double* r, int n, int lanes, double* out, 
     memcpy(plain + 20 * i, (const void*)&v, sizeof v);
   }
   return 1;
+}
+
+// rule_order of element s of geo for the node rt, and the 51 sums (AccI's layout: G, H, dG0, dH0, dG1, dH1
+// per shape function, F, dF0, dF1) of the pair by a rule of n points per direction, in extended
+// precision; size: the sums of the integrands' sizes, G, H and dG, dH.
+int sh_rule(const double* geo, int s, const double* rt, const double* v0, const double* v1, double kre, double kim, int n,
+            double* out, double* size)
+{
+  typedef std::complex<X> Z;
+  std::vector<X> x(n), w(n);
+  gauss(n, x.data(), w.data());
+  const X s3 = sqrtl(3.0L);
+  Elem e;
+  load_elem(geo, s, e);
+  const bool quad = e.nn == 4;
+  const Z k(kre, kim), I(0, 1);
+  Z sum[24] = {};
+  X F[3] = {}, sz[3] = {};
+  for (int q = 0; q < (quad ? n * n : 3 * n * n); q++) {
+    const int part = q / (n * n), i = q / n % n, j = q % n;
+    X z = x[i], t = x[j], wd = w[i] * w[j], N[4] = {};
+    if (quad) {
+      const X a = s3 * z, b = s3 * t;
+      N[0] = (1 - a) * (1 - b) / 4; N[1] = (1 + a) * (1 - b) / 4; N[2] = (1 + a) * (1 + b) / 4; N[3] = (1 - a) * (1 + b) / 4;
+    } else {
+      const X a = z, b = t;
+      wd *= 1 + a / 4 + b / 4;
+      if (part == 0) { z = (3 + 2 * a + 2 * b + a * b) / 8; t = s3 * (b - a) / 8; }
+      else if (part == 1) { z = (-3 + a - 5 * b - a * b) / 16; t = s3 * (3 + 3 * a + b + a * b) / 16; }
+      else { z = (-3 - 5 * a + b - a * b) / 16; t = s3 * (-3 - a - 3 * b - a * b) / 16; }
+      N[0] = (1 - 2.5L * (z + s3 * t)) / 3; N[1] = (1 + 5 * z) / 3; N[2] = (1 - 2.5L * (z - s3 * t)) / 3;
+    }
+    X W2 = 0, R2 = 0, RW = 0, Rv[2] = {}, Wv[2] = {};
+    for (int i = 0; i < 3; i++) {
+      const X W = quad ? e.cw[i][0] + z * e.cw[i][1] + t * e.cw[i][2] : (X)e.cw[i][0];
+      const X r = e.cr[i][0] + z * e.cr[i][1] + t * e.cr[i][2] + (quad ? z * t * e.cr[i][3] : 0) - rt[i];
+      W2 += W * W; R2 += r * r; RW += r * W;
+      Rv[0] += r * v0[i]; Rv[1] += r * v1[i]; Wv[0] += W * v0[i]; Wv[1] += W * v1[i];
+    }
+    const X R = sqrtl(R2), a = quad ? sqrtl(W2) : 1;
+    const Z u = std::exp(I * k * R) * wd, b = I * k * R - (X)1, c = k * k * R2 + (X)3 * b;
+    Z f[6] = {u * a / R, b * u * RW / (R2 * R)};
+    for (int j = 0; j < 2; j++) {
+      f[2 + 2 * j] = b * u * Rv[j] * a / (R2 * R);
+      f[3 + 2 * j] = u * (c * Rv[j] * RW / R2 - b * Wv[j]) / (R2 * R);
+      F[1 + j] += wd * (3 * Rv[j] * RW / R2 - Wv[j]) / (R2 * R);
+    }
+    F[0] += wd * RW / (R2 * R);
+    for (int j = 0; j < 6; j++)
+      for (int i = 0; i < 4; i++) sum[4 * j + i] += f[j] * N[i];
+    const X g = wd * a * expl(-kim * R) / R, d = std::abs(k) + 1 / R, m = quad ? 1 : fmaxl(1, sqrtl(W2));
+    sz[0] += g;
+    sz[1] += g * d * m;
+    sz[2] += 3 * g * d * d * m;
+  }
+  for (int i = 0; i < 24; i++) { out[2 * i] = (double)sum[i].real(); out[2 * i + 1] = (double)sum[i].imag(); }
+  for (int i = 0; i < 3; i++) { out[48 + i] = (double)F[i]; size[i] = (double)sz[i]; }
+  double d2 = 0.0;
+  for (int i = 0; i < 3; i++) d2 += (e.cr[i][0] - rt[i]) * (e.cr[i][0] - rt[i]);
+  return rule_order(e, d2, fabs(kre) + 2.5 * fabs(kim));
 }
 
 }

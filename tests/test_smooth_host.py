@@ -34,6 +34,7 @@ def sh():
     lib.sh_plan.argtypes = [vp, vp, i, d, i, vp]
     lib.sh_pair.argtypes = [vp, i, i, i, i, i, vp, vp, vp, vp]
     lib.sh_ewald.argtypes = [vp, vp, i, i, vp, vp]
+    lib.sh_rule.argtypes = [vp, i, vp, vp, vp, d, d, i, vp, vp]
     return lib
 
 
@@ -238,3 +239,57 @@ def test_warp_sums_equal_the_reference_and_the_plain_second_derivatives(sh, latt
     out, plain, ref = out.view(complex), plain.view(complex), _green(lat, r)
     assert np.max(np.abs(out[:, :4] - ref) / np.abs(ref).max(1, keepdims=True)) <= 1e-13
     assert np.max(np.abs(out - plain) / np.abs(plain).max(1, keepdims=True)) <= 1e-11
+
+
+# rule_order's limits: distance over the half edge, wave number times it
+RULES = {6: (33.0, 0.25), 7: (17.0, 0.55), 8: (10.5, 0.95), 9: (7.4, 1.45), 10: (5.6, 2.0), 11: (4.6, 2.7)}
+
+
+@pytest.mark.parametrize("tri", [False, True])
+@pytest.mark.parametrize("n", sorted(RULES))
+def test_fewer_points_for_distant_pairs(sh, tri, n):
+    """The n-point rule just inside its limits of distance and wave number, against 30 points, the
+    integrands in extended precision.  Tolerance: 2e-16 of the integrand's size for each of the two
+    directions, tripled for the shape functions (up to 1.4 a direction); just outside, more points are
+    taken."""
+    rng = np.random.default_rng(100 * n + tri)
+    q, kh = RULES[n]
+    s3 = math.sqrt(3)
+    for trial in range(24):
+        half = 10.0 ** rng.uniform(-2, -1)
+        geo = _elements(rng, tri, half, 0.6)
+        s = 1 + trial % 6
+        cr = geo[s, :12].reshape(3, 4)
+        if tri:
+            p, t = 0.375 * cr[:, 1], 0.125 * s3 * cr[:, 2]
+            h, off = math.sqrt(max(p @ p + t @ t + 2 * abs(p @ t), 4 * t @ t)), 2.0
+        else:
+            a, b, c = cr[:, 1], cr[:, 2], cr[:, 3]
+            h, off = math.sqrt(c @ c + max(a @ a + 2 * abs(a @ c), b @ b + 2 * abs(b @ c))), 1.0
+        part = rng.choice([0.0, 0.1, 1.0])  # of the imaginary part in the wave number's limit
+        k = rng.choice([0.05, 0.5, 0.999]) * kh / h
+        kre, kim = (1 - part) * k, part * k / 2.5
+        u = rng.normal(size=3)
+        if trial % 3 == 0:  # in line with an edge
+            u = cr[:, 1 + trial // 3 % 2]
+        u = u / np.linalg.norm(u)
+        v0, v1 = rng.normal(size=(2, 3))
+        v0, v1 = v0 / np.linalg.norm(v0), v1 / np.linalg.norm(v1)
+
+        def run(m, dist):
+            rt = np.ascontiguousarray(cr[:, 0] - u * dist)
+            out, size = np.zeros(51), np.zeros(3)
+            got = sh.sh_rule(geo.ctypes.data, s, rt.ctypes.data, v0.ctypes.data, v1.ctypes.data, kre, kim, m,
+                             out.ctypes.data, size.ctypes.data)
+            return got, out, size
+
+        dist = (q + off) * h * 1.0001
+        got, out, size = run(n, dist)
+        assert got == n, (trial, got)
+        _, ref, _ = run(30, dist)
+        scale = np.concatenate([np.repeat(size[[0, 1, 1, 2, 1, 2]], 8), [size[1], size[2], size[2]]])
+        # the solid angle is not damped
+        scale[48:] *= math.exp(kim * (dist + 2 * h))
+        assert (np.abs(out - ref) <= 1.2e-15 * scale).all(), (trial, (np.abs(out - ref) / scale).max())
+        assert run(n, (q + off) * h * 0.9999)[0] == n + 1
+        assert run(n, 1.0)[0] >= n or dist < 1.0
