@@ -337,9 +337,10 @@ __global__ void __launch_bounds__(256, 2) k_gh_periodic(AssembleArgs A, const __
 // e^{ikR} along a row is e^{ikR0} (its middle) times a Taylor sum in k (R - R0), without reductions and
 // branches, where every element of the warp is smaller than the sums' range.  At the end the warp writes
 // its row segments of each matrix from shared memory, 512 contiguous bytes an instruction.
-#define REGI_WARPS 4
+#define REGI_WARPS 1  // a CTA's warps would wait for the one whose pairs take the most points
 #define REGI_LD 33  // leading dimension of the sums (pad: the transposed read of the stores)
-#define REGI_SMEM_BYTES (sizeof(double) * 48 * REGI_LD * REGI_WARPS)
+#define REGI_SMEM (48 * REGI_LD + 21 * 32 + 10)  // doubles a warp: the sums, the lanes' elements, rt, v0, v1
+#define REGI_SMEM_BYTES (sizeof(double) * REGI_SMEM * REGI_WARPS)
 // Ranges of the Taylor sums: cos and sin to x^18 and x^17 (next terms below 1e-17 for |x| <= 0.9), e^-y
 // to y^10 (below 1e-17 for |y| <= 0.12).
 #define REGI_XMAX 0.9
@@ -391,11 +392,45 @@ struct RegiRow {
   double F, s0, s1, t0, t1;  // (R.W) / R^3; 3 (R.W) / R^5 and 1 / R^3: sum, b
 };
 
-// Row a (coordinate a of part `part` of a triangle's rule) of element e seen from rt: the linear forms,
-// the weight factor and the shape functions N_i = al[i] + be[i] b.
+// Row a (coordinate a of part `part` of a triangle's rule) of element e seen from rt: the linear forms
+// and the weight factor.
 struct RegiLine {
-  double P[3], Q[3], C[3], D[3], wf0, wf1, al[4], be[4];
+  double P[3], Q[3], C[3], D[3], wf0, wf1;
 };
+// lit_part_point along a row: zeta = z0 + z1 b, eta = n0 + n1 b
+__device__ __forceinline__ void regi_part(int part, double a, double& z0, double& z1, double& n0, double& n1)
+{
+  if (part == 0) {
+    z0 = 0.125 * (3.0 + 2.0 * a); z1 = 0.125 * (2.0 + a);
+    n0 = -0.125 * EL_SQ3 * a; n1 = 0.125 * EL_SQ3;
+  } else if (part == 1) {
+    z0 = 0.0625 * (-3.0 + a); z1 = 0.0625 * (-5.0 - a);
+    n0 = 0.0625 * EL_SQ3 * (3.0 + 3.0 * a); n1 = 0.0625 * EL_SQ3 * (1.0 + a);
+  } else {
+    z0 = 0.0625 * (-3.0 - 5.0 * a); z1 = 0.0625 * (1.0 - a);
+    n0 = 0.0625 * EL_SQ3 * (-3.0 - a); n1 = 0.0625 * EL_SQ3 * (-3.0 - a);
+  }
+}
+// Its shape functions N_i = al[i] + be[i] b.
+__device__ __forceinline__ void regi_shape(bool tri, int part, double a, double* al, double* be)
+{
+  if (!tri) {
+    const double i_a = 1.0 / EL_P44_N;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      al[i] = (i == 0 || i == 3) ? 0.25 * (1.0 - a * i_a) : 0.25 * (1.0 + a * i_a);
+      be[i] = (i < 2) ? -al[i] * i_a : al[i] * i_a;
+    }
+    return;
+  }
+  double z0, z1, n0, n1;
+  regi_part(part, a, z0, z1, n0, n1);
+  const double h = 0.5 / EL_P34_N0 / 3.0;
+  al[0] = 1.0 / 3.0 - h * (z0 + EL_SQ3 * n0); be[0] = -h * (z1 + EL_SQ3 * n1);
+  al[1] = 1.0 / 3.0 + 2.0 * h * z0;           be[1] = 2.0 * h * z1;
+  al[2] = 1.0 / 3.0 - h * (z0 - EL_SQ3 * n0); be[2] = -h * (z1 - EL_SQ3 * n1);
+  al[3] = be[3] = 0.0;
+}
 __device__ __forceinline__ void regi_line(const Elem& e, const double* rt, int part, double a, RegiLine& y)
 {
   if (e.nn == 4) {
@@ -408,25 +443,10 @@ __device__ __forceinline__ void regi_line(const Elem& e, const double* rt, int p
       y.C[i] = e.cw[i][0] + e.cw[i][1] * a;
       y.D[i] = e.cw[i][2];
     }
-    const double i_a = 1.0 / EL_P44_N;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      y.al[i] = (i == 0 || i == 3) ? 0.25 * (1.0 - a * i_a) : 0.25 * (1.0 + a * i_a);
-      y.be[i] = (i < 2) ? -y.al[i] * i_a : y.al[i] * i_a;
-    }
     return;
   }
-  double z0, z1, n0, n1;  // lit_part_point: zeta = z0 + z1 b, eta = n0 + n1 b
-  if (part == 0) {
-    z0 = 0.125 * (3.0 + 2.0 * a); z1 = 0.125 * (2.0 + a);
-    n0 = -0.125 * EL_SQ3 * a; n1 = 0.125 * EL_SQ3;
-  } else if (part == 1) {
-    z0 = 0.0625 * (-3.0 + a); z1 = 0.0625 * (-5.0 - a);
-    n0 = 0.0625 * EL_SQ3 * (3.0 + 3.0 * a); n1 = 0.0625 * EL_SQ3 * (1.0 + a);
-  } else {
-    z0 = 0.0625 * (-3.0 - 5.0 * a); z1 = 0.0625 * (1.0 - a);
-    n0 = 0.0625 * EL_SQ3 * (-3.0 - a); n1 = 0.0625 * EL_SQ3 * (-3.0 - a);
-  }
+  double z0, z1, n0, n1;
+  regi_part(part, a, z0, z1, n0, n1);
   y.wf0 = 1.0 + 0.25 * a;
   y.wf1 = 0.25;
 #pragma unroll
@@ -436,11 +456,6 @@ __device__ __forceinline__ void regi_line(const Elem& e, const double* rt, int p
     y.C[i] = e.cw[i][0];
     y.D[i] = 0.0;
   }
-  const double h = 0.5 / EL_P34_N0 / 3.0;
-  y.al[0] = 1.0 / 3.0 - h * (z0 + EL_SQ3 * n0); y.be[0] = -h * (z1 + EL_SQ3 * n1);
-  y.al[1] = 1.0 / 3.0 + 2.0 * h * z0;           y.be[1] = 2.0 * h * z1;
-  y.al[2] = 1.0 / 3.0 - h * (z0 - EL_SQ3 * n0); y.be[2] = -h * (z1 - EL_SQ3 * n1);
-  y.al[3] = y.be[3] = 0.0;
 }
 
 // Points j0 .. j1 - 1 of a row (nodes xs, weights ws).  SHORT: the Taylor sums' range holds.
@@ -517,10 +532,10 @@ __device__ __forceinline__ bool regi_brief(const Elem& e, double kre, double kim
   return fabs(kre) * reach <= REGI_XMAX && fabs(kim) * reach <= REGI_YMAX;
 }
 
-// Adds a row's moments, times its weight wr, to the 48 shape-function sums v[(8 q + 2 i + part) ld] of the
+// Adds the moments of row a, times its weight wr, to the 48 shape-function sums v[(8 q + 2 i + part) ld] of the
 // quantities q = G, H, dG0, dG1, dH0, dH1, and to F, dF0, dF1.
-__device__ __forceinline__ void regi_add(const RegiLine& y, const RegiRow& m, const double* v0, const double* v1, double wr,
-                                         double* v, int ld, double& F, double& dF0, double& dF1)
+__device__ __forceinline__ void regi_add(const RegiLine& y, const RegiRow& m, bool tri, int part, double a,
+                                         const double* v0, const double* v1, double wr, double* v, int ld, double& F, double& dF0, double& dF1)
 {
   const double C0 = dot3(y.C, v0), D0 = dot3(y.D, v0), C1 = dot3(y.C, v1), D1 = dot3(y.D, v1);
   const double P0 = dot3(y.P, v0), Q0 = dot3(y.Q, v0), P1 = dot3(y.P, v1), Q1 = dot3(y.Q, v1);
@@ -532,15 +547,42 @@ __device__ __forceinline__ void regi_add(const RegiLine& y, const RegiRow& m, co
   F += wr * m.F;
   dF0 += wr * (P0 * m.s0 + Q0 * m.s1 - (C0 * m.t0 + D0 * m.t1));
   dF1 += wr * (P1 * m.s0 + Q1 * m.s1 - (C1 * m.t0 + D1 * m.t1));
+  double sa[4], sb[4];
+  regi_shape(tri, part, a, sa, sb);
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const double al = wr * y.al[i], be = wr * y.be[i];
+    const double al = wr * sa[i], be = wr * sb[i];
 #pragma unroll
     for (int c = 0; c < 6; c++) {
       double* p = v + (c * 8 + 2 * i) * ld;
       p[0] += al * f0[c].re + be * f1[c].re;
       p[ld] += al * f0[c].im + be * f1[c].im;
     }
+  }
+}
+
+// load_elem where every lane has its own element: 32-byte loads where the records lie on such
+// boundaries (a caller's array need not), a quarter of the sectors.
+__device__ __forceinline__ void load_elem_wide(const double* __restrict__ geo, int id, Elem& e)
+{
+  if ((reinterpret_cast<uintptr_t>(geo) & 31) != 0) {
+    load_elem(geo, id, e);
+    return;
+  }
+  const double* g = geo + (size_t)id * GEO_STRIDE;
+  double v[21];
+#pragma unroll
+  for (int i = 0; i < 20; i += 4)
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[i]), "=d"(v[i + 1]), "=d"(v[i + 2]), "=d"(v[i + 3]) : "l"(g + i));
+  v[20] = g[20];
+  e.nn = (int)g[GEO_NN];
+  const bool tri = e.nn == 3;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) e.cr[d][c] = (tri && c == 3) ? 0.0 : v[4 * d + c];
+#pragma unroll
+    for (int c = 0; c < 3; c++) e.cw[d][c] = (tri && c > 0) ? 0.0 : v[12 + 3 * d + c];
   }
 }
 
@@ -556,9 +598,16 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
   const bool blank = (tn == 3 && tnn == 3);  // a triangle's fourth row stays zero
   const int sd = A.sid[in ? s : 0];
   Elem e;
-  load_elem(A.geo, abs(sd), e);
+  load_elem_wide(A.geo, abs(sd), e);
   const bool tri = e.nn == 3;
-  double* my = acc + lane;
+  // What is not needed within a row waits in shared memory: the row's moments and linear forms take 100
+  // registers, and spilled values would go through L2 (the sums leave L1 little room).
+  double *my = acc + lane, *me = acc + 48 * REGI_LD + lane, *mu = acc + 48 * REGI_LD + 21 * 32;
+#pragma unroll
+  for (int i = 0; i < 12; i++) me[32 * i] = e.cr[i / 4][i % 4];
+#pragma unroll
+  for (int i = 0; i < 9; i++) me[32 * (12 + i)] = e.cw[i / 3][i % 3];
+  if (lane < 3) { mu[lane] = rt[lane]; mu[3 + lane] = v0[lane]; mu[6 + lane] = v1[lane]; }
 #pragma unroll
   for (int i = 0; i < 48; i++) my[i * REGI_LD] = 0.0;
   double F = 0.0, dF0 = 0.0, dF1 = 0.0;
@@ -570,21 +619,28 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
       0xffffffffu, none ? RULE_NMIN : rule_order(e, dx * dx + dy * dy + dz * dz, fabs(A.kre) + 2.5 * fabs(A.kim)));
   const double *xn = c_xr + RULE_OFF(n), *wn = c_wr + RULE_OFF(n);
   const int nrow = none ? 0 : (tri ? 3 * n : n);
+  __syncwarp();
 #pragma unroll 1
   for (int ar = 0; ar < nrow; ar++) {
     const int part = (ar >= n) + (ar >= 2 * n), ia = ar - n * part;
+    Elem er;
+#pragma unroll
+    for (int i = 0; i < 12; i++) er.cr[i / 4][i % 4] = me[32 * i];
+#pragma unroll
+    for (int i = 0; i < 9; i++) er.cw[i / 3][i % 3] = me[32 * (12 + i)];
+    er.nn = tri ? 3 : 4;
     RegiLine y;
-    regi_line(e, rt, part, xn[ia], y);
+    regi_line(er, mu, part, xn[ia], y);
     RegiRow m;
     memset(&m, 0, sizeof m);
     if (brief) regi_row<true>(y, xn, wn, 0, n, tri, A.kre, A.kim, m);
     else regi_row<false>(y, xn, wn, 0, n, tri, A.kre, A.kim, m);
-    regi_add(y, m, v0, v1, wn[ia], my, REGI_LD, F, dF0, dF1);
+    regi_add(y, m, tri, part, xn[ia], mu + 3, mu + 6, wn[ia], my, REGI_LD, F, dF0, dF1);
   }
   // scalings of acci_finish; an element seen from its other side flips H and F
   double cg = EL_I_FP, ch = EL_I_FP, cf = EL_I_FP;
   if (tri) {
-    const double V[3] = {e.cw[0][0], e.cw[1][0], e.cw[2][0]}, c = 0.0625 * EL_SQ3 * EL_I_SPSQ3;
+    const double V[3] = {me[32 * 12], me[32 * 15], me[32 * 18]}, c = 0.0625 * EL_SQ3 * EL_I_SPSQ3;
     cg = c * vnorm3(V);
     ch = cf = c;
   }
@@ -626,10 +682,9 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
 
 // Regular interior pairs of one chunk (rows r0 .. r0 + nr - 1).  One B200, the shell of 1,728 quads
 // (11.9 M pairs, complex wave number): 38.5 -> 25.2 ms by the moments, -> 18.7 ms by fewer points for
-// distant pairs (rule_order; 7 to 9 per direction for most).
-#ifndef REGI_BLOCKS
-#define REGI_BLOCKS 4
-#endif
+// distant pairs (rule_order; 7 to 9 per direction for most), -> 13.5 ms with a warp per CTA, the elements
+// in shared memory in place of spilled registers, and read by 32-byte loads.  FP64 pipe 45 % busy before.
+#define REGI_BLOCKS 9  // up to 224 registers; 11 CTAs (13.8 ms) and 16 with spilled registers (18.7) are slower
 __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_reg_interior(AssembleArgs A, int r0, int nr, double3* Fp,
                                                                      unsigned* gh_list, unsigned* gh_count, unsigned gh_cap,
                                                                      int* status)
@@ -640,7 +695,7 @@ __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_reg_interior(A
   if (w >= (long long)wpr * nr) return;  // uniform across the warp
   const int rr = (int)(w / wpr), s = (int)(w - (long long)rr * wpr) * 32 + lane;
   reg_interior_warp(A, r0 + rr, s, lane, Fp, (long long)rr * A.ne + s, gh_list, gh_count, gh_cap, status,
-                    regi_smem + wib * 48 * REGI_LD);
+                    regi_smem + wib * REGI_SMEM);
 }
 
 // Near-singular interior pair w of the chunk starting at pair p0, 64 x 64 rule, by the whole CTA
@@ -671,7 +726,7 @@ __device__ __forceinline__ void gh_interior_pair(const AssembleArgs& A, long lon
     memset(&m, 0, sizeof m);
     if (brief) regi_row<true>(y, xh, wh, 32 * half, 32 * half + 32, tri, A.kre, A.kim, m);
     else regi_row<false>(y, xh, wh, 32 * half, 32 * half + 32, tri, A.kre, A.kim, m);
-    regi_add(y, m, v0, v1, wh[ia], v, 1, v[48], v[49], v[50]);
+    regi_add(y, m, tri, part, xh[ia], v0, v1, wh[ia], v, 1, v[48], v[49], v[50]);
   }
   warp_sum_arr<51>(v);
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -281,9 +281,9 @@ __global__ void __launch_bounds__(SMT_PROJ_THREADS) k_smooth_project(const __gri
 // The smooth points' values go to shared memory, from where two lanes per (pair, shape function) add
 // them up: no reduction over lanes.
 #define SMT_PAIRS 4
-#define SMT_WARPS 4
+#define SMT_WARPS 1
 #ifndef SMT_BLOCKS
-#define SMT_BLOCKS 4
+#define SMT_BLOCKS 16  // 128 registers; with 168 (12 warps) 864 quads take 35.7 ms, with 96 (20, spills) 41.7, so 31.3
 #endif
 #define SMT_BUF 160  // smooth points of a pass over the list
 struct SmoothWarp {
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS)
   if (!M.plan->on) return;
   extern __shared__ __align__(16) unsigned char smt_smem[];
   __shared__ double xr[RULE_TAB], wr[RULE_TAB];
-  if (threadIdx.x < RULE_TAB) { xr[threadIdx.x] = c_xr[threadIdx.x]; wr[threadIdx.x] = c_wr[threadIdx.x]; }
+  for (int i = threadIdx.x; i < RULE_TAB; i += SMT_WARPS * 32) { xr[i] = c_xr[i]; wr[i] = c_wr[i]; }
   __syncthreads();
   const int wib = threadIdx.x >> 5;
   const long long unit = (long long)blockIdx.x * SMT_WARPS + wib;

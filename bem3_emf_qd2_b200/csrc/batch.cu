@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth
 {
   extern __shared__ __align__(16) unsigned char smt_smem[];
   __shared__ double xr[RULE_TAB], wr[RULE_TAB];
-  if (threadIdx.x < RULE_TAB) { xr[threadIdx.x] = c_xr[threadIdx.x]; wr[threadIdx.x] = c_wr[threadIdx.x]; }
+  for (int i = threadIdx.x; i < RULE_TAB; i += SMT_WARPS * 32) { xr[i] = c_xr[i]; wr[i] = c_wr[i]; }
   __syncthreads();
   const int wib = threadIdx.x >> 5;
   const long long u = (long long)blockIdx.x * SMT_WARPS + wib;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_batch_reg_inte
   const long long u = w - S.base[i];
   const int row = (int)(u / wpr), s = (int)(u - (long long)row * wpr) * 32 + lane;
   reg_interior_warp(d.A, row, s, lane, d.Fp, (long long)row * d.A.ne + s, d.gh_list, d.gh_count, d.gh_cap, d.status,
-                    regi_smem + wib * 48 * REGI_LD);
+                    regi_smem + wib * REGI_SMEM);
 }
 
 // Near-singular pairs: the domains' lists in turn, CTAs striding over each.
