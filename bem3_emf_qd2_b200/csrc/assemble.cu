@@ -32,6 +32,7 @@
 // Constant tables: Gauss-Legendre nodes (12, 64) and the open-domain lattice.
 __constant__ double c_xl[12], c_wl[12], c_xh[64], c_wh[64];
 __constant__ double c_xr[RULE_TAB], c_wr[RULE_TAB];  // the rules of 6 to 12 points
+__constant__ double c_xs[SELF_NLOG], c_ws[SELF_NLOG];
 
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v)
@@ -902,6 +903,10 @@ static int ensure_tables(void)
   for (int n = RULE_NMIN; n <= RULE_NMAX; n++) gauleg_host(n, xr + RULE_OFF(n), wr + RULE_OFF(n));
   if (cudaMemcpyToSymbol(c_xr, xr, sizeof xr) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_wr, wr, sizeof wr) != cudaSuccess) return -1;
+  double xs[SELF_NLOG], ws[SELF_NLOG];
+  gauleg_host(SELF_NLOG, xs, ws);
+  if (cudaMemcpyToSymbol(c_xs, xs, sizeof xs) != cudaSuccess) return -1;
+  if (cudaMemcpyToSymbol(c_ws, ws, sizeof ws) != cudaSuccess) return -1;
   // k_reg_periodic keeps ~80 KB of shared memory per block (dynamic, above the 48 KB static
   // limit): allow it, and ask for the largest carve-out so the L1 split does not cut occupancy
   if (cudaFuncSetAttribute(k_reg_periodic, cudaFuncAttributePreferredSharedMemoryCarveout,

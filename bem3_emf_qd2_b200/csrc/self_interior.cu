@@ -6,7 +6,7 @@
 #include "self.cuh"
 #include "bem3_internal.h"
 
-// c_xl, c_wl, c_xh, c_wh: Gauss-Legendre tables defined in assemble.cu (same translation unit,
+// c_xl, c_wl, c_xh, c_wh, c_xs, c_ws: Gauss-Legendre tables defined in assemble.cu (same translation unit,
 // see bem3_lib.cu).
 
 #define SI_THREADS 256
@@ -53,7 +53,7 @@ __device__ __forceinline__ void self_interior_row(const AssembleArgs& A, int row
   block_sum<17>(v, red, res[0]);
 
   for (int i = 0; i < SELF_NV; i++) v[i] = 0.0;
-  self_int_piece2(S, c_xh, c_wh, threadIdx.x, blockDim.x, v);
+  self_int_piece2(S, c_xh, c_wh, threadIdx.x, blockDim.x, v, c_xs, c_ws);
   block_sum<34>(v, red, res[1]);
 
   for (int i = 0; i < SELF_NV; i++) v[i] = 0.0;

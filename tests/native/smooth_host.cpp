@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "ewald_warp.cuh"
+#include "self.cuh"
 #include "smooth.cuh"
 
 namespace {
@@ -260,6 +261,19 @@ int sh_rule(const double* geo, int s, const double* rt, const double* v0, const 
   double d2 = 0.0;
   for (int i = 0; i < 3; i++) d2 += (e.cr[i][0] - rt[i]) * (e.cr[i][0] - rt[i]);
   return rule_order(e, d2, fabs(kre) + 2.5 * fabs(kim));
+}
+
+// Piece 2 of the interior self pair of element s, node tn, by the 24-point (out) and the 64-point rule
+// (ref); returns whether the 24-point rule may stand for it.
+int sh_self2(const double* geo, int s, int tn, double kre, double kim, const double* xs, const double* ws, const double* xh,
+             const double* wh, double* out, double* ref)
+{
+  SelfInfo S;
+  self_setup(geo, s, tn, mk(kre, kim), S);
+  for (int i = 0; i < SELF_NV; i++) out[i] = ref[i] = 0.0;
+  self_int_piece2(S, xh, wh, 0, 1, out, xs, ws);
+  self_int_piece2(S, xh, wh, 0, 1, ref);
+  return self_log_rule(S);
 }
 
 }

@@ -35,6 +35,7 @@ def sh():
     lib.sh_pair.argtypes = [vp, i, i, i, i, i, vp, vp, vp, vp]
     lib.sh_ewald.argtypes = [vp, vp, i, i, vp, vp]
     lib.sh_rule.argtypes = [vp, i, vp, vp, vp, d, d, i, vp, vp]
+    lib.sh_self2.argtypes = [vp, i, i, d, d, vp, vp, vp, vp, vp, vp]
     return lib
 
 
@@ -293,3 +294,41 @@ def test_fewer_points_for_distant_pairs(sh, tri, n):
         assert (np.abs(out - ref) <= 1.2e-15 * scale).all(), (trial, (np.abs(out - ref) / scale).max())
         assert run(n, (q + off) * h * 0.9999)[0] == n + 1
         assert run(n, 1.0)[0] >= n or dist < 1.0
+
+
+@pytest.mark.parametrize("shape", ["quad", "twisted", "trapezoid", "triangle"])
+@pytest.mark.parametrize("kr", [0.01, 1.0, 3.95, 4.05])
+def test_self_rays_in_the_logarithm(sh, shape, kr):
+    """The 24-point rule in ln r against the 64-point rule in r, up to the limits of |k K| r and of the
+    distortion.  Tolerance: the rules agree to 5e-17 of the sums of sizes; the rounding of 64 values (a few
+    units each) per ray and the cancellation of opposite rays are covered by 2e-14 of the largest sum."""
+    from bem3_emf_qd2_b200 import gauss_legendre
+    from bem3_emf_qd2_b200.dqd2 import element_constants
+    (xs, ws), (xh, wh) = gauss_legendre(24), gauss_legendre(64)
+    rng = np.random.default_rng(11)
+    corners = {"quad": [(-1, -1, 0), (1, -1, 0), (1, 0.9, 0), (-1, 0.9, 0)],
+               "twisted": [(-1, -1, 0.1), (1, -1, -0.1), (1.1, 1, 0.1), (-1, 1, -0.1)],
+               "trapezoid": [(-1, -1, 0), (1, -1, 0), (0.72, 1, 0), (-0.72, 1, 0)],
+               "triangle": [(-1, -0.8, 0), (1, -0.9, 0), (0.1, 1, 0)]}[shape]
+    for half in (0.02, 1.0):
+        q, _ = np.linalg.qr(rng.normal(size=(3, 3)))
+        rn = np.vstack([np.zeros(3), half * np.array(corners) @ q.T])
+        nv = len(corners)
+        ed = np.array([[0, 0, 0, 0], [1, 2, 3, 4 if nv == 4 else 0]], np.int32)
+        cr, cw = element_constants(rn, ed)
+        geo = np.zeros((2, 48))
+        geo[1, :12], geo[1, 12:21], geo[1, 45] = cr[1].ravel(), cw[1].ravel(), nv
+        c = cr[1] * (np.array([1, 1, 1, 1]) if nv == 4 else np.array([1, 1, 1, 0]))
+        for tn in range(nv):
+            z, e = ((-1, 1, 1, -1)[tn] / math.sqrt(3), (-1, -1, 1, 1)[tn] / math.sqrt(3)) if nv == 4 else (0, 0)
+            hi = np.linalg.norm(np.stack([c[:, 1] + c[:, 3] * e, c[:, 2] + c[:, 3] * z]), 2)
+            k = kr / (2.24 * hi)
+            for ph in (0.0, 0.1, 1.2):
+                out, ref = np.zeros(40), np.zeros(40)
+                got = sh.sh_self2(geo.ctypes.data, 1, tn, k * math.cos(ph), k * math.sin(ph), xs.ctypes.data, ws.ctypes.data,
+                                  xh.ctypes.data, wh.ctypes.data, out.ctypes.data, ref.ctypes.data)
+                assert got == (kr < 4.0)
+                if not got:
+                    assert np.array_equal(out, ref)
+                for lo, hi_ in ((0, 16), (16, 32), (32, 34)):
+                    assert np.abs(out - ref)[lo:hi_].max() <= 2e-14 * np.abs(ref)[lo:hi_].max(), (tn, lo)
