@@ -319,6 +319,21 @@ struct RowCopies {
 };
 }  // namespace
 
+// Rows per chunk where finished chunks are copied to the host during the later ones: about 8 chunks a
+// domain, fewer (down to 4) where a chunk would not give the GPU two rounds of the regular kernel's warps
+// (16 a multiprocessor with 4 sources each, 9 with 32).  At least 64 rows.
+static int copied_rows_per_chunk(int Ne, bool periodic)
+{
+  const int N = 4 * Ne, wpr = periodic ? (Ne + 3) / 4 : (Ne + 31) / 32;
+  const int fill = (2 * 148 * (periodic ? 16 : 9) + wpr - 1) / wpr;
+  int r = (N + 7) / 8;
+  const int most = (N + 3) / 4;
+  if (r < fill) r = fill < most ? fill : most;
+  if (r < 64) r = 64;
+  const int top = default_rows_per_chunk(Ne);
+  return r > top ? top : r;
+}
+
 extern "C" int bem3_assemble_domain(const bem3_mesh* mesh, const int* sid, int Ne_d, int did, int periodic,
                                     const bem3_qpd2* qd, double kre, double kim, double* G, double* H, double* dG,
                                     double* dH, double* dF)
@@ -338,10 +353,7 @@ extern "C" int bem3_assemble_domain(const bem3_mesh* mesh, const int* sid, int N
   RowCopies rcp;
   rcp.N = N;
   const ChunkHook hook = {RowCopies::hook, &rcp};
-  // about 8 row chunks per domain (at least 64 rows each), so that copies overlap the kernels
-  int rows = (int)((N + 7) / 8);
-  rows = rows < 64 ? 64 : rows;
-  rows = rows > default_rows_per_chunk(Ne_d) ? default_rows_per_chunk(Ne_d) : rows;
+  const int rows = copied_rows_per_chunk(Ne_d, periodic != 0);
   DomainRun run;
   if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) { cs = nullptr; goto done; }
   if (cudaMalloc(&dgeo, geo.size() * sizeof(double)) != cudaSuccess) goto done;
@@ -379,6 +391,9 @@ done:
   return rc;
 }
 
+// Matrices and inputs of bem3_assemble_domains up to this size stay in the thread's scratch between calls.
+#define DOMAINS_KEPT_BYTES ((size_t)512 << 20)
+
 // Every domain of a problem through host pointers: the reference's create_cmatrix, the loop of
 // create_cmatrix_domain over did = 0..MN (d3qd2_solve_bieq.c:155-163).  The domains' kernels run back
 // to back on this thread's stream, the interior domains first: their matrices are large and quick to
@@ -408,11 +423,8 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
   size_t need = 0;
   for (int d = 0; d < nd; d++) {
     N[d] = (size_t)4 * Ne_d[d];
-    int r = (int)((N[d] + 7) / 8);  // about 8 row chunks per domain, as bem3_assemble_domain
-    r = r < 64 ? 64 : r;
-    r = r > default_rows_per_chunk(Ne_d[d]) ? default_rows_per_chunk(Ne_d[d]) : r;
-    rows[d] = r;
-    const size_t b = bem3_scratch_bytes(Ne_d[d], r, (periodic && d == 0) ? bem3_smooth_cap(Ne_d[d]) : 0);
+    rows[d] = copied_rows_per_chunk(Ne_d[d], periodic && d == 0);
+    const size_t b = bem3_scratch_bytes(Ne_d[d], rows[d], (periodic && d == 0) ? bem3_smooth_cap(Ne_d[d]) : 0);
     need = b > need ? b : need;
   }
   double* dgeo = nullptr;
@@ -428,20 +440,45 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
   const cudaStream_t st = cudaStreamPerThread;
   int rc = BEM3_ERR_CUDA;
   DevRes* R = nullptr;
-  // the scratch at its largest before the first launch: no domain may reallocate it under another's kernels
-  if ((rc = ensure_scratch(need, &R))) goto done;
-  rc = BEM3_ERR_CUDA;
-  if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) { cs = nullptr; goto done; }
-  if (cudaMalloc(&dgeo, geo.size() * sizeof(double)) != cudaSuccess) goto done;
-  if (cudaMalloc(&dstat, nd * sizeof(int)) != cudaSuccess) goto done;
-  if (cudaMalloc(&dgh, nd * sizeof(unsigned long long)) != cudaSuccess) goto done;
+  void* own = nullptr;
+  // the matrices and inputs in one piece: behind the scratch where they are small (13 allocations and
+  // their release take 5.3 ms, the whole call for 216 quads 7.5 ms without them), else allocated here
+  size_t bytes = 0;
+  auto take = [&](size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t ogeo = take(geo.size() * sizeof(double)), ostat = take(nd * sizeof(int)), ogh = take(nd * sizeof(unsigned long long));
+  std::vector<size_t> osid(nd), oG(nd), oH(nd), odG(nd), odH(nd), odF(nd);
   for (int d = 0; d < nd; d++) {
     const size_t n2 = N[d] * N[d] * 16;
-    if (cudaMalloc(&dsid[d], Ne_d[d] * sizeof(int)) != cudaSuccess) goto done;
-    if (cudaMalloc(&dG_[d], n2) != cudaSuccess || cudaMalloc(&dH_[d], n2) != cudaSuccess) goto done;
-    if (opt(dG, d) && cudaMalloc(&ddG[d], 2 * n2) != cudaSuccess) goto done;
-    if (opt(dH, d) && cudaMalloc(&ddH[d], 2 * n2) != cudaSuccess) goto done;
-    if (opt(dF, d) && cudaMalloc(&ddF[d], 3 * N[d] * sizeof(double)) != cudaSuccess) goto done;
+    osid[d] = take(Ne_d[d] * sizeof(int));
+    oG[d] = take(n2);
+    oH[d] = take(n2);
+    if (opt(dG, d)) odG[d] = take(2 * n2);
+    if (opt(dH, d)) odH[d] = take(2 * n2);
+    if (opt(dF, d)) odF[d] = take(3 * N[d] * sizeof(double));
+  }
+  const bool kept = bytes <= DOMAINS_KEPT_BYTES;
+  char* base = nullptr;
+  need = (need + 255) & ~(size_t)255;
+  // the scratch at its largest before the first launch: no domain may reallocate it under another's kernels
+  if ((rc = ensure_scratch(need + (kept ? bytes : 0), &R))) goto done;
+  rc = BEM3_ERR_CUDA;
+  if (!kept && cudaMalloc(&own, bytes) != cudaSuccess) { own = nullptr; goto done; }
+  base = kept ? (char*)R->scratch + need : (char*)own;
+  if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) { cs = nullptr; goto done; }
+  dgeo = (double*)(base + ogeo);
+  dstat = (int*)(base + ostat);
+  dgh = (unsigned long long*)(base + ogh);
+  for (int d = 0; d < nd; d++) {
+    dsid[d] = (int*)(base + osid[d]);
+    dG_[d] = (double*)(base + oG[d]);
+    dH_[d] = (double*)(base + oH[d]);
+    if (opt(dG, d)) ddG[d] = (double*)(base + odG[d]);
+    if (opt(dH, d)) ddH[d] = (double*)(base + odH[d]);
+    if (opt(dF, d)) ddF[d] = (double*)(base + odF[d]);
     if (cudaMemcpy(dsid[d], sid[d], Ne_d[d] * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) goto done;
     rcp[d].N = N[d];
   }
@@ -492,11 +529,8 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
     if (hs[d]) { rc = hs[d]; break; }
 done:
   if (cs) { cudaStreamSynchronize(cs); cudaStreamDestroy(cs); }
-  cudaDeviceSynchronize();  // nothing of this call may still use the buffers freed below
-  cudaFree(dgeo); cudaFree(dstat); cudaFree(dgh);
-  for (int d = 0; d < nd; d++) {
-    cudaFree(dsid[d]); cudaFree(dG_[d]); cudaFree(dH_[d]); cudaFree(ddG[d]); cudaFree(ddH[d]); cudaFree(ddF[d]);
-  }
+  cudaStreamSynchronize(st);  // nothing of this call may still use its buffers
+  cudaFree(own);
   return rc;
 }
 
