@@ -38,6 +38,8 @@ UNIT = "pairs/s"
 # over a seeded sample of 96 of the workload's regular periodic pairs, with the assembly's method
 # choice.  Fixed: the kernel's own instruction count is reported beside it, not in its place.
 ALG_OPS_PER_TERM = {"twolayer3072": 378.23, "sphere384": 377.03, "cone3360": 398.91}
+# operations of one rule point with the Green's function in closed form
+FLOOR_OPS_PER_POINT = 150.0
 # FP64 operations per term the hardware executed in k_reg_periodic (ncu: 2 x DFMA + DADD + DMUL,
 # thread level, over the kernel's own term counter), from the capture of the workload's /stride8
 # subsample in profiles/; None where no capture of the current kernel exists.
@@ -355,6 +357,16 @@ def run_ours(args):
                 "hw_ops_per_term": hw,
                 "hw_frac": terms_per_launch * hw / (per_launch_ms * 1e-3) / 1e12 / peak if hw else None,
                 "terms_per_s": terms_per_launch / (per_launch_ms * 1e-3)}
+        # pairs by the table of the smooth remainder have no lattice terms to count: their roofline is the
+        # closed-form floor, one evaluation of the kernel, the geometry and the sums per point of the rule
+        n_reg = counts[(0, "periodic", "regular")]
+        quads = np.array([p.nv[abs(t)] == 4 for t in p.sid[0]])
+        points = float(n_reg) * (144.0 * quads.mean() + 432.0 * (1.0 - quads.mean()))
+        if terms < points:
+            achieved = points / reg_launches * FLOOR_OPS_PER_POINT / (per_launch_ms * 1e-3) / 1e12
+            roof.update(achieved=achieved, frac=achieved / peak, traffic=None, kernel="k_reg_smooth", alg_ops_per_term=None,
+                        ops_basis="150 operations per rule point (closed-form floor)", hw_ops_per_term=None, hw_frac=None,
+                        terms_per_s=None)
         roof["launch_ms"] = per_launch_ms
         roof["terms_per_launch"] = terms_per_launch
 
