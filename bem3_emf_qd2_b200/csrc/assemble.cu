@@ -95,6 +95,9 @@ __device__ __forceinline__ void accp_unpack(const double* v, AccP& a)
   for (int i = 0; i < 4; i++) { a.G[i] = mk(v[2 * i], v[2 * i + 1]); a.H[i] = mk(v[8 + 2 * i], v[9 + 2 * i]); }
   a.F = v[16]; a.dF0 = v[17]; a.dF1 = v[18];
 }
+// A complex matrix whose entries may be stored 16 bytes at a time: a caller's array of doubles need not
+// start on such a boundary.
+__device__ __forceinline__ bool wide_cplx(const double* m) { return (reinterpret_cast<uintptr_t>(m) & 15) == 0; }
 // Store one pair's coefficients in the reference layout.  Done by lanes of a warp (lane l
 // stores item l) or by a single thread (lane = -1 stores all).
 __device__ __forceinline__ void store_pair(const AssembleArgs& A, int row, int s, const cplx* CC, const cplx* dCz,
@@ -670,12 +673,14 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
     if (!mat[q]) continue;
     const size_t r = (q < 2) ? (size_t)row : (size_t)2 * row + (q & 1);
     cplx* out = (cplx*)mat[q] + r * N + (size_t)4 * s0;
+    const bool wide = wide_cplx(mat[q]);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int k = c * 32 + lane, sl = k >> 2, i = k & 3;
       if (s0 + sl >= A.ne || (s0 + sl == t && !blank)) continue;
       const double* v = acc + (q * 8 + 2 * i) * REGI_LD + sl;
-      *reinterpret_cast<double2*>(out + k) = make_double2(v[0], v[REGI_LD]);
+      if (wide) *reinterpret_cast<double2*>(out + k) = make_double2(v[0], v[REGI_LD]);
+      else out[k] = mk(v[0], v[REGI_LD]);
     }
   }
   __syncwarp();

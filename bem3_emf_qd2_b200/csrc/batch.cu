@@ -91,15 +91,19 @@ __global__ void k_batch_zero(const BatchDomain* __restrict__ D)
   const size_t nn = N * N;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const double2 z = make_double2(0.0, 0.0);
-  double2* G = (double2*)d.A.G;
-  double2* H = (double2*)d.A.H;
-  double2* dG = (double2*)d.A.dG;
-  double2* dH = (double2*)d.A.dH;
+  auto zero = [&](double* m, size_t n) {  // n complex entries
+    if (!m) return;
+    if (wide_cplx(m)) {
+      for (size_t i = i0; i < n; i += stride) ((double2*)m)[i] = make_double2(0.0, 0.0);
+    } else {
+      for (size_t i = i0; i < 2 * n; i += stride) m[i] = 0.0;
+    }
+  };
   if (d.A.periodic) {  // the interior kernels write every entry
-    for (size_t i = i0; i < nn; i += stride) { G[i] = z; H[i] = z; }
-    if (dG) for (size_t i = i0; i < 2 * nn; i += stride) dG[i] = z;
-    if (dH) for (size_t i = i0; i < 2 * nn; i += stride) dH[i] = z;
+    zero(d.A.G, nn);
+    zero(d.A.H, nn);
+    zero(d.A.dG, 2 * nn);
+    zero(d.A.dH, 2 * nn);
   }
   if (d.A.dF) for (size_t i = i0; i < 3 * N; i += stride) d.A.dF[i] = 0.0;
   for (size_t i = i0; i < N; i += stride) d.Fself[i] = make_double3(0.0, 0.0, 0.0);
