@@ -143,29 +143,33 @@ extern "C" int bem3_qpgf(const bem3_qpd2* qd, int n, const double* r, double* ou
 {
   if (n < 0 || (n > 0 && (!r || !out || !ret))) return BEM3_ERR_ARG;
   if (n == 0) return 0;
+  QPLattice L;
+  int rc = lattice_from(qd, &L);  // before the first copy: nothing is in flight when a lattice is refused
+  if (rc) return rc;
   // the points and results in this thread's scratch, QPGF_CHUNK points (24 MB) at a time
   const int chunk = n < QPGF_CHUNK ? n : QPGF_CHUNK;
   const size_t m = (size_t)chunk;
   DevRes* R = nullptr;
-  int rc = ensure_scratch(m * (3 + 8) * sizeof(double) + m * sizeof(int), &R);
-  if (rc) return rc;
+  if ((rc = ensure_scratch(m * (3 + 8) * sizeof(double) + m * sizeof(int), &R))) return rc;
   double* dout = (double*)R->scratch;
   double* dr = dout + 8 * m;
   int* dret = (int*)(dr + 3 * m);
   const cudaStream_t st = cudaStreamPerThread;
-  for (int i = 0; i < n; i += chunk) {
+  for (int i = 0; rc == 0; i += chunk) {
     const int c = n - i < chunk ? n - i : chunk;
     const size_t b = (size_t)c;
-    if (cudaMemcpyAsync(dr, r + 3 * (size_t)i, 3 * sizeof(double) * b, cudaMemcpyHostToDevice, st) != cudaSuccess)
-      return BEM3_ERR_CUDA;
-    if ((rc = bem3_qpgf_dev(qd, c, dr, dout, dret, mode, st))) return rc;
-    if (cudaMemcpyAsync(out + 8 * (size_t)i, dout, 8 * sizeof(double) * b, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaMemcpyAsync(ret + i, dret, sizeof(int) * b, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return BEM3_ERR_CUDA;
+    if (cudaMemcpyAsync(dr, r + 3 * (size_t)i, 3 * sizeof(double) * b, cudaMemcpyHostToDevice, st) != cudaSuccess) {
+      rc = BEM3_ERR_CUDA;
+    } else if ((rc = bem3_qpgf_dev(qd, c, dr, dout, dret, mode, st)) == 0 &&
+               (cudaMemcpyAsync(out + 8 * (size_t)i, dout, 8 * sizeof(double) * b, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaMemcpyAsync(ret + i, dret, sizeof(int) * b, cudaMemcpyDeviceToHost, st) != cudaSuccess)) {
+      rc = BEM3_ERR_CUDA;
+    }
+    // on every way out: the copies read and write the caller's arrays
+    if (cudaStreamSynchronize(st) != cudaSuccess && rc == 0) rc = BEM3_ERR_CUDA;
     if (n - i <= chunk) break;
   }
-  return 0;
+  return rc;
 }
 
 // ------------------------------------------------------------------------------------------
