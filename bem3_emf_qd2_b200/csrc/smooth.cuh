@@ -42,6 +42,8 @@
 #define SMT_QTOL 5e-16  // worst-direction error of the smooth rules
 #define SMT_EXPM 1.0     // bound of (k veps)^2 of the table's Ewald sums
 #define SMT_CUT 38.5     // their terms below e^-38.5 = 2e-17 are left out
+#define SMT_NNEAR 21
+#define SMT_TNEAR 0.5    // R / (2 ve) up to which `near` is used (its next term is below 1e-17 of the first)
 #define SMT_ORDERS 5000  // most spectral orders (of the rectangle that holds them) of a table: shared memory
 
 // c_lm = ((l - 1)^2 - m^2) / ((2l - 1)(2l - 3)) of the monic recurrence
@@ -73,6 +75,7 @@ struct SmoothLat {
   double ve, rmax;     // split parameter; reach of the real-space terms
   int m1, m2;          // images |p| <= m1, |q| <= m2 hold that reach around every table point
   int o1, o2, no1, no2;  // spectral orders o1 .. o1 + no1 - 1, o2 .. o2 + no2 - 1
+  double near[SMT_NNEAR];  // an image's real-space term without the image itself, by powers of R / (2 ve)
 };
 
 // A domain's grid of expansion centres and sampling sphere, and their tables (device memory, written
@@ -156,6 +159,24 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S, double expm = SMT_E
   S.ve = sqrt(expm) / L.k;
   if (S.ve > L.veps0) S.ve = L.veps0;
   S.rmax = 2.0 * S.ve * sqrt(SMT_CUT + L.k * L.k * S.ve * S.ve);
+  // v(R) - cos kR of smooth_real, over R / (2 ve) = t: with v = Re e^{-ikR} erfc(t - i k ve) it is F(t) =
+  // -Re e^{-ikR} erf(t - i k ve), which solves F' = 2 k ve D - (2 / sqrt(pi)) e^{(k ve)^2 - t^2},
+  // D' = -2 k ve F, F(0) = 0, D(0) = erfi(k ve).
+  {
+    const double ke = L.k * S.ve, g0 = 2.0 * QP_INV_SQRTPI * exp(ke * ke);
+    double D = 0.0, term = ke, F = 0.0, E[2] = {1.0, 0.0};
+    for (int m = 0; m < 60; m++) {
+      D += term / (2 * m + 1);
+      term *= ke * ke / (m + 1);
+    }
+    D *= 2.0 * QP_INV_SQRTPI;
+    for (int n = 0; n < SMT_NNEAR; n++) {
+      const double f = (2.0 * ke * D - g0 * E[n & 1]) / (n + 1);
+      D = -2.0 * ke * F / (n + 1);
+      E[n & 1] *= -2.0 / (n + 2);
+      S.near[n] = F = f;
+    }
+  }
   const double l1 = sqrt(L.d1x * L.d1x + L.d1y * L.d1y), l2 = sqrt(L.ad22);
   // table points lie within a cell and a half of the origin
   const double b1 = S.rmax * l2 / det + 1.5, b2 = S.rmax * l1 / det + 1.5;
@@ -499,7 +520,8 @@ BEM_HD void smooth_sample_point(const SmoothPlan& P, const SmoothCell& c, int p,
   r[2] = c.cz + P.rs * P.cth[t];
 }
 
-// Real-space part of the table's sums at r, minus the block's four images.
+// Real-space part of the table's sums at r, minus the block's four images.  Within SMT_TNEAR of an image both are
+// nearly 1 / R: their difference comes from its series (SmoothLat::near), without the cancellation.
 BEM_HD cplx smooth_real(const QPLattice& L, const SmoothLat& S, const SmoothCell& c, const double* r)
 {
   const double ke = L.k * S.ve, h = 0.5 / S.ve, c4 = EL_I_FP, z2 = r[2] * r[2], r2max = S.rmax * S.rmax;
@@ -510,13 +532,16 @@ BEM_HD cplx smooth_real(const QPLattice& L, const SmoothLat& S, const SmoothCell
       const double x = r[0] + X, y = r[1] + Y, R2 = x * x + y * y + z2;
       const int img = (p == 0 || p == (int)c.su) && (q == 0 || q == (int)c.sv);
       if (!img && R2 > r2max) continue;
-      const double iR = rsqrt_(R2), R = R2 * iR;
+      const double Rc = fmax(R2, 1e-200), iR = rsqrt_(Rc), R = Rc * iR, t = R * h;
       cplx v = mk(0.0, 0.0);
-      if (R2 <= r2max) {
-        const double t = R * h;
-        v.re = exp(ke * ke - t * t) * faddeeva_w_upper(ke, t).re;
+      if (img && t < SMT_TNEAR) {  // close to the image: the difference of two 1 / R by its series
+        double f = S.near[SMT_NNEAR - 1];
+        for (int n = SMT_NNEAR - 2; n >= 0; n--) f = fma(f, t, S.near[n]);
+        v = mk(f * t, -expi(L.k * R).im);
+      } else {
+        if (R2 <= r2max) v.re = exp(ke * ke - t * t) * faddeeva_w_upper(ke, t).re;
+        if (img) v -= expi(L.k * R);
       }
-      if (img) v -= expi(L.k * R);
       s += (expi(L.vkx * X + L.vky * Y) * v) * (c4 * iR);
     }
   return s;
@@ -587,22 +612,11 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.e1 = S.e1; P.e2 = S.e2;
   P.top = L.k / 3.0;
   for (int l = 1; l <= degree; l++) P.top *= L.k / (2.0 * l + 3.0);
-  // the sphere: the ball of the grid cell's half diagonal, off the origin's image by 5 % of it
+  // the sphere: the ball of the grid cell's half diagonal (it may pass as close to an image as it likes:
+  // smooth_real)
   const double ax = L.d1x / P.n1, ay = L.d1y / P.n1, bx = L.d2x / P.n2, by = L.d2y / P.n2;
   const double dp = (ax + bx) * (ax + bx) + (ay + by) * (ay + by), dm = (ax - bx) * (ax - bx) + (ay - by) * (ay - by);
-  const double rg = 0.5 * sqrt((dp > dm ? dp : dm) + P.hz * P.hz);
-  P.rs = rg;
-  for (int it = 0; it < 8; it++) {
-    double gap = 1e300;
-    for (int i = -2; i <= 2; i++)
-      for (int j = -2; j <= 2; j++)
-        for (int m = 0; m <= 2; m++) {
-          const double cx = i * ax + j * bx, cy = i * ay + j * by, cz = m * P.hz;
-          gap = fmin(gap, fabs(sqrt(cx * cx + cy * cy + cz * cz) - P.rs));
-        }
-    if (gap > 0.05 * rg) break;
-    P.rs *= 1.02;
-  }
+  P.rs = 0.5 * sqrt((dp > dm ? dp : dm) + P.hz * P.hz);
 }
 // sphere nodes and smooth rules
 BEM_HD void smooth_tables_a(SmoothPlan& P, int part, int nparts)
