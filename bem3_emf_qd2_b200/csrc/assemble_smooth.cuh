@@ -169,7 +169,7 @@ __device__ __forceinline__ void smooth_spectral_block(const QPLattice& L, const 
     __syncthreads();
     for (int i = threadIdx.x; i < no; i += blockDim.x) {
       double ax, ay;
-      F[i] = smooth_order(L, S, S.o1 + i / S.no2, S.o2 + i % S.no2, z, &ax, &ay);
+      F[i] = smooth_order<true>(L, S, S.o1 + i / S.no2, S.o2 + i % S.no2, z, &ax, &ay);
     }
     for (int f = g; f < P.nph; f += SMT_FG) {
       const double rx = P.rs * P.sth[t] * P.cph[f], ry = P.rs * P.sth[t] * P.sph[f];
@@ -238,10 +238,14 @@ __device__ __forceinline__ void smooth_project_block(const QPLattice& L, const S
     const cplx* in = M.smp + (size_t)slot * ns;
     SmoothCell c;
     smooth_slot(L, P, slot, c);
+    const cplx K = smooth_wave_centre(L, c);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < ns; i += blockDim.x) smp[i] = in[i] + smooth_wave_diff(L, P, c, i, K);
+#pragma unroll 1
     for (int i = threadIdx.x; i < ns; i += blockDim.x) {
       double r[3];
       smooth_sample_point(P, c, i, r);
-      smp[i] = in[i] + smooth_real(L, M.S, c, r);
+      smp[i] += smooth_real(L, M.S, c, r);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < P.nth * L1; i += blockDim.x) smooth_azimuth(P, smp, i / L1, i % L1, ca[i], cb[i]);
@@ -258,7 +262,7 @@ __device__ __forceinline__ void smooth_project_block(const QPLattice& L, const S
         b += cb[t * L1 + m] * w[t];
       }
       if (m == 0) {
-        al[l] = a;
+        al[l] = l == 0 ? a + K * P.c00 : a;
       } else {  // m >= 1: A, B in turn; (m, l) of m >= 1 start at L + 1
         const int o = L1 + 2 * (lm - L1);
         al[o] = a;

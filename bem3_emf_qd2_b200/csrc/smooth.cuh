@@ -95,6 +95,7 @@ struct SmoothGrid {
 struct SmoothPlan : SmoothGrid {
   double cth[SMT_LMAX + 1], sth[SMT_LMAX + 1], wth[SMT_LMAX + 1];
   double cph[2 * SMT_LMAX + 2], sph[2 * SMT_LMAX + 2];  // cos, sin of 2 pi i / nph
+  double c00;                            // coefficient (0, 0) of a sample value constant over the sphere, 1 / f_0(rs)
   double q4[3 * SMT_NQMAX * SMT_NQMAX];  // zeta, eta, weight
   double q3[3 * SMT_PMAX];
   double proj[(SMT_LMAX + 1) * (SMT_LMAX + 2) / 2 * (SMT_LMAX + 1)];  // [(m, l)][theta node]
@@ -178,8 +179,10 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S, double expm = SMT_E
     }
   }
   const double l1 = sqrt(L.d1x * L.d1x + L.d1y * L.d1y), l2 = sqrt(L.ad22);
-  // table points lie within a cell and a half of the origin
-  const double b1 = S.rmax * l2 / det + 1.5, b2 = S.rmax * l1 / det + 1.5;
+  // table points: within half a cell, an element's radius (0.46 dimg at most with a smooth rule), half a
+  // grid cell's diagonal and the sampling sphere's radius (smooth_choose) of the origin
+  const double ext = 0.46 * S.dimg + (0.145 + 0.29) * S.dblk;
+  const double b1 = S.rmax * l2 / det + fmax(1.5, 0.5 + ext * l2 / det), b2 = S.rmax * l1 / det + fmax(1.5, 0.5 + ext * l1 / det);
   const double amax = sqrt(SMT_CUT / (S.ve * S.ve) + L.k * L.k);
   const double c1 = (L.vkx * L.d1x + L.vky * L.d1y) / (2.0 * QP_PI), c2 = (L.vkx * L.d2x + L.vky * L.d2y) / (2.0 * QP_PI);
   const double w1 = amax * l1 / (2.0 * QP_PI), w2 = amax * l2 / (2.0 * QP_PI);
@@ -490,7 +493,9 @@ BEM_HD double smt_add(double a, double b)
 }
 
 // Height function of spectral order (q1, q2) of the table's sums at height z >= 0, times i / (4 |cell|):
-// the order's share of G is this times e^{i a.rho}, a = (*ax, *ay).  Zero beyond the cut.
+// the order's share of G is this times e^{i a.rho}, a = (*ax, *ay).  Zero beyond the cut.  SPLIT: without
+// the wave of order (0, 0) (smooth_wave_diff).
+template <bool SPLIT = false>
 BEM_HD cplx smooth_order(const QPLattice& L, const SmoothLat& S, int q1, int q2, double z, double* ax, double* ay)
 {
   *ax = smt_add(smt_add(-L.vkx, smt_mul(q1, L.g1x)), smt_mul(q2, L.g2x));
@@ -503,6 +508,7 @@ BEM_HD cplx smooth_order(const QPLattice& L, const SmoothLat& S, int q1, int q2,
     const cplx ff = expi(bn * z);
     const cplx w = faddeeva_w_upper(x, y);
     const double ef = exp(x * x - y * y), f = 2.0 * c / bn;
+    if (SPLIT && q1 == 0 && q2 == 0) return mk(-f * ef * w.im, 0.0);
     return mk(-f * (ef * w.im + ff.im), f * ff.re);  // i c F, F = (2 / bn) (i ef Im w + ff)
   }
   const double E = exp(-(x * x + y * y));
@@ -518,6 +524,37 @@ BEM_HD void smooth_sample_point(const SmoothPlan& P, const SmoothCell& c, int p,
   r[0] = c.cx + P.rs * P.sth[t] * P.cph[f];
   r[1] = c.cy + P.rs * P.sth[t] * P.sph[f];
   r[2] = c.cz + P.rs * P.cth[t];
+}
+
+// The plane wave of order (0, 0), f_0 e^{i (beta |z| + a.rho)} with f_0 = i / (2 beta |cell|): its value K at
+// centre c and, for sample p, the difference from it.  Where the wavelength is above the period this wave is
+// large (1 / (2 k |cell|)) and nearly constant: its rounding in the samples, over the sphere's radius, would be
+// the error of the table's gradients.  K belongs to degree 0 alone (c00), the differences are taken without
+// cancellation.  With it and the wider sphere (smooth_choose) H of 96 quads, period 1, differs from 64-bit sums
+// by 5e-15, 7e-15, 6e-15 of a pair's largest at wavelengths 3, 10, 50 (1.7e-14, 8e-14, 4e-13 before; the
+// point-by-point sums 2e-15), and as before below 1.
+BEM_HD int smooth_wave0(const QPLattice& L, double* beta)
+{
+  const double b2 = smt_add(smt_add(smt_mul(L.k, L.k), -smt_mul(L.vkx, L.vkx)), -smt_mul(L.vky, L.vky));
+  *beta = sqrt(fabs(b2));
+  return b2 > 0.0;
+}
+BEM_HD cplx smooth_wave_centre(const QPLattice& L, const SmoothCell& c)
+{
+  double beta;
+  if (!smooth_wave0(L, &beta)) return mk(0.0, 0.0);
+  return mul_i(expi(beta * c.cz - L.vkx * c.cx - L.vky * c.cy)) * (0.5 * fabs(L.idd) / beta);
+}
+BEM_HD cplx smooth_wave_diff(const QPLattice& L, const SmoothPlan& P, const SmoothCell& c, int p, cplx K)
+{
+  double beta;
+  if (!smooth_wave0(L, &beta)) return mk(0.0, 0.0);
+  const int t = p / P.nph, f = p - t * P.nph;
+  const double dz = P.rs * P.cth[t], dx = P.rs * P.sth[t] * P.cph[f], dy = P.rs * P.sth[t] * P.sph[f];
+  // |cz + dz| - cz: below the plane the wave is the mirror image
+  const double d = beta * (c.cz + dz < 0.0 ? -dz - 2.0 * c.cz : dz) - L.vkx * dx - L.vky * dy;
+  const cplx h = expi(0.5 * d);  // e^{id} - 1 = 2i sin(d/2) e^{id/2}
+  return K * mk(-2.0 * h.im * h.im, 2.0 * h.im * h.re);
 }
 
 // Real-space part of the table's sums at r, minus the block's four images.  Within SMT_TNEAR of an image both are
@@ -612,11 +649,15 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.e1 = S.e1; P.e2 = S.e2;
   P.top = L.k / 3.0;
   for (int l = 1; l <= degree; l++) P.top *= L.k / (2.0 * l + 3.0);
-  // the sphere: the ball of the grid cell's half diagonal (it may pass as close to an image as it likes:
-  // smooth_real)
+  // The sphere: twice the grid cell's half diagonal rg, so that the samples' rounding reaches the cell damped
+  // by 2^-l at degree l (over the cell's own sphere the gradients' error was L / rg times it), but within
+  // the first zero of the Bessel functions.  The neglected degrees reach the kept ones only by aliasing,
+  // (rg / d)^l (rs / d)^(2 (L + 1 - l)) for images at distance d: below the truncation (rg / d)^(L + 1) as
+  // long as rs^2 <= rg d.
   const double ax = L.d1x / P.n1, ay = L.d1y / P.n1, bx = L.d2x / P.n2, by = L.d2y / P.n2;
   const double dp = (ax + bx) * (ax + bx) + (ay + by) * (ay + by), dm = (ax - bx) * (ax - bx) + (ay - by) * (ay - by);
-  P.rs = 0.5 * sqrt((dp > dm ? dp : dm) + P.hz * P.hz);
+  const double rg = 0.5 * sqrt((dp > dm ? dp : dm) + P.hz * P.hz);
+  P.rs = fmin(fmin(2.0 * rg, sqrt(rg * S.dblk)), 2.5 / L.k);
 }
 // sphere nodes and smooth rules
 BEM_HD void smooth_tables_a(SmoothPlan& P, int part, int nparts)
@@ -671,6 +712,7 @@ BEM_HD void smooth_tables_c(SmoothPlan& P, double k, int part, int nparts)
 {
   double rad[SMT_LMAX + 2];
   smooth_radial(k, P.rs * P.rs, P.L, P.top, rad, 1);
+  if (part == 0) P.c00 = 1.0 / rad[0];
   for (int i = part; i < (P.L + 1) * (P.L + 1); i += nparts) {
     const int m = i / (P.L + 1), l = i - m * (P.L + 1);
     if (l < m) continue;

@@ -1,5 +1,46 @@
-// Host build of the samples of the assembly's table (csrc/smooth.cuh, csrc/assemble_smooth.cuh).
+// Host build of the assembly's table as its kernels make it (csrc/smooth.cuh, csrc/assemble_smooth.cuh): the
+// centres a pair needs are filled with the spectral samples without the wave of order (0, 0), that wave's
+// differences from its value at the centre, and that value in degree 0.
 #include "smooth_host.cpp"
+
+namespace {
+void table_centre(int slot)
+{
+  SmoothPlan& P = D.P;
+  if (D.have[slot]) return;
+  D.have[slot] = 1;
+  SmoothCell c;
+  smooth_centre(D.L, P, slot % P.N1 - P.I, slot / P.N1 % P.N2 - P.J, slot / P.N1 / P.N2, c);
+  const cplx K = smooth_wave_centre(D.L, c);
+  std::vector<cplx> smp(P.nth * P.nph), a(P.nth), b(P.nth);
+  std::vector<double> pts(3 * P.nth * P.nph);
+  for (int t = 0; t < P.nth; t++) {
+    for (int q = t * P.nph; q < (t + 1) * P.nph; q++) smooth_sample_point(P, c, q, &pts[3 * q]);
+    for (int i = 0; i < D.S.no1 * D.S.no2; i++) {
+      double ax, ay;
+      const cplx f = smooth_order<true>(D.L, D.S, D.S.o1 + i / D.S.no2, D.S.o2 + i % D.S.no2,
+                                        fabs(c.cz + P.rs * P.cth[t]), &ax, &ay);
+      if (f.re == 0.0 && f.im == 0.0) continue;
+      for (int q = t * P.nph; q < (t + 1) * P.nph; q++) smp[q] += f * expi(ax * pts[3 * q] + ay * pts[3 * q + 1]);
+    }
+    for (int q = t * P.nph; q < (t + 1) * P.nph; q++)
+      smp[q] += smooth_wave_diff(D.L, P, c, q, K) + smooth_real(D.L, D.S, c, &pts[3 * q]);
+  }
+  cplx* al = D.tab.data() + (size_t)slot * smt_ncoef(P.L);
+  for (int m = 0; m <= P.L; m++) {
+    for (int t = 0; t < P.nth; t++) smooth_azimuth(P, smp.data(), t, m, a[t], b[t]);
+    for (int l = m; l <= P.L; l++) {
+      cplx A = (m == 0 && l == 0) ? K * P.c00 : mk(0, 0), B = mk(0, 0);
+      for (int t = 0; t < P.nth; t++) {
+        A += a[t] * P.proj[(size_t)smt_lm(P.L, m, l) * P.nth + t];
+        B += b[t] * P.proj[(size_t)smt_lm(P.L, m, l) * P.nth + t];
+      }
+      *al++ = A;
+      if (m) *al++ = B;
+    }
+  }
+}
+}  // namespace
 
 extern "C" {
 
@@ -20,6 +61,27 @@ int st_real(const double* lat, const double* r, double su, double sv, double* ou
   out[0] = v.re; out[1] = v.im;
   *ve = S.ve;
   return S.ok;
+}
+
+// sh_pair by the table as the kernels make it.
+int st_pair(const double* geo, int t, int tn, int s, int n, const double* x, const double* w, double* out)
+{
+  Elem es;
+  load_elem(geo, s, es);
+  const double* rt = geo + (size_t)t * GEO_STRIDE + GEO_REN + 3 * tn;
+  const double v[3] = {es.cr[0][0] - rt[0], es.cr[1][0] - rt[1], es.cr[2][0] - rt[2]};
+  double sx, sy;
+  smooth_shift(D.L, v, &sx, &sy);
+  const double* tq = es.nn == 4 ? D.P.q4 : D.P.q3;
+  for (int q = 0; q < (es.nn == 4 ? D.P.nq4 : D.P.nq3); q++) {
+    double r[3], W[3];
+    point_geom(es, tq[3 * q], tq[3 * q + 1], rt, r, W);
+    SmoothCell c;
+    smooth_cell(D.L, D.P, r[0] + sx, r[1] + sy, fabs(r[2]), c);
+    table_centre(c.slot);
+  }
+  int ip;
+  return sh_pair(geo, t, tn, s, 0, n, x, w, out, &ip);
 }
 
 }

@@ -8,19 +8,21 @@ import subprocess
 import numpy as np
 import pytest
 
-from conftest import BUILD, REPO
+import test_smooth_host as pairs
+from conftest import REPO
 
 
 @pytest.fixture(scope="module")
-def st():
-    os.makedirs(BUILD, exist_ok=True)
-    so = os.path.join(BUILD, "libsmooth_table_host.so")
+def st(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("table") / "libsmooth_table_host.so")
     native, hdr = os.path.join(REPO, "tests", "native"), os.path.join(REPO, "bem3_emf_qd2_b200", "csrc")
     subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + hdr,
                     os.path.join(native, "smooth_table_host.cpp"), "-o", so], check=True)
     lib = C.CDLL(so)
     vp, i, d = C.c_void_p, C.c_int, C.c_double
     lib.st_real.argtypes = [vp, vp, d, d, vp, vp]
+    lib.st_pair.argtypes = [vp, i, i, i, i, vp, vp, vp]
+    lib.sh_plan.argtypes = [vp, vp, i, d, i, vp]
     return lib
 
 
@@ -58,3 +60,49 @@ def test_samples_close_to_an_image_keep_their_digits(st, lam):
                     ref += ph * t / (4 * mp.pi * R)
                     size += min(1 / R, 1 / v) / (4 * mp.pi) * mp.exp((kk * v) ** 2) if image else abs(t) / (4 * mp.pi * R)
             assert abs(complex(*out) - complex(ref)) <= 32 * 1.1e-16 * float(size), (at, dist)
+
+
+def _sphere(n, lam, lattice):
+    """Geometry records of a cube-sphere of 6 n^2 quads and the lattice's seven numbers."""
+    from bem3_emf_qd2_b200 import meshgen
+    from bem3_emf_qd2_b200.dqd2 import element_constants
+    nodes = meshgen._Nodes()
+    els = meshgen.cube_sphere(nodes, 0.3 * min(lattice[0], lattice[3]), n)
+    rn = np.vstack([np.zeros(3), np.array(nodes.pts)])
+    ed = np.vstack([np.zeros(4, int), np.array(els)]).astype(np.int32)
+    cr, cw = element_constants(rn, ed)
+    geo = np.zeros((len(ed), 48))
+    geo[1:, 0:12], geo[1:, 12:21], geo[1:, 45] = cr[1:].reshape(-1, 12), cw[1:].reshape(-1, 9), 4
+    g = 1 / math.sqrt(3)
+    for j, (z, e) in enumerate(((-g, -g), (g, -g), (g, g), (-g, g))):
+        geo[:, 21 + 3 * j:24 + 3 * j] = cr[:, :, 0] + cr[:, :, 1] * z + cr[:, :, 2] * e + cr[:, :, 3] * z * e
+    k = 2 * math.pi * 1.33 / lam
+    return np.ascontiguousarray(geo), np.array([k, 0.35 * k, -0.2 * k, *lattice])
+
+
+@pytest.mark.parametrize("n,lam,lattice", [
+    (4, 0.6, (1.0, 0.0, 0.0, 1.0)), (4, 3.0, (0.8, 0.0, 0.0, 1.5)), (8, 3.0, (1.0, 0.0, 0.0, 1.0)),
+    (4, 10.0, (1.0, 0.0, 0.0, 1.0)), (4, 50.0, (1.0, 0.0, 0.0, 1.0)), (4, 2000.0, (1.0, 0.0, 0.4, 0.9))])
+def test_gradients_of_the_table_where_the_wavelength_is_above_the_period(st, n, lam, lattice):
+    """H of sampled pairs against 64-bit sums.  Tolerance: 8 roundings (1.8e-15) of the size of the parts the
+    sum consists of, the normal weight W times the gradients of the four nearest images, 1 / (4 pi R^2), and of
+    the wave of order (0, 0), 1 / (2 |cell|); above k = 2 pi / period the images' gradients are (1 + k R) as large."""
+    from bem3_emf_qd2_b200 import gauss_legendre
+    geo, lat = _sphere(n, lam, lattice)
+    ne, info = len(geo) - 1, np.zeros(8, np.int32)
+    assert st.sh_plan(lat.ctypes.data, geo.ctypes.data, ne, 4.0 * ne * ne, 0, info.ctypes.data) == 1 and info[0] == 1
+    x, w = gauss_legendre(12)
+    d1, d2 = np.array([*lattice[:2], 0]), np.array([*lattice[2:], 0])
+    rng = np.random.default_rng(n)
+    for _ in range(40):
+        t, s = rng.choice(ne, 2, replace=False) + 1
+        tn = int(rng.integers(4))
+        out = np.zeros(19)
+        st.st_pair(geo.ctypes.data, t, tn, s, 12, x.ctypes.data, w.ctypes.data, out.ctypes.data)
+        _, ref = pairs._reference(lat, geo, t, tn, s)
+        v = geo[s, [0, 4, 8]] - geo[t, 21 + 3 * tn:24 + 3 * tn]
+        R = np.sort([np.linalg.norm(v + a * d1 + b * d2) for a in (-1, 0, 1) for b in (-1, 0, 1)])[:4]
+        size = ((1 + lat[0] * R) / (4 * math.pi * R * R)).sum() + 0.5 / abs(lattice[0] * lattice[3] - lattice[1] * lattice[2])
+        size *= np.linalg.norm(geo[s, 12:21:3])
+        H = out[8:16:2] + 1j * out[9:16:2]
+        assert np.abs(H - ref).max() <= 1.8e-15 * size, (t, tn, s)
