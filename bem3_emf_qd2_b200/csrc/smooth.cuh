@@ -201,30 +201,44 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S, double expm = SMT_E
   S.ok = 1;
 }
 
+// Gauss points per direction for the images on an element whose half edges are at most 1, the nearest q away
+// from its middle: the n x n rule's error is below SMT_QTOL of the integrand's size, for 1 / R and r / R^3 times
+// the shape functions, rows up to 1 nearer than the middle, in the worst direction (extended precision, squares
+// and rhombi down to 45 degrees, and the triangle's rule, which needs less).
+BEM_HD int smooth_nq_image(double q)
+{
+  if (q >= 91.0) return 4;
+  if (q >= 30.1) return 5;
+  if (q >= 14.6) return 6;
+  if (q >= 9.05) return 7;
+  if (q >= 6.45) return 8;
+  if (q >= 5.05) return 9;
+  if (q >= 4.27) return 10;
+  if (q >= 3.72) return 11;
+  return q >= 3.34 ? 12 : 0;
+}
 // Gauss points per direction for a smooth integrand on an edge of half length h: a wave of number k and
-// images at distance d, times the (linear) shape functions, and the area factor |W| of an element whose
-// normal turns by `bend`.  The error of the n-point rule is K_n f^{(2n)} h^{2n} / (2n)!, K_n = 2^{2n}
-// (n!)^4 / ((2n+1) ((2n)!)^2) (mean over the edge); for the images it is the ellipse of analyticity
-// through one on the edge's line; |W| = |W0| sqrt(1 + bend^2 x^2) has the Taylor coefficient
-// binom(1/2, n) bend^{2n} ~ bend^{2n} / (2 sqrt(pi) n^{3/2}).  The smallest n whose errors, for the worst
-// direction, stay below SMT_QTOL; 0 when SMT_NQMAX points do not reach it.
+// images at distance d (smooth_nq_image), times the (linear) shape functions, and the area factor |W| of an
+// element whose normal turns by `bend`.  The error of the n-point rule is K_n f^{(2n)} h^{2n} / (2n)!,
+// K_n = 2^{2n} (n!)^4 / ((2n+1) ((2n)!)^2) (mean over the edge); |W| = |W0| sqrt(1 + bend^2 x^2) has the
+// Taylor coefficient binom(1/2, n) bend^{2n} ~ bend^{2n} / (2 sqrt(pi) n^{3/2}).  The smallest n whose errors,
+// for the worst direction, stay below SMT_QTOL; 0 when SMT_NQMAX points do not reach it.
 BEM_HD int smooth_nq(double k, double h, double d, double bend)
 {
-  const double x = k * h, q = d / h;
-  if (!(q > 1.5)) return 0;
-  const double rho = q + sqrt(q * q - 1.0);
-  const double lb = log(bend > 1e-9 ? bend : 1e-9), lx = log(x), lr = log(rho);
+  const double x = k * h;
+  const int ni = smooth_nq_image(d / h);
+  if (ni == 0) return 0;
+  const double lb = log(bend > 1e-9 ? bend : 1e-9), lx = log(x);
   double lf = 0.0;   // ln n!
   double lf2 = 0.0;  // ln (2n)!
   for (int n = 1; n <= SMT_NQMAX; n++) {
     lf += log((double)n);
     lf2 += log((double)(2 * n - 1)) + log((double)(2 * n));
-    if (n < 4) continue;
+    if (n < ni) continue;
     const double K = (2 * n) * 0.6931471805599453 + 4.0 * lf - log(2.0 * n + 1.0) - 2.0 * lf2;
     const double e1 = exp(K - lf2 + (2 * n - 1) * lx) * (x + 2 * n);
-    const double e2 = 4.0 * exp(-(2 * n - 1) * lr);
     const double e3 = exp(K + 2 * n * lb) * 0.29 / (n * sqrt((double)n));
-    if (e1 <= SMT_QTOL && e2 <= SMT_QTOL && e3 <= SMT_QTOL) return n;
+    if (e1 <= SMT_QTOL && e3 <= SMT_QTOL) return n;
   }
   return 0;
 }

@@ -63,6 +63,9 @@ int st_real(const double* lat, const double* r, double su, double sv, double* ou
   return S.ok;
 }
 
+// Points per direction of the smooth rule.
+int st_nq(double k, double h, double d, double bend) { return smooth_nq(k, h, d, bend); }
+
 // sh_pair by the table as the kernels make it.
 int st_pair(const double* geo, int t, int tn, int s, int n, const double* x, const double* w, double* out)
 {

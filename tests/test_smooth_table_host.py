@@ -21,6 +21,7 @@ def st(tmp_path_factory):
     lib = C.CDLL(so)
     vp, i, d = C.c_void_p, C.c_int, C.c_double
     lib.st_real.argtypes = [vp, vp, d, d, vp, vp]
+    lib.st_nq.argtypes = [d, d, d, d]
     lib.st_pair.argtypes = [vp, i, i, i, i, vp, vp, vp]
     lib.sh_plan.argtypes = [vp, vp, i, d, i, vp]
     return lib
@@ -106,3 +107,59 @@ def test_gradients_of_the_table_where_the_wavelength_is_above_the_period(st, n, 
         size *= np.linalg.norm(geo[s, 12:21:3])
         H = out[8:16:2] + 1j * out[9:16:2]
         assert np.abs(H - ref).max() <= 1.8e-15 * size, (t, tn, s)
+
+
+def _gauss(n):
+    """Nodes and weights of the n-point rule in extended precision."""
+    x = np.cos(np.pi * (np.arange(n) + 0.75) / (n + 0.5)).astype(np.longdouble)
+    for _ in range(8):
+        p, q = np.ones(n, np.longdouble), np.zeros(n, np.longdouble)
+        for j in range(1, n + 1):
+            p, q = ((2 * j - 1) * x * p - (j - 1) * q) / np.longdouble(j), p
+        d = n * (x * p - q) / (x * x - 1)
+        x = x - p / d
+    return x, 2 / ((1 - x * x) * d * d)
+
+
+@pytest.mark.parametrize("shape", ["square", "rhombus", "rectangle", "triangle"])
+@pytest.mark.parametrize("n", range(4, 13))
+def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
+    """The rule that smooth_nq gives with an image as near as it accepts for n points, against 40 points in
+    extended precision: 1 / R and r / R^3 times the shape functions, the image in any direction.  Tolerance:
+    SMT_QTOL = 5e-16 of the integrands' sizes, the bound smooth_nq states.  Nearer images take more points, and
+    below the last bound there is no rule."""
+    near, far = 1.5, 1000.0
+    assert st.st_nq(1e-3, 1.0, near, 0.0) == 0
+    for _ in range(60):
+        mid = math.sqrt(near * far)
+        got = st.st_nq(1e-3, 1.0, mid, 0.0)
+        near, far = (near, mid) if 0 < got <= n else (mid, far)
+    s3 = np.sqrt(np.longdouble(3))
+
+    def rule(m):
+        x, w = _gauss(m)
+        if shape != "triangle":
+            a, b = np.meshgrid(x, x, indexing="ij")
+            W = np.outer(w, w)
+            N = np.stack([(1 - s3 * a) * (1 - s3 * b), (1 + s3 * a) * (1 - s3 * b), (1 + s3 * a) * (1 + s3 * b), (1 - s3 * a) * (1 + s3 * b)]) / 4
+            ang = {"square": 90, "rhombus": 60, "rectangle": 90}[shape]
+            h = 0.4 if shape == "rectangle" else 1.0
+            P = np.stack([a + math.cos(math.radians(ang)) * h * b, math.sin(math.radians(ang)) * h * b, 0 * a])
+        else:  # collapsed square, side 2
+            x1, w1 = _gauss(m + 1)
+            a, b = np.meshgrid(x1, x, indexing="ij")
+            u, v = (1 + a) / 2, (1 + b) / 2
+            W = np.outer(w1, w) * u
+            z, e = -0.5 + 1.5 * u - 1.5 * u * v, s3 * (-0.5 + 0.5 * u + 0.5 * u * v)
+            N = np.stack([1 - 2.5 * (z + s3 * e), 1 + 5 * z, 1 - 2.5 * (z - s3 * e)]) / 3
+            P = np.stack([z, e, 0 * z]) * 2 / s3
+        v = P[None] - at[:, :, None, None]
+        R = np.sqrt((v * v).sum(1))
+        f = np.concatenate([(1 / R)[:, None], v / R[:, None] ** 3], 1)
+        return np.einsum("mfij,kij,ij->mfk", f, N, W), (W / R).sum((1, 2)), (W / R ** 2).sum((1, 2))
+
+    ph, th = np.linspace(0, 2 * np.pi, 37), np.linspace(0, np.pi / 2, 5)
+    at = np.array([[np.sin(t) * np.cos(p), np.sin(t) * np.sin(p), np.cos(t)] for t in th for p in ph]).astype(np.longdouble) * far
+    got, ref = rule(n)[0], rule(40)
+    err = np.abs(got - ref[0]).max(2)
+    assert (err[:, 0] <= 5e-16 * ref[1]).all() and (err[:, 1:].max(1) <= 5e-16 * ref[2]).all()
