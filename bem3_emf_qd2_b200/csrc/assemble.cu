@@ -401,20 +401,6 @@ struct RegiRow {
 struct RegiLine {
   double P[3], Q[3], C[3], D[3], wf0, wf1;
 };
-// lit_part_point along a row: zeta = z0 + z1 b, eta = n0 + n1 b
-__device__ __forceinline__ void regi_part(int part, double a, double& z0, double& z1, double& n0, double& n1)
-{
-  if (part == 0) {
-    z0 = 0.125 * (3.0 + 2.0 * a); z1 = 0.125 * (2.0 + a);
-    n0 = -0.125 * EL_SQ3 * a; n1 = 0.125 * EL_SQ3;
-  } else if (part == 1) {
-    z0 = 0.0625 * (-3.0 + a); z1 = 0.0625 * (-5.0 - a);
-    n0 = 0.0625 * EL_SQ3 * (3.0 + 3.0 * a); n1 = 0.0625 * EL_SQ3 * (1.0 + a);
-  } else {
-    z0 = 0.0625 * (-3.0 - 5.0 * a); z1 = 0.0625 * (1.0 - a);
-    n0 = 0.0625 * EL_SQ3 * (-3.0 - a); n1 = 0.0625 * EL_SQ3 * (-3.0 - a);
-  }
-}
 // Its shape functions N_i = al[i] + be[i] b.
 __device__ __forceinline__ void regi_shape(bool tri, int part, double a, double* al, double* be)
 {
@@ -523,16 +509,10 @@ __device__ __forceinline__ void regi_row(const RegiLine& line, const double* xs,
   }
 }
 
-// |r - r(b = 0)| <= regi_reach along every row: the Taylor sums' range
+// The Taylor sums' range holds along every row of the element.
 __device__ __forceinline__ bool regi_brief(const Elem& e, double kre, double kim)
 {
-  double reach = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const double d = (e.nn == 3) ? 0.4 * fabs(e.cr[i][1]) + 0.4 * fabs(e.cr[i][2]) : fabs(e.cr[i][2]) + fabs(e.cr[i][3]);
-    reach += d * d;
-  }
-  reach = sqrt(reach);
+  const double reach = regi_reach(e);
   return fabs(kre) * reach <= REGI_XMAX && fabs(kim) * reach <= REGI_YMAX;
 }
 

@@ -159,6 +159,33 @@ BEM_HD void rule_point(int nn, int n, const double* x, const double* wgt, int q,
   }
 }
 
+// lit_part_point along a row: zeta = z0 + z1 b, eta = n0 + n1 b
+BEM_HD void regi_part(int part, double a, double& z0, double& z1, double& n0, double& n1)
+{
+  if (part == 0) {
+    z0 = 0.125 * (3.0 + 2.0 * a); z1 = 0.125 * (2.0 + a);
+    n0 = -0.125 * EL_SQ3 * a; n1 = 0.125 * EL_SQ3;
+  } else if (part == 1) {
+    z0 = 0.0625 * (-3.0 + a); z1 = 0.0625 * (-5.0 - a);
+    n0 = 0.0625 * EL_SQ3 * (3.0 + 3.0 * a); n1 = 0.0625 * EL_SQ3 * (1.0 + a);
+  } else {
+    z0 = 0.0625 * (-3.0 - 5.0 * a); z1 = 0.0625 * (1.0 - a);
+    n0 = 0.0625 * EL_SQ3 * (-3.0 - a); n1 = 0.0625 * EL_SQ3 * (-3.0 - a);
+  }
+}
+// Bound of |r - r(b = 0)| along every row: half a row is cr2 + cr3 a on quads, z1 cr1 + n1 cr2 with |z1| <=
+// 3/8, |n1| <= sqrt(3)/4 on triangles.
+BEM_HD double regi_reach(const Elem& e)
+{
+  double reach = 0.0;
+  for (int i = 0; i < 3; i++) {
+    const double d = (e.nn == 3) ? 0.375 * fabs(e.cr[i][1]) + 0.25 * EL_SQ3 * fabs(e.cr[i][2])
+                                 : fabs(e.cr[i][2]) + fabs(e.cr[i][3]);
+    reach += d * d;
+  }
+  return sqrt(reach);
+}
+
 // Points per direction of a regular pair's rule: 12, or fewer where the element is far away.  The
 // integrands along a row are e^{ikR} / R times 1, 1/R, 1/R^2 and products of the position with vectors,
 // times polynomials up to degree 2 (shape functions, a triangle part's area factor) and, on quads, |W|.

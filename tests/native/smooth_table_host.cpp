@@ -63,6 +63,25 @@ int st_real(const double* lat, const double* r, double su, double sv, double* ou
   return S.ok;
 }
 
+// Bound of the interior kernel's rows on element s, and the longest half of its rows at the coordinates a[n].
+double st_reach(const double* geo, int s, int n, const double* a, double* longest)
+{
+  Elem e;
+  load_elem(geo, s, e);
+  *longest = 0.0;
+  for (int part = 0; part < (e.nn == 3 ? 3 : 1); part++)
+    for (int q = 0; q < n; q++) {
+      double d2 = 0.0, z0, z1 = 0.0, n0, n1 = 1.0;
+      if (e.nn == 3) regi_part(part, a[q], z0, z1, n0, n1);
+      for (int i = 0; i < 3; i++) {
+        const double d = e.cr[i][1] * z1 + (e.cr[i][2] + e.cr[i][3] * a[q]) * n1;
+        d2 += d * d;
+      }
+      *longest = fmax(*longest, sqrt(d2));
+    }
+  return regi_reach(e);
+}
+
 // Points per direction of the smooth rule.
 int st_nq(double k, double h, double d, double bend) { return smooth_nq(k, h, d, bend); }
 

@@ -21,6 +21,8 @@ def st(tmp_path_factory):
     lib = C.CDLL(so)
     vp, i, d = C.c_void_p, C.c_int, C.c_double
     lib.st_real.argtypes = [vp, vp, d, d, vp, vp]
+    lib.st_reach.argtypes = [vp, i, i, vp, vp]
+    lib.st_reach.restype = d
     lib.st_nq.argtypes = [d, d, d, d]
     lib.st_pair.argtypes = [vp, i, i, i, i, vp, vp, vp]
     lib.sh_plan.argtypes = [vp, vp, i, d, i, vp]
@@ -163,3 +165,20 @@ def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
     got, ref = rule(n)[0], rule(40)
     err = np.abs(got - ref[0]).max(2)
     assert (err[:, 0] <= 5e-16 * ref[1]).all() and (err[:, 1:].max(1) <= 5e-16 * ref[2]).all()
+
+
+@pytest.mark.parametrize("tri", [False, True])
+def test_reach_bounds_every_row(st, tri):
+    """The interior kernel's bound of its rows' half lengths, which its Taylor sums' range is tested against,
+    on elements whose one direction is much longer than the other."""
+    rng = np.random.default_rng(17)
+    a = np.linspace(-1.0, 1.0, 41)
+    for trial in range(60):
+        geo = np.zeros((2, 48))
+        cr = rng.normal(size=(3, 4)) * np.array([1.0, *10.0 ** rng.uniform(-3, 0, 3)])
+        if tri:
+            cr[:, 3] = 0.0
+        geo[1, :12], geo[1, 45] = cr.ravel(), 3 if tri else 4
+        longest = C.c_double()
+        reach = st.st_reach(geo.ctypes.data, 1, 41, a.ctypes.data, C.byref(longest))
+        assert longest.value <= reach * (1 + 1e-12), trial
