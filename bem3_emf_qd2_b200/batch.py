@@ -49,8 +49,8 @@ PLAN_BYTES = 48 << 10
 
 
 def table_coefficients(ne: int) -> int:
-    """Coefficients a periodic domain's table may hold (48 bytes each with its samples)."""
-    return 1 << 19 if ne < 256 else (1 << 21 if ne < 640 else 1 << 22)
+    """Most coefficients a periodic domain's table may hold (48 bytes each with its samples)."""
+    return 1 << 22
 
 
 def domain_scratch_bytes(ne: int, periodic: bool) -> int:

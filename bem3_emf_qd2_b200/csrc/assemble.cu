@@ -943,10 +943,6 @@ static ScratchLayout scratch_layout(int ne, int rows, long long cap)
 }
 size_t bem3_scratch_bytes(int ne, int rows, long long cap) { return scratch_layout(ne, rows, cap).end; }
 
-// Coefficients a domain's table may hold (48 bytes of scratch each, with the samples): enough for the
-// cheapest plans of the configurations (0.4 M for 96 elements, 1.1 M for 384, 2.1 M for 864).
-long long bem3_smooth_cap(int ne) { return ne < 256 ? 1LL << 19 : ne < 640 ? 1LL << 21 : 1LL << 22; }
-
 // Runs the whole domain on `stream` using caller-provided scratch (see bem3_scratch_bytes).
 // Returns 0, or a negative code (see bem3_qd2_b200.h).
 // Adds a chunk's near-singular count to the domain's total (no host round trip per chunk).
@@ -955,8 +951,9 @@ __global__ void k_acc_count(const unsigned* __restrict__ cnt, unsigned long long
   *total += *cnt;
 }
 
-int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, size_t scratch_bytes, int rows_per_chunk,
-                      long long cap, int* d_status, cudaStream_t st, AssembleStats* stats, const ChunkHook* hook)
+int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, const SmoothLat* S, void* scratch, size_t scratch_bytes,
+                      int rows_per_chunk, long long cap, int* d_status, cudaStream_t st, AssembleStats* stats,
+                      const ChunkHook* hook)
 {
   if (ensure_tables() != 0) return BEM3_ERR_CUDA;
   const int ne = A.ne;
@@ -964,7 +961,7 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, 
   if (rows_per_chunk <= 0 || rows_per_chunk > nrows) rows_per_chunk = nrows;
   SmoothArgs M;
   memset(&M, 0, sizeof M);
-  if (A.periodic && cap > 0) smooth_lattice(*L, M.S);
+  if (A.periodic && S) M.S = *S;
   if (!M.S.ok) cap = 0;
   const ScratchLayout lay = scratch_layout(ne, rows_per_chunk, cap);
   if (lay.end > scratch_bytes) return BEM3_ERR_SCRATCH;  // every part below ends inside the scratch

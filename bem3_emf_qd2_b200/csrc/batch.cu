@@ -344,7 +344,7 @@ extern "C" size_t bem3_batch_scratch_bytes(const bem3_batch_domain* doms, int n)
     if (doms[i].periodic) {
       total += (sizeof(QPProp) * QP_PROP_CAP + 255) & ~(size_t)255;
       // the table (48 bytes a coefficient with its samples), its plan and lists
-      total += (size_t)bem3_smooth_cap((int)ne) * 48 + ((sizeof(SmoothPlan) + 255) & ~(size_t)255) + np * sizeof(unsigned) +
+      total += (size_t)SMT_CAPMAX * 48 + ((sizeof(SmoothPlan) + 255) & ~(size_t)255) + np * sizeof(unsigned) +
                (np / 8 + 4096) * sizeof(unsigned) + 1024;
     }
   }
@@ -420,7 +420,7 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
       smtP.add(i, 4 * ne * ((ne + SMT_PAIRS - 1) / SMT_PAIRS));
       smooth_lattice(B.L, B.M.S);
       if (B.M.S.ok) {
-        B.M.cap = bem3_smooth_cap((int)ne);
+        B.M.cap = smooth_capacity(B.L, B.M.S, (int)ne, 4.0 * (double)ne * ne, 144.0, 0.0);
         spec_smem = std::max(spec_smem, smooth_spec_smem(B.M.S));
       }
       pdom.push_back(i);

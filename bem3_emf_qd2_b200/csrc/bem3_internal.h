@@ -40,9 +40,10 @@ struct ChunkHook {
   void* user;
 };
 
-// cap: coefficients of the periodic domain's table of the smooth remainder (0: none)
-long long bem3_smooth_cap(int ne);
+// S, cap: the lattice's part of a periodic domain's table and the coefficients it has room for (nullptr, 0: none)
+struct SmoothLat;
 size_t bem3_scratch_bytes(int ne, int rows, long long cap);
-int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, void* scratch, size_t scratch_bytes, int rows_per_chunk,
-                      long long cap, int* d_status, cudaStream_t st, AssembleStats* stats, const ChunkHook* hook = nullptr);
+int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, const SmoothLat* S, void* scratch, size_t scratch_bytes,
+                      int rows_per_chunk, long long cap, int* d_status, cudaStream_t st, AssembleStats* stats,
+                      const ChunkHook* hook = nullptr);
 void bem3_launch_self_interior(const AssembleArgs& A, double3* Fself, int* d_status, cudaStream_t st);

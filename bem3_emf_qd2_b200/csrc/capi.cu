@@ -213,6 +213,35 @@ static int default_rows_per_chunk(int ne)
   return (int)rows;
 }
 
+// A periodic domain's lattice and the room for its table (cap coefficients; 0: summed point by point).
+struct PeriodicHost {
+  QPLattice L;
+  SmoothLat S;
+  long long cap = 0;
+};
+static int periodic_host(const bem3_qpd2* qd, int ne, PeriodicHost& P)
+{
+  memset(&P.L, 0, sizeof P.L);
+  int e = lattice_from(qd, &P.L);
+  if (e) return e;
+  smooth_lattice(P.L, P.S);
+  P.cap = smooth_capacity(P.L, P.S, ne, 4.0 * (double)ne * ne, 144.0, 0.0);
+  return 0;
+}
+
+// This thread's scratch for `rows` rows a chunk of a domain of ne elements, with `extra` bytes behind it.  The
+// table is what may be left out: where the memory cannot be had, less room for it (*cap), then none.
+static int table_scratch(int ne, int rows, size_t extra, long long* cap, DevRes** R)
+{
+  for (;;) {
+    const size_t need = ((bem3_scratch_bytes(ne, rows, *cap) + 255) & ~(size_t)255) + extra;
+    const int e = ensure_scratch(need, R);
+    if (e != BEM3_ERR_CUDA || *cap == 0) return e;
+    cudaGetLastError();  // the failed allocation's error must not be found after a later launch
+    *cap = *cap > SMT_CAPMIN ? SMT_CAPMIN : 0;
+  }
+}
+
 // One domain's assembly in flight on a stream: its per-thread resources and counters.
 struct DomainRun {
   DevRes* R = nullptr;
@@ -221,24 +250,23 @@ struct DomainRun {
 };
 
 // Enqueues the assembly of one domain on `st` (device inputs and outputs) without waiting for it;
-// `hook` (optional) sees every row chunk as its kernels are enqueued.
+// `hook` (optional) sees every row chunk as its kernels are enqueued.  given: the periodic domain's lattice and
+// table where the caller has set them up and holds the scratch already.
 static int enqueue_domain(const double* geo_dev, int Ne, const int* sid_dev, int Ne_d, int did, int periodic,
                           const bem3_qpd2* qd, double kre, double kim, double* G_dev, double* H_dev, double* dG_dev,
                           double* dH_dev, double* dF_dev, cudaStream_t st, int rows, const ChunkHook* hook,
-                          DomainRun& run)
+                          DomainRun& run, const PeriodicHost* given = nullptr)
 {
   if (!geo_dev || !sid_dev || Ne <= 0 || Ne_d <= 0 || Ne_d > 2 * Ne || !G_dev || !H_dev) return BEM3_ERR_ARG;
-  QPLattice L;
-  memset(&L, 0, sizeof L);
-  if (periodic) {
-    int e = lattice_from(qd, &L);
-    if (e) return e;
-  }
-  const long long cap = periodic ? bem3_smooth_cap(Ne_d) : 0;
-  size_t need = bem3_scratch_bytes(Ne_d, rows, cap);
+  PeriodicHost own;
+  int e = 0;
+  if (!periodic) given = nullptr;
+  else if (!given && (e = periodic_host(qd, Ne_d, own))) return e;
+  long long cap = given ? given->cap : own.cap;
   DevRes* R = nullptr;
-  int e = ensure_scratch(need, &R);
-  if (e) return e;
+  if ((e = table_scratch(Ne_d, rows, 0, &cap, &R))) return e;
+  QPLattice L = given ? given->L : own.L;
+  const SmoothLat* S = given ? &given->S : periodic ? &own.S : nullptr;
   AssembleArgs A;
   A.geo = geo_dev; A.sid = sid_dev; A.ne = Ne_d; A.did = did; A.periodic = periodic ? 1 : 0;
   A.kre = kre; A.kim = kim;
@@ -258,7 +286,7 @@ static int enqueue_domain(const double* geo_dev, int Ne, const int* sid_dev, int
   memset(&run.S, 0, sizeof run.S);
   run.S.time_kernels = t_profiling;
   run.R = R;
-  return bem3_assemble_run(A, &L, R->scratch, R->scratch_bytes, rows, cap, R->status, st, &run.S, hook);
+  return bem3_assemble_run(A, &L, S, R->scratch, R->scratch_bytes, rows, cap, R->status, st, &run.S, hook);
 }
 
 // Waits for `st` and returns the kernels' status; fills this thread's counters.
@@ -424,11 +452,13 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
   order.push_back(0);
   std::vector<size_t> N(nd);
   std::vector<int> rows(nd);
-  size_t need = 0;
+  PeriodicHost per;
+  if (periodic && (e = periodic_host(qd, Ne_d[0], per))) return e;
+  size_t need = 0;  // of the domains without a table
   for (int d = 0; d < nd; d++) {
     N[d] = (size_t)4 * Ne_d[d];
     rows[d] = copied_rows_per_chunk(Ne_d[d], periodic && d == 0);
-    const size_t b = bem3_scratch_bytes(Ne_d[d], rows[d], (periodic && d == 0) ? bem3_smooth_cap(Ne_d[d]) : 0);
+    const size_t b = bem3_scratch_bytes(Ne_d[d], rows[d], 0);
     need = b > need ? b : need;
   }
   double* dgeo = nullptr;
@@ -468,7 +498,14 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
   char* base = nullptr;
   need = (need + 255) & ~(size_t)255;
   // the scratch at its largest before the first launch: no domain may reallocate it under another's kernels
-  if ((rc = ensure_scratch(need + (kept ? bytes : 0), &R))) goto done;
+  {
+    const size_t first = (bem3_scratch_bytes(Ne_d[0], rows[0], per.cap) + 255) & ~(size_t)255;
+    const size_t more = need > first ? need - first : 0;  // another domain's scratch where it is the larger
+    if ((rc = table_scratch(Ne_d[0], rows[0], more + (kept ? bytes : 0), &per.cap, &R))) goto done;
+    const size_t now = (bem3_scratch_bytes(Ne_d[0], rows[0], per.cap) + 255) & ~(size_t)255;
+    need = now > need ? now : need;
+    if ((rc = ensure_scratch(need + (kept ? bytes : 0), &R))) goto done;  // with a smaller table another may need more
+  }
   rc = BEM3_ERR_CUDA;
   if (!kept && cudaMalloc(&own, bytes) != cudaSuccess) { own = nullptr; goto done; }
   base = kept ? (char*)R->scratch + need : (char*)own;
@@ -490,7 +527,7 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
   for (int d : order) {
     const ChunkHook hook = {RowCopies::hook, &rcp[d]};
     rc = enqueue_domain(dgeo, Ne, dsid[d], Ne_d[d], d, (periodic && d == 0) ? 1 : 0, qd, kn[2 * d], kn[2 * d + 1],
-                        dG_[d], dH_[d], ddG[d], ddH[d], ddF[d], st, rows[d], &hook, run[d]);
+                        dG_[d], dH_[d], ddG[d], ddH[d], ddF[d], st, rows[d], &hook, run[d], periodic && d == 0 ? &per : nullptr);
     if (rc) goto done;
     rc = BEM3_ERR_CUDA;
     if (rcp[d].failed) goto done;
@@ -603,10 +640,12 @@ extern "C" int bem3_assemble_domain_dev_noalloc(const double* geo_dev, int Ne, c
 {
   if (!geo_dev || !sid_dev || Ne <= 0 || Ne_d <= 0 || Ne_d > 2 * Ne || !G_dev || !H_dev) return BEM3_ERR_ARG;
   QPLattice L;
+  SmoothLat S;
   memset(&L, 0, sizeof L);
   if (periodic) {
     int e = lattice_from(qd, &L);
     if (e) return e;
+    smooth_lattice(L, S);
   }
   // The array's device address: host code may not use the symbol itself (that is a host-side
   // stand-in, not a device pointer), so resolve it once per device with that device current.
@@ -632,12 +671,12 @@ extern "C" int bem3_assemble_domain_dev_noalloc(const double* geo_dev, int Ne, c
   int rows = default_rows_per_chunk(Ne_d);
   while (rows > 4 && bem3_scratch_bytes(Ne_d, rows, 0) > avail) rows = rows / 2 > 4 ? rows / 2 : 4;
   if (bem3_scratch_bytes(Ne_d, rows, 0) > avail) return BEM3_ERR_SCRATCH;  // domain too large for the array
-  // a table of up to 0.25 M coefficients where at least 64 rows still fit beside it
+  // a table of up to SMT_CAPMIN coefficients where at least 64 rows still fit beside it
   long long cap = 0;
   if (periodic) {
     int rc = default_rows_per_chunk(Ne_d);
-    while (rc > 64 && bem3_scratch_bytes(Ne_d, rc, 1LL << 18) > avail) rc = rc / 2 > 64 ? rc / 2 : 64;
-    if (bem3_scratch_bytes(Ne_d, rc, 1LL << 18) <= avail) { cap = 1LL << 18; rows = rc; }
+    while (rc > 64 && bem3_scratch_bytes(Ne_d, rc, SMT_CAPMIN) > avail) rc = rc / 2 > 64 ? rc / 2 : 64;
+    if (bem3_scratch_bytes(Ne_d, rc, SMT_CAPMIN) <= avail) { cap = SMT_CAPMIN; rows = rc; }
   }
   cudaStream_t st = (cudaStream_t)stream;
   AssembleArgs A;
@@ -652,19 +691,19 @@ extern "C" int bem3_assemble_domain_dev_noalloc(const double* geo_dev, int Ne, c
   // the array keeps the previous call's contents: the status word must start at zero (the
   // run itself clears its row-sum slots and work-list counter before use)
   if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return BEM3_ERR_CUDA;
-  AssembleStats S;
-  memset(&S, 0, sizeof S);
-  int e = bem3_assemble_run(A, &L, scratch, avail, rows, cap, status, st, &S);
+  AssembleStats run;
+  memset(&run, 0, sizeof run);
+  int e = bem3_assemble_run(A, &L, periodic ? &S : nullptr, scratch, avail, rows, cap, status, st, &run);
   if (e) return e;
   int hs = 0;
   unsigned long long gh = 0;
   if (cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return BEM3_ERR_CUDA;
-  if (cudaMemcpyAsync(&gh, S.d_gh_total, sizeof gh, cudaMemcpyDeviceToHost, st) != cudaSuccess) return BEM3_ERR_CUDA;
+  if (cudaMemcpyAsync(&gh, run.d_gh_total, sizeof gh, cudaMemcpyDeviceToHost, st) != cudaSuccess) return BEM3_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return BEM3_ERR_CUDA;
   // this thread's counters, as the allocating entry fills them (no term counter or kernel timing:
   // bem3_set_profiling does not apply to this entry point)
   memset(&t_last_stats, 0, sizeof t_last_stats);
   t_last_stats.gh_pairs = gh;
-  t_last_stats.launches = S.launches;
+  t_last_stats.launches = run.launches;
   return hs;
 }

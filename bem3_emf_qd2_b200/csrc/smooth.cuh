@@ -288,15 +288,21 @@ BEM_HD double smooth_grid(const QPLattice& L, const SmoothExt& X, double a, Smoo
   return 0.0;
 }
 
-// Time of a degree-L plan in units of FP64 instructions (lane level): the evaluations at the pairs'
-// smooth points, and the table's samples (the transform's two steps, the real-space terms and the
-// images of each).
-BEM_HD double smooth_cost(const SmoothLat& S, double det, double pts, double ncent, int L)
+// Time of a degree-L plan in ps of one B200, fitted to the kernels' times (CUPTI) at degrees 9 to 18 for 24 to 864
+// quads, periods over wavelengths 1.2 to 3.75 (63 points, 0.2 to 52 ms): the evaluations at the pairs' smooth points
+// (k_reg_smooth; within 10 % above 0.7 ms), and the table's samples: the transform's orders and its two steps
+// (k_smooth_spectral, 30 %), the real-space terms within reach and the images (k_smooth_project, 20 % above
+// 0.1 ms).  A plan for 384 quads at 0.63: degree 12 8.5 ms, 11 9.2, 13 8.7; a count of operations without the
+// kernels' rates preferred 11 and below.
+BEM_HD double smooth_cost(const SmoothLat& S, const SmoothGrid& P, double det, double pts, int L)
 {
-  const double nc = smt_ncoef(L);
-  const double real = QP_PI * S.rmax * S.rmax / det * 400.0 + 600.0;
-  return pts * (14.0 * nc + 400.0) + ncent * 2.0 * nc * (8.0 * (S.no1 + S.no2) + real);
+  const double ns = 2.0 * (L + 1) * (L + 1), o1 = S.no1, o2 = S.no2;
+  const double real = QP_PI * S.rmax * S.rmax / det * 111.0 + 41.0;
+  const double spec = 2.4 * o1 * o2 * P.N2 + 0.94 * o1 * P.N1 * P.N2 + 8.2 * o1 * o2;
+  return pts * (0.96 * smt_ncoef(L) + 104.0) + ns * (P.ncent * real + P.N3 * spec);
 }
+// ... of one lattice sum point by point, per term (k_reg_periodic: 10 to 18 from 1,090 to 160 terms)
+#define SMT_TERM_PS 14.0
 
 // f_l(r) = j_l(k r) / r^l for l = 0 .. L + 1 into out[l * st], r2 = r^2 (k r <= 2.5): the top two from
 // the series j_l(x) = x^l / (2l+1)!! (1 - x^2 / (2 (2l+3)) + ...), the rest by f_{l-1} = ((2l+1) f_l -
@@ -656,8 +662,8 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.nq4 = n4 * n4;
   P.nq3 = n4 * (n4 + 1);
   const double nq = near > 0.0 ? (tri ? P.nq3 : P.nq4) : 1.0;
-  cost = smooth_cost(S, fabs(L.detd), npairs * nq, nc, degree);
-  const double plain = npairs * (near > 0.0 ? (tri ? 3.0 * near : near) : 1.0) * S.terms * 200.0;
+  cost = smooth_cost(S, P, fabs(L.detd), npairs * nq, degree);
+  const double plain = npairs * (near > 0.0 ? (tri ? 3.0 * near : near) : 1.0) * S.terms * SMT_TERM_PS;
   if (cost < 0.8 * plain) P.on = 1;
   P.rn1 = 1.0 / P.n1; P.rn2 = 1.0 / P.n2; P.rhz = 1.0 / P.hz;
   P.e1 = S.e1; P.e2 = S.e2;
@@ -673,6 +679,32 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   const double rg = 0.5 * sqrt((dp > dm ? dp : dm) + P.hz * P.hz);
   P.rs = fmin(fmin(2.0 * rg, sqrt(rg * S.dblk)), 2.5 / L.k);
 }
+// Coefficients that a domain's table should have room for (48 bytes each with the samples), from what the host
+// knows before the elements are looked at: the cheapest plan for `npairs` evaluations by `ne` elements on a surface
+// of about the cell's size, as tall as the cell is wide or (zlen > 0) zlen, and half as much again (90 seeded
+// spheres and cones of 24 to 864 elements want 0.4 to 1.9 times that plan's, nine in ten up to 1.4).  At least
+// SMT_CAPMIN, also where no table would pay (the elements may be smaller), and at most SMT_CAPMAX; 0 where the
+// lattice has none.
+#define SMT_CAPMIN (1LL << 18)  // 13 MB
+#define SMT_CAPMAX (1LL << 22)  // 200 MB
+inline long long smooth_capacity(const QPLattice& L, const SmoothLat& S, int ne, double npairs, double near, double zlen)
+{
+  if (!S.ok) return 0;
+  const double w = sqrt(fabs(L.detd)), h = 0.53 * w / sqrt((double)ne);
+  const SmoothExt X = {h, zlen > 0.0 ? zlen : w, 1.0, 1.0, 1.42 * h, 0.2};
+  double best = 1e300, want = 0.0;
+  for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
+    SmoothGrid g;
+    double c;
+    smooth_choose(L, S, X, npairs, near, 0, 1LL << 40, d, g, c);
+    if (g.on && c < best) {
+      best = c;
+      want = 1.5 * g.ncent * smt_ncoef(d);
+    }
+  }
+  return want < (double)SMT_CAPMIN ? SMT_CAPMIN : want > (double)SMT_CAPMAX ? SMT_CAPMAX : (long long)want;
+}
+
 // sphere nodes and smooth rules
 BEM_HD void smooth_tables_a(SmoothPlan& P, int part, int nparts)
 {

@@ -82,6 +82,45 @@ double st_reach(const double* geo, int s, int n, const double* a, double* longes
   return regi_reach(e);
 }
 
+// The room the host gives a domain's table (coefficients), and what the plan of the elements 1..ne of geo makes of
+// `cap` coefficients: its own number, 0 when the domain is left to the point-by-point sums.
+double st_capacity(const double* lat, int ne)
+{
+  QPLattice L;
+  memset((void*)&L, 0, sizeof L);
+  if (qp_lattice_init(L, lat[0], lat[1], lat[2], lat[3], lat[4], lat[5], lat[6]) != 0) return -1.0;
+  SmoothLat S;
+  smooth_lattice(L, S);
+  return (double)smooth_capacity(L, S, ne, 4.0 * (double)ne * ne, 144.0, 0.0);
+}
+double st_plan_size(const double* lat, const double* geo, int ne, double cap)
+{
+  QPLattice L;
+  memset((void*)&L, 0, sizeof L);
+  if (qp_lattice_init(L, lat[0], lat[1], lat[2], lat[3], lat[4], lat[5], lat[6]) != 0) return -1.0;
+  SmoothLat S;
+  smooth_lattice(L, S);
+  double he = 0, ra = 0, be = 0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, best = 1e300, size = 0.0;
+  int tri = 0;
+  for (int i = 1; i <= ne; i++) {
+    Elem e;
+    load_elem(geo, i, e);
+    smooth_extent(L, e, &he, &ra, &be, lo, hi);
+    tri |= (e.nn == 3);
+  }
+  const SmoothExt X = {he, hi[2] - lo[2], hi[0] - lo[0], hi[1] - lo[1], ra, be};
+  for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
+    SmoothGrid g;
+    double c;
+    smooth_choose(L, S, X, 4.0 * (double)ne * ne, 144.0, tri, (long long)cap, d, g, c);
+    if (g.on && c < best) {
+      best = c;
+      size = (double)g.ncent * smt_ncoef(d);
+    }
+  }
+  return size;
+}
+
 // Points per direction of the smooth rule.
 int st_nq(double k, double h, double d, double bend) { return smooth_nq(k, h, d, bend); }
 

@@ -21,6 +21,9 @@ def st(tmp_path_factory):
     lib = C.CDLL(so)
     vp, i, d = C.c_void_p, C.c_int, C.c_double
     lib.st_real.argtypes = [vp, vp, d, d, vp, vp]
+    lib.st_capacity.argtypes = [vp, i]
+    lib.st_plan_size.argtypes = [vp, vp, i, d]
+    lib.st_capacity.restype = lib.st_plan_size.restype = d
     lib.st_reach.argtypes = [vp, i, i, vp, vp]
     lib.st_reach.restype = d
     lib.st_nq.argtypes = [d, d, d, d]
@@ -182,3 +185,43 @@ def test_reach_bounds_every_row(st, tri):
         longest = C.c_double()
         reach = st.st_reach(geo.ctypes.data, 1, 41, a.ctypes.data, C.byref(longest))
         assert longest.value <= reach * (1 + 1e-12), trial
+
+
+def _cone(n, r):
+    """Geometry records of a triangulated cone, height 2 r."""
+    from bem3_emf_qd2_b200 import meshgen
+    from bem3_emf_qd2_b200.dqd2 import element_constants
+    nodes = meshgen._Nodes()
+    els = meshgen.cone(nodes, r, 2 * r, -r, n, 2 * n, 4 * n, 0.01, 3)
+    rn = np.vstack([np.zeros(3), np.array(nodes.pts)])
+    ed = np.array([[0, 0, 0, 0]] + [list(e) + [0] * (4 - len(e)) for e in els], np.int32)
+    cr, cw = element_constants(rn, ed)
+    geo = np.zeros((len(ed), 48))
+    geo[1:, 0:12], geo[1:, 12:21], geo[1:, 45] = cr[1:].reshape(-1, 12), cw[1:].reshape(-1, 9), 3
+    return np.ascontiguousarray(geo)
+
+
+@pytest.mark.parametrize("shape,n", [("sphere", 2), ("sphere", 3), ("sphere", 4), ("sphere", 5), ("sphere", 6), ("sphere", 7),
+                                     ("sphere", 10), ("cone", 2), ("cone", 3), ("cone", 4)])
+@pytest.mark.parametrize("lam,period", [(0.8, 0.8), (0.6328, 1.0), (0.5, 1.2), (0.4, 1.5)])
+def test_table_has_room_whatever_the_number_of_elements(st, shape, n, lam, period):
+    """Meshes of every size keep their table over the whole range of wavelengths and periods: the room the host
+    gives it holds a plan wherever the elements admit one at all."""
+    geo, lat = _sphere(n, lam, (period, 0.0, 0.0, period))
+    if shape == "cone":
+        geo = _cone(n, 0.3 * period)
+        lat[0] /= 1.33
+    ne = len(geo) - 1
+    cap = st.st_capacity(lat.ctypes.data, ne)
+    assert 0 < cap <= 1 << 22
+    assert 0 < st.st_plan_size(lat.ctypes.data, geo.ctypes.data, ne, cap) <= cap
+
+
+def test_plan_is_refused_by_the_capacity_or_fits_it(st):
+    """A smaller room gives a plan of a higher degree with fewer coefficients, a still smaller one none."""
+    geo, lat = _sphere(8, 0.6328, (1.0, 0.0, 0.0, 1.0))
+    free = st.st_plan_size(lat.ctypes.data, geo.ctypes.data, 384, 1e12)
+    assert st.st_plan_size(lat.ctypes.data, geo.ctypes.data, 384, free + 4) == free
+    less = st.st_plan_size(lat.ctypes.data, geo.ctypes.data, 384, free - 1)
+    assert 0 < less < free
+    assert st.st_plan_size(lat.ctypes.data, geo.ctypes.data, 384, 1 << 15) == 0
