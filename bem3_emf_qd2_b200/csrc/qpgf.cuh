@@ -37,6 +37,7 @@
 #define QP_EW_EXPM 3.0
 #define QP_EFS 0.1
 #define QP_MEPS 1.0e-15
+#define QP_ZPLANE 1e-11  // heights, in periods, that count as the node's plane
 #define QP_PROP_CAP 2048  // most propagating orders a hoisted lattice list holds
 #ifndef QP_FD_ZFAC
 // Fourier-domain sum in the assembly's evaluation (OPT) only for |z| > QP_FD_ZFAC x split parameter:
@@ -411,7 +412,12 @@ BEM_HD int qp_ew1_sum_body(const QPLattice& L, const double* r, double veps, dou
 // passes over the propagating positions (they still count for the row rule).  The stop rules see
 // the propagating contributions earlier than the reference's order, so a sum may stop a term
 // sooner or later; every neglected term is still below the rule's relative threshold (1e-16 of
-// the running sum).  OPT callers must attach the list (qp_prop_list); OPT also selects the
+// the running sum).  The row rule compares the sums before and after a row; a row's propagating orders no longer
+// change them there, so a row that has any, its centre included, does not end the walk: the rows after it hold
+// evanescent orders close to grazing, which far points still need (period 1.5, wavelength 0.4 in index 1.33, z = 3:
+// 1e-5 of G was missing).  In the plane of the node (z within QP_ZPLANE periods), where the rule decides on
+// rounding noise, only the reference's own count of such orders, without the centre, keeps its values.
+// OPT callers must attach the list (qp_prop_list); OPT also selects the
 // division-light w(z) (faddeeva_w_t<true>).
 template <int MODE, int FD, bool OPT = false>
 BEM_HD int qp_spec_sum_body(const QPLattice& L, const double* r, double veps, double eps, cplx& S, cplx* dS)
@@ -421,6 +427,8 @@ BEM_HD int qp_spec_sum_body(const QPLattice& L, const double* r, double veps, do
   const int ELIM = FD ? -1 : -2;
   S = mk(0, 0); dS[0] = mk(0, 0); dS[1] = mk(0, 0); dS[2] = mk(0, 0);
   const bool hoist = OPT;  // OPT callers always attach the list (L.nprop >= 0)
+  const bool plane = OPT && r[2] * r[2] < QP_ZPLANE * QP_ZPLANE * fabs(L.detd);
+  bool own = false;  // the row has propagating orders, summed before (not in the plane)
   int cc = 0;
   if (hoist) {
 #pragma unroll 1
@@ -454,6 +462,7 @@ BEM_HD int qp_spec_sum_body(const QPLattice& L, const double* r, double veps, do
       const double bn2 = L.k * L.k - an0 * an0 - an1 * an1;
       if (bn2 > 0.0) {
         e = 2;
+        own = !plane;
       } else if (bn2 < 0.0) {
         // 1/|beta_n| from one reciprocal square root, |beta_n| = -beta_n^2 / |beta_n|
         const double ibn = rsqrt_(-bn2);
@@ -498,7 +507,7 @@ BEM_HD int qp_spec_sum_body(const QPLattice& L, const double* r, double veps, do
     bool rstop = true;
     if (dir != 0) {
       rstop = false;
-      if (FD || flg == 0) {
+      if ((FD || flg == 0) && !own) {
         rstop = qp_comp(dS[2], od2, eps);
         if (MODE == QP_BOTH) rstop = rstop && qp_comp(S, oS, eps);
       }
@@ -513,6 +522,7 @@ BEM_HD int qp_spec_sum_body(const QPLattice& L, const double* r, double veps, do
     }
     oS = S; od2 = dS[2];
     flg = 0;
+    own = false;
     if (FD) nc2 = (int)round((L.vkx * L.g2x + L.vky * L.g2y - (double)n1 * L.g12) / L.g22);
     else nc2 = (int)round(-((-L.vkx + (double)n1 * L.g1x) * L.g2x + (-L.vky + (double)n1 * L.g1y) * L.g2y) / L.g22);
     ph0 = expi((-L.vkx + (double)n1 * L.g1x + (double)nc2 * L.g2x) * r[0] +

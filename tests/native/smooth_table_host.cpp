@@ -121,6 +121,26 @@ double st_plan_size(const double* lat, const double* geo, int ne, double cap)
   return size;
 }
 
+// G, grad G (8 doubles a point) by the lattice sums with the propagating orders taken first; returns the lowest
+// status.
+int st_sums(const double* lat, const double* r, int n, double* out)
+{
+  QPLattice L;
+  memset((void*)&L, 0, sizeof L);
+  if (qp_lattice_init(L, lat[0], lat[1], lat[2], lat[3], lat[4], lat[5], lat[6]) != 0) return -1;
+  std::vector<QPProp> prop(QP_PROP_CAP);
+  L.nprop = qp_prop_list(L, prop.data(), QP_PROP_CAP);
+  L.prop = prop.data();
+  int worst = 0;
+  for (int i = 0; i < n; i++) {
+    QPVal v;
+    const int e = qpgf_eval<QP_V1, true>(L, r + 3 * i, v);
+    if (e < worst) worst = e;
+    memcpy((void*)(out + 8 * i), (const void*)&v, sizeof v);
+  }
+  return worst;
+}
+
 // Points per direction of the smooth rule.
 int st_nq(double k, double h, double d, double bend) { return smooth_nq(k, h, d, bend); }
 

@@ -21,6 +21,7 @@ def st(tmp_path_factory):
     lib = C.CDLL(so)
     vp, i, d = C.c_void_p, C.c_int, C.c_double
     lib.st_real.argtypes = [vp, vp, d, d, vp, vp]
+    lib.st_sums.argtypes = [vp, vp, i, vp]
     lib.st_capacity.argtypes = [vp, i]
     lib.st_plan_size.argtypes = [vp, vp, i, d]
     lib.st_capacity.restype = lib.st_plan_size.restype = d
@@ -225,3 +226,25 @@ def test_plan_is_refused_by_the_capacity_or_fits_it(st):
     less = st.st_plan_size(lat.ctypes.data, geo.ctypes.data, 384, free - 1)
     assert 0 < less < free
     assert st.st_plan_size(lat.ctypes.data, geo.ctypes.data, 384, 1 << 15) == 0
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_sums_with_the_propagating_orders_first_reach_far_points(st, seed):
+    """The lattice sums that take the propagating orders first, at heights of 0.001 to 8 over seeded lattices (sides
+    1 : 0.2 to 1 : 5, skewed, wavelengths 0.35 to 4), against 64-bit sums.  At far points the evanescent orders close to
+    grazing lie behind rows of propagating ones, which must not end the walk.  Tolerance: 1e-11 of the largest
+    value, as the plain sums' terms reach e^3 times a sum that may be small."""
+    rng = np.random.default_rng(seed)
+    for _ in range(25):
+        d1, asp, sk = rng.uniform(0.5, 2), math.exp(rng.uniform(-1.6, 1.6)), rng.uniform(-0.5, 0.5)
+        k = 2 * math.pi * rng.choice([1, 1.33]) / math.exp(rng.uniform(math.log(0.35), math.log(4)))
+        th, ph = rng.uniform(0.001, 1.2), rng.uniform(0, 2 * math.pi)
+        if k * k * d1 * d1 * asp > 600:
+            continue
+        lat = np.array([k, k * math.sin(th) * math.cos(ph), k * math.sin(th) * math.sin(ph), d1, 0, sk * d1, asp * d1])
+        r = np.concatenate([rng.uniform(-1.5, 1.5, (5, 2)), np.exp(rng.uniform(math.log(1e-3), math.log(8), (5, 1)))], 1)
+        r[::2, 2] *= -1
+        r, out = np.ascontiguousarray(r), np.zeros((5, 8))
+        assert st.st_sums(lat.ctypes.data, r.ctypes.data, 5, out.ctypes.data) >= 0
+        ref = pairs._green(lat, r)
+        assert (np.abs(out.view(complex) - ref).max(1) <= 1e-11 * np.abs(ref).max(1)).all(), (lat, r)
