@@ -49,14 +49,14 @@ __device__ __forceinline__ double block_reduce(double v, double* red, bool mx)
 
 // What the table is for: the pairs of a domain, or (points) evaluations at points of heights zlo .. zhi
 // against every element, `evals` of them (near = 0: each a single point; else elements with a rule of
-// `near` points per quad).
+// `near` points per quad), `chain` in turn by a thread.
 struct SmoothUse {
   int points;
-  double zlo, zhi, evals, near;
+  double zlo, zhi, evals, near, chain;
 };
 
 __device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const QPLattice& L, const SmoothArgs& M,
-                                                  const SmoothUse U = SmoothUse{0, 0.0, 0.0, 0.0, 0.0})
+                                                  const SmoothUse U = SmoothUse{0, 0.0, 0.0, 0.0, 0.0, 0.0})
 {
   __shared__ double red[SMT_PLAN_THREADS];
   __shared__ SmoothGrid best;
@@ -86,7 +86,7 @@ __device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const Q
   g.on = 0;
   double c = 1e300;
   if (d <= SMT_LMAX) {
-    smooth_choose(L, M.S, X, np, near, tri > 0.0, M.cap, d, g, c);
+    smooth_choose(L, M.S, X, np, near, tri > 0.0, M.cap, d, g, c, U.chain);
     if (!g.on) c = 1e300;
     costs[d] = c;
   }
@@ -126,9 +126,10 @@ __global__ void __launch_bounds__(SMT_PLAN_THREADS) k_smooth_plan(AssembleArgs A
 
 // A table for evaluations at field points.
 __global__ void __launch_bounds__(SMT_PLAN_THREADS) k_field_plan(AssembleArgs A, const __grid_constant__ QPLattice L,
-                                                                 SmoothArgs M, double zlo, double zhi, double evals, double near)
+                                                                 SmoothArgs M, double zlo, double zhi, double evals, double near,
+                                                                 double chain)
 {
-  smooth_plan_block(A, L, M, SmoothUse{1, zlo, zhi, evals, near});
+  smooth_plan_block(A, L, M, SmoothUse{1, zlo, zhi, evals, near, chain});
 }
 
 __device__ __forceinline__ void smooth_slot(const QPLattice& L, const SmoothPlan& P, int slot, SmoothCell& c)

@@ -25,6 +25,10 @@ struct bem3_ctx_s {
   double lambda0 = 0.0;
   bem3_qpd2 qd;
   QPLattice L;
+  SmoothLat lat_w, lat_t;              // (ps == 1) splits of the fields' warp sums and tables
+  SmoothExt ext;                       // of the open region's elements, for the fields' tables
+  double zlo = 0.0, zhi = 0.0;         // their heights
+  int tri = 0;                         // triangles among them
   std::vector<int> nv;                 // [(Ne+1)]
   std::vector<std::vector<int>> sid;   // per domain, signed ids
   std::vector<double> kn;              // [2 (MN+1)]
@@ -118,6 +122,20 @@ extern "C" int bem3_ctx_create(const bem3_problem* P, bem3_ctx* out)
   }
   std::vector<double> geo((size_t)(Ne + 1) * GEO_STRIDE);
   if ((rc = bem3_pack_geometry(&P->mesh, geo.data()))) return fail(rc);
+  if (P->ps == 1) {
+    smooth_lattice(c->L, c->lat_w, EWW_EXPM);
+    smooth_lattice(c->L, c->lat_t);
+    double he = 0.0, ra = 0.0, be = 0.0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    for (int s : c->sid[0]) {
+      Elem e;
+      load_elem(geo.data(), abs(s), e);
+      smooth_extent(c->L, e, &he, &ra, &be, lo, hi);
+      if (e.nn == 3) c->tri = 1;
+    }
+    c->ext = SmoothExt{he, 0.0, 1.0, 1.0, ra, be};  // points anywhere in the cell
+    c->zlo = lo[2];
+    c->zhi = hi[2];
+  }
   if ((rc = upload(c->geo, geo.data(), geo.size())) || (rc = upload(c->md, P->md, (size_t)Ne + 1)) ||
       (rc = upload(c->sd, P->sd, (size_t)Ne + 1)) || (rc = upload(c->eni, P->eni, (size_t)(Ne + 1) * 4)) ||
       (rc = upload(c->knd, P->kn, (size_t)2 * (MN + 1))) || (rc = upload(c->Ui, P->Ui, (size_t)(Ne + 1) * 32)) ||
@@ -791,10 +809,22 @@ extern "C" int bem3_ctx_domain_id(bem3_ctx c, int n, const double* r, int* did)
 
 namespace {
 
-// How the open region's Green's function is evaluated at n field points (rule `type`): by warps where
-// the rule's points are few (FIELD_WARP_MAX evaluations: 17 ns each against ~1.3 ms for a table and its
-// plan), else from a table of the smooth remainder made for the points' heights.
-#define FIELD_WARP_MAX 60000
+// How the open region's Green's function is evaluated at n field points (rule `type`): the cheapest of a warp per
+// evaluation, a table of the smooth remainder made for the points' heights, and the lattice sums by a thread an
+// element.  Times in ps, measured on a B200 through bem3_ctx_field (96 to 864 quads, periods over wavelengths 1 to
+// 3.75, 2,600 to 100,000 evaluations):
+//   warps   14.5 ns and 23.5 ps a spectral order (of the rectangle that is walked) per evaluation: 19 ns at 169
+//           orders, 38 at 1,024, 61 at 2,025
+//   table   140 us for the plan and the launches, the table and its evaluations (smooth_choose: about 40 us a point of
+//           the rule, a thread's chain, or 0.55 ns per evaluation)
+//   plain   1.2 us a term and point of the rule (the chain) or 14 ps a term per evaluation
+// 4 points an element, call by call: 0.63 um, period 1: 30,000 evaluations 759 us by warps, 684 by a table; 100,000:
+// 2,060 and 690.  0.4 um, period 1.5: 36,000 2,490 and 2,700, 100,000 6,100 and 2,720.  (One line at 60,000
+// for every lattice left calls between 30,000 and 60,000 at up to twice the time, and above it took the plain sums where
+// their operations, not their chains, were the fewer: 4,810 us at 100,000 of the latter.)
+// Rules 2 and 3 (144 and 4,096 points a thread) always take the table.
+#define FIELD_WARP_PS(S) (14500.0 + 23.5 * (S).no1 * (S).no2)
+#define FIELD_TABLE_LEAST 200e6  // no table is made in less: not worth planning
 struct FieldPlanHost {
   FieldGreen g;
   bool warp = false;
@@ -806,34 +836,56 @@ int field_plan(bem3_ctx c, const FieldArgs& A, int n, const double* r, int type,
   P.warp = false;
   if (c->ps != 1) return 0;
   const int ne = (int)c->sid[0].size();
+  const double npt = type == 0 ? 4.0 : type == 1 ? 9.0 : 1.0, evals = npt * n * ne;
+  double by_warp = 1e300;
   if (type <= 1) {
-    smooth_lattice(c->L, P.g.W, EWW_EXPM);
-    if (P.g.W.ok && (grad || (double)n * ne * (type == 0 ? 4 : 9) <= FIELD_WARP_MAX)) {
+    P.g.W = c->lat_w;
+    if (P.g.W.ok) by_warp = evals * FIELD_WARP_PS(P.g.W);
+    if (P.g.W.ok && (grad || by_warp < FIELD_TABLE_LEAST)) {
       P.warp = true;
       return 0;
     }
   }
   if (grad) return 0;
   SmoothArgs& M = P.g.M;
-  smooth_lattice(c->L, M.S);
+  M.S = c->lat_t;
+  const double plain = M.S.terms * fmax(1.2e6 * npt, SMT_TERM_PS * evals);
+  const double near = type == 2 ? 144.0 : type == 3 ? 4096.0 : 0.0;
+  double zlo = r[2], zhi = r[2], by_table = 1e300;
+  for (int i = 1; i < n; i++) { zlo = fmin(zlo, r[3 * i + 2]); zhi = fmax(zhi, r[3 * i + 2]); }
+  if (M.S.ok) {
+    SmoothExt X = c->ext;
+    X.zlen = fmax(fmax(zhi - c->zlo, c->zhi - zlo), 0.0);
+    M.cap = smooth_field_room(c->L, M.S, X, evals, near, c->tri, npt, by_table);
+    by_table += 140e6;
+  }
+  if (by_warp < 1e300 && by_warp <= (M.cap ? by_table : plain)) {
+    P.warp = true;
+    return 0;
+  }
   if (!M.S.ok) return 0;
-  M.cap = 1LL << 21;
+  // the plan, and (M.cap) the table; what memory cannot be had is left out, down to the plain sums
   const size_t plan = round256(sizeof(SmoothPlan));
   DevRes* R = nullptr;
-  int rc = ensure_scratch(plan + (size_t)M.cap * 48, &R);
-  if (rc) return rc;
+  for (;;) {
+    const int rc = ensure_scratch(plan + (size_t)M.cap * 48, &R);
+    if (rc == 0) break;
+    if (rc != BEM3_ERR_CUDA) return rc;
+    cudaGetLastError();
+    if (M.cap == 0) return 0;
+    M.cap = M.cap > SMT_CAPMIN ? SMT_CAPMIN : 0;
+  }
   M.plan = (SmoothPlan*)R->scratch;
   M.tab = (cplx*)((char*)R->scratch + plan);
   M.smp = M.tab + M.cap;
-  double zlo = r[2], zhi = r[2];
-  for (int i = 1; i < n; i++) { zlo = fmin(zlo, r[3 * i + 2]); zhi = fmax(zhi, r[3 * i + 2]); }
   AssembleArgs B;
   memset(&B, 0, sizeof B);
   B.geo = A.geo; B.sid = A.sid[0]; B.ne = ne;
-  const double evals = (double)n * ne * (type == 0 ? 4 : type == 1 ? 9 : 1);
-  k_field_plan<<<1, SMT_PLAN_THREADS>>>(B, c->L, M, zlo, zhi, evals, type >= 2 ? (type == 2 ? 144.0 : 4096.0) : 0.0);
-  k_smooth_spectral<<<148 * 4, SMT_SPEC_THREADS, smooth_spec_smem(M.S)>>>(c->L, M);
-  k_smooth_project<<<148 * 8, SMT_PROJ_THREADS>>>(c->L, M);
+  k_field_plan<<<1, SMT_PLAN_THREADS>>>(B, c->L, M, zlo, zhi, evals, near, npt);
+  if (M.cap) {
+    k_smooth_spectral<<<148 * 4, SMT_SPEC_THREADS, smooth_spec_smem(M.S)>>>(c->L, M);
+    k_smooth_project<<<148 * 8, SMT_PROJ_THREADS>>>(c->L, M);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : BEM3_ERR_CUDA;
 }
 

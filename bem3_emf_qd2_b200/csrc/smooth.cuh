@@ -643,10 +643,11 @@ BEM_HD void smooth_gauss(int n, int i, double& x, double& w)
 // The plan's choice of degree and grid, then its tables; the tables are filled by part = 0, 1, ... of
 // nparts (threads), with a barrier between the two stages (smooth_tables_a, _b).
 BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothExt& X, double npairs, double near, int tri,
-                          long long cap, int degree, SmoothGrid& P, double& cost)
+                          long long cap, int degree, SmoothGrid& P, double& cost, double chain = 0.0)
 {
   // degree L alone (the caller takes the cheapest).  near: points of a quad's rule, three times that on a
-  // triangle; 0 where each "pair" is one point
+  // triangle; 0 where each "pair" is one point.  chain > 0: field points, a thread taking `chain` rule points in
+  // turn (their latency counts: 105,000 times the rate's time for each), made without regard to the plain sums
   cost = 1e300;
   P.on = 0;
   if (!S.ok) return;
@@ -662,9 +663,10 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.nq4 = n4 * n4;
   P.nq3 = n4 * (n4 + 1);
   const double nq = near > 0.0 ? (tri ? P.nq3 : P.nq4) : 1.0;
-  cost = smooth_cost(S, P, fabs(L.detd), npairs * nq, degree);
+  const double pts = npairs * nq;
+  cost = smooth_cost(S, P, fabs(L.detd), chain > 0.0 ? fmax(1.7 * pts, 1.05e5 * chain * nq) : pts, degree);
   const double plain = npairs * (near > 0.0 ? (tri ? 3.0 * near : near) : 1.0) * S.terms * SMT_TERM_PS;
-  if (cost < 0.8 * plain) P.on = 1;
+  if (chain > 0.0 || cost < 0.8 * plain) P.on = 1;
   P.rn1 = 1.0 / P.n1; P.rn2 = 1.0 / P.n2; P.rhz = 1.0 / P.hz;
   P.e1 = S.e1; P.e2 = S.e2;
   P.top = L.k / 3.0;
@@ -703,6 +705,25 @@ inline long long smooth_capacity(const QPLattice& L, const SmoothLat& S, int ne,
     }
   }
   return want < (double)SMT_CAPMIN ? SMT_CAPMIN : want > (double)SMT_CAPMAX ? SMT_CAPMAX : (long long)want;
+}
+
+// A table for `evals` evaluations at field points within the domain's extents X (zlen: the largest height of a point
+// against an element): its coefficients (0: none holds) and its cost.
+inline long long smooth_field_room(const QPLattice& L, const SmoothLat& S, const SmoothExt& X, double evals, double near,
+                                   int tri, double chain, double& cost)
+{
+  cost = 1e300;
+  double want = 0.0;
+  for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
+    SmoothGrid g;
+    double c;
+    smooth_choose(L, S, X, evals, near, tri, SMT_CAPMAX, d, g, c, chain);
+    if (g.on && c < cost) {
+      cost = c;
+      want = (double)g.ncent * smt_ncoef(d);
+    }
+  }
+  return want > 0.0 ? (long long)(1.125 * want) + SMT_PAD : 0;  // the device's rounding may add a row of centres
 }
 
 // sphere nodes and smooth rules
