@@ -43,9 +43,11 @@ def domain_output_bytes(ne: int) -> int:
 
 # scratch the batch allocates for a domain (bem3_batch_scratch_bytes, per domain): per-pair F
 # terms (24 B per pair), self-pair terms, the near-singular list; for periodic domains the
-# propagating-order list and the table of the smooth remainder with its plan and lists
+# propagating-order list, the list of pairs in one plane and, in a pool that all tables of a batch
+# share, the table of the smooth remainder with its plan and near-singular list
 PROP_LIST_BYTES = 32 * 2048
 PLAN_BYTES = 48 << 10
+TABLE_POOL_BYTES = 2 << 30  # most that a batch's tables take together
 
 
 def table_coefficients(ne: int) -> int:
@@ -53,11 +55,20 @@ def table_coefficients(ne: int) -> int:
     return 1 << 22
 
 
-def domain_scratch_bytes(ne: int, periodic: bool) -> int:
+def domain_core_bytes(ne: int, periodic: bool) -> int:
+    """Scratch of a domain without its table."""
     np_ = 4 * ne * ne
     b = 24 * np_ + 96 * ne + 4 * (np_ // 8 + 4096) + 4 * 256
     if periodic:
-        b += PROP_LIST_BYTES + PLAN_BYTES + 48 * table_coefficients(ne) + 4 * np_ + 4 * (np_ // 8 + 4096)
+        b += PROP_LIST_BYTES + 4 * np_ + 512
+    return b
+
+
+def domain_scratch_bytes(ne: int, periodic: bool) -> int:
+    """Upper bound of a domain's scratch, whatever its lattice."""
+    b = domain_core_bytes(ne, periodic)
+    if periodic:
+        b += PLAN_BYTES + 48 * table_coefficients(ne) + 4 * (ne * ne // 2 + 4096)
     return b
 
 
@@ -66,8 +77,19 @@ def instance_domains(p) -> List[Tuple[int, int, bool]]:
     return [(d, len(p.sid[d]), d == 0 and p.ps == 1) for d in range(p.MN + 1)]
 
 
+def instance_core_bytes(p) -> int:
+    """Matrices and scratch of an instance without its table (which a batch's pool holds)."""
+    return sum(domain_output_bytes(ne) + domain_core_bytes(ne, per) for _, ne, per in instance_domains(p))
+
+
 def instance_bytes(p) -> int:
-    return sum(domain_output_bytes(ne) + domain_scratch_bytes(ne, per) for _, ne, per in instance_domains(p))
+    """Matrices and scratch of an instance in a batch of its own, the table sized for its lattice."""
+    from . import bem3_batch_domain, lib, make_qpd
+    doms = instance_domains(p)
+    arr = (bem3_batch_domain * len(doms))()
+    for e, (did, ne, per) in zip(arr, doms):
+        e.Ne, e.Ne_d, e.did, e.periodic, e.qd = p.Ne, ne, did, int(per), make_qpd(p.qpd)
+    return sum(domain_output_bytes(ne) for _, ne, _ in doms) + int(lib().bem3_batch_scratch_bytes(arr, len(doms)))
 
 
 def size_class(p) -> str:
@@ -97,13 +119,20 @@ def plan_waves(sizes: Sequence[int], budget: int) -> List[List[int]]:
 
 
 def plan(problems: Sequence, budget: int) -> List[Tuple[str, List[int]]]:
-    """Waves per size class: [(class, instance indices)], classes in a fixed order."""
+    """Waves per size class: [(class, instance indices)], classes in a fixed order.  Where the budget
+    has room for the pool of tables beside the largest instance, the pool is taken off it once and the
+    instances count without their tables; else each counts with its own."""
+    core = [instance_core_bytes(p) for p in problems]
+    if problems and max(core) + TABLE_POOL_BYTES <= budget:
+        sizes, room = core, budget - TABLE_POOL_BYTES
+    else:
+        sizes, room = [instance_bytes(p) for p in problems], budget
     out = []
     for cls in ("large", "medium", "small"):
         idx = [i for i, p in enumerate(problems) if size_class(p) == cls]
         if not idx:
             continue
-        for w in plan_waves([instance_bytes(problems[i]) for i in idx], budget):
+        for w in plan_waves([sizes[i] for i in idx], room):
             out.append((cls, [idx[j] for j in w]))
     return out
 

@@ -47,7 +47,7 @@ struct BatchDomain {
   SmoothArgs M;        // periodic domains: plan and table (plan == nullptr: none)
   unsigned* ip_list;   // [4 ne * ne] pairs in one plane, left to the point-by-point sums
   unsigned* smt_list;  // [gh_cap] near-singular pairs of the tabulated ones
-  unsigned* smt_count; // entries of smt_list, then of ip_list
+  unsigned* smt_count; // entries of smt_list, then of ip_list; then whether the domain has a table (its plan's `on`)
 };
 
 // Cumulative work of the domains of one class: base[0] = 0, base[n] = total, domain dom[i]
@@ -77,7 +77,7 @@ __global__ void k_batch_reset(BatchDomain* D, int nd, unsigned long long* next)
   if (i == 0) next[0] = 0ull;
   if (i < nd) {
     *D[i].gh_count = 0u;
-    if (D[i].smt_count) D[i].smt_count[0] = D[i].smt_count[1] = 0u;
+    if (D[i].smt_count) D[i].smt_count[0] = D[i].smt_count[1] = D[i].smt_count[2] = 0u;
     *D[i].status = 0;
   }
 }
@@ -109,12 +109,16 @@ __global__ void k_batch_zero(const BatchDomain* __restrict__ D)
   for (size_t i = i0; i < N; i += stride) d.Fself[i] = make_double3(0.0, 0.0, 0.0);
 }
 
-// Tables of the periodic domains dom[blockIdx.y].
+// Tables of the periodic domains dom[blockIdx.y].  The tables of a batch share one pool of memory: the domains go
+// through it in groups, plan to near-singular pairs, group after group (bem3_batch_create).
 __global__ void __launch_bounds__(SMT_PLAN_THREADS) k_batch_smooth_plan(const BatchDomain* __restrict__ D,
                                                                         const int* __restrict__ dom)
 {
   const BatchDomain& d = D[dom[blockIdx.x]];
-  if (d.M.plan) smooth_plan_block(d.A, d.L, d.M);
+  if (!d.M.plan) return;
+  smooth_plan_block(d.A, d.L, d.M);
+  __syncthreads();
+  if (threadIdx.x == 0) d.smt_count[2] = (unsigned)d.M.plan->on;  // the plan's memory is another domain's later
 }
 __global__ void __launch_bounds__(SMT_SPEC_THREADS) k_batch_smooth_spectral(const BatchDomain* __restrict__ D,
                                                                             const int* __restrict__ dom)
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(SMT_PROJ_THREADS) k_batch_smooth_project(const
   if (d.M.plan) smooth_project_block(d.L, d.M, blockIdx.x, gridDim.x);
 }
 
-__device__ __forceinline__ bool batch_smooth(const BatchDomain& d) { return d.M.plan && d.M.plan->on; }
+__device__ __forceinline__ bool batch_smooth(const BatchDomain& d) { return d.smt_count && d.smt_count[2] != 0u; }
 
 __global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_periodic(const BatchDomain* __restrict__ D, BatchSeg S)
 {
@@ -143,11 +147,13 @@ __global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_periodic(const B
   self_periodic_row(d.A, d.L, (int)(g - S.base[i]), d.Fself, d.status, red, serr);
 }
 
-__global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_smooth(const BatchDomain* __restrict__ D, BatchSeg S)
+// Self pairs of the rows first, first + 1, ... of all periodic domains' rows.
+__global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_smooth(const BatchDomain* __restrict__ D, BatchSeg S,
+                                                                       long long first)
 {
   __shared__ double red[SELF_THREADS / 32][24];
   __shared__ double xl[12], wl[12], xh[64], wh[64];
-  const long long g = blockIdx.x;
+  const long long g = first + blockIdx.x;
   const int i = seg_find(S, g);
   const BatchDomain& d = D[S.dom[i]];
   if (!batch_smooth(d)) return;
@@ -157,16 +163,18 @@ __global__ void __launch_bounds__(SELF_THREADS, 2) k_batch_self_smooth(const Bat
   self_smooth_row(d.A, d.L, *d.M.plan, d.M.tab, (int)(g - S.base[i]), d.Fself, red, xl, wl, xh, wh);
 }
 
-// Tabulated regular pairs: S counts units of SMT_PAIRS sources (reg_smooth_unit), one warp each.
-__global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth(const BatchDomain* __restrict__ D, BatchSeg S)
+// Tabulated regular pairs: S counts units of SMT_PAIRS sources (reg_smooth_unit), one warp each, from unit `first`
+// to before `end`.
+__global__ void __launch_bounds__(SMT_WARPS * 32, SMT_BLOCKS) k_batch_reg_smooth(const BatchDomain* __restrict__ D, BatchSeg S,
+                                                                                 long long first, long long end)
 {
   extern __shared__ __align__(16) unsigned char smt_smem[];
   __shared__ double xr[RULE_TAB], wr[RULE_TAB];
   for (int i = threadIdx.x; i < RULE_TAB; i += SMT_WARPS * 32) { xr[i] = c_xr[i]; wr[i] = c_wr[i]; }
   __syncthreads();
   const int wib = threadIdx.x >> 5;
-  const long long u = (long long)blockIdx.x * SMT_WARPS + wib;
-  if (u >= S.base[S.n]) return;  // uniform across the warp
+  const long long u = first + (long long)blockIdx.x * SMT_WARPS + wib;
+  if (u >= end) return;  // uniform across the warp
   const int i = seg_find(S, u);
   const BatchDomain& d = D[S.dom[i]];
   if (!batch_smooth(d)) return;
@@ -332,10 +340,36 @@ void batch_free(bem3_batch b)
 
 }  // namespace
 
+namespace {
+
+// The pool that the batch's tables share: at most this many bytes, where one domain does not need more.
+#define BATCH_POOL_BYTES ((size_t)2 << 30)
+
+// A periodic domain's share of the pool, from its first byte: plan, table, samples, near-singular list.
+struct PoolPart {
+  size_t tab, smp, list, end;
+};
+PoolPart pool_part(long long cap, unsigned gh_cap)
+{
+  PoolPart p;
+  p.tab = round256(sizeof(SmoothPlan));
+  p.smp = p.tab + round256(sizeof(cplx) * (size_t)cap);
+  p.list = p.smp + round256(sizeof(cplx) * 2 * (size_t)cap);
+  p.end = p.list + round256(sizeof(unsigned) * (size_t)gh_cap);
+  return p;
+}
+
+long long batch_table_room(const QPLattice& L, const SmoothLat& S, int ne)
+{
+  return smooth_capacity(L, S, ne, 4.0 * (double)ne * ne, 144.0, 0.0);
+}
+
+}  // namespace
+
 extern "C" size_t bem3_batch_scratch_bytes(const bem3_batch_domain* doms, int n)
 {
   if (!doms || n <= 0) return 0;
-  size_t total = 0;
+  size_t total = 0, pool = 0, largest = 0;
   for (int i = 0; i < n; i++) {
     const size_t ne = (size_t)(doms[i].Ne_d > 0 ? doms[i].Ne_d : 0);
     const size_t np = 4 * ne * ne;
@@ -343,11 +377,20 @@ extern "C" size_t bem3_batch_scratch_bytes(const bem3_batch_domain* doms, int n)
              (((np / 8 + 4096) * sizeof(unsigned) + 255) & ~(size_t)255) + 256;
     if (doms[i].periodic) {
       total += (sizeof(QPProp) * QP_PROP_CAP + 255) & ~(size_t)255;
-      // the table (48 bytes a coefficient with its samples), its plan and lists
-      total += (size_t)SMT_CAPMAX * 48 + ((sizeof(SmoothPlan) + 255) & ~(size_t)255) + np * sizeof(unsigned) +
-               (np / 8 + 4096) * sizeof(unsigned) + 1024;
+      QPLattice L;
+      SmoothLat S;
+      memset(&L, 0, sizeof L);
+      if (ne == 0 || lattice_from(&doms[i].qd, &L) != 0) continue;  // refused by bem3_batch_create
+      smooth_lattice(L, S);
+      const long long cap = batch_table_room(L, S, (int)ne);
+      if (cap == 0) continue;
+      total += round256(np * sizeof(unsigned)) + 256;
+      const size_t part = pool_part(cap, (unsigned)(np / 8 + 4096)).end;
+      pool += part;
+      largest = std::max(largest, part);
     }
   }
+  total += std::min(pool, std::max(largest, BATCH_POOL_BYTES));
   // table, status words and segments
   total += (((sizeof(BatchDomain) + 2 * sizeof(long long) + 5 * sizeof(int)) * (size_t)n + 8 * sizeof(long long)) * 5 +
             255) & ~(size_t)255;
@@ -420,7 +463,7 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
       smtP.add(i, 4 * ne * ((ne + SMT_PAIRS - 1) / SMT_PAIRS));
       smooth_lattice(B.L, B.M.S);
       if (B.M.S.ok) {
-        B.M.cap = smooth_capacity(B.L, B.M.S, (int)ne, 4.0 * (double)ne * ne, 144.0, 0.0);
+        B.M.cap = batch_table_room(B.L, B.M.S, (int)ne);
         spec_smem = std::max(spec_smem, smooth_spec_smem(B.M.S));
       }
       pdom.push_back(i);
@@ -447,7 +490,7 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
   const size_t oPdom = Lay.take(sizeof(int) * (pdom.size() + 1));
   const size_t oIdom = Lay.take(sizeof(int) * (idom.size() + 1));
   std::vector<size_t> oFp((size_t)n), oFself((size_t)n), oList((size_t)n), oCount((size_t)n), oProp((size_t)n, 0);
-  std::vector<size_t> oPlan((size_t)n), oTab((size_t)n), oSmp((size_t)n), oIp((size_t)n), oSl((size_t)n), oSc((size_t)n);
+  std::vector<size_t> oPool((size_t)n, 0), oIp((size_t)n, 0), oSc((size_t)n, 0);
   for (int i = 0; i < n; i++) {
     const size_t ne = (size_t)doms[i].Ne_d, np = 4 * ne * ne;
     oFp[(size_t)i] = Lay.take(np * sizeof(double3));
@@ -457,16 +500,40 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     oCount[(size_t)i] = Lay.take(sizeof(unsigned));
     if (doms[i].periodic && !props[(size_t)i].empty()) oProp[(size_t)i] = Lay.take(sizeof(QPProp) * props[(size_t)i].size());
     if (hD[(size_t)i].M.cap) {
-      oPlan[(size_t)i] = Lay.take(sizeof(SmoothPlan));
-      oTab[(size_t)i] = Lay.take(sizeof(cplx) * (size_t)hD[(size_t)i].M.cap);
-      oSmp[(size_t)i] = Lay.take(sizeof(cplx) * 2 * (size_t)hD[(size_t)i].M.cap);
       oIp[(size_t)i] = Lay.take(np * sizeof(unsigned));
-      oSl[(size_t)i] = Lay.take((size_t)hD[(size_t)i].gh_cap * sizeof(unsigned));
-      oSc[(size_t)i] = Lay.take(2 * sizeof(unsigned));
+      oSc[(size_t)i] = Lay.take(3 * sizeof(unsigned));
     }
   }
-  b->bytes = Lay.off;
-  if (cudaMalloc(&b->mem, b->bytes) != cudaSuccess) { b->mem = nullptr; batch_free(b); return BEM3_ERR_CUDA; }
+  // the pool, and the groups of periodic domains that go through it (from groups[k] to before groups[k + 1] of pdom).
+  // Where the memory cannot be had: a smaller pool and more groups; domains that do not fit it, then all of them, are
+  // summed point by point.
+  std::vector<int> groups;
+  for (size_t limit = BATCH_POOL_BYTES;; limit = limit > ((size_t)32 << 20) ? limit / 4 : 0) {
+    groups.assign(1, 0);
+    size_t pool = 0, at = 0;
+    for (int q = 0; q < (int)pdom.size(); q++) {
+      BatchDomain& B = hD[(size_t)pdom[(size_t)q]];
+      if (!B.M.cap) continue;
+      const size_t part = pool_part(B.M.cap, B.gh_cap).end;
+      if (part > limit && limit < BATCH_POOL_BYTES) {
+        B.M.cap = 0;
+        continue;
+      }
+      if (at > 0 && at + part > limit) {
+        groups.push_back(q);
+        at = 0;
+      }
+      oPool[(size_t)pdom[(size_t)q]] = Lay.off + at;
+      at += part;
+      pool = std::max(pool, at);
+    }
+    groups.push_back((int)pdom.size());
+    b->bytes = Lay.off + pool;
+    if (cudaMalloc(&b->mem, b->bytes) == cudaSuccess) break;
+    b->mem = nullptr;
+    if (limit == 0) { batch_free(b); return BEM3_ERR_CUDA; }
+    cudaGetLastError();
+  }
   char* m = (char*)b->mem;
   b->dD = (BatchDomain*)(m + oD);
   b->dstatus = (int*)(m + oStatus);
@@ -479,11 +546,13 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     B.gh_count = (unsigned*)(m + oCount[(size_t)i]);
     B.status = b->dstatus + i;
     if (B.M.cap) {
-      B.M.plan = (SmoothPlan*)(m + oPlan[(size_t)i]);
-      B.M.tab = (cplx*)(m + oTab[(size_t)i]);
-      B.M.smp = (cplx*)(m + oSmp[(size_t)i]);
+      const PoolPart part = pool_part(B.M.cap, B.gh_cap);
+      char* at = m + oPool[(size_t)i];
+      B.M.plan = (SmoothPlan*)at;
+      B.M.tab = (cplx*)(at + part.tab);
+      B.M.smp = (cplx*)(at + part.smp);
+      B.smt_list = (unsigned*)(at + part.list);
       B.ip_list = (unsigned*)(m + oIp[(size_t)i]);
-      B.smt_list = (unsigned*)(m + oSl[(size_t)i]);
       B.smt_count = (unsigned*)(m + oSc[(size_t)i]);
     }
     if (doms[i].periodic) B.L.prop = props[(size_t)i].empty() ? nullptr : (QPProp*)(m + oProp[(size_t)i]);
@@ -531,15 +600,19 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     cudaEventRecord(fork, s0);
     cudaStreamWaitEvent(s1, fork, 0);
     // periodic branch
-    if (spec_smem > 0) {
-      const unsigned npd = (unsigned)pdom.size();
-      const int* dp = (const int*)(m + oPdom);
+    for (size_t q = 0; spec_smem > 0 && q + 1 < groups.size(); q++) {
+      const int p0 = groups[q], p1 = groups[q + 1];
+      const unsigned npd = (unsigned)(p1 - p0);
+      if (npd == 0) continue;
+      const int* dp = (const int*)(m + oPdom) + p0;
+      const long long r0 = selfP.base[(size_t)p0], rows = selfP.base[(size_t)p1] - r0;
+      const long long u0 = smtP.base[(size_t)p0], u1 = smtP.base[(size_t)p1];
       k_batch_smooth_plan<<<npd, SMT_PLAN_THREADS, 0, s0>>>(b->dD, dp);
       k_batch_smooth_spectral<<<dim3((unsigned)(4 * sms), npd), SMT_SPEC_THREADS, spec_smem, s0>>>(b->dD, dp);
       k_batch_smooth_project<<<dim3((unsigned)(8 * sms), npd), SMT_PROJ_THREADS, 0, s0>>>(b->dD, dp);
-      k_batch_self_smooth<<<(unsigned)selfP.total(), SELF_THREADS, 0, s0>>>(b->dD, S[0]);
-      k_batch_reg_smooth<<<(unsigned)((smtP.total() + SMT_WARPS - 1) / SMT_WARPS), SMT_WARPS * 32,
-                           SMT_WARPS * sizeof(SmoothWarp), s0>>>(b->dD, S[5]);
+      k_batch_self_smooth<<<(unsigned)rows, SELF_THREADS, 0, s0>>>(b->dD, S[0], r0);
+      k_batch_reg_smooth<<<(unsigned)((u1 - u0 + SMT_WARPS - 1) / SMT_WARPS), SMT_WARPS * 32,
+                           SMT_WARPS * sizeof(SmoothWarp), s0>>>(b->dD, S[5], u0, u1);
       k_batch_gh_smooth<<<(unsigned)(sms * T.gh_blocks_per_sm), 256, 0, s0>>>(b->dD, dp, (int)npd);
       launches += 6;
     }

@@ -819,9 +819,8 @@ namespace {
 //           the rule, a thread's chain, or 0.55 ns per evaluation)
 //   plain   1.2 us a term and point of the rule (the chain) or 14 ps a term per evaluation
 // 4 points an element, call by call: 0.63 um, period 1: 30,000 evaluations 759 us by warps, 684 by a table; 100,000:
-// 2,060 and 690.  0.4 um, period 1.5: 36,000 2,490 and 2,700, 100,000 6,100 and 2,720.  (One line at 60,000
-// for every lattice left calls between 30,000 and 60,000 at up to twice the time, and above it took the plain sums where
-// their operations, not their chains, were the fewer: 4,810 us at 100,000 of the latter.)
+// 2,060 and 690.  0.4 um, period 1.5: 36,000 2,490 and 2,700, 100,000 6,100 and 2,720.  (With one line at 60,000
+// for every lattice, calls between 25,000 and 60,000 took up to twice the time.)
 // Rules 2 and 3 (144 and 4,096 points a thread) always take the table.
 #define FIELD_WARP_PS(S) (14500.0 + 23.5 * (S).no1 * (S).no2)
 #define FIELD_TABLE_LEAST 200e6  // no table is made in less: not worth planning
