@@ -61,18 +61,20 @@ __device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const Q
   __shared__ double red[SMT_PLAN_THREADS];
   __shared__ SmoothGrid best;
   __shared__ double costs[SMT_LMAX + 1];
-  double he = 0.0, ra = 0.0, be = 0.0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, tri = 0.0;
+  double he = 0.0, ra = 0.0, be = 0.0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, tri = 0.0, quad = 0.0;
   for (int i = threadIdx.x; i < A.ne; i += blockDim.x) {
     Elem e;
     load_elem(A.geo, abs(A.sid[i]), e);
     smooth_extent(L, e, &he, &ra, &be, lo, hi);
-    if (e.nn == 3) tri = 1.0;
+    (e.nn == 3 ? tri : quad) = 1.0;
   }
   SmoothExt X;
   X.half_edge = block_reduce(he, red, true);
   X.radius = block_reduce(ra, red, true);
   X.bend = block_reduce(be, red, true);
   tri = block_reduce(tri, red, true);
+  quad = block_reduce(quad, red, true);
+  const int kinds = tri > 0.0 ? (quad > 0.0 ? 1 : 2) : 0;
   for (int i = 0; i < 3; i++) {
     const double a = block_reduce(lo[i], red, false), b = block_reduce(hi[i], red, true);
     (i == 0 ? X.ulen : i == 1 ? X.vlen : X.zlen) = b - a;
@@ -86,7 +88,7 @@ __device__ __forceinline__ void smooth_plan_block(const AssembleArgs& A, const Q
   g.on = 0;
   double c = 1e300;
   if (d <= SMT_LMAX) {
-    smooth_choose(L, M.S, X, np, near, tri > 0.0, M.cap, d, g, c, U.chain);
+    smooth_choose(L, M.S, X, np, near, kinds, M.cap, d, g, c, U.chain);
     if (!g.on) c = 1e300;
     costs[d] = c;
   }

@@ -28,7 +28,7 @@ struct bem3_ctx_s {
   SmoothLat lat_w, lat_t;              // (ps == 1) splits of the fields' warp sums and tables
   SmoothExt ext;                       // of the open region's elements, for the fields' tables
   double zlo = 0.0, zhi = 0.0;         // their heights
-  int tri = 0;                         // triangles among them
+  int tri = 0;                         // triangles among them: 1 some, 2 all
   std::vector<int> nv;                 // [(Ne+1)]
   std::vector<std::vector<int>> sid;   // per domain, signed ids
   std::vector<double> kn;              // [2 (MN+1)]
@@ -126,12 +126,14 @@ extern "C" int bem3_ctx_create(const bem3_problem* P, bem3_ctx* out)
     smooth_lattice(c->L, c->lat_w, EWW_EXPM);
     smooth_lattice(c->L, c->lat_t);
     double he = 0.0, ra = 0.0, be = 0.0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    size_t tri = 0;
     for (int s : c->sid[0]) {
       Elem e;
       load_elem(geo.data(), abs(s), e);
       smooth_extent(c->L, e, &he, &ra, &be, lo, hi);
-      if (e.nn == 3) c->tri = 1;
+      if (e.nn == 3) tri++;
     }
+    c->tri = tri == 0 ? 0 : tri == c->sid[0].size() ? 2 : 1;
     c->ext = SmoothExt{he, 0.0, 1.0, 1.0, ra, be};  // points anywhere in the cell
     c->zlo = lo[2];
     c->zhi = hi[2];

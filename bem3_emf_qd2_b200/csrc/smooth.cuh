@@ -202,20 +202,20 @@ inline void smooth_lattice(const QPLattice& L, SmoothLat& S, double expm = SMT_E
 }
 
 // Gauss points per direction for the images on an element whose half edges are at most 1, the nearest q away
-// from its middle: the n x n rule's error is below SMT_QTOL of the integrand's size, for 1 / R and r / R^3 times
-// the shape functions, rows up to 1 nearer than the middle, in the worst direction (extended precision, squares
-// and rhombi down to 45 degrees, and the triangle's rule, which needs less).
-BEM_HD int smooth_nq_image(double q)
+// from its middle: the rule's error is below SMT_QTOL of the integrand's size, for 1 / R and r / R^3 times the shape
+// functions, rows up to 1 nearer than the middle, in the worst direction (extended precision; squares and rhombi
+// down to 45 degrees; triangles, whose rule has n + 1 by n points: equilateral to 150 degrees, and slivers).
+BEM_HD int smooth_nq_image(double q, int tri)
 {
-  if (q >= 91.0) return 4;
-  if (q >= 30.1) return 5;
-  if (q >= 14.6) return 6;
-  if (q >= 9.05) return 7;
-  if (q >= 6.45) return 8;
-  if (q >= 5.05) return 9;
-  if (q >= 4.27) return 10;
-  if (q >= 3.72) return 11;
-  return q >= 3.34 ? 12 : 0;
+  if (q >= (tri ? 83.0 : 91.0)) return 4;
+  if (q >= (tri ? 27.0 : 30.1)) return 5;
+  if (q >= (tri ? 13.3 : 14.6)) return 6;
+  if (q >= (tri ? 8.25 : 9.05)) return 7;
+  if (q >= (tri ? 5.85 : 6.45)) return 8;
+  if (q >= (tri ? 4.55 : 5.05)) return 9;
+  if (q >= (tri ? 3.75 : 4.27)) return 10;
+  if (q >= (tri ? 3.22 : 3.72)) return 11;
+  return q >= (tri ? 2.85 : 3.34) ? 12 : 0;
 }
 // Gauss points per direction for a smooth integrand on an edge of half length h: a wave of number k and
 // images at distance d (smooth_nq_image), times the (linear) shape functions, and the area factor |W| of an
@@ -223,10 +223,10 @@ BEM_HD int smooth_nq_image(double q)
 // K_n = 2^{2n} (n!)^4 / ((2n+1) ((2n)!)^2) (mean over the edge); |W| = |W0| sqrt(1 + bend^2 x^2) has the
 // Taylor coefficient binom(1/2, n) bend^{2n} ~ bend^{2n} / (2 sqrt(pi) n^{3/2}).  The smallest n whose errors,
 // for the worst direction, stay below SMT_QTOL; 0 when SMT_NQMAX points do not reach it.
-BEM_HD int smooth_nq(double k, double h, double d, double bend)
+BEM_HD int smooth_nq(double k, double h, double d, double bend, int tri = 0)
 {
   const double x = k * h;
-  const int ni = smooth_nq_image(d / h);
+  const int ni = smooth_nq_image(d / h, tri);
   if (ni == 0) return 0;
   const double lb = log(bend > 1e-9 ? bend : 1e-9), lx = log(x);
   double lf = 0.0;   // ln n!
@@ -645,14 +645,15 @@ BEM_HD void smooth_gauss(int n, int i, double& x, double& w)
 BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothExt& X, double npairs, double near, int tri,
                           long long cap, int degree, SmoothGrid& P, double& cost, double chain = 0.0)
 {
-  // degree L alone (the caller takes the cheapest).  near: points of a quad's rule, three times that on a
+  // degree L alone (the caller takes the cheapest).  tri: 1 some of the elements are triangles, 2 all.  near: points of a quad's rule, three times that on a
   // triangle; 0 where each "pair" is one point.  chain > 0: field points, a thread taking `chain` rule points in
   // turn (their latency counts: 105,000 times the rate's time for each), made without regard to the plain sums
   cost = 1e300;
   P.on = 0;
   if (!S.ok) return;
-  const int n4 = smooth_nq(L.k, X.half_edge, S.dimg, X.bend);
-  if (n4 == 0) return;
+  const int n3 = tri ? smooth_nq(L.k, X.half_edge, S.dimg, X.bend, 1) : 1;
+  const int n4 = tri == 2 ? n3 : smooth_nq(L.k, X.half_edge, S.dimg, X.bend);
+  if (n4 == 0 || n3 == 0) return;
   const double a = smooth_radius(degree, L.k, S.dblk);
   const double nc = smooth_grid(L, X, a, P);
   if (!(nc > 0.0) || nc * smt_ncoef(degree) + SMT_PAD > (double)cap) return;
@@ -661,7 +662,7 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.nph = 2 * degree + 2;
   P.ncent = (int)nc;
   P.nq4 = n4 * n4;
-  P.nq3 = n4 * (n4 + 1);
+  P.nq3 = n3 * (n3 + 1);
   const double nq = near > 0.0 ? (tri ? P.nq3 : P.nq4) : 1.0;
   const double pts = npairs * nq;
   cost = smooth_cost(S, P, fabs(L.detd), chain > 0.0 ? fmax(1.7 * pts, 1.05e5 * chain * nq) : pts, degree);
@@ -746,6 +747,8 @@ BEM_HD void smooth_tables_a(SmoothPlan& P, int part, int nparts)
     smooth_gauss(n, q % n, b, wb);
     P.q4[3 * q] = a; P.q4[3 * q + 1] = b; P.q4[3 * q + 2] = wa * wb;
   }
+  n = 1;
+  while (n * (n + 1) < P.nq3) n++;
   // triangle: u along the edge direction from vertex 0, v across (collapsed square), weights summing
   // to 12 as those of the 3 x 12 x 12 rule
   for (int q = part; q < P.nq3; q += nparts) {

@@ -112,7 +112,7 @@ double st_plan_size(const double* lat, const double* geo, int ne, double cap)
   for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
     SmoothGrid g;
     double c;
-    smooth_choose(L, S, X, 4.0 * (double)ne * ne, 144.0, tri, (long long)cap, d, g, c);
+    smooth_choose(L, S, X, 4.0 * (double)ne * ne, 144.0, 2 * tri, (long long)cap, d, g, c);
     if (g.on && c < best) {
       best = c;
       size = (double)g.ncent * smt_ncoef(d);
@@ -142,7 +142,7 @@ int st_sums(const double* lat, const double* r, int n, double* out)
 }
 
 // Points per direction of the smooth rule.
-int st_nq(double k, double h, double d, double bend) { return smooth_nq(k, h, d, bend); }
+int st_nq(double k, double h, double d, double bend, int tri) { return smooth_nq(k, h, d, bend, tri); }
 
 // sh_pair by the table as the kernels make it.
 int st_pair(const double* geo, int t, int tn, int s, int n, const double* x, const double* w, double* out)

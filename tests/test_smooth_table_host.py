@@ -27,7 +27,7 @@ def st(tmp_path_factory):
     lib.st_capacity.restype = lib.st_plan_size.restype = d
     lib.st_reach.argtypes = [vp, i, i, vp, vp]
     lib.st_reach.restype = d
-    lib.st_nq.argtypes = [d, d, d, d]
+    lib.st_nq.argtypes = [d, d, d, d, i]
     lib.st_pair.argtypes = [vp, i, i, i, i, vp, vp, vp]
     lib.sh_plan.argtypes = [vp, vp, i, d, i, vp]
     return lib
@@ -127,7 +127,7 @@ def _gauss(n):
     return x, 2 / ((1 - x * x) * d * d)
 
 
-@pytest.mark.parametrize("shape", ["square", "rhombus", "rectangle", "triangle"])
+@pytest.mark.parametrize("shape", ["square", "rhombus", "rectangle", "triangle", "right", "obtuse"])
 @pytest.mark.parametrize("n", range(4, 13))
 def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
     """The rule that smooth_nq gives with an image as near as it accepts for n points, against 40 points in
@@ -135,16 +135,17 @@ def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
     SMT_QTOL = 5e-16 of the integrands' sizes, the bound smooth_nq states.  Nearer images take more points, and
     below the last bound there is no rule."""
     near, far = 1.5, 1000.0
-    assert st.st_nq(1e-3, 1.0, near, 0.0) == 0
+    tri = int(shape in ("triangle", "right", "obtuse"))
+    assert st.st_nq(1e-3, 1.0, near, 0.0, tri) == 0
     for _ in range(60):
         mid = math.sqrt(near * far)
-        got = st.st_nq(1e-3, 1.0, mid, 0.0)
+        got = st.st_nq(1e-3, 1.0, mid, 0.0, tri)
         near, far = (near, mid) if 0 < got <= n else (mid, far)
     s3 = np.sqrt(np.longdouble(3))
 
     def rule(m):
         x, w = _gauss(m)
-        if shape != "triangle":
+        if not tri:
             a, b = np.meshgrid(x, x, indexing="ij")
             W = np.outer(w, w)
             N = np.stack([(1 - s3 * a) * (1 - s3 * b), (1 + s3 * a) * (1 - s3 * b), (1 + s3 * a) * (1 + s3 * b), (1 - s3 * a) * (1 + s3 * b)]) / 4
@@ -158,7 +159,11 @@ def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
             W = np.outer(w1, w) * u
             z, e = -0.5 + 1.5 * u - 1.5 * u * v, s3 * (-0.5 + 0.5 * u + 0.5 * u * v)
             N = np.stack([1 - 2.5 * (z + s3 * e), 1 + 5 * z, 1 - 2.5 * (z - s3 * e)]) / 3
-            P = np.stack([z, e, 0 * z]) * 2 / s3
+            V = {"triangle": [(-1, -1), (1, -1), (0, 3 ** 0.5 - 1)], "right": [(-1, 0), (1, 0), (0, 1)],
+                 "obtuse": [(-1, 0), (1, 0), (0, 0.4)]}[shape]  # longest edge 2
+            V = np.array(V) - np.mean(V, 0)
+            w0, w1_, w2 = (1 - z - s3 * e) / 3, (1 + 2 * z) / 3, (1 - z + s3 * e) / 3
+            P = np.stack([w0 * V[0, q] + w1_ * V[1, q] + w2 * V[2, q] for q in (0, 1)] + [0 * z])
         v = P[None] - at[:, :, None, None]
         R = np.sqrt((v * v).sum(1))
         f = np.concatenate([(1 / R)[:, None], v / R[:, None] ** 3], 1)
