@@ -83,6 +83,10 @@ class bem3_stats(C.Structure):
                 ("class_ms", C.c_double * 4)]
 
 
+class bem3_table_stats(C.Structure):
+    _fields_ = [("on", C.c_int), ("plane_pairs", C.c_ulonglong), ("reg_smooth_ms", C.c_double)]
+
+
 class bem3_batch_domain(C.Structure):
     _fields_ = [("geo", C.c_void_p), ("Ne", C.c_int), ("sid", C.c_void_p), ("Ne_d", C.c_int), ("did", C.c_int),
                 ("periodic", C.c_int), ("qd", bem3_qpd2), ("kre", C.c_double), ("kim", C.c_double),
@@ -142,6 +146,7 @@ def lib():
         L.bem3_version.restype = C.c_char_p
         L.bem3_set_profiling.argtypes = [i]
         L.bem3_last_stats.argtypes = [C.POINTER(bem3_stats)]
+        L.bem3_last_table_stats.argtypes = [C.POINTER(bem3_table_stats)]
         L.bem3_fp64_peak_tflops.restype = d
         L.bem3_batch_scratch_bytes.argtypes = [C.POINTER(bem3_batch_domain), i]
         L.bem3_batch_scratch_bytes.restype = C.c_size_t
@@ -525,6 +530,12 @@ def last_stats() -> dict:
     out = {f: getattr(st, f) for f, _ in bem3_stats._fields_}
     out["class_ms"] = list(out["class_ms"])
     return out
+
+
+def last_table_stats() -> dict:
+    st = bem3_table_stats()
+    lib().bem3_last_table_stats(C.byref(st))
+    return {f: getattr(st, f) for f, _ in bem3_table_stats._fields_}
 
 
 def set_profiling(on: bool) -> None:

@@ -1019,6 +1019,8 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, const SmoothLat
     k_smooth_project<<<148 * 8, SMT_PROJ_THREADS, 0, st>>>(*L, M);
     toc(1);
     launches += 3;
+    if (timing && cudaMemcpy(&stats->table_on, &M.plan->on, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+      return BEM3_ERR_CUDA;
   }
   // self pairs
   tic();
@@ -1048,7 +1050,13 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, const SmoothLat
             A, *L, M, r0, nr, Fp, gh_list, smt_count, gh_cap, ip_list, ip_count, d_status);
         launches++;
       }
-      float ms = toc(1);
+      const float sms = toc(1);
+      if (timing && M.plan) {
+        unsigned left = 0;
+        if (cudaMemcpy(&left, ip_count, sizeof left, cudaMemcpyDeviceToHost) != cudaSuccess) return BEM3_ERR_CUDA;
+        stats->reg_smooth_ms += sms;
+        stats->plane_pairs += left;
+      }
       tic();
       if (M.plan) {
         k_gh_smooth<<<148 * 4, 256, 0, st>>>(A, *L, M, p0, Fp, gh_list, smt_count, gh_cap);
@@ -1059,7 +1067,7 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, const SmoothLat
       tic();
       k_reg_periodic<<<blocks, 256, REGP_SMEM_BYTES, st>>>(A, *L, M.plan, ip_list, ip_count, p0, np, Fp, gh_list, gh_count,
                                                            gh_cap, d_status);
-      ms += toc(1);
+      const float ms = toc(1);
       if (timing) {
         stats->reg_periodic_ms += ms;
         stats->reg_periodic_launches++;

@@ -29,6 +29,9 @@ struct AssembleStats {
   int time_kernels;              // in: 1 = time every kernel with CUDA events (synchronising)
   double reg_periodic_ms;        // out: summed duration of k_reg_periodic launches
   int reg_periodic_launches;     // out: number of k_reg_periodic launches
+  double reg_smooth_ms;          // out: summed duration of k_reg_smooth launches (pairs by the table)
+  int table_on;                  // out (with time_kernels): 1 when the periodic domain's plan was on
+  unsigned long long plane_pairs;  // out (with time_kernels): regular pairs that the table left to k_reg_periodic
   double class_ms[4];            // out: self, regular, near-singular, row-sum kernels (any domain)
   unsigned long long* d_gh_total;  // out: device counter of near-singular pairs (read it after the stream syncs)
 };

@@ -47,6 +47,7 @@ struct ThreadRes {
 };
 thread_local ThreadRes t_res;
 thread_local bem3_stats t_last_stats;
+thread_local bem3_table_stats t_last_table;
 thread_local int t_profiling = 0;
 
 int cur_dev()
@@ -204,6 +205,13 @@ extern "C" int bem3_last_stats(bem3_stats* out)
   return 0;
 }
 
+extern "C" int bem3_last_table_stats(bem3_table_stats* out)
+{
+  if (!out) return BEM3_ERR_ARG;
+  *out = t_last_table;
+  return 0;
+}
+
 // Rows per chunk so that the per-pair scratch stays near 384 MB.
 static int default_rows_per_chunk(int ne)
 {
@@ -300,12 +308,16 @@ static int finish_domain(cudaStream_t st, const DomainRun& run)
   if (cudaMemcpyAsync(&gh, run.S.d_gh_total, sizeof gh, cudaMemcpyDeviceToHost, st) != cudaSuccess) return BEM3_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return BEM3_ERR_CUDA;
   memset(&t_last_stats, 0, sizeof t_last_stats);
+  memset(&t_last_table, 0, sizeof t_last_table);
   t_last_stats.gh_pairs = gh;
   t_last_stats.qpgf_terms = terms;
   t_last_stats.launches = run.S.launches;
   t_last_stats.reg_periodic_launches = run.S.reg_periodic_launches;
   t_last_stats.reg_periodic_ms = run.S.reg_periodic_ms;
   for (int i = 0; i < 4; i++) t_last_stats.class_ms[i] = run.S.class_ms[i];
+  t_last_table.on = run.S.table_on;
+  t_last_table.plane_pairs = run.S.plane_pairs;
+  t_last_table.reg_smooth_ms = run.S.reg_smooth_ms;
   return hs;
 }
 
@@ -560,6 +572,7 @@ extern "C" int bem3_assemble_domains(const bem3_mesh* mesh, int MN, const int* c
       cudaMemcpy(hgh.data(), dgh, nd * sizeof(unsigned long long), cudaMemcpyDeviceToHost) != cudaSuccess)
     goto done;
   memset(&t_last_stats, 0, sizeof t_last_stats);
+  memset(&t_last_table, 0, sizeof t_last_table);
   for (int d = 0; d < nd; d++) {
     t_last_stats.gh_pairs += hgh[d];
     t_last_stats.launches += run[d].S.launches;
@@ -703,6 +716,7 @@ extern "C" int bem3_assemble_domain_dev_noalloc(const double* geo_dev, int Ne, c
   // this thread's counters, as the allocating entry fills them (no term counter or kernel timing:
   // bem3_set_profiling does not apply to this entry point)
   memset(&t_last_stats, 0, sizeof t_last_stats);
+  memset(&t_last_table, 0, sizeof t_last_table);
   t_last_stats.gh_pairs = gh;
   t_last_stats.launches = run.launches;
   return hs;

@@ -268,6 +268,32 @@ def served(requests):
     return serve.measure(meshes, probes, requests=requests, workers=8, budget_gb=120.0, load=0.8)
 
 
+def regular_roofline(config, table, pairs, quads, terms, reg_ms, launches, peak):
+    """Roofline of the kernel that does the open region's regular pairs: k_reg_smooth where the domain has a table
+    (table["on"]; no lattice terms to count, so the closed-form floor, one evaluation of the kernel, the geometry and
+    the sums per point of the rule), else k_reg_periodic (algorithmic operations per lattice term).  pairs: regular
+    pairs, `quads` of them (0 to 1) by quads; terms, reg_ms: lattice terms and time of k_reg_periodic."""
+    roof = {"bound": "fp64", "peak": peak, "unit": "TFLOP/s",
+            "peak_source": "measured DFMA probe on this GPU (MEASURED_PEAKS.json has no FP64 entry)",
+            "terms_per_launch": terms / launches}
+    if table["on"]:
+        ms = table["reg_smooth_ms"]
+        points = (pairs - table["plane_pairs"]) * (144.0 * quads + 432.0 * (1.0 - quads))
+        achieved = points * FLOOR_OPS_PER_POINT / (ms * 1e-3) / 1e12
+        roof.update(achieved=achieved, frac=achieved / peak, traffic=None, kernel="k_reg_smooth", alg_ops_per_term=None,
+                    ops_basis="150 operations per rule point (closed-form floor)", hw_ops_per_term=None, hw_frac=None,
+                    terms_per_s=None, launch_ms=ms / launches, plane_pairs=table["plane_pairs"], plane_pairs_ms=reg_ms)
+        return roof
+    ops, hw = ALG_OPS_PER_TERM.get(config), HW_OPS_PER_TERM.get(config)
+    rate = terms / (reg_ms * 1e-3)
+    achieved = rate * ops / 1e12 if ops else None
+    roof.update(achieved=achieved, frac=achieved / peak if achieved else None, traffic=TRAFFIC_PER_LAUNCH.get(config),
+                kernel="k_reg_periodic", alg_ops_per_term=ops,
+                ops_basis="oracle/opcount.py: restatement op count, seeded sample", hw_ops_per_term=hw,
+                hw_frac=rate * hw / 1e12 / peak if hw else None, terms_per_s=rate, launch_ms=reg_ms / launches)
+    return roof
+
+
 def run_ours(args):
     import torch
     import bem3_emf_qd2_b200 as B
@@ -318,12 +344,14 @@ def run_ours(args):
 
     # kernel launches per step and the roofline of the dominant kernel (profiling pass, not timed above)
     B.set_profiling(True)
-    reg_ms, reg_launches, terms, per_step_launches, gh = 0.0, 0, 0, 0, 0
+    reg_ms, reg_launches, terms, per_step_launches, gh, table = 0.0, 0, 0, 0, 0, None
     counts = class_counts(p)
     classes = {}
     for d in domains:
         dev.assemble(d, sptr)
         st = B.last_stats()
+        if d == 0 and p.ps == 1:
+            table = B.last_table_stats()
         reg_ms += st["reg_periodic_ms"]
         reg_launches += st["reg_periodic_launches"]
         terms += st["qpgf_terms"]
@@ -344,31 +372,8 @@ def run_ours(args):
     peak = B.fp64_peak_tflops()
     roof = None
     if reg_launches:
-        per_launch_ms = reg_ms / reg_launches
-        terms_per_launch = terms / reg_launches
-        ops = ALG_OPS_PER_TERM.get(args.config)
-        hw = HW_OPS_PER_TERM.get(args.config)
-        achieved = terms_per_launch * ops / (per_launch_ms * 1e-3) / 1e12 if ops else None
-        roof = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": achieved / peak if achieved else None,
-                "traffic": TRAFFIC_PER_LAUNCH.get(args.config), "kernel": "k_reg_periodic",
-                "peak_source": "measured DFMA probe on this GPU (MEASURED_PEAKS.json has no FP64 entry)",
-                "alg_ops_per_term": ops, "ops_basis": "oracle/opcount.py: restatement op count, seeded sample",
-                "hw_ops_per_term": hw,
-                "hw_frac": terms_per_launch * hw / (per_launch_ms * 1e-3) / 1e12 / peak if hw else None,
-                "terms_per_s": terms_per_launch / (per_launch_ms * 1e-3)}
-        # pairs by the table of the smooth remainder have no lattice terms to count: their roofline is the
-        # closed-form floor, one evaluation of the kernel, the geometry and the sums per point of the rule
-        n_reg = counts[(0, "periodic", "regular")]
-        quads = np.array([p.nv[abs(t)] == 4 for t in p.sid[0]])
-        points = float(n_reg) * (144.0 * quads.mean() + 432.0 * (1.0 - quads.mean()))
-        if terms < points:
-            achieved = points / reg_launches * FLOOR_OPS_PER_POINT / (per_launch_ms * 1e-3) / 1e12
-            roof.update(achieved=achieved, frac=achieved / peak, traffic=None, kernel="k_reg_smooth", alg_ops_per_term=None,
-                        ops_basis="150 operations per rule point (closed-form floor)", hw_ops_per_term=None, hw_frac=None,
-                        terms_per_s=None)
-        roof["launch_ms"] = per_launch_ms
-        roof["terms_per_launch"] = terms_per_launch
+        quads = float(np.mean([p.nv[abs(t)] == 4 for t in p.sid[0]]))
+        roof = regular_roofline(args.config, table, counts[(0, "periodic", "regular")], quads, terms, reg_ms, reg_launches, peak)
 
     # end to end through the host-pointer C ABI
     e2e = None

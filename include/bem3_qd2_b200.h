@@ -149,6 +149,16 @@ typedef struct {
 void bem3_set_profiling(int on);
 int bem3_last_stats(bem3_stats *out);
 
+/* The table of the smooth remainder in the last assembly on this thread, with bem3_set_profiling(1) (zeros else).
+ * A periodic domain with a table has its regular pairs in k_reg_smooth and only those in one plane with their
+ * node in the regular periodic kernel (whose lattice terms and duration bem3_stats has). */
+typedef struct {
+  int on;                          /* 1: the domain's pairs were done by the table */
+  unsigned long long plane_pairs;  /* regular pairs left to the regular periodic kernel */
+  double reg_smooth_ms;            /* summed duration of the tabulated pairs' kernel (CUDA events) */
+} bem3_table_stats;
+int bem3_last_table_stats(bem3_table_stats *out);
+
 /* Measures the FP64 FMA throughput of the current device (TFLOP/s), the denominator of the
  * FP64 roofline.  Runs a ~100 ms kernel. */
 double bem3_fp64_peak_tflops(void);
