@@ -9,8 +9,10 @@
 // the reference.
 //
 // Work decomposition (all FP64, no tensor cores -- none of this is a contraction):
+//   k_*_smooth     : the periodic domain's pairs by the nearest image and a table of the rest
+//                    (assemble_smooth.cuh); what it leaves, and domains without a table:
 //   k_self_periodic / k_self_interior : one CTA per self pair (t == s), polar rule;
-//   k_reg_periodic : one warp per regular pair, lanes over the 144 (quad) / 432 (triangle)
+//   k_reg_periodic : one warp per 2 regular pairs, lanes over the 144 (quad) / 432 (triangle)
 //                    Gauss points, one quasi-periodic Green's function per point;
 //   k_reg_interior : one thread per regular pair (free-space kernel), a warp per 32 sources of a row;
 //   k_gh_*         : pairs whose GL dF/dv exceeds CBD_SDF, recomputed with the 64x64 rule from a
@@ -669,8 +671,9 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
 // Regular interior pairs of one chunk (rows r0 .. r0 + nr - 1).  One B200, the shell of 1,728 quads
 // (11.9 M pairs, complex wave number): 38.5 -> 25.2 ms by the moments, -> 18.7 ms by fewer points for
 // distant pairs (rule_order; 7 to 9 per direction for most), -> 13.5 ms with a warp per CTA, the elements
-// in shared memory in place of spilled registers, and read by 32-byte loads.  FP64 pipe 45 % busy before.
-#define REGI_BLOCKS 9  // up to 224 registers; 11 CTAs (13.8 ms) and 16 with spilled registers (18.7) are slower
+// in shared memory in place of spilled registers, and read by 32-byte loads.  FP64 pipe 60 % busy (45 % before),
+// 168 registers, 12 CTAs a multiprocessor by registers and by shared memory.
+#define REGI_BLOCKS 9  // 168 registers (three warps a partition); 16 with spilled registers took 18.7 ms
 __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_reg_interior(AssembleArgs A, int r0, int nr, double3* Fp,
                                                                      unsigned* gh_list, unsigned* gh_count, unsigned gh_cap,
                                                                      int* status)

@@ -13,7 +13,9 @@
 // k_self_periodic, ~200 terms a point): the open region of 96 quads 41.4 -> 2.26 ms, of 864 quads
 // 1,767 -> 59.6 ms, of 352 triangles 437 -> 54 ms (33 ms of it the in-plane pairs, which stay there).
 // With k_reg_smooth's evaluation tuned since, 864 quads take 39.0 ms, and with eight lanes a pair and
-// fewer points for distant pairs in its nearest image (rule_order) 35.4 ms.
+// fewer points for distant pairs in its nearest image (rule_order) 35.1 ms; 96 quads 1.9 ms, 352 triangles 47 ms.
+// k_reg_smooth has the FP64 pipe 61 % busy with 16 warps a multiprocessor, k_smooth_project 40 %, k_smooth_spectral
+// 35 % (issue slots 61 %: index arithmetic of the transform).
 //
 // Every kernel returns at once when the plan is off (SmoothPlan::on == 0); the point-by-point kernels
 // then do the domain.  Nothing is kept between calls: plan and table are made again by each assembly.

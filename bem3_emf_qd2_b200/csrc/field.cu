@@ -2,7 +2,7 @@
 // potentials at points off the boundary (d3qd2_src/d3qd2_field.c:10-87, 203-300,
 // d3qd2_src/d3qd2_setup.c:157-238), on the device.
 //
-//   k_domain_id  one warp per point: solid angles of the domains' boundary elements, summed per
+//   k_domain_id  one CTA per point: solid angles of the domains' boundary elements, summed per
 //                domain in the reference's domain order (a point on a vertex or in an element's
 //                plane belongs to the domain being scanned)
 //   k_field_part one CTA per (point, FIELD_THREADS elements of its domain): a thread evaluates its

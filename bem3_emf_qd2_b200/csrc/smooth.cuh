@@ -35,7 +35,7 @@
 
 #define SMT_LMIN 8
 #define SMT_LMAX 18
-#define SMT_NQMAX 12
+#define SMT_NQMAX 16
 #define SMT_ZPLANE 1e-11
 #define SMT_PMAX (SMT_NQMAX * (SMT_NQMAX + 1))
 #define SMT_TOL 1e-16   // truncation of the expansions
@@ -213,9 +213,13 @@ BEM_HD int smooth_nq_image(double q, int tri)
   if (q >= (tri ? 8.25 : 9.05)) return 7;
   if (q >= (tri ? 5.85 : 6.45)) return 8;
   if (q >= (tri ? 4.55 : 5.05)) return 9;
-  if (q >= (tri ? 3.75 : 4.27)) return 10;
-  if (q >= (tri ? 3.22 : 3.72)) return 11;
-  return q >= (tri ? 2.85 : 3.34) ? 12 : 0;
+  if (q >= (tri ? 3.75 : 4.28)) return 10;
+  if (q >= (tri ? 3.22 : 3.75)) return 11;
+  if (q >= (tri ? 2.85 : 3.38)) return 12;
+  if (q >= (tri ? 2.58 : 3.10)) return 13;
+  if (q >= (tri ? 2.38 : 2.90)) return 14;
+  if (q >= (tri ? 2.22 : 2.75)) return 15;
+  return q >= (tri ? 2.09 : 2.63) ? 16 : 0;
 }
 // Gauss points per direction for a smooth integrand on an edge of half length h: a wave of number k and
 // images at distance d (smooth_nq_image), times the (linear) shape functions, and the area factor |W| of an
@@ -645,8 +649,8 @@ BEM_HD void smooth_gauss(int n, int i, double& x, double& w)
 BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothExt& X, double npairs, double near, int tri,
                           long long cap, int degree, SmoothGrid& P, double& cost, double chain = 0.0)
 {
-  // degree L alone (the caller takes the cheapest).  tri: 1 some of the elements are triangles, 2 all.  near: points of a quad's rule, three times that on a
-  // triangle; 0 where each "pair" is one point.  chain > 0: field points, a thread taking `chain` rule points in
+  // degree L alone (the caller takes the cheapest).  tri: 1 some of the elements are triangles, 2 all.  near:
+  // points of a quad's rule, three times that on a triangle; 0 where each "pair" is one point.  chain > 0: field points, a thread taking `chain` rule points in
   // turn (their latency counts: 105,000 times the rate's time for each), made without regard to the plain sums
   cost = 1e300;
   P.on = 0;
@@ -666,7 +670,10 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   const double nq = near > 0.0 ? (tri ? P.nq3 : P.nq4) : 1.0;
   const double pts = npairs * nq;
   cost = smooth_cost(S, P, fabs(L.detd), chain > 0.0 ? fmax(1.7 * pts, 1.05e5 * chain * nq) : pts, degree);
-  const double plain = npairs * (near > 0.0 ? (tri ? 3.0 * near : near) : 1.0) * S.terms * SMT_TERM_PS;
+  // point by point the regular pairs' points and the self pairs' (6,144 a row, 24 in turn by a thread at 1 us a term:
+  // 5.4 of the 7.6 ms of 24 quads at 0.63, where the table's way takes 0.8)
+  const double points = npairs * (near > 0.0 ? (tri ? 3.0 * near : near) : 1.0) + 2.0 * sqrt(npairs) * 6144.0;
+  const double plain = S.terms * fmax(SMT_TERM_PS * points, 24e6);
   if (chain > 0.0 || cost < 0.8 * plain) P.on = 1;
   P.rn1 = 1.0 / P.n1; P.rn2 = 1.0 / P.n2; P.rhz = 1.0 / P.hz;
   P.e1 = S.e1; P.e2 = S.e2;
@@ -683,28 +690,33 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.rs = fmin(fmin(2.0 * rg, sqrt(rg * S.dblk)), 2.5 / L.k);
 }
 // Coefficients that a domain's table should have room for (48 bytes each with the samples), from what the host
-// knows before the elements are looked at: the cheapest plan for `npairs` evaluations by `ne` elements on a surface
-// of about the cell's size, as tall as the cell is wide or (zlen > 0) zlen, and half as much again (90 seeded
-// spheres and cones of 24 to 864 elements want 0.4 to 1.9 times that plan's, nine in ten up to 1.4).  At least
-// SMT_CAPMIN, also where no table would pay (the elements may be smaller), and at most SMT_CAPMAX; 0 where the
-// lattice has none.
+// knows before the elements are looked at: plans for `npairs` evaluations by `ne` elements on a surface of about the
+// cell's size, as tall as the cell is wide or (zlen > 0) zlen.  Half as much again as the cheapest (90 seeded
+// spheres and cones of 24 to 864 elements want 0.4 to 1.9 times that plan's, nine in ten up to 1.4; a domain that
+// wants more takes a higher degree), and 2.5 times the smallest, which has no higher degree to turn to.  At least
+// SMT_CAPMIN and at most SMT_CAPMAX; 0 where the lattice has none.
 #define SMT_CAPMIN (1LL << 18)  // 13 MB
 #define SMT_CAPMAX (1LL << 22)  // 200 MB
 inline long long smooth_capacity(const QPLattice& L, const SmoothLat& S, int ne, double npairs, double near, double zlen)
 {
   if (!S.ok) return 0;
-  const double w = sqrt(fabs(L.detd)), h = 0.53 * w / sqrt((double)ne);
+  // (elements small enough for a smooth rule: the real ones may be)
+  const double w = sqrt(fabs(L.detd)), h = fmin(0.53 * w / sqrt((double)ne), 0.29 * S.dimg);
   const SmoothExt X = {h, zlen > 0.0 ? zlen : w, 1.0, 1.0, 1.42 * h, 0.2};
-  double best = 1e300, want = 0.0;
+  double best = 1e300, want = 0.0, least = 1e300;
   for (int d = SMT_LMIN; d <= SMT_LMAX; d++) {
     SmoothGrid g;
     double c;
     smooth_choose(L, S, X, npairs, near, 0, 1LL << 40, d, g, c);
-    if (g.on && c < best) {
+    if (!(c < 1e300)) continue;
+    const double n = (double)g.ncent * smt_ncoef(d);
+    least = fmin(least, n);
+    if (c < best) {
       best = c;
-      want = 1.5 * g.ncent * smt_ncoef(d);
+      want = 1.5 * n;
     }
   }
+  if (least < 1e300) want = fmax(want, 2.5 * least);
   return want < (double)SMT_CAPMIN ? SMT_CAPMIN : want > (double)SMT_CAPMAX ? SMT_CAPMAX : (long long)want;
 }
 

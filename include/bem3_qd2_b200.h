@@ -86,8 +86,9 @@ int bem3_assemble_domain(const bem3_mesh *mesh, const int *sid, int Ne_d, int di
  * dH[d], dF[d] as bem3_assemble_domain's (dG, dH, dF: NULL arrays, or NULL entries, skip them);
  * domain 0 is the quasi-periodic open region when periodic != 0.  The domains' kernels run back to
  * back, the interior domains first, and the row chunks of every domain are copied to the host
- * while later chunks compute; the device holds every domain's matrices at once.  Host pointers;
- * synchronous.  Returns the first failing domain's status.  Fills bem3_last_gh_pairs and the
+ * while later chunks compute; the device holds every domain's matrices at once.  Matrices and inputs of
+ * up to 512 MB stay in the calling thread's scratch for its next call; larger ones are allocated and freed by
+ * the call.  Host pointers; synchronous.  Returns the first failing domain's status.  Fills bem3_last_gh_pairs and the
  * gh_pairs / launches of bem3_last_stats, summed over the domains (no term counter or kernel times). */
 int bem3_assemble_domains(const bem3_mesh *mesh, int MN, const int *const *sid, const int *Ne_d, int periodic,
                           const bem3_qpd2 *qd, const double *kn, double *const *G, double *const *H,
@@ -95,8 +96,10 @@ int bem3_assemble_domains(const bem3_mesh *mesh, int MN, const int *const *sid, 
 
 /* Device-resident variant.  geo_dev: packed geometry from bem3_pack_geometry (uploaded by the
  * caller); sid_dev: [Ne_d] ints; outputs in device memory.  The library allocates its scratch
- * with cudaMalloc on a calling thread's first use and keeps it, per host thread and device, for
- * that thread's later calls; calls from different threads may run concurrently. */
+ * with cudaMalloc on a calling thread's first use and keeps it, per host thread and device, until the
+ * thread ends: the per-pair terms of a row chunk (up to about 480 MB) and, for periodic domains, the table of
+ * the Green's function's smooth remainder (13 to 200 MB; left out where it cannot be had, the pairs are then
+ * summed point by point).  Calls from different threads may run concurrently. */
 int bem3_assemble_domain_dev(const double *geo_dev, int Ne, const int *sid_dev, int Ne_d, int did, int periodic,
                              const bem3_qpd2 *qd, double kre, double kim, double *G_dev, double *H_dev,
                              double *dG_dev, double *dH_dev, double *dF_dev, void *stream);
@@ -271,7 +274,9 @@ int bem3_ctx_domain_id(bem3_ctx c, int n, const double *r, int *did);
  * boundary.  (The reference's type 4, double-exponential integration, is not provided.)
  * total 0: scattered / internal field (EH_s); 1: plus the incident field in the open region
  * (EH_t); 2: the incident field alone, at every point (EH_i).
- * Points outside every domain get did = -1 and zero fields (except with total 2). */
+ * Points outside every domain get did = -1 and zero fields (except with total 2).
+ * Calls with many points of the quasi-periodic region make a table in the calling thread's scratch (up to
+ * 200 MB, by the points' heights; left out where it cannot be had). */
 int bem3_ctx_field(bem3_ctx c, int n, const double *r, int type, int total, double *E, double *H, int *did);
 
 /* Modified electromagnetic potentials at n points (mEMP_s / mEMP_t / mEMP_i,
@@ -343,8 +348,11 @@ typedef struct {
 typedef struct bem3_batch_s *bem3_batch;
 
 /* Device bytes bem3_batch_create allocates for these domains (an upper bound): per domain
- * 96 Ne_d^2 bytes of per-pair F terms, its near-singular work list and self-pair terms, plus the
- * descriptor table.  The outputs are the caller's. */
+ * 96 Ne_d^2 bytes of per-pair F terms, its near-singular work list (2 Ne_d^2 bytes + 16 KB) and self-pair
+ * terms, plus the descriptor table; per periodic domain 16 Ne_d^2 bytes for the pairs in one plane and
+ * up to 64 KB of propagating orders; and one pool of at most 2 GB that the periodic domains' tables
+ * (13 to 200 MB each) share.  Where the device has no memory for the pool, bem3_batch_create takes a smaller
+ * one, in the end none: the domains are then summed point by point.  The outputs are the caller's. */
 size_t bem3_batch_scratch_bytes(const bem3_batch_domain *doms, int n);
 
 /* Builds a batch over n <= 65535 domains: descriptor table, work segments, scratch (one

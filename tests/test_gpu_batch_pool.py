@@ -8,12 +8,12 @@ pytestmark = pytest.mark.gpu
 KEYS = ("G", "H", "dF")
 
 
-def _problem(tmp_path, n, lam, period, theta=0.4):
+def _problem(tmp_path, n, lam, period, theta=0.4, radius=0.3):
     from bem3_emf_qd2_b200 import meshgen
     from bem3_emf_qd2_b200.dqd2 import Problem
-    cfg = dict(surfaces=[("sphere", 0.3 * period, n, 1, 99)], media=[1.6 + 0.0j], lambda0=lam, ni=1.33, theta=theta,
+    cfg = dict(surfaces=[("sphere", radius * period, n, 1, 99)], media=[1.6 + 0.0j], lambda0=lam, ni=1.33, theta=theta,
                phi=2.2, d1=(period, 0.0), d2=(0.0, period), e0=[(1.0, 0.0)])
-    return Problem.from_files(*meshgen.write_config("b", cfg, str(tmp_path / ("%d_%g_%g" % (n, lam, theta)))))
+    return Problem.from_files(*meshgen.write_config("b", cfg, str(tmp_path / ("%d_%g_%g_%g" % (n, lam, theta, radius)))))
 
 
 def _run(insts, tol):
@@ -45,8 +45,8 @@ def test_tables_go_through_the_pool_in_groups(cuda_lib, tmp_path):
     table: those are summed point by point in the batch as alone."""
     from bem3_emf_qd2_b200 import batch
     probs = [_problem(tmp_path, 4, 0.4, 1.5, 0.1 + 0.02 * i) for i in range(40)]
-    probs.insert(7, _problem(tmp_path, 1, 0.5, 1.0))
-    probs.insert(30, _problem(tmp_path, 1, 0.7, 1.2))
+    probs.insert(7, _problem(tmp_path, 1, 0.5, 1.0, radius=0.42))
+    probs.insert(30, _problem(tmp_path, 1, 0.7, 1.2, radius=0.42))
     launches, nbytes = _run([batch.InstanceDevice(p, derivatives=False) for p in probs], 1e-13)
     assert launches >= 15 + 6
     assert nbytes < (2 << 30) + 42 * (2 << 20)

@@ -26,5 +26,5 @@ def test_table_and_plane_pairs(cuda_lib, tmp_path):
 
 
 def test_domain_without_a_table(cuda_lib, tmp_path):
-    st, tb = _stats(cuda_lib, tmp_path, ("sphere", 0.3, 1, 1, 99))
+    st, tb = _stats(cuda_lib, tmp_path, ("sphere", 0.42, 1, 1, 99))  # an image 2.1 half edges away
     assert tb["on"] == 0 and tb["plane_pairs"] == 0 and st["reg_periodic_ms"] > tb["reg_smooth_ms"]

@@ -128,9 +128,9 @@ def _gauss(n):
 
 
 @pytest.mark.parametrize("shape", ["square", "rhombus", "rectangle", "triangle", "right", "obtuse"])
-@pytest.mark.parametrize("n", range(4, 13))
+@pytest.mark.parametrize("n", range(4, 17))
 def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
-    """The rule that smooth_nq gives with an image as near as it accepts for n points, against 40 points in
+    """The rule that smooth_nq gives with an image as near as it accepts for n points, against 56 points in
     extended precision: 1 / R and r / R^3 times the shape functions, the image in any direction.  Tolerance:
     SMT_QTOL = 5e-16 of the integrands' sizes, the bound smooth_nq states.  Nearer images take more points, and
     below the last bound there is no rule."""
@@ -171,7 +171,7 @@ def test_smooth_rule_at_the_nearest_image_it_accepts(st, shape, n):
 
     ph, th = np.linspace(0, 2 * np.pi, 37), np.linspace(0, np.pi / 2, 5)
     at = np.array([[np.sin(t) * np.cos(p), np.sin(t) * np.sin(p), np.cos(t)] for t in th for p in ph]).astype(np.longdouble) * far
-    got, ref = rule(n)[0], rule(40)
+    got, ref = rule(n)[0], rule(56)
     err = np.abs(got - ref[0]).max(2)
     assert (err[:, 0] <= 5e-16 * ref[1]).all() and (err[:, 1:].max(1) <= 5e-16 * ref[2]).all()
 
@@ -209,13 +209,15 @@ def _cone(n, r):
 
 @pytest.mark.parametrize("shape,n", [("sphere", 2), ("sphere", 3), ("sphere", 4), ("sphere", 5), ("sphere", 6), ("sphere", 7),
                                      ("sphere", 10), ("cone", 2), ("cone", 3), ("cone", 4)])
+@pytest.mark.parametrize("hexagonal", [False, True])
 @pytest.mark.parametrize("lam,period", [(0.8, 0.8), (0.6328, 1.0), (0.5, 1.2), (0.4, 1.5)])
-def test_table_has_room_whatever_the_number_of_elements(st, shape, n, lam, period):
+def test_table_has_room_whatever_the_number_of_elements(st, shape, n, lam, period, hexagonal):
     """Meshes of every size keep their table over the whole range of wavelengths and periods: the room the host
     gives it holds a plan wherever the elements admit one at all."""
-    geo, lat = _sphere(n, lam, (period, 0.0, 0.0, period))
+    lattice = (period, 0.0, 0.5 * period, 0.866 * period) if hexagonal else (period, 0.0, 0.0, period)
+    geo, lat = _sphere(n, lam, lattice)
     if shape == "cone":
-        geo = _cone(n, 0.3 * period)
+        geo = _cone(n, 0.3 * min(lattice[0], lattice[3]))
         lat[0] /= 1.33
     ne = len(geo) - 1
     cap = st.st_capacity(lat.ctypes.data, ne)
