@@ -99,7 +99,11 @@ __device__ __forceinline__ void accp_unpack(const double* v, AccP& a)
 }
 // A complex matrix whose entries may be stored 16 bytes at a time: a caller's array of doubles need not
 // start on such a boundary.
-__device__ __forceinline__ bool wide_cplx(const double* m) { return (reinterpret_cast<uintptr_t>(m) & 15) == 0; }
+__host__ __device__ __forceinline__ bool wide_cplx(const double* m) { return (reinterpret_cast<uintptr_t>(m) & 15) == 0; }
+static inline bool wide_outputs(const AssembleArgs& A)
+{
+  return wide_cplx(A.G) && wide_cplx(A.H) && wide_cplx(A.dG) && wide_cplx(A.dH);
+}
 // Store one pair's coefficients in the reference layout.  Done by lanes of a warp (lane l
 // stores item l) or by a single thread (lane = -1 stores all).
 __device__ __forceinline__ void store_pair(const AssembleArgs& A, int row, int s, const cplx* CC, const cplx* dCz,
@@ -572,6 +576,8 @@ __device__ __forceinline__ void load_elem_wide(const double* __restrict__ geo, i
   }
 }
 
+// WIDE: every matrix starts on 16 bytes (tested on the host: a test here costs the kernel 1 %).
+template <bool WIDE>
 __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row, int s, int lane, double3* Fp,
                                                   long long fidx, unsigned* gh_list, unsigned* gh_count, unsigned gh_cap,
                                                   int* status, double* acc)
@@ -655,13 +661,12 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
     if (!mat[q]) continue;
     const size_t r = (q < 2) ? (size_t)row : (size_t)2 * row + (q & 1);
     cplx* out = (cplx*)mat[q] + r * N + (size_t)4 * s0;
-    const bool wide = wide_cplx(mat[q]);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int k = c * 32 + lane, sl = k >> 2, i = k & 3;
       if (s0 + sl >= A.ne || (s0 + sl == t && !blank)) continue;
       const double* v = acc + (q * 8 + 2 * i) * REGI_LD + sl;
-      if (wide) *reinterpret_cast<double2*>(out + k) = make_double2(v[0], v[REGI_LD]);
+      if (WIDE) *reinterpret_cast<double2*>(out + k) = make_double2(v[0], v[REGI_LD]);
       else out[k] = mk(v[0], v[REGI_LD]);
     }
   }
@@ -674,6 +679,7 @@ __device__ __forceinline__ void reg_interior_warp(const AssembleArgs& A, int row
 // in shared memory in place of spilled registers, and read by 32-byte loads.  FP64 pipe 60 % busy (45 % before),
 // 168 registers, 12 CTAs a multiprocessor by registers and by shared memory.
 #define REGI_BLOCKS 9  // 168 registers (three warps a partition); 16 with spilled registers took 18.7 ms
+template <bool WIDE>
 __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_reg_interior(AssembleArgs A, int r0, int nr, double3* Fp,
                                                                      unsigned* gh_list, unsigned* gh_count, unsigned gh_cap,
                                                                      int* status)
@@ -683,7 +689,7 @@ __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_reg_interior(A
   const long long w = (long long)blockIdx.x * REGI_WARPS + wib;
   if (w >= (long long)wpr * nr) return;  // uniform across the warp
   const int rr = (int)(w / wpr), s = (int)(w - (long long)rr * wpr) * 32 + lane;
-  reg_interior_warp(A, r0 + rr, s, lane, Fp, (long long)rr * A.ne + s, gh_list, gh_count, gh_cap, status,
+  reg_interior_warp<WIDE>(A, r0 + rr, s, lane, Fp, (long long)rr * A.ne + s, gh_list, gh_count, gh_cap, status,
                     regi_smem + wib * REGI_SMEM);
 }
 
@@ -907,11 +913,11 @@ static int ensure_tables(void)
                            (int)(SMT_WARPS * sizeof(SmoothWarp))) != cudaSuccess ||
       cudaFuncSetAttribute(k_smooth_spectral, cudaFuncAttributeMaxDynamicSharedMemorySize, SMT_SPEC_SMEM) != cudaSuccess)
     return -1;
-  if (cudaFuncSetAttribute(k_reg_interior, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-      cudaFuncSetAttribute(k_reg_interior, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGI_SMEM_BYTES) !=
-          cudaSuccess)
-    return -1;
+  for (auto reg : {k_reg_interior<true>, k_reg_interior<false>})
+    if (cudaFuncSetAttribute(reg, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(reg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGI_SMEM_BYTES) != cudaSuccess)
+      return -1;
   if (dev < 64) g_tables_ready[dev] = 1;
   return 0;
 }
@@ -1081,7 +1087,8 @@ int bem3_assemble_run(const AssembleArgs& A, const QPLattice* L, const SmoothLat
     } else {
       const long long warps = (long long)((ne + 31) / 32) * nr;
       tic();
-      k_reg_interior<<<(unsigned)((warps + REGI_WARPS - 1) / REGI_WARPS), REGI_WARPS * 32, REGI_SMEM_BYTES, st>>>(
+      const auto reg = wide_outputs(A) ? k_reg_interior<true> : k_reg_interior<false>;
+      reg<<<(unsigned)((warps + REGI_WARPS - 1) / REGI_WARPS), REGI_WARPS * 32, REGI_SMEM_BYTES, st>>>(
           A, r0, nr, Fp, gh_list, gh_count, gh_cap, d_status);
       toc(1);
       tic();

@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(256, REGP_MIN_BLOCKS) k_batch_reg_periodic(con
 }
 
 // Regular interior pairs: S counts warps, each 32 sources of a row (reg_interior_warp).
+template <bool WIDE>
 __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_batch_reg_interior(const BatchDomain* __restrict__ D, BatchSeg S)
 {
   extern __shared__ __align__(16) double regi_smem[];
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(REGI_WARPS * 32, REGI_BLOCKS) k_batch_reg_inte
   const int wpr = (d.A.ne + 31) >> 5;
   const long long u = w - S.base[i];
   const int row = (int)(u / wpr), s = (int)(u - (long long)row * wpr) * 32 + lane;
-  reg_interior_warp(d.A, row, s, lane, d.Fp, (long long)row * d.A.ne + s, d.gh_list, d.gh_count, d.gh_cap, d.status,
+  reg_interior_warp<WIDE>(d.A, row, s, lane, d.Fp, (long long)row * d.A.ne + s, d.gh_list, d.gh_count, d.gh_cap, d.status,
                     regi_smem + wib * REGI_SMEM);
 }
 
@@ -423,10 +424,16 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
       cudaFuncSetAttribute(k_batch_reg_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)(SMT_WARPS * sizeof(SmoothWarp))) != cudaSuccess ||
       cudaFuncSetAttribute(k_batch_smooth_spectral, cudaFuncAttributeMaxDynamicSharedMemorySize, SMT_SPEC_SMEM) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_batch_reg_interior, cudaFuncAttributePreferredSharedMemoryCarveout,
+          cudaSuccess)
+    return BEM3_ERR_CUDA;
+  bool wide = true;  // every matrix of the interior domains starts on 16 bytes
+  for (int i = 0; i < n; i++)
+    if (!doms[i].periodic)
+      wide = wide && wide_cplx(doms[i].G) && wide_cplx(doms[i].H) && wide_cplx(doms[i].dG) && wide_cplx(doms[i].dH);
+  const auto batch_reg_interior = wide ? k_batch_reg_interior<true> : k_batch_reg_interior<false>;
+  if (cudaFuncSetAttribute(batch_reg_interior, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-      cudaFuncSetAttribute(k_batch_reg_interior, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGI_SMEM_BYTES) !=
+      cudaFuncSetAttribute(batch_reg_interior, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REGI_SMEM_BYTES) !=
           cudaSuccess)
     return BEM3_ERR_CUDA;
 
@@ -628,7 +635,7 @@ extern "C" int bem3_batch_create(const bem3_batch_domain* doms, int n, const bem
     // interior branch
     if (selfI.total() > 0) { k_batch_self_interior<<<(unsigned)selfI.total(), SI_THREADS, 0, s1>>>(b->dD, S[1]); launches++; }
     if (regI.total() > 0) {
-      k_batch_reg_interior<<<(unsigned)((regI.total() + REGI_WARPS - 1) / REGI_WARPS), REGI_WARPS * 32, REGI_SMEM_BYTES, s1>>>(
+      batch_reg_interior<<<(unsigned)((regI.total() + REGI_WARPS - 1) / REGI_WARPS), REGI_WARPS * 32, REGI_SMEM_BYTES, s1>>>(
           b->dD, S[3]);
       k_batch_gh_interior<<<(unsigned)(2 * sms * T.gh_blocks_per_sm), GHI_THREADS, 0, s1>>>(b->dD, (const int*)(m + oIdom),
                                                                              (int)idom.size());
