@@ -680,14 +680,14 @@ BEM_HD void smooth_choose(const QPLattice& L, const SmoothLat& S, const SmoothEx
   P.top = L.k / 3.0;
   for (int l = 1; l <= degree; l++) P.top *= L.k / (2.0 * l + 3.0);
   // The sphere: twice the grid cell's half diagonal rg, so that the samples' rounding reaches the cell damped
-  // by 2^-l at degree l (over the cell's own sphere the gradients' error was L / rg times it), but within
-  // the first zero of the Bessel functions.  The neglected degrees reach the kept ones only by aliasing,
+  // by 2^-l at degree l (over the cell's own sphere the gradients' error was L / rg times it), but well within
+  // the first zero of the Bessel functions (j_0 at pi; at k rs = 3.1 the constant part's error is 15 times as large).  The neglected degrees reach the kept ones only by aliasing,
   // (rg / d)^l (rs / d)^(2 (L + 1 - l)) for images at distance d: below the truncation (rg / d)^(L + 1) as
   // long as rs^2 <= rg d.
   const double ax = L.d1x / P.n1, ay = L.d1y / P.n1, bx = L.d2x / P.n2, by = L.d2y / P.n2;
   const double dp = (ax + bx) * (ax + bx) + (ay + by) * (ay + by), dm = (ax - bx) * (ax - bx) + (ay - by) * (ay - by);
   const double rg = 0.5 * sqrt((dp > dm ? dp : dm) + P.hz * P.hz);
-  P.rs = fmin(fmin(2.0 * rg, sqrt(rg * S.dblk)), 2.5 / L.k);
+  P.rs = fmin(fmin(2.0 * rg, sqrt(rg * S.dblk)), fmax(2.0 / L.k, rg));
 }
 // Coefficients that a domain's table should have room for (48 bytes each with the samples), from what the host
 // knows before the elements are looked at: plans for `npairs` evaluations by `ne` elements on a surface of about the
