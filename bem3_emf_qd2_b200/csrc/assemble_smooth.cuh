@@ -243,14 +243,17 @@ __device__ __forceinline__ void smooth_project_block(const QPLattice& L, const S
     const cplx* in = M.smp + (size_t)slot * ns;
     SmoothCell c;
     smooth_slot(L, P, slot, c);
-    const cplx K = smooth_wave_centre(L, c);
-#pragma unroll 1
-    for (int i = threadIdx.x; i < ns; i += blockDim.x) smp[i] = in[i] + smooth_wave_diff(L, P, c, i, K);
+    cplx K = mk(0.0, 0.0);
+    if (smooth_split(L)) {
+      K = smooth_wave_centre(L, c);
+      for (int i = threadIdx.x; i < ns; i += blockDim.x) smp[i] = smooth_wave_diff(L, P, c, i, K);
+    }
 #pragma unroll 1
     for (int i = threadIdx.x; i < ns; i += blockDim.x) {
       double r[3];
       smooth_sample_point(P, c, i, r);
-      smp[i] += smooth_real(L, M.S, c, r);
+      const cplx v = in[i] + smooth_real(L, M.S, c, r);
+      smp[i] = smooth_split(L) ? smp[i] + v : v;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < P.nth * L1; i += blockDim.x) smooth_azimuth(P, smp, i / L1, i % L1, ca[i], cb[i]);

@@ -518,7 +518,8 @@ BEM_HD double smt_add(double a, double b)
 
 // Height function of spectral order (q1, q2) of the table's sums at height z >= 0, times i / (4 |cell|):
 // the order's share of G is this times e^{i a.rho}, a = (*ax, *ay).  Zero beyond the cut.  SPLIT: without
-// the wave of order (0, 0) (smooth_wave_diff).
+// the wave of order (0, 0) where smooth_wave_diff has it (smooth_split).
+BEM_HD int smooth_split(const QPLattice& L) { return L.k * L.k * fabs(L.detd) < 1.0; }
 template <bool SPLIT = false>
 BEM_HD cplx smooth_order(const QPLattice& L, const SmoothLat& S, int q1, int q2, double z, double* ax, double* ay)
 {
@@ -532,7 +533,7 @@ BEM_HD cplx smooth_order(const QPLattice& L, const SmoothLat& S, int q1, int q2,
     const cplx ff = expi(bn * z);
     const cplx w = faddeeva_w_upper(x, y);
     const double ef = exp(x * x - y * y), f = 2.0 * c / bn;
-    if (SPLIT && q1 == 0 && q2 == 0) return mk(-f * ef * w.im, 0.0);
+    if (SPLIT && q1 == 0 && q2 == 0 && smooth_split(L)) return mk(-f * ef * w.im, 0.0);
     return mk(-f * (ef * w.im + ff.im), f * ff.re);  // i c F, F = (2 / bn) (i ef Im w + ff)
   }
   const double E = exp(-(x * x + y * y));
@@ -551,17 +552,18 @@ BEM_HD void smooth_sample_point(const SmoothPlan& P, const SmoothCell& c, int p,
 }
 
 // The plane wave of order (0, 0), f_0 e^{i (beta |z| + a.rho)} with f_0 = i / (2 beta |cell|): its value K at
-// centre c and, for sample p, the difference from it.  Where the wavelength is above the period this wave is
+// centre c and, for sample p, the difference from it.  Where the wavelength is far above the period this wave is
 // large (1 / (2 k |cell|)) and nearly constant: its rounding in the samples, over the sphere's radius, would be
 // the error of the table's gradients.  K belongs to degree 0 alone (c00), the differences are taken without
-// cancellation.  With it and the wider sphere (smooth_choose) H of 96 quads, period 1, differs from 64-bit sums
-// by 5e-15, 7e-15, 6e-15 of a pair's largest at wavelengths 3, 10, 50 (1.7e-14, 8e-14, 4e-13 before; the
-// point-by-point sums 2e-15), and as before below 1.
+// cancellation.  Only for k^2 |cell| < 1 (smooth_split): above, the wider sphere (smooth_choose) is enough, and the
+// differences would cost k_smooth_project 2 % (384 quads at 0.63: 867 -> 886 us).  H of 96 quads, period 1,
+// against 64-bit sums, of a pair's largest: 4e-15 at wavelength 3 (no split), 7e-15, 6e-15 at 10, 50 (1.7e-14, 8e-14,
+// 4e-13 with neither; the point-by-point sums 2e-15).
 BEM_HD int smooth_wave0(const QPLattice& L, double* beta)
 {
   const double b2 = smt_add(smt_add(smt_mul(L.k, L.k), -smt_mul(L.vkx, L.vkx)), -smt_mul(L.vky, L.vky));
   *beta = sqrt(fabs(b2));
-  return b2 > 0.0;
+  return smooth_split(L) && b2 > 0.0;
 }
 BEM_HD cplx smooth_wave_centre(const QPLattice& L, const SmoothCell& c)
 {
