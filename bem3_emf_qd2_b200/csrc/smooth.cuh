@@ -303,7 +303,8 @@ BEM_HD double smooth_cost(const SmoothLat& S, const SmoothGrid& P, double det, d
   const double ns = 2.0 * (L + 1) * (L + 1), o1 = S.no1, o2 = S.no2;
   const double real = QP_PI * S.rmax * S.rmax / det * 111.0 + 41.0;
   const double spec = 2.4 * o1 * o2 * P.N2 + 0.94 * o1 * P.N1 * P.N2 + 8.2 * o1 * o2;
-  return pts * (0.96 * smt_ncoef(L) + 104.0) + ns * (P.ncent * real + P.N3 * spec);
+  // fewer than 640 centres take no less: one centre's samples by its CTA (722 of them 162 us)
+  return pts * (0.96 * smt_ncoef(L) + 104.0) + ns * (fmax((double)P.ncent, 640.0) * real + P.N3 * spec);
 }
 // ... of one lattice sum point by point, per term (k_reg_periodic: 10 to 18 from 1,090 to 160 terms)
 #define SMT_TERM_PS 14.0
